@@ -985,7 +985,8 @@ struct VolTanArgs {
     const double* dG[12];
 };
 
-/* shared layout per node: dfr[3] dfm[9] dft[3] jin[9] */
+/* shared record per node: per direction the tangents of the flux columns as
+ * in the forward kernel; then jin[9] */
 constexpr int TAN_W = 24;
 
 __global__ void k_tan_volume(const NsemDev m, const NsemTables tab, VolTanArgs a) {
@@ -1007,24 +1008,25 @@ __global__ void k_tan_volume(const NsemDev m, const NsemTables tab, VolTanArgs a
         const double Fc[3] = {P.U[0] * P.r, P.U[1] * P.r, P.U[2] * P.r};
         double dFc[3];
         for (int c = 0; c < 3; c++) dFc[c] = d.U[c] * P.r + P.U[c] * d.r;
-        for (int c = 0; c < 3; c++) my[c] = dFc[c];
-        for (int r = 0; r < 3; r++)
-            for (int c = 0; c < 3; c++) {
-                const int idx = (r == c) ? r : (r == 0 && c == 1) ? XY : (r == 1 && c == 2) ? YZ
-                              : (r == 0 && c == 2) ? XZ : (r == 1 && c == 0) ? YX
-                              : (r == 2 && c == 1) ? ZY : ZX;
-                my[3 + idx] = dFc[r] * P.U[c] + Fc[r] * d.U[c] + (r == c ? d.p : 0.0);
-            }
-        for (int c = 0; c < 3; c++) my[12 + c] = dFc[c] * P.T + Fc[c] * d.T;
+        for (int c = 0; c < 3; c++) {
+            double* col = my + 5 * c;
+            col[0] = dFc[c];
+            for (int r = 0; r < 3; r++)
+                col[1 + r] = dFc[r] * P.U[c] + Fc[r] * d.U[c] + (r == c ? d.p : 0.0);
+            col[4] = dFc[c] * P.T + Fc[c] * d.T;
+        }
         if (a.G[0]) {
             const double mu = P.r * m.nu, dmu = d.r * m.nu;
-            for (int c = 0; c < 9; c++) my[3 + c] -= dmu * a.G[c][node] + mu * a.dG[c][node];
-            for (int c = 0; c < 3; c++)
-                my[12 + c] -= m.iPr * (dmu * a.G[9 + c][node] + mu * a.dG[9 + c][node]);
+            for (int c = 0; c < 3; c++) {
+                double* col = my + 5 * c;
+                for (int r = 0; r < 3; r++)
+                    col[1 + r] -= dmu * a.G[tix(r, c)][node] + mu * a.dG[tix(r, c)][node];
+                col[4] -= m.iPr * (dmu * a.G[9 + c][node] + mu * a.dG[9 + c][node]);
+            }
         }
         for (int c = 0; c < 9; c++) my[15 + c] = m.jin[(int64_t)c * m.n_int + node];
     }
-    __syncthreads();
+    const bool diag = __syncthreads_and(!active || nsem_node_diag<5>(sm + (size_t)t * TAN_W));
     if (!active) return;
     double r[5] = {0, 0, 0, 0, 0};
     /* surface lift (a coarse side of a non-conforming face lifts the
@@ -1041,15 +1043,7 @@ __global__ void k_tan_volume(const NsemDev m, const NsemTables tab, VolTanArgs a
         }
     }
     /* volume term: r[a] -= dF_b . (Jin_b dpsi(b -> a)) over the lines through a */
-    nsem_volume_gather<TAN_W, 15>(NPX, NPY, NPZ, sm, dps, t, [&](int lb, const double* dj) {
-        const double* sb = sm + (size_t)lb * TAN_W;
-        r[0] -= vdot3(sb, dj);
-        const double* F = sb + 3;
-        r[1] -= F[XX] * dj[0] + F[XY] * dj[1] + F[XZ] * dj[2];
-        r[2] -= F[YX] * dj[0] + F[YY] * dj[1] + F[YZ] * dj[2];
-        r[3] -= F[ZX] * dj[0] + F[ZY] * dj[1] + F[ZZ] * dj[2];
-        r[4] -= vdot3(sb + 12, dj);
-    });
+    nsem_volume_gather<5, TAN_W, 0xe>(NPX, NPY, NPZ, sm, dps, t, diag, r);
     /* gravity source: r_m -= g (rho - rho_ref) cV */
     const double cv = m.cv[node];
     for (int c = 0; c < 3; c++) r[1 + c] -= m.g[c] * drho * cv;

@@ -18,8 +18,9 @@
  *           order, weak volume term gathered in the order the reference's
  *           scatter loop (field.h:3440-3464) adds it, gravity source,
  *           L = -Su/cV, Shu-Osher combination, primitives of the new state.
- * Roofline: FP64-pipe bound (about 1e3 FP64 instructions per node-stage
- * against 40-80 bytes of traffic).
+ * Roofline: FP64-pipe bound (hundreds of FP64 instructions per node-stage
+ * against 40-80 bytes of traffic); products with the zeros of a diagonal
+ * metric or an axis normal are left out (nsem_gather.cuh).
  */
 #include <cuda_runtime.h>
 
@@ -217,6 +218,53 @@ __global__ void __launch_bounds__(256) k_face(const NsemDev m, FaceArgs a) {
     if (side == 2) { mu2 = a.mq[0][ms]; cs2 = a.mq[1][ms]; r2v = a.mq[5][ms]; }
     const double lam = ((mu1v * fi + mu2 * fo) + (cs1v * fi + cs2 * fo)) / 2;
 
+    /* a normal along one axis (FP64-pipe bound: about 60 operations instead of
+     * 190): only the flux tensor's column of that axis meets a nonzero
+     * normal component; the products left out are zeros that change no sum
+     * (the lift starts at +0), provided nothing can overflow */
+    const int ax = side == 0 ? nsem_axis_of(n, en) : -1;
+    bool gok = true;
+    if (ax >= 0 && a.G[0])
+        for (int c = 0; c < 12; c++)
+            gok = gok && nsem_bounded(a.G[c][c1]) && (c2 < 0 || nsem_bounded(a.G[c][c2]));
+    if (ax >= 0 && gok && nsem_bounded(r1) && nsem_bounded(r2) && nsem_bounded(T1) && nsem_bounded(T2) &&
+        nsem_bounded(p1) && nsem_bounded(p2) && nsem_bounded(lam) && nsem_bounded(U1[0]) &&
+        nsem_bounded(U1[1]) && nsem_bounded(U1[2]) && nsem_bounded(U2[0]) && nsem_bounded(U2[1]) &&
+        nsem_bounded(U2[2])) {
+        const double na = nsem_pick(ax, n[0], n[1], n[2]), ea = nsem_pick(ax, en[0], en[1], en[2]);
+        const double Ua1 = nsem_pick(ax, U1[0], U1[1], U1[2]), Ua2 = nsem_pick(ax, U2[0], U2[1], U2[2]);
+        const double Fc1[3] = {U1[0] * r1, U1[1] * r1, U1[2] * r1};
+        const double Fc2[3] = {U2[0] * r2, U2[1] * r2, U2[2] * r2};
+        const double Fa1 = nsem_pick(ax, Fc1[0], Fc1[1], Fc1[2]);
+        const double Fa2 = nsem_pick(ax, Fc2[0], Fc2[1], Fc2[2]);
+        /* artificial viscosity: mu = rho nu */
+        const double mu1 = a.G[0] ? r1 * m.nu : 0.0, mu2 = a.G[0] ? r2 * m.nu : 0.0;
+        a.d[0][k] = ((Fa1 * fi + Fa2 * fo) - nsem_signed(ea, lam * (r2 - r1))) * na;
+        const double dq = nsem_signed(ea, (Fa2 - Fa1) * lam);
+        for (int r = 0; r < 3; r++) {
+            double A = Fc1[r] * Ua1, B = Fc2[r] * Ua2;
+            /* the pressure sits on the diagonal: p added there, 0 elsewhere */
+            const double A1 = A + p1, B1 = B + p2;
+            if (r == ax) { A = A1; B = B1; }
+            if (a.G[0]) {
+                const double* g = r == ax ? a.G[r] : a.G[r == 0 ? (ax == 1 ? XY : XZ)
+                                                         : r == 1 ? (ax == 2 ? YZ : YX) : (ax == 0 ? ZX : ZY)];
+                A = A - mu1 * g[c1];
+                B = B - mu2 * (c2 >= 0 ? g[c2] : 0.0);
+            }
+            const double F = A * fi + B * fo;
+            const double Fj = F - dq;
+            a.d[1 + r][k] = (r == ax ? Fj : F) * na;
+        }
+        double x = Fa1 * T1, y = Fa2 * T2;
+        if (a.G[0]) {
+            x = x - (mu1 * m.iPr) * a.G[9 + ax][c1];
+            y = y - (mu2 * m.iPr) * (c2 >= 0 ? a.G[9 + ax][c2] : 0.0);
+        }
+        a.d[4][k] = ((x * fi + y * fo) - nsem_signed(ea, lam * (r2 * T2 - r1 * T1))) * na;
+        return;
+    }
+
     /* continuity: flux U rho, state rho */
     {
         double F[3];
@@ -305,8 +353,10 @@ struct VolArgs {
     const double* dC[5];    /* non-conforming faces: the coarse side's lifted values */
 };
 
-/* shared layout per node: fr[3] fm[9] ft[3] jin[9] = 24 doubles */
+/* shared record per node: per direction c the flux column (U rho)_c, the
+ * momentum tensor's column c, the theta flux' component c; then jin[9] */
 constexpr int SM_W = 24;
+constexpr unsigned SM_ROWS = 0xe;   /* the momentum equations are tensor rows */
 
 __global__ void k_volume(const NsemDev m, const NsemTables tab, VolArgs a) {
     extern __shared__ double sm[];
@@ -327,9 +377,8 @@ __global__ void k_volume(const NsemDev m, const NsemTables tab, VolArgs a) {
         pp = a.prim[4][node];
         double* my = sm + (size_t)t * SM_W;
         const double Fc[3] = {U[0] * rho, U[1] * rho, U[2] * rho};
-        my[0] = Fc[0]; my[1] = Fc[1]; my[2] = Fc[2];          /* U*rho == rho*U */
         double fm[9];
-        outer(Fc, U, fm);
+        outer(Fc, U, fm);                                     /* U*rho == rho*U */
         for (int c = 0; c < 9; c++) fm[c] = fm[c] + ((c < 3) ? 1.0 : 0.0) * pp;
         double ft[3] = {Fc[0] * T, Fc[1] * T, Fc[2] * T};
         if (a.G[0]) {
@@ -337,54 +386,45 @@ __global__ void k_volume(const NsemDev m, const NsemTables tab, VolArgs a) {
             for (int c = 0; c < 9; c++) fm[c] = fm[c] - mu * a.G[c][node];
             for (int c = 0; c < 3; c++) ft[c] = ft[c] - (mu * m.iPr) * a.G[9 + c][node];
         }
-        for (int c = 0; c < 9; c++) my[3 + c] = fm[c];
-        my[12] = ft[0]; my[13] = ft[1]; my[14] = ft[2];
+        const int col[3][3] = {{XX, YX, ZX}, {XY, YY, ZY}, {XZ, YZ, ZZ}};
+        for (int c = 0; c < 3; c++) {
+            my[5 * c] = Fc[c];
+            for (int r = 0; r < 3; r++) my[5 * c + 1 + r] = fm[col[c][r]];
+            my[5 * c + 4] = ft[c];
+        }
         for (int c = 0; c < 9; c++) my[15 + c] = m.jin[(int64_t)c * m.n_int + node];
     }
-    __syncthreads();
+    const bool diag = __syncthreads_and(!active || nsem_node_diag<5>(sm + (size_t)t * SM_W));
     if (!active) return;
 
     /* surface lift, in the order div_flux visits the element's faces */
-    double r0 = 0.0, r1 = 0.0, r2 = 0.0, r3 = 0.0, r4 = 0.0;
+    double r[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     for (int j = 0; j < m.n_lift; j++) {
         const int32_t code = m.lift[(int64_t)j * m.n_int + node];
         if (code < 0) break;
         const int64_t k = code >> 2;
-        double v0, v1, v2, v3, v4;
-        if (code & 2) {
-            v0 = a.dC[0][k]; v1 = a.dC[1][k]; v2 = a.dC[2][k]; v3 = a.dC[3][k]; v4 = a.dC[4][k];
-        } else {
-            v0 = a.d[0][k]; v1 = a.d[1][k]; v2 = a.d[2][k]; v3 = a.d[3][k]; v4 = a.d[4][k];
-        }
-        if (code & 1) {
-            r0 -= v0; r1 -= v1; r2 -= v2; r3 -= v3; r4 -= v4;
-        } else {
-            r0 += v0; r1 += v1; r2 += v2; r3 += v3; r4 += v4;
+        for (int v = 0; v < 5; v++) {
+            const double x = (code & 2) ? a.dC[v][k] : a.d[v][k];
+            /* r - x is r + (-x): one add, the sign flipped in the bits */
+            r[v] += __hiloint2double(__double2hiint(x) ^ (code << 31), __double2loint(x));
         }
     }
 
     /* weak volume term.  Source b adds -F_b . (Jin_b . dpsi(b->a)); sources
      * arrive in lexicographic order of b: X-line below, Y-line below, Z-line
      * below, self, Z above, Y above, X above. */
-    nsem_volume_gather<SM_W, 15>(NPX, NPY, NPZ, sm, dps, t, [&](int lb, const double* dj) {
-        const double* sb = sm + (size_t)lb * SM_W;
-        double tv[3];
-        r0 -= vdot3(sb, dj);
-        tdot(sb + 3, dj, tv);
-        r1 -= tv[0]; r2 -= tv[1]; r3 -= tv[2];
-        r4 -= vdot3(sb + 12, dj);
-    });
+    nsem_volume_gather<5, SM_W, SM_ROWS>(NPX, NPY, NPZ, sm, dps, t, diag, r);
 
     /* gravity source: Su -= ((rho - rho_ref) g) cV */
     const double cv = m.cv[node];
     {
         const double s = rho - m.rho_ref[node];
         const double sc0 = 0.0 + m.g[0] * s, sc1 = 0.0 + m.g[1] * s, sc2 = 0.0 + m.g[2] * s;
-        r1 = r1 - sc0 * cv;
-        r2 = r2 - sc1 * cv;
-        r3 = r3 - sc2 * cv;
+        r[1] = r[1] - sc0 * cv;
+        r[2] = r[2] - sc1 * cv;
+        r[3] = r[3] - sc2 * cv;
     }
-    const double L[5] = {-(r0 / cv), -(r1 / cv), -(r2 / cv), -(r3 / cv), -(r4 / cv)};
+    const double L[5] = {-(r[0] / cv), -(r[1] / cv), -(r[2] / cv), -(r[3] / cv), -(r[4] / cv)};
 
     if (a.stage == 0) {
         for (int c = 0; c < 5; c++) a.out[c][node] = L[c];

@@ -267,19 +267,22 @@ __global__ void __launch_bounds__(256) k_seg_face_rho(const NsemDev m, SegArgs a
     }
     const double lam = ((mu1v * fi + mu2 * fo) + (cs1v * fi + cs2 * fo)) / 2;
     a.lam[k] = lam;
-    double F[3];
     const double jump = lam * (r2 - r1v);
+    /* a normal along one axis meets one component of the flux (the others'
+     * products are zeros that change no sum) */
+    const int ax = ms < 0 ? nsem_axis_of(n, en) : -1;
+    if (ax >= 0 && nsem_bounded(jump) && nsem_bounded(X1[0]) && nsem_bounded(X1[1]) &&
+        nsem_bounded(X1[2]) && nsem_bounded(X2[0]) && nsem_bounded(X2[1]) && nsem_bounded(X2[2])) {
+        a.d[0][k] = ((nsem_pick(ax, X1[0], X1[1], X1[2]) * fi + nsem_pick(ax, X2[0], X2[1], X2[2]) * fo) -
+                     nsem_signed(nsem_pick(ax, en[0], en[1], en[2]), jump)) *
+                    nsem_pick(ax, n[0], n[1], n[2]);
+        return;
+    }
+    double F[3];
     for (int c = 0; c < 3; c++) F[c] = (X1[c] * fi + X2[c] * fo) - en[c] * jump;
     a.d[0][k] = vdot3(F, n);
     if (ms >= 0)
         for (int c = 0; c < 3; c++) a.mf[c][ms] = F[c];
-}
-
-/* weak volume term of one node, sources in the reference's scatter order */
-template <int W, int JOFF, typename Apply>
-__device__ __forceinline__ void volume_gather(const NsemDev& m, const double* sm, const double* dps,
-                                              int t, Apply apply) {
-    nsem_volume_gather<W, JOFF>(m.npx, m.npy, m.npz, sm, dps, t, apply);
 }
 
 /* inputs and outputs of the strong-form gradients of U and theta */
@@ -369,7 +372,15 @@ __global__ void k_seg_grad_vol(const NsemDev m, const NsemTables tab, GradArgs a
         my[3] = a.Tf[node];
         for (int c = 0; c < 9; c++) my[4 + c] = m.jin[(int64_t)c * m.n_int + node];
     }
-    __syncthreads();
+    /* a diagonal metric (see nsem_volume_gather): only row r of the gradients
+     * takes line r's terms, 1 + 4 products a source instead of 3 + 12 */
+    bool ok = true;
+    if (active) {
+        const double* my = sm + (size_t)t * W_GRAD;
+        for (int c = 0; c < 7; c++) ok = ok && nsem_bounded(my[c]);
+        for (int c = 7; c < 13; c++) ok = ok && nsem_is_zero(my[c]);
+    }
+    const bool diag = __syncthreads_and(ok);
     if (!active) return;
     const double* me = sm + (size_t)t * W_GRAD;
     double gU[9], gT[3];
@@ -388,6 +399,24 @@ __global__ void k_seg_grad_vol(const NsemDev m, const NsemTables tab, GradArgs a
         const double n[3] = {m.fn[k], m.fn[m.n_slot + k], m.fn[2 * m.n_slot + k]};
         const double dU[3] = {f4[0] - me[0], f4[1] - me[1], f4[2] - me[2]};
         const double dT = f4[3] - me[3];
+        /* a normal along one axis reaches that axis' row only */
+        const double en[3] = {m.en[k], m.en[m.n_slot + k], m.en[2 * m.n_slot + k]};
+        const int ax = nsem_bounded(dU[0]) && nsem_bounded(dU[1]) && nsem_bounded(dU[2]) &&
+                               nsem_bounded(dT) ? nsem_axis_of(n, en) : -1;
+        if (ax >= 0) {
+            /* r - x is r + (-x): the sign goes into the normal's bits */
+            const double na = nsem_pick(ax, n[0], n[1], n[2]);
+            const double ns = __hiloint2double(__double2hiint(na) ^ (code << 31), __double2loint(na));
+            const double x[4] = {ns * dU[0], ns * dU[1], ns * dU[2], ns * dT};
+            if (ax == 0) {
+                gU[XX] += x[0]; gU[XY] += x[1]; gU[XZ] += x[2]; gT[0] += x[3];
+            } else if (ax == 1) {
+                gU[YX] += x[0]; gU[YY] += x[1]; gU[YZ] += x[2]; gT[1] += x[3];
+            } else {
+                gU[ZX] += x[0]; gU[ZY] += x[1]; gU[ZZ] += x[2]; gT[2] += x[3];
+            }
+            continue;
+        }
         double tU[9];
         outer(n, dU, tU);
         if (code & 1) {
@@ -413,6 +442,33 @@ __global__ void k_seg_grad_vol(const NsemDev m, const NsemTables tab, GradArgs a
         for (int c = 0; c < 3; c++) gT[c] += dj[c] * sb[3];
     };
     const int sx = NPY * NPZ, sy = NPZ;
+    if (diag) {
+        /* row r: the node's own term, which the x line's order puts first in
+         * rows y and z, then line r's sources in order */
+        auto row = [&](int lb, double dj, double& g0, double& g1, double& g2, double& gt) {
+            const double* sb = sm + (size_t)lb * W_GRAD;
+            g0 += dj * sb[0];
+            g1 += dj * sb[1];
+            g2 += dj * sb[2];
+            gt += dj * sb[3];
+        };
+        for (int ii = 0; ii < NPX; ii++)
+            row(t + (ii - ia) * sx, J[XX] * Dx[ia * NPX + ii], gU[XX], gU[XY], gU[XZ], gT[0]);
+        row(t, J[YY] * Dy[ja * NPY + ja], gU[YX], gU[YY], gU[YZ], gT[1]);
+        for (int q = 0; q + 1 < NPY; q++) {
+            const int jj = q < ja ? q : q + 1;
+            row(t + (jj - ja) * sy, J[YY] * Dy[ja * NPY + jj], gU[YX], gU[YY], gU[YZ], gT[1]);
+        }
+        row(t, J[ZZ] * Dz[ka * NPZ + ka], gU[ZX], gU[ZY], gU[ZZ], gT[2]);
+        for (int q = 0; q + 1 < NPZ; q++) {
+            const int kk = q < ka ? q : q + 1;
+            row(t + (kk - ka), J[ZZ] * Dz[ka * NPZ + kk], gU[ZX], gU[ZY], gU[ZZ], gT[2]);
+        }
+        const double cv = m.cv[node];
+        for (int c = 0; c < 9; c++) a.G[c][node] = gU[c] / cv;
+        for (int c = 0; c < 3; c++) a.G[9 + c][node] = gT[c] / cv;
+        return;
+    }
     /* every thread runs the same trip counts: the node's own term is selected
      * on the x line, and the y and z loops map past the node's index */
     double dj_self[3];
@@ -445,7 +501,8 @@ __global__ void k_seg_grad_vol(const NsemDev m, const NsemTables tab, GradArgs a
 }
 
 constexpr int W_RHO = 12;   /* fr[3] jin[9] */
-constexpr int W_UT = 21;    /* fm[9] ft[3] jin[9] */
+constexpr int W_UT = 21;    /* per direction: momentum tensor column [3], ft; then jin[9] */
+constexpr unsigned UT_ROWS = 0x7;   /* the U equations are tensor rows */
 
 __global__ void k_seg_vol_rho(const NsemDev m, const NsemTables tab, SegArgs a) {
     extern __shared__ double sm[];
@@ -464,7 +521,7 @@ __global__ void k_seg_vol_rho(const NsemDev m, const NsemTables tab, SegArgs a) 
         for (int c = 0; c < 3; c++) my[c] = a.U[c][node] * rho;     /* U * rho */
         for (int c = 0; c < 9; c++) my[3 + c] = m.jin[(int64_t)c * m.n_int + node];
     }
-    __syncthreads();
+    const bool diag = __syncthreads_and(!active || nsem_node_diag<1>(sm + (size_t)t * W_RHO));
     if (!active) return;
     double r = 0.0;
     for (int j = 0; j < m.n_lift; j++) {
@@ -475,9 +532,7 @@ __global__ void k_seg_vol_rho(const NsemDev m, const NsemTables tab, SegArgs a) 
         if (code & 1) r -= v;
         else r += v;
     }
-    volume_gather<W_RHO, 3>(m, sm, dps, t, [&](int lb, const double* dj) {
-        r -= vdot3(sm + (size_t)lb * W_RHO, dj);
-    });
+    nsem_volume_gather<1, W_RHO, 0>(m.npx, m.npy, m.npz, sm, dps, t, diag, &r);
     const double cv = m.cv[node];
     const double ap = a.c_dt * cv;
     const double rn = (r + rho * ap) / (0.0 + ap);
@@ -518,6 +573,43 @@ __global__ void __launch_bounds__(256) k_seg_face_ut(const NsemDev m, SegArgs a)
     /* a mortar's coarse side: interpolated from the coarse face's nodes */
     const int32_t ms = m.n_ms ? m.ms_of[k] : -1;
     const int mside = ms >= 0 ? ms_field(m, NSEM_MS_SIDE, ms) : 0;
+    /* a normal along one axis: only the flux tensor's column of that axis
+     * meets a nonzero normal component (about 45 operations instead of 160);
+     * the products left out are zeros that change no sum */
+    const int ax = mside == 0 ? nsem_axis_of(n, en) : -1;
+    bool ok = ax >= 0 && nsem_bounded(lam) && nsem_bounded(r1) && nsem_bounded(r2) &&
+              nsem_bounded(T1) && nsem_bounded(T2) && nsem_bounded(p1) && nsem_bounded(p2);
+    for (int c = 0; c < 3; c++)
+        ok = ok && nsem_bounded(U1[c]) && nsem_bounded(U2[c]) && nsem_bounded(Fc1[c]) && nsem_bounded(Fc2[c]);
+    if (a.visc && ok)
+        for (int c = 0; c < 12; c++)
+            ok = ok && nsem_bounded(a.G[c][c1]) && (c2 < 0 || nsem_bounded(a.G[c][c2]));
+    if (ok) {
+        const double na = nsem_pick(ax, n[0], n[1], n[2]), ea = nsem_pick(ax, en[0], en[1], en[2]);
+        const double Ua1 = nsem_pick(ax, U1[0], U1[1], U1[2]), Ua2 = nsem_pick(ax, U2[0], U2[1], U2[2]);
+        const double dq = nsem_signed(ea, (r2 * Ua2 - r1 * Ua1) * lam);
+        for (int r = 0; r < 3; r++) {
+            double A = Fc1[r] * Ua1, B = Fc2[r] * Ua2;
+            const double A1 = A + p1, B1 = B + p2;
+            if (r == ax) { A = A1; B = B1; }
+            if (a.visc) {
+                const double* g = r == ax ? a.G[r] : a.G[r == 0 ? (ax == 1 ? XY : XZ)
+                                                         : r == 1 ? (ax == 2 ? YZ : YX) : (ax == 0 ? ZX : ZY)];
+                A = A - mu1 * g[c1];
+                B = B - mu2 * (c2 >= 0 ? g[c2] : 0.0);
+            }
+            const double F = A * fi + B * fo;
+            const double Fj = F - dq;
+            a.d[1 + r][k] = (r == ax ? Fj : F) * na;
+        }
+        double x = nsem_pick(ax, Fc1[0], Fc1[1], Fc1[2]) * T1, y = nsem_pick(ax, Fc2[0], Fc2[1], Fc2[2]) * T2;
+        if (a.visc) {
+            x = x - (mu1 * m.iPr) * a.G[9 + ax][c1];
+            y = y - (mu2 * m.iPr) * (c2 >= 0 ? a.G[9 + ax][c2] : 0.0);
+        }
+        a.d[4][k] = ((x * fi + y * fo) - nsem_signed(ea, lam * (r2 * T2 - r1 * T1))) * na;
+        return;
+    }
     /* U equation: flux Fc (x) U + p' I - mu grad U, state rho U */
     {
         double A[9], B[9], O[9], F[9], dq[3], out[3], q1[3], q2[3];
@@ -598,49 +690,42 @@ __global__ void k_seg_vol_ut(const NsemDev m, const NsemTables tab, SegArgs a) {
         for (int c = 0; c < 3; c++) { U[c] = a.U[c][node]; Fc[c] = a.Fc[c][node]; }
         Tf = a.Tf[node];
         const double p = a.pp[node];
-        outer(Fc, U, my);
-        for (int c = 0; c < 9; c++) my[c] = my[c] + ((c < 3) ? 1.0 : 0.0) * p;
-        for (int c = 0; c < 3; c++) my[9 + c] = Fc[c] * Tf;
+        double fm[9], ft[3];
+        outer(Fc, U, fm);
+        for (int c = 0; c < 9; c++) fm[c] = fm[c] + ((c < 3) ? 1.0 : 0.0) * p;
+        for (int c = 0; c < 3; c++) ft[c] = Fc[c] * Tf;
         if (a.visc) {
             const double mu = a.rho_o[node] * m.nu;
-            for (int c = 0; c < 9; c++) my[c] = my[c] - mu * a.G[c][node];
-            for (int c = 0; c < 3; c++) my[9 + c] = my[9 + c] - (mu * m.iPr) * a.G[9 + c][node];
+            for (int c = 0; c < 9; c++) fm[c] = fm[c] - mu * a.G[c][node];
+            for (int c = 0; c < 3; c++) ft[c] = ft[c] - (mu * m.iPr) * a.G[9 + c][node];
+        }
+        const int col[3][3] = {{XX, YX, ZX}, {XY, YY, ZY}, {XZ, YZ, ZZ}};
+        for (int c = 0; c < 3; c++) {
+            for (int q = 0; q < 3; q++) my[4 * c + q] = fm[col[c][q]];
+            my[4 * c + 3] = ft[c];
         }
         for (int c = 0; c < 9; c++) my[12 + c] = m.jin[(int64_t)c * m.n_int + node];
     }
-    __syncthreads();
+    const bool diag = __syncthreads_and(!active || nsem_node_diag<4>(sm + (size_t)t * W_UT));
     if (!active) return;
-    double r1 = 0.0, r2 = 0.0, r3 = 0.0, r4 = 0.0;
+    double r[4] = {0.0, 0.0, 0.0, 0.0};
     for (int j = 0; j < m.n_lift; j++) {
         const int32_t code = m.lift[(int64_t)j * m.n_int + node];
         if (code < 0) break;
         const int64_t idx = code >> 2;
-        double v1, v2, v3, v4;
-        if (code & 2) {
-            v1 = a.dC[1][idx]; v2 = a.dC[2][idx]; v3 = a.dC[3][idx]; v4 = a.dC[4][idx];
-        } else {
-            v1 = a.d[1][idx]; v2 = a.d[2][idx]; v3 = a.d[3][idx]; v4 = a.d[4][idx];
-        }
-        if (code & 1) {
-            r1 -= v1; r2 -= v2; r3 -= v3; r4 -= v4;
-        } else {
-            r1 += v1; r2 += v2; r3 += v3; r4 += v4;
+        for (int v = 0; v < 4; v++) {
+            const double x = (code & 2) ? a.dC[1 + v][idx] : a.d[1 + v][idx];
+            /* r - x is r + (-x): one add, the sign flipped in the bits */
+            r[v] += __hiloint2double(__double2hiint(x) ^ (code << 31), __double2loint(x));
         }
     }
-    volume_gather<W_UT, 12>(m, sm, dps, t, [&](int lb, const double* dj) {
-        const double* sb = sm + (size_t)lb * W_UT;
-        double tv[3];
-        tdot(sb, dj, tv);
-        r1 -= tv[0]; r2 -= tv[1]; r3 -= tv[2];
-        r4 -= vdot3(sb + 9, dj);
-    });
+    nsem_volume_gather<4, W_UT, UT_ROWS>(m.npx, m.npy, m.npz, sm, dps, t, diag, r);
     const double cv = m.cv[node];
     const double rn = a.rho_n[node];
     const double ro = a.rho_o[node];
     const double s = rn - m.rho_ref[node];
     const double ap0 = a.c_dt * cv;
     const double ap = ap0 * rn;
-    const double r[3] = {r1, r2, r3};
     bool finite = isfinite(rn);
     for (int c = 0; c < 3; c++) {
         const double sc = 0.0 + m.g[c] * s;
@@ -649,7 +734,7 @@ __global__ void k_seg_vol_ut(const NsemDev m, const NsemTables tab, SegArgs a) {
         a.U[c][node] = un;
         finite = finite && isfinite(un);
     }
-    const double Tn = (r4 + (Tf * ro) * ap0) / (0.0 + ap);
+    const double Tn = (r[3] + (Tf * ro) * ap0) / (0.0 + ap);
     a.Tp[node] = Tn - m.T0;
     finite = finite && isfinite(Tn);
     if (!finite) atomicOr(m.status, NSEM_STATUS_NONFINITE);
@@ -836,8 +921,17 @@ __global__ void __launch_bounds__(256) k_conv_face(const NsemDev m, AdvArgs a) {
         for (int c = 0; c < 3; c++) X2[c] = a.mq[c][ms];
         T2v = a.mq[3][ms];
     }
-    double F[3];
     const double jump = a.lam[k] * (T2v - T1v);
+    /* a normal along one axis: one flux component (as k_seg_face_rho) */
+    const int ax = side == 0 ? nsem_axis_of(n, en) : -1;
+    if (ax >= 0 && nsem_bounded(jump) && nsem_bounded(X1[0]) && nsem_bounded(X1[1]) &&
+        nsem_bounded(X1[2]) && nsem_bounded(X2[0]) && nsem_bounded(X2[1]) && nsem_bounded(X2[2])) {
+        a.d[k] = ((nsem_pick(ax, X1[0], X1[1], X1[2]) * fi + nsem_pick(ax, X2[0], X2[1], X2[2]) * fo) -
+                  nsem_signed(nsem_pick(ax, en[0], en[1], en[2]), jump)) *
+                 nsem_pick(ax, n[0], n[1], n[2]);
+        return;
+    }
+    double F[3];
     for (int c = 0; c < 3; c++) F[c] = (X1[c] * fi + X2[c] * fo) - en[c] * jump;
     a.d[k] = vdot3(F, n);
     if (side)
@@ -863,7 +957,7 @@ __global__ void k_conv_vol(const NsemDev m, const NsemTables tab, AdvArgs a) {
         for (int c = 0; c < 3; c++) my[c] = a.U[c][node] * T;
         for (int c = 0; c < 9; c++) my[3 + c] = m.jin[(int64_t)c * m.n_int + node];
     }
-    __syncthreads();
+    const bool diag = __syncthreads_and(!active || nsem_node_diag<1>(sm + (size_t)t * W_CONV));
     if (!active) return;
     double r = 0.0;
     for (int j = 0; j < m.n_lift; j++) {
@@ -874,9 +968,7 @@ __global__ void k_conv_vol(const NsemDev m, const NsemTables tab, AdvArgs a) {
         if (code & 1) r -= v;
         else r += v;
     }
-    volume_gather<W_CONV, 3>(m, sm, dps, t, [&](int lb, const double* dj) {
-        r -= vdot3(sm + (size_t)lb * W_CONV, dj);
-    });
+    nsem_volume_gather<1, W_CONV, 0>(m.npx, m.npy, m.npz, sm, dps, t, diag, &r);
     const double ap = a.c_dt * m.cv[node];
     double Tn;
     if (a.ab2) {
