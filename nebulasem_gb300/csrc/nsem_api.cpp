@@ -151,6 +151,7 @@ nsem_status build_device_mesh(nsem_ctx* ctx, const nsem_mesh_desc* m, const nsem
     D.gamma = p->cp / p->cv;
     D.gR = D.gamma * D.R;
     D.P0 = p->P0;
+    D.dP0 = nsem_make_divisor(p->P0);
     D.cp = p->cp;
     D.T0 = p->T0;
     D.nu = p->viscosity;

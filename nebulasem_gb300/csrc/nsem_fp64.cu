@@ -55,10 +55,9 @@ __device__ __forceinline__ void outer(const double* p, const double* q, double* 
     r[ZX] = p[2] * q[0];
 }
 
-/* ghost velocity of the SYMMETRY condition (src/tensor/tensor.h:486-494) */
-__device__ __forceinline__ void sym_vec(const double* p, const double* n, double* out) {
-    const double mg = sqrt(vdot3(n, n));
-    const double en[3] = {n[0] / mg, n[1] / mg, n[2] / mg};
+/* ghost velocity of the SYMMETRY condition (src/tensor/tensor.h:486-494), en
+ * the slot's unit normal */
+__device__ __forceinline__ void sym_vec(const double* p, const double* en, double* out) {
     const double A0 = 1.0 - en[0] * en[0];
     const double A1 = 1.0 - en[1] * en[1];
     const double A2 = 1.0 - en[2] * en[2];
@@ -69,12 +68,12 @@ __device__ __forceinline__ void sym_vec(const double* p, const double* n, double
     r[0] = A0 * p[0] + A3 * p[1] + A5 * p[2];
     r[1] = A3 * p[0] + A1 * p[1] + A4 * p[2];
     r[2] = A5 * p[0] + A4 * p[1] + A2 * p[2];
-    const double magR = sqrt(vdot3(r, r));
+    const double magR = nsem_sqrt(vdot3(r, r));
     if (fabs(magR - 0.0) <= 1e-7) {
         out[0] = r[0]; out[1] = r[1]; out[2] = r[2];
         return;
     }
-    const double s = sqrt(vdot3(p, p)) / magR;
+    const double s = nsem_div(nsem_sqrt(vdot3(p, p)), magR);
     out[0] = r[0] * s; out[1] = r[1] * s; out[2] = r[2] * s;
 }
 
@@ -86,19 +85,20 @@ struct PrimArgs {
 __device__ __forceinline__ void prim_at(const NsemDev& m, const double* const* S,
                                         double* const* prim, int64_t i) {
     const double r = S[0][i];
+    const nsem_divisor dr = nsem_make_divisor(r);
     double U[3];
-    U[0] = S[1][i] / r;
-    U[1] = S[2][i] / r;
-    U[2] = S[3][i] / r;
-    const double T = S[4][i] / r;
-    const double p = m.P0 * nsem_pow(((r * T) * m.R) / m.P0, m.gamma);
+    U[0] = nsem_div_by(S[1][i], dr);
+    U[1] = nsem_div_by(S[2][i], dr);
+    U[2] = nsem_div_by(S[3][i], dr);
+    const double T = nsem_div_by(S[4][i], dr);
+    const double p = m.P0 * nsem_pow(nsem_div_by((r * T) * m.R, m.dP0), m.gamma);
     prim[0][i] = U[0];
     prim[1][i] = U[1];
     prim[2][i] = U[2];
     prim[3][i] = T;
     prim[4][i] = p - m.p_ref[i];
-    prim[5][i] = sqrt(vdot3(U, U));
-    prim[6][i] = sqrt(m.gR * T);
+    prim[5][i] = nsem_sqrt(vdot3(U, U));
+    prim[6][i] = nsem_sqrt(m.gR * T);
 }
 
 __global__ void __launch_bounds__(256) k_prim(const NsemDev m, PrimArgs a) {
@@ -203,12 +203,12 @@ __global__ void __launch_bounds__(256) k_face(const NsemDev m, FaceArgs a) {
         T2 = T1 + 0.0;
         p2 = p1;
         if (m.bc[k] == 2) {
-            sym_vec(U1, n, U2);
+            sym_vec(U1, en, U2);
         } else {
             U2[0] = U1[0] + 0.0; U2[1] = U1[1] + 0.0; U2[2] = U1[2] + 0.0;
         }
-        mu2 = sqrt(vdot3(U2, U2));
-        cs2 = sqrt(m.gR * T2);
+        mu2 = nsem_sqrt(vdot3(U2, U2));
+        cs2 = cs1;   /* sqrt(gamma R theta) of the same theta */
     }
     /* a mortar's coarse side (1: c1, 2: c2) takes interpolated quantities */
     const int32_t ms = m.n_ms ? m.ms_of[k] : -1;
@@ -424,7 +424,9 @@ __global__ void k_volume(const NsemDev m, const NsemTables tab, VolArgs a) {
         r[2] = r[2] - sc1 * cv;
         r[3] = r[3] - sc2 * cv;
     }
-    const double L[5] = {-(r[0] / cv), -(r[1] / cv), -(r[2] / cv), -(r[3] / cv), -(r[4] / cv)};
+    const nsem_divisor dcv = nsem_make_divisor(cv);
+    double L[5];
+    for (int v = 0; v < 5; v++) L[v] = -nsem_div_by(r[v], dcv);
 
     if (a.stage == 0) {
         for (int c = 0; c < 5; c++) a.out[c][node] = L[c];

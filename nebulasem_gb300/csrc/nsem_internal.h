@@ -20,6 +20,8 @@
 
 #include <stdint.h>
 
+#include "nsem_intfp.h"
+
 #define NSEM_MAX_NPD 10          /* up to order 9 per direction */
 #define NSEM_NPRIM 7
 #define NSEM_STATUS_NONFINITE 1u
@@ -40,6 +42,7 @@ struct NsemDev {
     int64_t n_elem, n_int, n_slot;
     /* physical constants */
     double P0, R, gamma, gR, cv_heat, cp, T0;
+    nsem_divisor dP0;  /* P0 prepared for nsem_div_by */
     double nu, iPr;    /* artificial viscosity (segregated scheme), 1 / Pr */
     double g[3];
     /* node arrays */

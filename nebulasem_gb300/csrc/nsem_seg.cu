@@ -71,10 +71,9 @@ __device__ __forceinline__ void outer(const double* p, const double* q, double* 
     r[ZX] = p[2] * q[0];
 }
 
-/* SYMMETRY ghost velocity (src/tensor/tensor.h:486-494) */
-__device__ __forceinline__ void sym_vec(const double* p, const double* n, double* out) {
-    const double mg = sqrt(vdot3(n, n));
-    const double en[3] = {n[0] / mg, n[1] / mg, n[2] / mg};
+/* SYMMETRY ghost velocity (src/tensor/tensor.h:486-494), en the slot's unit
+ * normal */
+__device__ __forceinline__ void sym_vec(const double* p, const double* en, double* out) {
     const double A0 = 1.0 - en[0] * en[0];
     const double A1 = 1.0 - en[1] * en[1];
     const double A2 = 1.0 - en[2] * en[2];
@@ -85,20 +84,20 @@ __device__ __forceinline__ void sym_vec(const double* p, const double* n, double
     r[0] = A0 * p[0] + A3 * p[1] + A5 * p[2];
     r[1] = A3 * p[0] + A1 * p[1] + A4 * p[2];
     r[2] = A5 * p[0] + A4 * p[1] + A2 * p[2];
-    const double magR = sqrt(vdot3(r, r));
+    const double magR = nsem_sqrt(vdot3(r, r));
     if (fabs(magR - 0.0) <= 1e-7) {
         out[0] = r[0]; out[1] = r[1]; out[2] = r[2];
         return;
     }
-    const double s = sqrt(vdot3(p, p)) / magR;
+    const double s = nsem_div(nsem_sqrt(vdot3(p, p)), magR);
     out[0] = r[0] * s; out[1] = r[1] * s; out[2] = r[2] * s;
 }
 
 /* ghost velocity of slot k from the owner's */
-__device__ __forceinline__ void ghost_U(const NsemDev& m, int64_t k, const double* n,
-                                        const double* U1, double* U2) {
+__device__ __forceinline__ void ghost_U(const NsemDev& m, int64_t k, const double* U1, double* U2) {
     if (m.bc[k] == 2) {
-        sym_vec(U1, n, U2);
+        const double en[3] = {m.en[k], m.en[m.n_slot + k], m.en[2 * m.n_slot + k]};
+        sym_vec(U1, en, U2);
     } else {
         U2[0] = U1[0] + 0.0; U2[1] = U1[1] + 0.0; U2[2] = U1[2] + 0.0;
     }
@@ -219,8 +218,8 @@ __global__ void __launch_bounds__(256) k_seg_prep(const NsemDev m, SegArgs a) {
     const double Tf = a.Tp[i] + m.T0;
     a.Tf[i] = Tf;
     for (int c = 0; c < 3; c++) a.Fc[c][i] = r * U[c];
-    a.mu[i] = sqrt(vdot3(U, U));
-    a.cs[i] = sqrt(m.gR * Tf);
+    a.mu[i] = nsem_sqrt(vdot3(U, U));
+    a.cs[i] = nsem_sqrt(m.gR * Tf);
 }
 
 __global__ void __launch_bounds__(256) k_seg_face_rho(const NsemDev m, SegArgs a) {
@@ -240,9 +239,9 @@ __global__ void __launch_bounds__(256) k_seg_face_rho(const NsemDev m, SegArgs a
         mu2 = a.mu[c2]; cs2 = a.cs[c2];
     } else {
         r2 = r1 + 0.0;
-        ghost_U(m, k, n, U1, U2);
-        mu2 = sqrt(vdot3(U2, U2));
-        cs2 = sqrt(m.gR * (a.Tf[c1] + 0.0));
+        ghost_U(m, k, U1, U2);
+        mu2 = nsem_sqrt(vdot3(U2, U2));
+        cs2 = cs1;   /* sqrt(gamma R theta) of the same theta */
     }
     double X1[3], X2[3];
     for (int c = 0; c < 3; c++) {
@@ -338,7 +337,6 @@ __global__ void __launch_bounds__(256) k_seg_grad_face(const NsemDev m, GradArgs
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= m.n_slot) return;
     const int32_t c1 = m.c1[k], c2 = m.c2[k];
-    const double n[3] = {m.fn[k], m.fn[m.n_slot + k], m.fn[2 * m.n_slot + k]};
     const double fi = m.fi[k], fo = 1 - fi;
     const double U1[3] = {a.U[0][c1], a.U[1][c1], a.U[2][c1]};
     const double T1 = a.Tf[c1];
@@ -347,7 +345,7 @@ __global__ void __launch_bounds__(256) k_seg_grad_face(const NsemDev m, GradArgs
         U2[0] = a.U[0][c2]; U2[1] = a.U[1][c2]; U2[2] = a.U[2][c2];
         T2 = a.Tf[c2];
     } else {
-        ghost_U(m, k, n, U1, U2);
+        ghost_U(m, k, U1, U2);
         T2 = T1 + 0.0;
     }
     for (int c = 0; c < 3; c++) a.fF[c][k] = (U1[c] * fi) + (U2[c] * fo);
@@ -465,8 +463,9 @@ __global__ void k_seg_grad_vol(const NsemDev m, const NsemTables tab, GradArgs a
             row(t + (kk - ka), J[ZZ] * Dz[ka * NPZ + kk], gU[ZX], gU[ZY], gU[ZZ], gT[2]);
         }
         const double cv = m.cv[node];
-        for (int c = 0; c < 9; c++) a.G[c][node] = gU[c] / cv;
-        for (int c = 0; c < 3; c++) a.G[9 + c][node] = gT[c] / cv;
+        const nsem_divisor dcv = nsem_make_divisor(cv);
+        for (int c = 0; c < 9; c++) a.G[c][node] = nsem_div_by(gU[c], dcv);
+        for (int c = 0; c < 3; c++) a.G[9 + c][node] = nsem_div_by(gT[c], dcv);
         return;
     }
     /* every thread runs the same trip counts: the node's own term is selected
@@ -496,8 +495,9 @@ __global__ void k_seg_grad_vol(const NsemDev m, const NsemTables tab, GradArgs a
         add(t + (kk - ka), dj);
     }
     const double cv = m.cv[node];
-    for (int c = 0; c < 9; c++) a.G[c][node] = gU[c] / cv;
-    for (int c = 0; c < 3; c++) a.G[9 + c][node] = gT[c] / cv;
+    const nsem_divisor dcv = nsem_make_divisor(cv);
+    for (int c = 0; c < 9; c++) a.G[c][node] = nsem_div_by(gU[c], dcv);
+    for (int c = 0; c < 3; c++) a.G[9 + c][node] = nsem_div_by(gT[c], dcv);
 }
 
 constexpr int W_RHO = 12;   /* fr[3] jin[9] */
@@ -535,9 +535,9 @@ __global__ void k_seg_vol_rho(const NsemDev m, const NsemTables tab, SegArgs a) 
     nsem_volume_gather<1, W_RHO, 0>(m.npx, m.npy, m.npz, sm, dps, t, diag, &r);
     const double cv = m.cv[node];
     const double ap = a.c_dt * cv;
-    const double rn = (r + rho * ap) / (0.0 + ap);
+    const double rn = nsem_div(r + rho * ap, 0.0 + ap);
     a.rho_n[node] = rn;
-    const double p = m.P0 * nsem_pow(((rn * a.Tf[node]) * m.R) / m.P0, m.gamma);
+    const double p = m.P0 * nsem_pow(nsem_div_by((rn * a.Tf[node]) * m.R, m.dP0), m.gamma);
     a.pp[node] = p - m.p_ref[node];
 }
 
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(256) k_seg_face_ut(const NsemDev m, SegArgs a)
         p2 = a.pp[c2];
     } else {
         r2 = r1 + 0.0;
-        ghost_U(m, k, n, U1, U2);
+        ghost_U(m, k, U1, U2);
         const double ro2 = a.rho_o[c1] + 0.0;
         for (int c = 0; c < 3; c++) Fc2[c] = ro2 * U2[c];
         T2 = T1 + 0.0;
@@ -726,15 +726,16 @@ __global__ void k_seg_vol_ut(const NsemDev m, const NsemTables tab, SegArgs a) {
     const double s = rn - m.rho_ref[node];
     const double ap0 = a.c_dt * cv;
     const double ap = ap0 * rn;
+    const nsem_divisor dap = nsem_make_divisor(0.0 + ap);
     bool finite = isfinite(rn);
     for (int c = 0; c < 3; c++) {
         const double sc = 0.0 + m.g[c] * s;
         const double su = r[c] - sc * cv;
-        const double un = (su + (U[c] * ro) * ap0) / (0.0 + ap);
+        const double un = nsem_div_by(su + (U[c] * ro) * ap0, dap);
         a.U[c][node] = un;
         finite = finite && isfinite(un);
     }
-    const double Tn = (r[3] + (Tf * ro) * ap0) / (0.0 + ap);
+    const double Tn = nsem_div_by(r[3] + (Tf * ro) * ap0, dap);
     a.Tp[node] = Tn - m.T0;
     finite = finite && isfinite(Tn);
     if (!finite) atomicOr(m.status, NSEM_STATUS_NONFINITE);
@@ -763,8 +764,9 @@ __global__ void __launch_bounds__(256) k_cons_to_seg(const NsemDev m, ConvArgs a
     if (i >= m.n_int) return;
     const double r = a.u[0][i];
     a.rho_w[i] = r;
-    for (int c = 0; c < 3; c++) a.U[c][i] = a.u[1 + c][i] / r;
-    a.Tp[i] = a.u[4][i] / r - m.T0;
+    const nsem_divisor dr = nsem_make_divisor(r);
+    for (int c = 0; c < 3; c++) a.U[c][i] = nsem_div_by(a.u[1 + c][i], dr);
+    a.Tp[i] = nsem_div_by(a.u[4][i], dr) - m.T0;
 }
 
 SegArgs seg_args(const NsemDev* m, NsemSegBuf* b, int cur, double dt) {
@@ -843,7 +845,7 @@ __global__ void __launch_bounds__(128) k_conv_mortar(const NsemDev m, AdvArgs a)
     mortar_interp<1>(m, ms, [&](int64_t node, double* v) {
         if (STAGE == 0) {
             const double U[3] = {a.U[0][node], a.U[1][node], a.U[2][node]};
-            v[0] = sqrt(vdot3(U, U));
+            v[0] = nsem_sqrt(vdot3(U, U));
         } else {
             v[0] = c < 3 ? a.U[c][node] * a.T_o[node] : a.T_o[node];
         }
@@ -865,7 +867,6 @@ __global__ void __launch_bounds__(256) k_conv_lambda(const NsemDev m, AdvArgs a)
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= m.n_slot) return;
     const int32_t c1 = m.c1[k], c2 = m.c2[k];
-    const double n[3] = {m.fn[k], m.fn[m.n_slot + k], m.fn[2 * m.n_slot + k]};
     const double fi = m.fi[k], fo = 1 - fi;
     const double U1[3] = {a.U[0][c1], a.U[1][c1], a.U[2][c1]};
     double U2[3];
@@ -874,9 +875,9 @@ __global__ void __launch_bounds__(256) k_conv_lambda(const NsemDev m, AdvArgs a)
     } else if (a.Ug[0]) {
         U2[0] = a.Ug[0][k]; U2[1] = a.Ug[1][k]; U2[2] = a.Ug[2][k];
     } else {
-        ghost_U(m, k, n, U1, U2);
+        ghost_U(m, k, U1, U2);
     }
-    double u1 = sqrt(vdot3(U1, U1)), u2 = sqrt(vdot3(U2, U2));
+    double u1 = nsem_sqrt(vdot3(U1, U1)), u2 = nsem_sqrt(vdot3(U2, U2));
     const int32_t ms = m.n_ms ? m.ms_of[k] : -1;
     if (ms >= 0) {
         if (ms_field(m, NSEM_MS_SIDE, ms) == 1) u1 = a.mq[0][ms];
@@ -902,7 +903,7 @@ __global__ void __launch_bounds__(256) k_conv_face(const NsemDev m, AdvArgs a) {
         if (a.Ug[0]) {
             U2[0] = a.Ug[0][k]; U2[1] = a.Ug[1][k]; U2[2] = a.Ug[2][k];
         } else {
-            ghost_U(m, k, n, U1, U2);
+            ghost_U(m, k, U1, U2);
         }
         T2 = T1 + 0.0;
     }
@@ -973,10 +974,10 @@ __global__ void k_conv_vol(const NsemDev m, const NsemTables tab, AdvArgs a) {
     double Tn;
     if (a.ab2) {
         /* AB2: Su = T ap + (3 R^n - R^{n-1}) / 2, T = Su / ap */
-        Tn = (T * ap + (3.0 * r - a.R_o[node]) / 2.0) / ap;
+        Tn = nsem_div(T * ap + (3.0 * r - a.R_o[node]) / 2.0, ap);
     } else {
         /* BDF1 / AB1 (the same sum in either order): T = (R + T ap) / ap */
-        Tn = (r + T * ap) / (0.0 + ap);
+        Tn = nsem_div(r + T * ap, 0.0 + ap);
     }
     if (a.R_n) a.R_n[node] = r;
     a.T_n[node] = Tn;

@@ -294,6 +294,34 @@ def pow_fast_sweep(n, seed, xlo, xhi, y):
     return fb.value, mm.value
 
 
+def pow_int_sweep(n, seed, xlo, xhi, y):
+    """(fallbacks, mismatches) of the fixed-point phase over n log-uniform x."""
+    fb, mm = ctypes.c_int64(), ctypes.c_int64()
+    lib().nsem_oracle_pow_int_sweep(ctypes.c_int64(n), ctypes.c_uint64(seed), ctypes.c_double(xlo),
+                                    ctypes.c_double(xhi), ctypes.c_double(y), ctypes.byref(fb),
+                                    ctypes.byref(mm))
+    return fb.value, mm.value
+
+
+def intfp_sweep(n, seed):
+    """Mismatches (div, sqrt, mul) of the integer operations with the hardware's."""
+    bad = (ctypes.c_int64 * 3)()
+    lib().nsem_oracle_intfp_sweep(ctypes.c_int64(n), ctypes.c_uint64(seed), bad)
+    return tuple(bad)
+
+
+def intfp_div(a, b):
+    f = lib().nsem_oracle_intfp_div
+    f.restype, f.argtypes = ctypes.c_double, [ctypes.c_double] * 2
+    return f(a, b)
+
+
+def intfp_sqrt(a):
+    f = lib().nsem_oracle_intfp_sqrt
+    f.restype, f.argtypes = ctypes.c_double, [ctypes.c_double]
+    return f(a)
+
+
 def load_dump(path):
     """Read a harness dump directory (raw .f64/.u32 files) into a dict."""
     out = {}
