@@ -28,6 +28,7 @@
 #include <cuda_runtime.h>
 
 #include "nsem_adjoint.h"
+#include "nsem_ddpow.h"
 #include "nsem_seg.h"
 #include "nsem_gather.cuh"
 #include "nsem_mortar.cuh"
@@ -50,17 +51,26 @@ struct NodePrim {
     double r, U[3], T, p, pp, mu, c;   /* p: full pressure, pp = p - p_ref */
 };
 
+/* EOS: false leaves the pressures out, where a caller has no use for them.
+ * Divisions, roots and the power run on the integer pipes (nsem_intfp.h): the
+ * FP64 pipe bounds these kernels. */
+template <bool EOS = true>
 __device__ __forceinline__ NodePrim node_prim(const NsemDev& m, const double* const* S, int64_t i) {
     NodePrim q;
     q.r = S[0][i];
-    q.U[0] = S[1][i] / q.r;
-    q.U[1] = S[2][i] / q.r;
-    q.U[2] = S[3][i] / q.r;
-    q.T = S[4][i] / q.r;
-    q.p = m.P0 * pow(((q.r * q.T) * m.R) / m.P0, m.gamma);
-    q.pp = q.p - m.p_ref[i];
-    q.mu = sqrt(vdot3(q.U, q.U));
-    q.c = sqrt(m.gR * q.T);
+    const nsem_divisor dr = nsem_make_divisor(q.r);
+    q.U[0] = nsem_div_by(S[1][i], dr);
+    q.U[1] = nsem_div_by(S[2][i], dr);
+    q.U[2] = nsem_div_by(S[3][i], dr);
+    q.T = nsem_div_by(S[4][i], dr);
+    if constexpr (EOS) {
+        q.p = m.P0 * nsem_pow(nsem_div_by((q.r * q.T) * m.R, m.dP0), m.gamma);
+        q.pp = q.p - m.p_ref[i];
+    } else {
+        q.p = q.pp = 0.0;
+    }
+    q.mu = nsem_sqrt(vdot3(q.U, q.U));
+    q.c = nsem_sqrt(m.gR * q.T);
     return q;
 }
 
@@ -72,8 +82,8 @@ __device__ __forceinline__ void sym_fwd(const double* p, const double* en, doubl
     r[0] = p[0] - en[0] * dn;
     r[1] = p[1] - en[1] * dn;
     r[2] = p[2] - en[2] * dn;
-    magR = sqrt(vdot3(r, r));
-    magP = sqrt(vdot3(p, p));
+    magR = nsem_sqrt(vdot3(r, r));
+    magP = nsem_sqrt(vdot3(p, p));
     scaled = !(fabs(magR) <= 1e-7);
     const double s = scaled ? magP / magR : 1.0;
     out[0] = r[0] * s; out[1] = r[1] * s; out[2] = r[2] * s;
@@ -115,26 +125,28 @@ __global__ void __launch_bounds__(128) k_adj_face(const NsemDev m, FaceAdjArgs a
     const int32_t c1 = m.c1[k], c2 = m.c2[k];
     const double n[3] = {m.fn[k], m.fn[m.n_slot + k], m.fn[2 * m.n_slot + k]};
     const double en[3] = {m.en[k], m.en[m.n_slot + k], m.en[2 * m.n_slot + k]};
-    const double nmag = sqrt(vdot3(n, n));
     const double fi = m.fi[k], fo = 1 - fi;
 
-    const NodePrim P1 = node_prim(m, a.S, c1);
+    const NodePrim P1 = node_prim<false>(m, a.S, c1);
     NodePrim P2;
     double rsym[3] = {0, 0, 0}, magR = 0, magP = 0;
     bool scaled = false;
     if (c2 >= 0) {
-        P2 = node_prim(m, a.S, c2);
+        P2 = node_prim<false>(m, a.S, c2);
     } else {
         P2 = P1;
         if (m.bc[k] == 2) sym_fwd(P1.U, en, P2.U, rsym, magR, magP, scaled);
-        P2.mu = sqrt(vdot3(P2.U, P2.U));
+        P2.mu = nsem_sqrt(vdot3(P2.U, P2.U));
     }
     /* dbar from rbar = -w / cV */
     double db[5];
-    for (int v = 0; v < 5; v++) {
-        double x = -a.W[v][c1] / m.cv[c1];
-        if (c2 >= 0) x -= -a.W[v][c2] / m.cv[c2];
-        db[v] = x;
+    {
+        const nsem_divisor v1 = nsem_make_divisor(m.cv[c1]), v2 = nsem_make_divisor(m.cv[c2 >= 0 ? c2 : c1]);
+        for (int v = 0; v < 5; v++) {
+            double x = -nsem_div_by(a.W[v][c1], v1);
+            if (c2 >= 0) x += nsem_div_by(a.W[v][c2], v2);
+            db[v] = x;
+        }
     }
     if (a.dbv[0]) {
         for (int c = 0; c < 3; c++) a.dbv[c][k] = db[1 + c];
@@ -144,6 +156,56 @@ __global__ void __launch_bounds__(128) k_adj_face(const NsemDev m, FaceAdjArgs a
     /* primitive adjoints of both sides */
     double rb1 = 0, rb2 = 0, Ub1[3] = {0, 0, 0}, Ub2[3] = {0, 0, 0}, Tb1 = 0, Tb2 = 0, pb1 = 0,
            pb2 = 0, lamb = 0;
+    /* a normal along one axis: only that axis' flux components have adjoints
+     * (the products left out are zeros, as long as nothing overflows); about
+     * 110 FP64 instructions instead of 300.  Measured with the integer
+     * divisions and roots on 60 k slots: 101 -> 31 us. */
+    const int ax = nsem_axis_of(n, en);
+    bool bounded = ax >= 0 && nsem_bounded(lam) && nsem_bounded(P1.r) && nsem_bounded(P2.r) &&
+                   nsem_bounded(P1.T) && nsem_bounded(P2.T);
+    for (int v = 0; v < 5; v++) bounded = bounded && nsem_bounded(db[v]);
+    for (int c = 0; c < 3; c++) bounded = bounded && nsem_bounded(P1.U[c]) && nsem_bounded(P2.U[c]);
+    if (bounded) {
+        const double na = nsem_pick(ax, n[0], n[1], n[2]), ea = nsem_pick(ax, en[0], en[1], en[2]);
+        const double w1 = na * fi, w2 = na * fo, nm = fabs(na);
+        const double Ua1 = nsem_pick(ax, P1.U[0], P1.U[1], P1.U[2]);
+        const double Ua2 = nsem_pick(ax, P2.U[0], P2.U[1], P2.U[2]);
+        const double dba = nsem_pick(ax, db[1], db[2], db[3]);
+        /* the flux averages: mass, theta and momentum rows against the side's
+         * normal velocity, as sum_v db_v q_v with q = (1, U, theta) */
+        const double q1 = db[0] + vdot3(db + 1, P1.U) + db[4] * P1.T;
+        const double q2 = db[0] + vdot3(db + 1, P2.U) + db[4] * P2.T;
+        const double m1 = w1 * P1.r, m2 = w2 * P2.r;
+        const double Uax1 = m1 * q1, Uax2 = m2 * q2;
+        rb1 = w1 * Ua1 * q1;
+        rb2 = w2 * Ua2 * q2;
+        const double f1 = m1 * Ua1, f2 = m2 * Ua2;
+        Tb1 = f1 * db[4];
+        Tb2 = f2 * db[4];
+        pb1 = w1 * dba;
+        pb2 = w2 * dba;
+        /* the jumps: lambda times rho, normal momentum, rho theta, with
+         * en_c en_c |n| = |n| on the axis */
+        const double j0 = nm * db[0], jm = nm * dba, j4 = nm * db[4];
+        lamb = -(j0 * (P2.r - P1.r) + jm * (P2.r * Ua2 - P1.r * Ua1) + j4 * (P2.r * P2.T - P1.r * P1.T));
+        rb1 += lam * (j0 + jm * Ua1 + j4 * P1.T);
+        rb2 -= lam * (j0 + jm * Ua2 + j4 * P2.T);
+        Tb1 += lam * j4 * P1.r;
+        Tb2 -= lam * j4 * P2.r;
+        const double ja1 = lam * jm * P1.r, ja2 = -(lam * jm * P2.r);
+        /* lambda -> |U|, c */
+        const double h1 = lamb * fi / 2, h2 = lamb * fo / 2;
+        const double k1 = P1.mu > 0 ? nsem_div(h1, P1.mu) : 0.0, k2 = P2.mu > 0 ? nsem_div(h2, P2.mu) : 0.0;
+        if (P1.c > 0) Tb1 += nsem_div(h1 * m.gR, 2 * P1.c);
+        if (P2.c > 0) Tb2 += nsem_div(h2 * m.gR, 2 * P2.c);
+        for (int c = 0; c < 3; c++) {
+            Ub1[c] = f1 * db[1 + c] + k1 * P1.U[c];
+            Ub2[c] = f2 * db[1 + c] + k2 * P2.U[c];
+            const double x1 = Ub1[c] + (Uax1 + ja1), x2 = Ub2[c] + (Uax2 + ja2);
+            if (c == ax) { Ub1[c] = x1; Ub2[c] = x2; }
+        }
+    } else {
+    const double nmag = nsem_sqrt(vdot3(n, n));
     /* continuity */
     {
         const double A0 = db[0] * nmag;     /* sum_c Fbar_c en_c */
@@ -197,10 +259,14 @@ __global__ void __launch_bounds__(128) k_adj_face(const NsemDev m, FaceAdjArgs a
     {
         const double mub1 = lamb * fi / 2, mub2 = lamb * fo / 2;
         const double cb1 = lamb * fi / 2, cb2 = lamb * fo / 2;
-        if (P1.mu > 0) for (int c = 0; c < 3; c++) Ub1[c] += mub1 * P1.U[c] / P1.mu;
-        if (P2.mu > 0) for (int c = 0; c < 3; c++) Ub2[c] += mub2 * P2.U[c] / P2.mu;
-        if (P1.c > 0) Tb1 += cb1 * m.gR / (2 * P1.c);
-        if (P2.c > 0) Tb2 += cb2 * m.gR / (2 * P2.c);
+        const double k1 = P1.mu > 0 ? nsem_div(mub1, P1.mu) : 0.0, k2 = P2.mu > 0 ? nsem_div(mub2, P2.mu) : 0.0;
+        for (int c = 0; c < 3; c++) {
+            Ub1[c] += k1 * P1.U[c];
+            Ub2[c] += k2 * P2.U[c];
+        }
+        if (P1.c > 0) Tb1 += nsem_div(cb1 * m.gR, 2 * P1.c);
+        if (P2.c > 0) Tb2 += nsem_div(cb2 * m.gR, 2 * P2.c);
+    }
     }
     if (c2 < 0) {
         /* ghost: fold into the owner */
@@ -302,55 +368,61 @@ __global__ void __maxnreg__(VISC ? 128 : 88) k_adj_volume(const NsemDev m, const
     const int64_t node = e * NP + t;
     const bool active = t < NP;
     if (active) {
-        const double cv = m.cv[node];
-        for (int v = 0; v < 5; v++) rb[v * NP + t] = -a.W[v][node] / cv;
+        const nsem_divisor dcv = nsem_make_divisor(m.cv[node]);
+        for (int v = 0; v < 5; v++) rb[v * NP + t] = -nsem_div_by(a.W[v][node], dcv);
     }
     __syncthreads();
     if (!active) return;
     const int ia = t / (NPY * NPZ), ja = (t / NPZ) % NPY, ka = t % NPZ;
     const NodePrim P = node_prim(m, a.S, node);
-    double Jin[9];
-    for (int c = 0; c < 9; c++) Jin[c] = m.jin[(int64_t)c * m.n_int + node];
 
-    /* transposed volume gather: G_c, H_rc, K_c over the targets a of node b */
-    double Gv[3] = {0, 0, 0}, H[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, K[3] = {0, 0, 0};
-    const double* Dx = dps;
-    const double* Dy = dps + NSEM_MAX_NPD * NSEM_MAX_NPD;
-    const double* Dz = dps + 2 * NSEM_MAX_NPD * NSEM_MAX_NPD;
-    auto acc = [&](int la, const double* dj) {
-        const double r0 = rb[la], r4 = rb[4 * NP + la];
-        const double rm[3] = {rb[NP + la], rb[2 * NP + la], rb[3 * NP + la]};
-        for (int c = 0; c < 3; c++) {
-            Gv[c] += r0 * dj[c];
-            K[c] += r4 * dj[c];
-            for (int r = 0; r < 3; r++) H[r][c] += rm[r] * dj[c];
+    /* transposed volume gather: G_c, H_rc, K_c over the targets a of node b.
+     * dj = Jin_b dpsi(b -> a) carries the node's own metric, so each
+     * direction d's line is summed first, s_d[v] = sum_a rbar_v[a] D_d(b -> a)
+     * (5 FMAs a target), and the metric applied once:
+     * (G, H, K)_c = sum_d Jin[c][d] s_d, of which a diagonal metric keeps one
+     * term (FP64-pipe bound; 720 elements of order 4: 112 -> 56 us,
+     * the integer divisions and power included). */
+    double Gv[3], H[3][3], K[3];
+    {
+        const double* Dx = dps;
+        const double* Dy = dps + NSEM_MAX_NPD * NSEM_MAX_NPD;
+        const double* Dz = dps + 2 * NSEM_MAX_NPD * NSEM_MAX_NPD;
+        double sd[3][5] = {{0, 0, 0, 0, 0}, {0, 0, 0, 0, 0}, {0, 0, 0, 0, 0}};
+        auto line = [&](int first, int stride, int n, const double* D, double* s) {
+            for (int q = 0; q < n; q++) {
+                const double w = D[q];
+                const double* r = rb + first + q * stride;
+#pragma unroll
+                for (int v = 0; v < 5; v++) s[v] += r[v * NP] * w;
+            }
+        };
+        line(t - ia * NPY * NPZ, NPY * NPZ, NPX, Dx + ia * NPX, sd[0]);
+        line(t - ja * NPZ, NPZ, NPY, Dy + ja * NPY, sd[1]);
+        line(t - ka, 1, NPZ, Dz + ka * NPZ, sd[2]);
+        bool diag = true;
+        for (int c = 3; c < 9; c++) diag = diag && nsem_is_zero(m.jin[(int64_t)c * m.n_int + node]);
+        for (int d = 0; d < 3; d++)
+            for (int v = 0; v < 5; v++) diag = diag && nsem_bounded(sd[d][v]);
+        if (diag) {
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const double J = m.jin[(int64_t)c * m.n_int + node];
+                Gv[c] = J * sd[c][0];
+                for (int r = 0; r < 3; r++) H[r][c] = J * sd[c][1 + r];
+                K[c] = J * sd[c][4];
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                double J[3];
+                for (int d = 0; d < 3; d++) J[d] = m.jin[(int64_t)tix(c, d) * m.n_int + node];
+                Gv[c] = J[0] * sd[0][0] + J[1] * sd[1][0] + J[2] * sd[2][0];
+                for (int r = 0; r < 3; r++)
+                    H[r][c] = J[0] * sd[0][1 + r] + J[1] * sd[1][1 + r] + J[2] * sd[2][1 + r];
+                K[c] = J[0] * sd[0][4] + J[1] * sd[1][4] + J[2] * sd[2][4];
+            }
         }
-    };
-    /* targets on the x line (including self), then y and z lines */
-    for (int im = 0; im < NPX; im++) {
-        double dv[3];
-        dv[0] = Dx[ia * NPX + im];
-        dv[1] = (im == ia) ? Dy[ja * NPY + ja] : 0.0;
-        dv[2] = (im == ia) ? Dz[ka * NPZ + ka] : 0.0;
-        double dj[3];
-        dj[0] = Jin[XX] * dv[0] + Jin[XY] * dv[1] + Jin[XZ] * dv[2];
-        dj[1] = Jin[YX] * dv[0] + Jin[YY] * dv[1] + Jin[YZ] * dv[2];
-        dj[2] = Jin[ZX] * dv[0] + Jin[ZY] * dv[1] + Jin[ZZ] * dv[2];
-        acc(t + (im - ia) * NPY * NPZ, dj);
-    }
-    /* the y and z lines without the node itself: the same trip count on
-     * every thread, the node's own index skipped by the mapping */
-    for (int q = 0; q + 1 < NPY; q++) {
-        const int jm = q < ja ? q : q + 1;
-        const double D = Dy[ja * NPY + jm];
-        const double dj[3] = {Jin[XY] * D, Jin[YY] * D, Jin[ZY] * D};
-        acc(t + (jm - ja) * NPZ, dj);
-    }
-    for (int q = 0; q + 1 < NPZ; q++) {
-        const int km = q < ka ? q : q + 1;
-        const double D = Dz[ka * NPZ + km];
-        const double dj[3] = {Jin[XZ] * D, Jin[YZ] * D, Jin[ZZ] * D};
-        acc(t + (km - ka), dj);
     }
     /* viscous fluxes fm -= mu grad U, ft -= (mu / Pr) grad theta (volume) and the
      * node's side of its face fluxes: adjoints of the node's gradients and of mu */
@@ -464,10 +536,12 @@ __global__ void __maxnreg__(VISC ? 128 : 88) k_adj_volume(const NsemDev m, const
         face_q_vjp(m, P, q, rbar, Ub, Tb, pb);
     }
     /* EOS: p = P0 (rho theta R / P0)^gamma */
-    rbar += pb * m.gamma * P.p / P.r;
-    Tb += pb * m.gamma * P.p / P.T;
+    const nsem_divisor dr = nsem_make_divisor(P.r);
+    const double pg = pb * m.gamma * P.p;
+    rbar += nsem_div_by(pg, dr);
+    Tb += nsem_div(pg, P.T);
     /* U = m / rho, theta = E / rho */
-    const double inv = 1.0 / P.r;
+    const double inv = nsem_div_by(1.0, dr);
     double g0 = rbar - inv * vdot3(Ub, P.U) - inv * Tb * P.T;
     a.G[0][node] = g0;
     a.G[1][node] = Ub[0] * inv;
@@ -915,7 +989,7 @@ __global__ void __launch_bounds__(128) k_tan_face(const NsemDev m, FaceTanArgs a
             sym_fwd(P1.U, en, P2.U, rsym, magR, magP, scaled);
             sym_jvp(P1.U, en, rsym, magR, magP, scaled, d1.U, d2.U);
         }
-        P2.mu = sqrt(vdot3(P2.U, P2.U));
+        P2.mu = nsem_sqrt(vdot3(P2.U, P2.U));
         d2.mu = P2.mu > 0 ? vdot3(P2.U, d2.U) / P2.mu : 0.0;
     }
     const double lam = ((P1.mu * fi + P2.mu * fo) + (P1.c * fi + P2.c * fo)) / 2;
@@ -1047,7 +1121,8 @@ __global__ void k_tan_volume(const NsemDev m, const NsemTables tab, VolTanArgs a
     /* gravity source: r_m -= g (rho - rho_ref) cV */
     const double cv = m.cv[node];
     for (int c = 0; c < 3; c++) r[1 + c] -= m.g[c] * drho * cv;
-    for (int v = 0; v < 5; v++) a.out[v][node] = -(r[v] / cv);
+    const nsem_divisor dcv = nsem_make_divisor(cv);
+    for (int v = 0; v < 5; v++) a.out[v][node] = -nsem_div_by(r[v], dcv);
 }
 
 /* Transpose of the strong-form gradient (gradf<true>) for the viscous

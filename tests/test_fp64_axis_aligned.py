@@ -100,3 +100,22 @@ def test_non_finite_values_spread_as_in_the_full_products(var, value, visc):
     for a, b in zip(got, want):
         assert np.array_equal(np.isfinite(a), np.isfinite(b))
         assert np.array_equal(a[np.isfinite(b)], b[np.isfinite(b)])
+
+
+@pytest.mark.parametrize("n,dim,order,visc,tilt", [((3, 2, 2), 3, 4, 0.0, 0.0), ((2, 2, 3), 3, 3, 1.5, 0.0),
+                                                   ((4, 1, 3), 2, 5, 0.0, 0.0), ((2, 2, 2), 3, 4, 0.0, 30.0)])
+def test_transpose_of_the_tangent(n, dim, order, visc, tilt):
+    """<w, J dv> = <J^T w, dv>: each side sums n_int products of rounding error
+    below 1e-14 of its terms, so 1e-12 of the sum of magnitudes bounds it."""
+    m, u, dt = _setup(n, order, dim, visc, tilt)
+    rng = np.random.default_rng(3)
+    s = ng.Solver(m, dt=dt)
+    s.set_state(u)
+    dv = [a * rng.standard_normal(len(a)) * 1e-3 + (1e-3 if c in (1, 3) else 0.0) for c, a in enumerate(u)]
+    w = [rng.standard_normal(len(u[0])) for _ in range(5)]
+    Jd, Jw = s.jvp(dv), s.vjp(w)
+    s.close()
+    lhs = sum(np.dot(a, b) for a, b in zip(w, Jd))
+    rhs = sum(np.dot(a, b) for a, b in zip(Jw, dv))
+    scale = sum(np.abs(a * b).sum() for a, b in zip(w, Jd))
+    assert abs(lhs - rhs) <= 1e-12 * scale
