@@ -479,9 +479,6 @@ __global__ void k_pert_to_host(const double* U, double* rho, double* mom, double
     }
 }
 
-/* launch configuration of the stage kernels: tensor-core line sums (order 7),
- * persistent CTAs and their grid per stage (resident CTAs x SMs) */
-
 }  // namespace
 
 bool nsem_mixed_supported(int nx, int ny, int nz) {
@@ -493,8 +490,8 @@ bool nsem_mixed_supported(int nx, int ny, int nz) {
 
 namespace {
 
-int prepare(int nx, int ny, int nz, LaunchCfg* c) {
-    const int e = prepare_aligned(nx, ny, nz, c);
+int prepare(int nx, int ny, int nz) {
+    const int e = prepare_aligned(nx, ny, nz);
     return e ? e : prepare_general(nx, ny, nz);
 }
 
@@ -963,20 +960,9 @@ nsem_status nsem_mixed_setup(const NsemDev& dev, const nsem_mesh_desc* m, NsemMi
         err = "precision form: device allocation failed";
         return NSEM_NO_MEMORY;
     }
-    /* persistent stage kernels only with NSEM_MIXED_PERSIST=1: measured on
-     * GB300 (32^3, N = 4) they are slower than one CTA per element -- the
-     * register cap of 8 resident CTAs makes the element loop spill, and with
-     * fewer CTAs the prefetch only breaks even */
-    {
-        const char* pers = std::getenv("NSEM_MIXED_PERSIST");
-        LaunchCfg c{};
-        c.persist = pers && std::string(pers) == "1";
-        if (prepare(NX, NY, NZ, &c) != 0) {
-            err = "precision form: cannot reserve the kernel's shared memory";
-            return NSEM_CUDA_ERROR;
-        }
-        mb->persist = c.persist;
-        for (int q = 0; q < 4; q++) mb->pgrid[q] = c.pgrid[q];
+    if (prepare(NX, NY, NZ) != 0) {
+        err = "precision form: cannot reserve the kernel's shared memory";
+        return NSEM_CUDA_ERROR;
     }
     /* order 7: line sums on the FP32 pipes (measured faster than the
      * tensor-core variant on GB300); NSEM_MIXED_LINES=tensor selects the
@@ -1110,9 +1096,7 @@ int launch_args(const NsemMixedBuf* mb, const StageArgs& a, int stage, cudaStrea
     }
     c.visc = mb->visc;
     c.tc = mb->tc;
-    c.persist = mb->persist;
     c.gen = mb->gen;
-    for (int q = 0; q < 4; q++) c.pgrid[q] = mb->pgrid[q];
     return dispatch_stage(mb->npd[0], mb->npd[1], mb->npd[2], a, stage, st, c);
 }
 

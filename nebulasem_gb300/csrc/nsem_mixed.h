@@ -36,11 +36,9 @@ struct NsemMixedBuf {
     float* G = nullptr;           /* viscous runs: [n_elem][12][NP] gradients of the stage state */
     bool visc = false;            /* artificial viscosity (diffusion YES)   */
     bool tc = false;              /* order-7 line sums on the tensor cores  */
-    bool persist = false;         /* persistent stage kernels               */
     bool gen = false;             /* general geometry (inclined, curved)    */
     float* Jg = nullptr;          /* gen: [n_elem][10][NP] Jinv cV, 1/cV    */
     float* Fn = nullptr;          /* gen: [n_elem][3][NFS] outward fN       */
-    int pgrid[4] = {0, 0, 0, 0};  /* their grids (resident CTAs), per stage */
     /* non-conforming (2:1) faces (inviscid runs on axis-aligned elements):
      * per mortar slot the fine node, the coarse face and the interpolation
      * indices; the flux vectors, the fine side's F.n and the coarse side's

@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include "nsem_mixed_kern.cuh"
+#include "nsem_pdl.cuh"
 
 using namespace nsem_mx;
 
@@ -30,10 +31,11 @@ struct GenSmem {
     using G = Geo<NX, NY, NZ>;
     static constexpr int NP = G::NP, NFS = G::NFS;
     /* floats: contravariant fluxes, line-major per direction [3][n][5][NL];
-     * own values P[4][NP] (x4); face fluxes FF4[NFS] (x4) + FF1[NFS];
-     * viscous runs: the nodes' gradients GV[12][NP] */
-    static constexpr int OFF_P = (line_floats<NX, NY, NZ>() + 3) / 4 * 4;
-    static constexpr int OFF_FF4 = OFF_P + 16 * NP;
+     * own values P[12][NP] (viscous runs 13): rho', rho u (3), Theta', u (3),
+     * p', theta, |u|, c, rho; face fluxes FF4[NFS] (x4) + FF1[NFS]; viscous runs:
+     * the nodes' gradients GV[12][NP] */
+    static constexpr int OFF_P = line_floats<NX, NY, NZ>();
+    static constexpr int OFF_FF4 = (OFF_P + (VISC ? 13 : 12) * NP + 3) / 4 * 4;
     static constexpr int OFF_FF1 = OFF_FF4 + 4 * NFS;
     static constexpr int OFF_GV = OFF_FF1 + NFS;
     static constexpr size_t BYTES = sizeof(float) * (OFF_GV + (VISC ? 12 * NP : 0));
@@ -73,7 +75,7 @@ k_mixed_stage_gen(StageArgs a) {
     constexpr int NFS = G::NFS;
     extern __shared__ float4 gen4[];
     float* smem = reinterpret_cast<float*>(gen4);
-    float4* sP = reinterpret_cast<float4*>(smem + SM::OFF_P);
+    float* sP = smem + SM::OFF_P;       /* [12 or 13][NP] */
     float4* sFF4 = reinterpret_cast<float4*>(smem + SM::OFF_FF4);
     float* sFF1 = smem + SM::OFF_FF1;
     float* sGV = smem + SM::OFF_GV;     /* viscous runs: [12][NP] */
@@ -81,20 +83,11 @@ k_mixed_stage_gen(StageArgs a) {
     const int64_t e = blockIdx.x;
     constexpr bool has_din = STAGE >= 2;
 
+    /* what no kernel of the chain writes, before the wait for the previous
+     * kernel: background, metric, neighbours, normals */
     float own[5], din[5] = {0, 0, 0, 0, 0}, bgs[4] = {0, 0, 0, 0}, jin[9], icv = 0.0f;
     float gown[12];
     if (t < NP) {
-        const float* sp = a.S + e * 5 * NP + t;
-#pragma unroll
-        for (int v = 0; v < 5; v++) own[v] = __ldg(sp + v * NP);
-        if constexpr (has_din) {
-            const float* d = a.Din + e * 5 * NP + t;
-#pragma unroll
-            for (int v = 0; v < 5; v++) {
-                din[v] = __ldg(d + v * NP);
-                own[v] = __fadd_rn(own[v], din[v]);
-            }
-        }
         const float* bg = a.bg + (int64_t)__ldg(a.layer + e) * 4 * NP + t;
 #pragma unroll
         for (int c = 0; c < 4; c++) bgs[c] = __ldg(bg + c * NP);
@@ -102,6 +95,38 @@ k_mixed_stage_gen(StageArgs a) {
 #pragma unroll
         for (int c = 0; c < 9; c++) jin[c] = __ldg(jg + c * NP);
         icv = __ldg(jg + 9 * NP);
+    }
+    FaceSlot fs{};
+    int32_t nb = -1;
+    /* the other side's node; a wall's flux is formed from the own trace */
+    int64_t eo = e;
+    int lo = 0;
+    float oth[5], bgo[4], fno[3] = {0, 0, 0};
+    if (t < NFS) {
+        fs = face_slot<NX, NY, NZ, STAGE == 1 || STAGE == 2>(t);
+        nb = __ldg(a.nbr + (int64_t)fs.face * a.n_elem + e);
+#pragma unroll
+        for (int c = 0; c < 3; c++) fno[c] = __ldg(a.Fn + (e * 3 + c) * NFS + t);
+        lo = fs.la;
+        if (nb >= 0) { eo = nb; lo = fs.lo; }
+        const float* bg = a.bg + (int64_t)__ldg(a.layer + eo) * 4 * NP + lo;
+#pragma unroll
+        for (int c = 0; c < 4; c++) bgo[c] = __ldg(bg + c * NP);
+    }
+    nsem_chain_wait();
+
+    if (t < NP) {
+        const float* sp = a.S + e * 5 * NP + t;
+#pragma unroll
+        for (int v = 0; v < 5; v++) own[v] = sp[v * NP];
+        if constexpr (has_din) {
+            const float* d = a.Din + e * 5 * NP + t;
+#pragma unroll
+            for (int v = 0; v < 5; v++) {
+                din[v] = d[v * NP];
+                own[v] = __fadd_rn(own[v], din[v]);
+            }
+        }
         if constexpr (STAGE == 3) {
             /* u'^n is needed only at the update: fetched into L2 here, loaded
              * there (with the increment reloaded), so that neither holds
@@ -114,37 +139,26 @@ k_mixed_stage_gen(StageArgs a) {
             const float* gr = a.G + e * 12 * NP + t;
 #pragma unroll
             for (int c = 0; c < 12; c++) {
-                gown[c] = __ldg(gr + c * NP);
+                gown[c] = gr[c * NP];
                 sGV[c * NP + t] = gown[c];
             }
         }
     }
-    FaceSlot fs{};
-    int32_t nb = -1;
-    float oth[5], bgo[4], fno[3] = {0, 0, 0};
     if (t < NFS) {
-        fs = face_slot<NX, NY, NZ, STAGE == 1 || STAGE == 2>(t);
-        nb = __ldg(a.nbr + (int64_t)fs.face * a.n_elem + e);
-#pragma unroll
-        for (int c = 0; c < 3; c++) fno[c] = __ldg(a.Fn + (e * 3 + c) * NFS + t);
         if (nb <= -2) {
             /* a face on a 2:1 mortar: its outward values from the mortar kernels */
             const float* mf = a.MF + (int64_t)(-2 - nb) * MF_ROWS_GEN * a.nfmax + face_local<NX, NY, NZ>(t);
 #pragma unroll
-            for (int v = 0; v < 5; v++) oth[v] = __ldg(mf + v * a.nfmax);
-        }
-        if (nb >= 0) {
-            const float* sp = a.S + (int64_t)nb * 5 * NP + fs.lo;
+            for (int v = 0; v < 5; v++) oth[v] = mf[v * a.nfmax];
+        } else {
+            const float* sp = a.S + eo * 5 * NP + lo;
 #pragma unroll
-            for (int v = 0; v < 5; v++) oth[v] = __ldg(sp + v * NP);
+            for (int v = 0; v < 5; v++) oth[v] = sp[v * NP];
             if constexpr (has_din) {
-                const float* d = a.Din + (int64_t)nb * 5 * NP + fs.lo;
+                const float* d = a.Din + eo * 5 * NP + lo;
 #pragma unroll
-                for (int v = 0; v < 5; v++) oth[v] = __fadd_rn(oth[v], __ldg(d + v * NP));
+                for (int v = 0; v < 5; v++) oth[v] = __fadd_rn(oth[v], d[v * NP]);
             }
-            const float* bg = a.bg + (int64_t)__ldg(a.layer + nb) * 4 * NP + fs.lo;
-#pragma unroll
-            for (int c = 0; c < 4; c++) bgo[c] = __ldg(bg + c * NP);
         }
     }
     /* viscous runs: the neighbour's gradients along the face node's normal,
@@ -155,7 +169,7 @@ k_mixed_stage_gen(StageArgs a) {
             const float* gr = a.G + (int64_t)nb * 12 * NP + fs.lo;
             float g[12];
 #pragma unroll
-            for (int c = 0; c < 12; c++) g[c] = __ldg(gr + c * NP);
+            for (int c = 0; c < 12; c++) g[c] = gr[c * NP];
             /* the same association as the own side's (exact antisymmetry) */
 #pragma unroll
             for (int r = 0; r < 3; r++)
@@ -168,10 +182,15 @@ k_mixed_stage_gen(StageArgs a) {
     /* phase 1: primitives and contravariant fluxes */
     if (t < NP) {
         const Pt p = pointwise(own, bgs, a.eos, a.gamma, a.gR);
-        sP[t] = make_float4(own[0], own[1], own[2], own[3]);
-        sP[NP + t] = make_float4(own[4], p.rho, p.umag, p.c);
-        sP[2 * NP + t] = make_float4(p.u[0], p.u[1], p.u[2], p.pp);
-        sP[3 * NP + t] = make_float4(p.th, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int v = 0; v < 5; v++) sP[v * NP + t] = own[v];
+#pragma unroll
+        for (int c = 0; c < 3; c++) sP[(5 + c) * NP + t] = p.u[c];
+        sP[8 * NP + t] = p.pp;
+        sP[9 * NP + t] = p.th;
+        sP[10 * NP + t] = p.umag;
+        sP[11 * NP + t] = p.c;
+        if constexpr (VISC) sP[12 * NP + t] = p.rho;
         const int i = t / (NY * NZ), j = (t / NZ) % NY, k = t % NZ;
         const int lpos[3] = {LineLay<NX, NY, NZ, 0>::at(i, j, k), LineLay<NX, NY, NZ, 1>::at(i, j, k),
                              LineLay<NX, NY, NZ, 2>::at(i, j, k)};
@@ -203,9 +222,6 @@ k_mixed_stage_gen(StageArgs a) {
 
     /* phase 2: Rusanov flux through every face node, dotted with its normal */
     if (t < NFS) {
-        const float4 P0 = sP[fs.la], P1 = sP[NP + fs.la], P2 = sP[2 * NP + fs.la];
-        const float th_s = sP[3 * NP + fs.la].x;
-        const float ms[3] = {P0.y, P0.z, P0.w}, us[3] = {P2.x, P2.y, P2.z};
         const float nrm = __fsqrt_rn(__fmaf_rn(fno[0], fno[0], __fmaf_rn(fno[1], fno[1], __fmul_rn(fno[2], fno[2]))));
         const float inrm = nrm > 0.0f ? 1.0f / nrm : 0.0f;
         const float en[3] = {__fmul_rn(fno[0], inrm), __fmul_rn(fno[1], inrm), __fmul_rn(fno[2], inrm)};
@@ -216,16 +232,24 @@ k_mixed_stage_gen(StageArgs a) {
             o1 = oth[4];
         } else if (nb >= 0) {
             const Pt q = pointwise(oth, bgo, a.eos, a.gamma, a.gR);
+            const float* own_p = sP + fs.la;
+            float ms[3], us[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                ms[c] = own_p[(1 + c) * NP];
+                us[c] = own_p[(5 + c) * NP];
+            }
             float4 A4, B4;
             float A1, B1;
-            normal_flux(ms, us, P2.w, th_s, fno, A4, A1);
+            normal_flux(ms, us, own_p[8 * NP], own_p[9 * NP], fno, A4, A1);
             normal_flux(oth + 1, q.u, q.pp, q.th, fno, B4, B1);
-            const float lam = __fmul_rn(0.25f, __fadd_rn(__fadd_rn(P1.z, q.umag), __fadd_rn(P1.w, q.c)));
+            const float lam = __fmul_rn(0.25f, __fadd_rn(__fadd_rn(own_p[10 * NP], q.umag),
+                                                         __fadd_rn(own_p[11 * NP], q.c)));
             const float dm0 = __fsub_rn(oth[1], ms[0]), dm1 = __fsub_rn(oth[2], ms[1]),
                         dm2 = __fsub_rn(oth[3], ms[2]);
             const float dmn = __fmaf_rn(dm0, fno[0], __fmaf_rn(dm1, fno[1], __fmul_rn(dm2, fno[2])));
-            const float jr = __fmul_rn(nrm, __fsub_rn(oth[0], P0.x));
-            const float jt = __fmul_rn(nrm, __fsub_rn(oth[4], P1.x));
+            const float jr = __fmul_rn(nrm, __fsub_rn(oth[0], own_p[0]));
+            const float jt = __fmul_rn(nrm, __fsub_rn(oth[4], own_p[4 * NP]));
             if constexpr (VISC) {
                 /* both sides' viscous normal fluxes, - mu (grad U) n and
                  * - (mu / Pr) (grad theta) . n, each side's from its own node */
@@ -236,8 +260,9 @@ k_mixed_stage_gen(StageArgs a) {
                     sn[r] = __fmaf_rn(gs[tidx(r, 0) * NP], fno[0],
                                       __fmaf_rn(gs[tidx(r, 1) * NP], fno[1], __fmul_rn(gs[tidx(r, 2) * NP], fno[2])));
                 sn[3] = __fmaf_rn(gs[9 * NP], fno[0], __fmaf_rn(gs[10 * NP], fno[1], __fmul_rn(gs[11 * NP], fno[2])));
-                const float mus = __fmul_rn(P1.y, a.nu), muo = __fmul_rn(q.rho, a.nu);
-                const float mts = __fmul_rn(P1.y, a.nu_pr), mto = __fmul_rn(q.rho, a.nu_pr);
+                const float rho_s = own_p[12 * NP];
+                const float mus = __fmul_rn(rho_s, a.nu), muo = __fmul_rn(q.rho, a.nu);
+                const float mts = __fmul_rn(rho_s, a.nu_pr), mto = __fmul_rn(q.rho, a.nu_pr);
                 A4.y = __fmaf_rn(-mus, sn[0], A4.y);
                 A4.z = __fmaf_rn(-mus, sn[1], A4.z);
                 A4.w = __fmaf_rn(-mus, sn[2], A4.w);
@@ -255,17 +280,18 @@ k_mixed_stage_gen(StageArgs a) {
         } else {
             /* wall ghost (SYMMETRY velocity, NEUMANN rho, theta, p): the ghost's
              * normal flux is p' fN, the jump term lam en (m.fN) */
-            const float un = __fmaf_rn(us[0], en[0], __fmaf_rn(us[1], en[1], __fmul_rn(us[2], en[2])));
-            const float r0 = __fmaf_rn(-un, en[0], us[0]), r1 = __fmaf_rn(-un, en[1], us[1]),
-                        r2 = __fmaf_rn(-un, en[2], us[2]);
+            const Pt q = pointwise(oth, bgo, a.eos, a.gamma, a.gR);
+            const float un = __fmaf_rn(q.u[0], en[0], __fmaf_rn(q.u[1], en[1], __fmul_rn(q.u[2], en[2])));
+            const float r0 = __fmaf_rn(-un, en[0], q.u[0]), r1 = __fmaf_rn(-un, en[1], q.u[1]),
+                        r2 = __fmaf_rn(-un, en[2], q.u[2]);
             const float mr = safe_sqrt(__fmaf_rn(r0, r0, __fmaf_rn(r1, r1, __fmul_rn(r2, r2))));
-            const float um_g = mr > 1e-7f ? P1.z : mr;
-            const float lam = __fmul_rn(0.5f, __fadd_rn(um_g, P1.w));
-            const float mn = __fmaf_rn(ms[0], fno[0], __fmaf_rn(ms[1], fno[1], __fmul_rn(ms[2], fno[2])));
+            const float um_g = mr > 1e-7f ? q.umag : mr;
+            const float lam = __fmul_rn(0.5f, __fadd_rn(um_g, q.c));
+            const float mn = __fmaf_rn(oth[1], fno[0], __fmaf_rn(oth[2], fno[1], __fmul_rn(oth[3], fno[2])));
             o4.x = 0.0f;
-            o4.y = __fmaf_rn(lam, __fmul_rn(en[0], mn), __fmul_rn(P2.w, fno[0]));
-            o4.z = __fmaf_rn(lam, __fmul_rn(en[1], mn), __fmul_rn(P2.w, fno[1]));
-            o4.w = __fmaf_rn(lam, __fmul_rn(en[2], mn), __fmul_rn(P2.w, fno[2]));
+            o4.y = __fmaf_rn(lam, __fmul_rn(en[0], mn), __fmul_rn(q.pp, fno[0]));
+            o4.z = __fmaf_rn(lam, __fmul_rn(en[1], mn), __fmul_rn(q.pp, fno[1]));
+            o4.w = __fmaf_rn(lam, __fmul_rn(en[2], mn), __fmul_rn(q.pp, fno[2]));
             o1 = 0.0f;
         }
         sFF4[t] = o4;
@@ -273,6 +299,7 @@ k_mixed_stage_gen(StageArgs a) {
     }
     __syncthreads();
 
+    nsem_chain_begin();   /* here: see k_mixed_stage */
     /* phase 3: line sums l_a'(x_m) G_d(m) (in-place line transform), lift,
      * 1/cV, buoyancy, update */
     line_transform<NX, NY, NZ, 0>(smem, a, t);
@@ -331,10 +358,17 @@ k_mixed_stage_gen(StageArgs a) {
         for (int v = 0; v < 5; v++) a.Dout[o + v * NP] = 0.25f * fmaf(dt, Lv[v], din[v]);
     } else {
         bool finite = true;
+        /* every load before the first store, which could alias them */
+        double u64[5];
 #pragma unroll
         for (int v = 0; v < 5; v++) {
-            const float D = (2.0f / 3.0f) * fmaf(dt, Lv[v], __ldg(a.Din + o + v * NP));
-            const double un = __ldg(a.U + o + v * NP) + f2d(D);
+            din[v] = a.Din[o + v * NP];
+            u64[v] = a.U[o + v * NP];
+        }
+#pragma unroll
+        for (int v = 0; v < 5; v++) {
+            const float D = (2.0f / 3.0f) * fmaf(dt, Lv[v], din[v]);
+            const double un = u64[v] + f2d(D);
             a.Unew[o + v * NP] = un;
             a.Snew[o + v * NP] = d2f_rn(un);
             finite = finite && ((__double2hiint(un) & 0x7ff00000) != 0x7ff00000);
@@ -365,14 +399,6 @@ k_mixed_grad_gen(StageArgs a) {
 
     float own[5], bgs0 = 0.0f, jin[9], icv = 0.0f;
     if (t < NP) {
-        const float* s = a.S + e * 5 * NP + t;
-#pragma unroll
-        for (int v = 0; v < 5; v++) own[v] = __ldg(s + v * NP);
-        if (has_din) {
-            const float* d = a.Din + e * 5 * NP + t;
-#pragma unroll
-            for (int v = 0; v < 5; v++) own[v] = __fadd_rn(own[v], __ldg(d + v * NP));
-        }
         bgs0 = __ldg(a.bg + (int64_t)__ldg(a.layer + e) * 4 * NP + t);
         const float* jg = a.Jg + e * 10 * NP + t;
 #pragma unroll
@@ -387,19 +413,30 @@ k_mixed_grad_gen(StageArgs a) {
         nb = __ldg(a.nbr + (int64_t)fs.face * a.n_elem + e);
 #pragma unroll
         for (int c = 0; c < 3; c++) fno[c] = __ldg(a.Fn + (e * 3 + c) * NFS + t);
-        if (nb >= 0) {
-            const float* s = a.S + (int64_t)nb * 5 * NP + fs.lo;
-#pragma unroll
-            for (int v = 0; v < 5; v++) oth[v] = __ldg(s + v * NP);
-            if (has_din) {
-                const float* d = a.Din + (int64_t)nb * 5 * NP + fs.lo;
-#pragma unroll
-                for (int v = 0; v < 5; v++) oth[v] = __fadd_rn(oth[v], __ldg(d + v * NP));
-            }
-            bgo0 = __ldg(a.bg + (int64_t)__ldg(a.layer + nb) * 4 * NP + fs.lo);
-        }
+        if (nb >= 0) bgo0 = __ldg(a.bg + (int64_t)__ldg(a.layer + nb) * 4 * NP + fs.lo);
     }
     for (int q = t; q < QTAB; q += G::BLOCK) sDg[q] = __ldg(a.Dg + q);
+    nsem_chain_wait();
+    if (t < NP) {
+        const float* s = a.S + e * 5 * NP + t;
+#pragma unroll
+        for (int v = 0; v < 5; v++) own[v] = s[v * NP];
+        if (has_din) {
+            const float* d = a.Din + e * 5 * NP + t;
+#pragma unroll
+            for (int v = 0; v < 5; v++) own[v] = __fadd_rn(own[v], d[v * NP]);
+        }
+    }
+    if (t < NFS && nb >= 0) {
+        const float* s = a.S + (int64_t)nb * 5 * NP + fs.lo;
+#pragma unroll
+        for (int v = 0; v < 5; v++) oth[v] = s[v * NP];
+        if (has_din) {
+            const float* d = a.Din + (int64_t)nb * 5 * NP + fs.lo;
+#pragma unroll
+            for (int v = 0; v < 5; v++) oth[v] = __fadd_rn(oth[v], d[v * NP]);
+        }
+    }
 
     const float T0 = a.T0;
     auto prim_ut = [T0](const float* s, float rref) {
@@ -436,6 +473,7 @@ k_mixed_grad_gen(StageArgs a) {
     }
     __syncthreads();
 
+    nsem_chain_begin();
     if (t >= NP) return;
     const int i = t / (NY * NZ), j = (t / NZ) % NY, k = t % NZ;
     /* derivatives along the reference directions */
@@ -488,10 +526,10 @@ k_mixed_grad_gen(StageArgs a) {
                               face_local<NX, NY, NZ>(slot);
 #pragma unroll
             for (int r = 0; r < 3; r++) {
-                g[r].x += __ldg(gf + (4 * r) * a.nfmax);
-                g[r].y += __ldg(gf + (4 * r + 1) * a.nfmax);
-                g[r].z += __ldg(gf + (4 * r + 2) * a.nfmax);
-                g[r].w += __ldg(gf + (4 * r + 3) * a.nfmax);
+                g[r].x += gf[(4 * r) * a.nfmax];
+                g[r].y += gf[(4 * r + 1) * a.nfmax];
+                g[r].z += gf[(4 * r + 2) * a.nfmax];
+                g[r].w += gf[(4 * r + 3) * a.nfmax];
             }
             return;
         }
@@ -526,26 +564,24 @@ k_mixed_grad_gen(StageArgs a) {
 
 template <int NX, int NY, int NZ>
 int launch_gen(const StageArgs& a, int stage, cudaStream_t st, bool visc) {
-    using G = Geo<NX, NY, NZ>;
+    constexpr unsigned B = Geo<NX, NY, NZ>::BLOCK;
     const unsigned grid = (unsigned)a.n_elem;
     if (visc) {
         constexpr size_t SMEM = GenSmem<NX, NY, NZ, true>::BYTES;
         switch (stage) {
-            case 0: k_mixed_stage_gen<NX, NY, NZ, 0, true><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-            case 1: k_mixed_stage_gen<NX, NY, NZ, 1, true><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-            case 2: k_mixed_stage_gen<NX, NY, NZ, 2, true><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-            default: k_mixed_stage_gen<NX, NY, NZ, 3, true><<<grid, G::BLOCK, SMEM, st>>>(a); break;
+            case 0: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 0, true>, grid, B, SMEM, st, a);
+            case 1: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 1, true>, grid, B, SMEM, st, a);
+            case 2: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 2, true>, grid, B, SMEM, st, a);
+            default: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 3, true>, grid, B, SMEM, st, a);
         }
-        return (int)cudaGetLastError();
     }
     constexpr size_t SMEM = GenSmem<NX, NY, NZ>::BYTES;
     switch (stage) {
-        case 0: k_mixed_stage_gen<NX, NY, NZ, 0, false><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-        case 1: k_mixed_stage_gen<NX, NY, NZ, 1, false><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-        case 2: k_mixed_stage_gen<NX, NY, NZ, 2, false><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-        default: k_mixed_stage_gen<NX, NY, NZ, 3, false><<<grid, G::BLOCK, SMEM, st>>>(a); break;
+        case 0: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 0, false>, grid, B, SMEM, st, a);
+        case 1: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 1, false>, grid, B, SMEM, st, a);
+        case 2: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 2, false>, grid, B, SMEM, st, a);
+        default: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 3, false>, grid, B, SMEM, st, a);
     }
-    return (int)cudaGetLastError();
 }
 
 template <int NX, int NY, int NZ>
@@ -553,9 +589,9 @@ int launch_grad_gen(const StageArgs& a, int stage, cudaStream_t st) {
     using G = Geo<NX, NY, NZ>;
     const unsigned grid = (unsigned)a.n_elem;
     constexpr size_t gs = grad_smem<NX, NY, NZ>();
-    if (stage <= 1) k_mixed_grad_gen<NX, NY, NZ, 1><<<grid, G::BLOCK, gs, st>>>(a);
-    else k_mixed_grad_gen<NX, NY, NZ, 2><<<grid, G::BLOCK, gs, st>>>(a);
-    return (int)cudaGetLastError();
+    constexpr unsigned B = G::BLOCK;
+    return stage <= 1 ? nsem_launch_chained(k_mixed_grad_gen<NX, NY, NZ, 1>, grid, B, gs, st, a)
+                      : nsem_launch_chained(k_mixed_grad_gen<NX, NY, NZ, 2>, grid, B, gs, st, a);
 }
 
 template <int NX, int NY, int NZ>

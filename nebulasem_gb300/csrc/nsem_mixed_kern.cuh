@@ -106,14 +106,13 @@ constexpr size_t grad_smem() {
 }
 
 struct LaunchCfg {
-    bool visc, tc, persist, gen;
-    int pgrid[4];
+    bool visc, tc, gen;
 };
 
-/* per translation unit: the kernels' shared-memory attributes (and the
- * persistent kernels' grids), the stage launches and the gradient launches
- * of viscous runs, each dispatched on the node counts per direction */
-int prepare_aligned(int nx, int ny, int nz, LaunchCfg* c);
+/* per translation unit: the kernels' shared-memory attributes, the stage
+ * launches and the gradient launches of viscous runs, each dispatched on the
+ * node counts per direction */
+int prepare_aligned(int nx, int ny, int nz);
 int prepare_general(int nx, int ny, int nz);
 int launch_stage_aligned(int nx, int ny, int nz, const StageArgs& a, int stage, cudaStream_t st,
                          const LaunchCfg& c);

@@ -1,13 +1,14 @@
 /*
  * Precision form on axis-aligned affine elements: the fused SSP-RK3 stage
  * kernel k_mixed_stage (FP32 line sums, or TF32 tensor-core line sums at
- * order 7; optional persistent CTAs) and the viscous runs' gradient kernel
+ * order 7) and the viscous runs' gradient kernel
  * k_mixed_grad, with their launches.  The algorithm is described in
  * nsem_mixed.cu.
  */
 #include <cuda_runtime.h>
 
 #include "nsem_mixed_kern.cuh"
+#include "nsem_pdl.cuh"
 
 using namespace nsem_mx;
 
@@ -18,34 +19,18 @@ struct StageSmem {
     using G = Geo<NX, NY, NZ>;
     static constexpr int NP = G::NP, NFS = G::NFS;
     /* floats: volume fluxes, line-major per direction [3][n][5][NL] (tensor-core
-     * line sums: F[3][5][TC_NP]); own values P[3][NP] (x4); face fluxes
-     * FF4[NFS] (x4) + FF1[NFS]; metric */
+     * line sums: F[3][5][TC_NP]); own values P[NP] (x4) of the faces' jumps and
+     * speeds: rho', Theta', |u|, c; face fluxes FF4[NFS] (x4) + FF1[NFS]; metric */
     static constexpr int FLUX = TC ? 15 * TC_NP : line_floats<NX, NY, NZ>();
     static constexpr int OFF_P = (FLUX + 3) / 4 * 4;
-    static constexpr int OFF_FF4 = OFF_P + 12 * NP;
+    static constexpr int OFF_FF4 = OFF_P + 4 * NP;
     static constexpr int OFF_FF1 = OFF_FF4 + 4 * NFS;
     static constexpr int OFF_META = OFF_FF1 + NFS;
-    static_assert(OFF_P % 4 == 0 && OFF_FF4 % 4 == 0, "float4 regions must be 16-byte aligned");
     /* tensor-core line sums: the B fragments of Q_d^T pre-split into TF32
      * high and low parts, [3][2][8][8] words after the metric */
     static constexpr int OFF_QTC = OFF_META + 4;
     static constexpr size_t BYTES = sizeof(float) * (OFF_QTC + (TC ? TC_QTAB : 0));
-    /* persistent kernels: the next element's stage base, increment and
-     * background, staged by asynchronous copies while the current element
-     * computes */
-    static constexpr int OFF_STG = OFF_META + 4;
-    static constexpr size_t BYTES_P = sizeof(float) * (OFF_STG + 14 * NP);
-    static_assert(BYTES_P > BYTES || TC, "the persistent layout extends the plain one");
 };
-
-/* 4-byte asynchronous copies global -> shared (no registers held while in
- * flight) */
-__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 /* Tensor-core line sums (order 7, 8 nodes per direction).  The volume term
  * of direction d is, per conserved variable v and line l through the
@@ -91,7 +76,7 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
 #ifndef NSEM_MIXED_MB3
 #define NSEM_MIXED_MB3 9
 #endif
-template <int NX, int NY, int NZ, int STAGE, bool VISC, bool PERSIST = false>
+template <int NX, int NY, int NZ, int STAGE, bool VISC>
 constexpr int stage_min_blocks() {
     /* order 7 (512 threads, 64 KB of shared memory): three CTAs, two for the
      * stages that hold more live values (no spills) */
@@ -99,8 +84,7 @@ constexpr int stage_min_blocks() {
         return min_blocks((VISC || STAGE == 0) ? 2 : 3, Geo<NX, NY, NZ>::BLOCK,
                           StageSmem<NX, NY, NZ>::BYTES);
     return min_blocks(VISC ? (STAGE == 3 ? 5 : 6) : (STAGE == 1 || STAGE == 2) ? NSEM_MIXED_MB12 : NSEM_MIXED_MB3,
-                      Geo<NX, NY, NZ>::BLOCK,
-                      PERSIST ? StageSmem<NX, NY, NZ>::BYTES_P : StageSmem<NX, NY, NZ>::BYTES);
+                      Geo<NX, NY, NZ>::BLOCK, StageSmem<NX, NY, NZ>::BYTES);
 }
 
 /* Strong-form DG gradients of U and theta of a stage state (gradf<true>,
@@ -228,28 +212,26 @@ __device__ __forceinline__ void grad_node(int i, int j, int k, const float4* sV,
  * axis is a run-time value (selects, no branches), so a warp whose face
  * nodes lie on faces of two axes runs one instruction stream; the operations
  * and their operands are those of the plain per-axis form, so the two
- * elements of a face still produce exact negatives. */
+ * elements of a face still produce exact negatives.  oth, bgo: the other
+ * side's state and background, on a wall (nb = -1) the own node's. */
 template <int NX, int NY, int NZ, bool VISC, bool TC>
 __device__ __forceinline__ void face_flux(const FaceSlot& fs, int32_t nb, const float* oth,
                                           const float* bgo, const float* gfo, const float* sF,
-                                          const float4* sP, const StageArgs& a,
-                                          float4& o4, float& o1) {
-    constexpr int NP = Geo<NX, NY, NZ>::NP;
+                                          const float4* sP, const StageArgs& a, float4& o4,
+                                          float& o1) {
     const int dir = fs.dir;
     const bool d0 = dir == 0, d1 = dir == 1, d2 = dir == 2;
     const float sg = fs.side ? 1.0f : -1.0f;   /* outward normal = sg e_dir */
-    const float4 P0 = sP[fs.la], P1 = sP[NP + fs.la];
-    const float md_s = d0 ? P0.y : d1 ? P0.z : P0.w;
-    const float um_s = P1.z, c_s = P1.w;
+    const Pt q = pointwise(oth, bgo, a.eos, a.gamma, a.gR);
+    const float mdo = d0 ? oth[1] : d1 ? oth[2] : oth[3];
     if (nb >= 0) {
-        float4 A4;
-        float A1;
+        float A[5];
         if constexpr (TC) {
             const int i = fs.la / (NY * NZ), j = (fs.la / NZ) % NY, k = fs.la % NZ;
             const float* f = sF + dir * 5 * TC_NP +
                              (d0 ? tc_idx<0>(i, j, k) : d1 ? tc_idx<1>(i, j, k) : tc_idx<2>(i, j, k));
-            A4 = make_float4(f[0], f[TC_NP], f[2 * TC_NP], f[3 * TC_NP]);
-            A1 = f[4 * TC_NP];
+#pragma unroll
+            for (int v = 0; v < 5; v++) A[v] = f[v * TC_NP];
         } else {
             /* the node's flux row along the face's axis: the face plane's
              * row (first or last) at the node's in-plane index */
@@ -261,37 +243,35 @@ __device__ __forceinline__ void face_flux(const FaceSlot& fs, int32_t nb, const 
                                : L2::BASE + (fs.side ? NZ - 1 : 0) * L2::ROW;
             const float* f = sF + row + fs.r;
             const int nl = d0 ? L0::NL : d1 ? L1::NL : L2::NL;
-            A4 = make_float4(f[0], f[nl], f[2 * nl], f[3 * nl]);
-            A1 = f[4 * nl];
+#pragma unroll
+            for (int v = 0; v < 5; v++) A[v] = f[v * nl];
         }
-        const Pt q = pointwise(oth, bgo, a.eos, a.gamma, a.gR);
         /* the neighbour's volume flux along the axis (vol_flux of its node) */
         const float ud = d0 ? q.u[0] : d1 ? q.u[1] : q.u[2];
-        const float mdo = d0 ? oth[1] : d1 ? oth[2] : oth[3];
-        float4 B4;
-        float B1;
-        B4.x = mdo;
-        B4.y = __fmaf_rn(oth[1], ud, d0 ? q.pp : 0.0f);
-        B4.z = __fmaf_rn(oth[2], ud, d1 ? q.pp : 0.0f);
-        B4.w = __fmaf_rn(oth[3], ud, d2 ? q.pp : 0.0f);
-        B1 = __fmul_rn(mdo, q.th);
+        float B[5];
+        B[0] = mdo;
+        B[1] = __fmaf_rn(oth[1], ud, d0 ? q.pp : 0.0f);
+        B[2] = __fmaf_rn(oth[2], ud, d1 ? q.pp : 0.0f);
+        B[3] = __fmaf_rn(oth[3], ud, d2 ? q.pp : 0.0f);
+        B[4] = __fmul_rn(mdo, q.th);
         if constexpr (VISC) {
             /* gfo: the neighbour's d_c U_dir (c = 0..2) and d_dir theta */
             const float mu = __fmul_rn(q.rho, a.nu), mt = __fmul_rn(q.rho, a.nu_pr);
-            B4.y = __fmaf_rn(-mu, gfo[0], B4.y);
-            B4.z = __fmaf_rn(-mu, gfo[1], B4.z);
-            B4.w = __fmaf_rn(-mu, gfo[2], B4.w);
-            B1 = __fmaf_rn(-mt, gfo[3], B1);
+            B[1] = __fmaf_rn(-mu, gfo[0], B[1]);
+            B[2] = __fmaf_rn(-mu, gfo[1], B[2]);
+            B[3] = __fmaf_rn(-mu, gfo[2], B[3]);
+            B[4] = __fmaf_rn(-mt, gfo[3], B[4]);
         }
-        const float lam = __fmul_rn(0.25f, __fadd_rn(__fadd_rn(um_s, q.umag), __fadd_rn(c_s, q.c)));
-        const float av0 = __fmul_rn(0.5f, __fadd_rn(A4.x, B4.x));
-        const float av1 = __fmul_rn(0.5f, __fadd_rn(A4.y, B4.y));
-        const float av2 = __fmul_rn(0.5f, __fadd_rn(A4.z, B4.z));
-        const float av3 = __fmul_rn(0.5f, __fadd_rn(A4.w, B4.w));
-        const float av4 = __fmul_rn(0.5f, __fadd_rn(A1, B1));
-        const float jr = __fsub_rn(oth[0], P0.x);
-        const float jm = __fsub_rn(mdo, md_s);
-        const float jt = __fsub_rn(oth[4], P1.x);
+        const float4 P = sP[fs.la];
+        const float lam = __fmul_rn(0.25f, __fadd_rn(__fadd_rn(P.z, q.umag), __fadd_rn(P.w, q.c)));
+        const float jr = __fsub_rn(oth[0], P.x);
+        const float jm = __fsub_rn(mdo, A[0]);      /* the mass flux is the normal momentum */
+        const float jt = __fsub_rn(oth[4], P.y);
+        const float av0 = __fmul_rn(0.5f, __fadd_rn(A[0], B[0]));
+        const float av1 = __fmul_rn(0.5f, __fadd_rn(A[1], B[1]));
+        const float av2 = __fmul_rn(0.5f, __fadd_rn(A[2], B[2]));
+        const float av3 = __fmul_rn(0.5f, __fadd_rn(A[3], B[3]));
+        const float av4 = __fmul_rn(0.5f, __fadd_rn(A[4], B[4]));
         const float s1 = sg * av1, s2 = sg * av2, s3 = sg * av3;
         o4.x = __fmaf_rn(-lam, jr, sg * av0);
         o4.y = d0 ? __fmaf_rn(-lam, jm, s1) : s1;
@@ -305,27 +285,21 @@ __device__ __forceinline__ void face_flux(const FaceSlot& fs, int32_t nb, const 
          * field.cpp:257-266), so only the normal momentum flux remains:
          * s p' + lam m_n, lam = (|U_ghost| + c) / 2.  No viscous wall flux
          * (zero ghost gradient). */
-        const float4 P2 = sP[2 * NP + fs.la];
-        const float r0 = d0 ? 0.0f : P2.x;
-        const float r1 = d1 ? 0.0f : P2.y;
-        const float r2 = d2 ? 0.0f : P2.z;
+        const float r0 = d0 ? 0.0f : q.u[0];
+        const float r1 = d1 ? 0.0f : q.u[1];
+        const float r2 = d2 ? 0.0f : q.u[2];
         const float mr = safe_sqrt(__fmaf_rn(r0, r0, __fmaf_rn(r1, r1, __fmul_rn(r2, r2))));
-        const float um_g = mr > 1e-7f ? um_s : mr;
-        const float lam = __fmul_rn(0.5f, __fadd_rn(um_g, c_s));
-        const float fn = __fmaf_rn(lam, md_s, sg * P2.w);
+        const float um_g = mr > 1e-7f ? q.umag : mr;
+        const float lam = __fmul_rn(0.5f, __fadd_rn(um_g, q.c));
+        const float fn = __fmaf_rn(lam, mdo, sg * q.pp);
         o4 = make_float4(0.0f, d0 ? fn : 0.0f, d1 ? fn : 0.0f, d2 ? fn : 0.0f);
         o1 = 0.0f;
     }
 }
 
 /* one kernel per stage (0: tendency only): the stage's own loads and update */
-/* PERSIST: a grid of resident CTAs walks the elements (e, e + grid, ...);
- * while one element computes, the next element's own stage base and
- * increment stream into shared memory, so their load latency is hidden; the
- * line-sum table is staged once per CTA. */
-template <int NX, int NY, int NZ, int STAGE, bool VISC, bool TC, bool PERSIST>
-__global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK,
-                                  (stage_min_blocks<NX, NY, NZ, STAGE, VISC, PERSIST>()))
+template <int NX, int NY, int NZ, int STAGE, bool VISC, bool TC>
+__global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK, (stage_min_blocks<NX, NY, NZ, STAGE, VISC>()))
 k_mixed_stage(StageArgs a) {
     static_assert(!TC || (NX == 8 && NY == 8 && NZ == 8), "tensor-core line sums: order 7");
     using G = Geo<NX, NY, NZ>;
@@ -334,79 +308,60 @@ k_mixed_stage(StageArgs a) {
     constexpr int NFS = G::NFS;
     extern __shared__ float4 smem4[];
     float* smem = reinterpret_cast<float*>(smem4);
-    float4* sP = reinterpret_cast<float4*>(smem + SM::OFF_P);     /* [3][NP] */
+    float4* sP = reinterpret_cast<float4*>(smem + SM::OFF_P);     /* [NP] */
     float4* sFF4 = reinterpret_cast<float4*>(smem + SM::OFF_FF4); /* [NFS] */
     float* sFF1 = smem + SM::OFF_FF1;                             /* [NFS] */
     float* sMeta = smem + SM::OFF_META;
 
     const int t = threadIdx.x;
+    const int64_t e = blockIdx.x;
     constexpr bool has_din = STAGE >= 2;
-    float* sStg = smem + SM::OFF_STG;                             /* [14][NP] (PERSIST) */
     if constexpr (TC) {
         float* sQtc = smem + SM::OFF_QTC;
         for (int q = t; q < TC_QTAB; q += G::BLOCK) sQtc[q] = __ldg(a.Qg + QTAB + q);
     }
-    auto prefetch = [&](int64_t en, int32_t lay) {
-        if (t < NP) {
-            const float* s = a.S + en * 5 * NP + t;
-#pragma unroll
-            for (int v = 0; v < 5; v++) cp_async4(sStg + v * NP + t, s + v * NP);
-            if constexpr (has_din) {
-                const float* d = a.Din + en * 5 * NP + t;
-#pragma unroll
-                for (int v = 0; v < 5; v++) cp_async4(sStg + (5 + v) * NP + t, d + v * NP);
-            }
-            const float* bg = a.bg + (int64_t)lay * 4 * NP + t;
-#pragma unroll
-            for (int c = 0; c < 4; c++) cp_async4(sStg + (10 + c) * NP + t, bg + c * NP);
-        }
-        cp_async_commit();
-    };
-    const int64_t e_step = gridDim.x;
-    auto element = [&](const int64_t e) {
-    int32_t lay_next = 0;
-    if constexpr (PERSIST) {
-        cp_async_wait_all();
-        __syncthreads();
-        /* the next element's background layer, needed when its copies start */
-        if (e + e_step < a.n_elem) lay_next = __ldg(a.layer + e + e_step);
-    }
 
-    /* issue every global load first: own node, face neighbour, stage-3 FP64 */
+    /* what no kernel of the chain writes, before the wait for the previous
+     * kernel: background, neighbours, metric */
     float own[5], din[5] = {0, 0, 0, 0, 0}, bgs[4] = {0, 0, 0, 0};
     double u64[5];
     float gown[12];
     if (t < NP) {
-        if constexpr (PERSIST) {
+        const float* bg = a.bg + (int64_t)__ldg(a.layer + e) * 4 * NP + t;
 #pragma unroll
-            for (int v = 0; v < 5; v++) own[v] = sStg[v * NP + t];
-            if constexpr (has_din) {
+        for (int c = 0; c < 4; c++) bgs[c] = __ldg(bg + c * NP);
+    }
+    FaceSlot fs{};
+    int32_t nb = -1;
+    /* the other side's node; a wall's flux is formed from the own trace */
+    int64_t eo = e;
+    int lo = 0;
+    float oth[5], bgo[4];
+    float gfo[4] = {0, 0, 0, 0};
+    if (t < NFS) {
+        fs = face_slot<NX, NY, NZ, STAGE == 1 || STAGE == 2>(t);
+        nb = __ldg(a.nbr + (int64_t)fs.face * a.n_elem + e);
+        lo = fs.la;
+        if (nb >= 0) { eo = nb; lo = fs.lo; }
+        const float* bg = a.bg + (int64_t)__ldg(a.layer + eo) * 4 * NP + lo;
 #pragma unroll
-                for (int v = 0; v < 5; v++) {
-                    din[v] = sStg[(5 + v) * NP + t];
-                    own[v] = __fadd_rn(own[v], din[v]);
-                }
+        for (int c = 0; c < 4; c++) bgo[c] = __ldg(bg + c * NP);
+    }
+    if (t < 3) sMeta[t] = __ldg(a.J + (int64_t)t * a.n_elem + e);
+    nsem_chain_wait();
+
+    /* every other global load: own node, face neighbour, stage-3 FP64 */
+    if (t < NP) {
+        const float* s = a.S + e * 5 * NP + t;
+#pragma unroll
+        for (int v = 0; v < 5; v++) own[v] = s[v * NP];
+        if constexpr (has_din) {
+            const float* d = a.Din + e * 5 * NP + t;
+#pragma unroll
+            for (int v = 0; v < 5; v++) {
+                din[v] = d[v * NP];
+                own[v] = __fadd_rn(own[v], din[v]);
             }
-        } else {
-            const float* s = a.S + e * 5 * NP + t;
-#pragma unroll
-            for (int v = 0; v < 5; v++) own[v] = __ldg(s + v * NP);
-            if constexpr (has_din) {
-                const float* d = a.Din + e * 5 * NP + t;
-#pragma unroll
-                for (int v = 0; v < 5; v++) {
-                    din[v] = __ldg(d + v * NP);
-                    own[v] = __fadd_rn(own[v], din[v]);
-                }
-            }
-        }
-        if constexpr (PERSIST) {
-#pragma unroll
-            for (int c = 0; c < 4; c++) bgs[c] = sStg[(10 + c) * NP + t];
-        } else {
-            const float* bg = a.bg + (int64_t)__ldg(a.layer + e) * 4 * NP + t;
-#pragma unroll
-            for (int c = 0; c < 4; c++) bgs[c] = __ldg(bg + c * NP);
         }
         if constexpr (STAGE == 3) {
             /* u'^n is needed only at the update: inviscid runs fetch it into L2
@@ -416,7 +371,7 @@ k_mixed_stage(StageArgs a) {
             const double* u = a.U + e * 5 * NP + t;
             if constexpr (VISC) {
 #pragma unroll
-                for (int v = 0; v < 5; v++) u64[v] = __ldg(u + v * NP);
+                for (int v = 0; v < 5; v++) u64[v] = u[v * NP];
             } else {
 #pragma unroll
                 for (int v = 0; v < 5; v++) asm volatile("prefetch.global.L2 [%0];" ::"l"(u + v * NP));
@@ -425,55 +380,42 @@ k_mixed_stage(StageArgs a) {
         if constexpr (VISC) {
             const float* gr = a.G + e * 12 * NP + t;
 #pragma unroll
-            for (int c = 0; c < 12; c++) gown[c] = __ldg(gr + c * NP);
+            for (int c = 0; c < 12; c++) gown[c] = gr[c * NP];
         }
     }
-    FaceSlot fs{};
-    int32_t nb = -1;
-    float oth[5], bgo[4];
-    float gfo[4] = {0, 0, 0, 0};
     if (t < NFS) {
-        fs = face_slot<NX, NY, NZ, STAGE == 1 || STAGE == 2>(t);
-        nb = __ldg(a.nbr + (int64_t)fs.face * a.n_elem + e);
         if (nb <= -2) {
             /* a face on a 2:1 mortar: its outward values come from the
              * mortar kernels */
             const float* mf = a.MF + (int64_t)(-2 - nb) * MF_ROWS * a.nfmax + face_local<NX, NY, NZ>(t);
 #pragma unroll
-            for (int v = 0; v < 5; v++) oth[v] = __ldg(mf + v * a.nfmax);
-        }
-        if (nb >= 0) {
-            const float* s = a.S + (int64_t)nb * 5 * NP + fs.lo;
+            for (int v = 0; v < 5; v++) oth[v] = mf[v * a.nfmax];
+        } else {
+            const float* s = a.S + eo * 5 * NP + lo;
 #pragma unroll
-            for (int v = 0; v < 5; v++) oth[v] = __ldg(s + v * NP);
+            for (int v = 0; v < 5; v++) oth[v] = s[v * NP];
             if constexpr (has_din) {
-                const float* d = a.Din + (int64_t)nb * 5 * NP + fs.lo;
+                const float* d = a.Din + eo * 5 * NP + lo;
 #pragma unroll
-                for (int v = 0; v < 5; v++) oth[v] = __fadd_rn(oth[v], __ldg(d + v * NP));
+                for (int v = 0; v < 5; v++) oth[v] = __fadd_rn(oth[v], d[v * NP]);
             }
-            const float* bg = a.bg + (int64_t)__ldg(a.layer + nb) * 4 * NP + fs.lo;
-#pragma unroll
-            for (int c = 0; c < 4; c++) bgo[c] = __ldg(bg + c * NP);
             if constexpr (VISC) {
                 /* the neighbour's gradients along the face's axis only:
                  * d_c U_dir (c = 0..2) and d_dir theta */
-                const float* gr = a.G + (int64_t)nb * 12 * NP + fs.lo;
+                const float* gr = a.G + eo * 12 * NP + lo;
                 const int d = fs.dir;
-                gfo[0] = __ldg(gr + tidx(0, d) * NP);
-                gfo[1] = __ldg(gr + tidx(1, d) * NP);
-                gfo[2] = __ldg(gr + tidx(2, d) * NP);
-                gfo[3] = __ldg(gr + (9 + d) * NP);
+                gfo[0] = gr[tidx(0, d) * NP];
+                gfo[1] = gr[tidx(1, d) * NP];
+                gfo[2] = gr[tidx(2, d) * NP];
+                gfo[3] = gr[(9 + d) * NP];
             }
         }
     }
-    if (t < 3) sMeta[t] = __ldg(a.J + (int64_t)t * a.n_elem + e);
 
     /* phase 1: own node primitives and volume fluxes */
     if (t < NP) {
         const Pt p = pointwise(own, bgs, a.eos, a.gamma, a.gR);
-        sP[t] = make_float4(own[0], own[1], own[2], own[3]);
-        sP[NP + t] = make_float4(own[4], p.rho, p.umag, p.c);
-        sP[2 * NP + t] = make_float4(p.u[0], p.u[1], p.u[2], p.pp);
+        sP[t] = make_float4(own[0], own[4], p.umag, p.c);
         float4 f4;
         float f1;
         if constexpr (TC) {
@@ -505,11 +447,6 @@ k_mixed_stage(StageArgs a) {
         }
     }
     __syncthreads();
-    if constexpr (PERSIST) {
-        /* the staging area is free: stream in the next element */
-        if (e + e_step < a.n_elem) prefetch(e + e_step, lay_next);
-    }
-
     /* phase 2: Rusanov flux on every face node */
     if (t < NFS) {
         float4 o4;
@@ -525,6 +462,11 @@ k_mixed_stage(StageArgs a) {
     }
     __syncthreads();
 
+    /* the next stage's CTAs may start: launched earlier (at the start, or after
+     * the wait) they take the slots of a grid below one wave unevenly
+     * (9 x 7 x 11 elements, 40 steps: 767 us at the start, 756 after the wait,
+     * 666 here, 679 never; 10 x 10 in 2D, 50 steps: 465, 443, 444, 515) */
+    nsem_chain_begin();
     /* phase 3: weak volume term (line sums with Q), lift, buoyancy, update */
     if constexpr (TC) {
         /* tensor-core line sums, results in place of the fluxes */
@@ -636,10 +578,18 @@ k_mixed_stage(StageArgs a) {
         for (int v = 0; v < 5; v++) a.Dout[o + v * NP] = 0.25f * fmaf(dt, Lv[v], din[v]);
     } else if constexpr (STAGE == 3) {
         bool finite = true;
+        /* every load before the first store, which could alias them */
+        if constexpr (!VISC) {
+#pragma unroll
+            for (int v = 0; v < 5; v++) {
+                din[v] = a.Din[o + v * NP];
+                u64[v] = a.U[o + v * NP];
+            }
+        }
 #pragma unroll
         for (int v = 0; v < 5; v++) {
-            const float D = (2.0f / 3.0f) * fmaf(dt, Lv[v], VISC ? din[v] : __ldg(a.Din + o + v * NP));
-            const double un = (VISC ? u64[v] : __ldg(a.U + o + v * NP)) + f2d(D);
+            const float D = (2.0f / 3.0f) * fmaf(dt, Lv[v], din[v]);
+            const double un = u64[v] + f2d(D);
             a.Unew[o + v * NP] = un;
             a.Snew[o + v * NP] = d2f_rn(un);
             /* exponent field all ones = inf or nan (integer test, no FP64 op) */
@@ -648,17 +598,7 @@ k_mixed_stage(StageArgs a) {
         if (!finite) atomicOr(a.status, NSEM_STATUS_NONFINITE);
     }
     }  /* t < NP */
-    };  /* element */
-    if constexpr (PERSIST) {
-        prefetch(blockIdx.x, __ldg(a.layer + blockIdx.x));
-        for (int64_t e = blockIdx.x; e < a.n_elem; e += e_step) element(e);
-        cp_async_wait_all();
-    } else {
-        element(blockIdx.x);
-    }
 }
-
-
 
 template <int NX, int NY, int NZ, int SIN>
 __global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK)
@@ -676,37 +616,38 @@ k_mixed_grad(StageArgs a) {
     const int64_t e = blockIdx.x;
 
     float own[5], bgs0 = 0.0f;
-    if (t < NP) {
-        const float* s = a.S + e * 5 * NP + t;
-#pragma unroll
-        for (int v = 0; v < 5; v++) own[v] = __ldg(s + v * NP);
-        if (has_din) {
-            const float* d = a.Din + e * 5 * NP + t;
-#pragma unroll
-            for (int v = 0; v < 5; v++) own[v] = __fadd_rn(own[v], __ldg(d + v * NP));
-        }
-        bgs0 = __ldg(a.bg + (int64_t)__ldg(a.layer + e) * 4 * NP + t);
-    }
+    if (t < NP) bgs0 = __ldg(a.bg + (int64_t)__ldg(a.layer + e) * 4 * NP + t);
     FaceSlot fs{};
     int32_t nb = -1;
     float oth[5], bgo0 = 0.0f;
     if (t < NFS) {
         fs = face_slot<NX, NY, NZ>(t);
         nb = __ldg(a.nbr + (int64_t)fs.face * a.n_elem + e);
-        if (nb >= 0) {
-            const float* s = a.S + (int64_t)nb * 5 * NP + fs.lo;
-#pragma unroll
-            for (int v = 0; v < 5; v++) oth[v] = __ldg(s + v * NP);
-            if (has_din) {
-                const float* d = a.Din + (int64_t)nb * 5 * NP + fs.lo;
-#pragma unroll
-                for (int v = 0; v < 5; v++) oth[v] = __fadd_rn(oth[v], __ldg(d + v * NP));
-            }
-            bgo0 = __ldg(a.bg + (int64_t)__ldg(a.layer + nb) * 4 * NP + fs.lo);
-        }
+        if (nb >= 0) bgo0 = __ldg(a.bg + (int64_t)__ldg(a.layer + nb) * 4 * NP + fs.lo);
     }
     for (int q = t; q < QTAB; q += G::BLOCK) sDg[q] = __ldg(a.Dg + q);
     if (t < 3) sJ[t] = __ldg(a.J + (int64_t)t * a.n_elem + e);
+    nsem_chain_wait();
+    if (t < NP) {
+        const float* s = a.S + e * 5 * NP + t;
+#pragma unroll
+        for (int v = 0; v < 5; v++) own[v] = s[v * NP];
+        if (has_din) {
+            const float* d = a.Din + e * 5 * NP + t;
+#pragma unroll
+            for (int v = 0; v < 5; v++) own[v] = __fadd_rn(own[v], d[v * NP]);
+        }
+    }
+    if (t < NFS && nb >= 0) {
+        const float* s = a.S + (int64_t)nb * 5 * NP + fs.lo;
+#pragma unroll
+        for (int v = 0; v < 5; v++) oth[v] = s[v * NP];
+        if (has_din) {
+            const float* d = a.Din + (int64_t)nb * 5 * NP + fs.lo;
+#pragma unroll
+            for (int v = 0; v < 5; v++) oth[v] = __fadd_rn(oth[v], d[v * NP]);
+        }
+    }
 
     if (t < NP) sV[t] = prim_ut(own, bgs0, a.T0);
     __syncthreads();
@@ -714,14 +655,14 @@ k_mixed_grad(StageArgs a) {
     if (t < NFS && nb <= -2) {
         /* a face on a 2:1 mortar: the projected values from the mortar kernels */
         const float* gf = a.MF + ((int64_t)(-2 - nb) * MF_ROWS + 5) * a.nfmax + face_local<NX, NY, NZ>(t);
-        sD[t] = make_float4(__ldg(gf), __ldg(gf + a.nfmax), __ldg(gf + 2 * a.nfmax),
-                            __ldg(gf + 3 * a.nfmax));
+        sD[t] = make_float4(gf[0], gf[a.nfmax], gf[2 * a.nfmax], gf[3 * a.nfmax]);
     } else if (t < NFS) {
         const float4 O = nb >= 0 ? prim_ut(oth, bgo0, a.T0) : make_float4(0, 0, 0, 0);
         sD[t] = cds_minus_own(sV[fs.la], nb >= 0 ? &O : nullptr, fs.dir);
     }
     __syncthreads();
 
+    nsem_chain_begin();
     if (t >= NP) return;
     const int i = t / (NY * NZ), j = (t / NZ) % NY, k = t % NZ;
     float g12[12];
@@ -731,55 +672,37 @@ k_mixed_grad(StageArgs a) {
     for (int c = 0; c < 12; c++) out[c * NP] = g12[c];
 }
 
-template <int NX, int NY, int NZ, bool VISC, bool TC, bool PERSIST>
-void launch_stage_v(const StageArgs& a, int stage, cudaStream_t st, const LaunchCfg& c) {
-    using G = Geo<NX, NY, NZ>;
-    constexpr size_t SMEM = PERSIST ? StageSmem<NX, NY, NZ>::BYTES_P : StageSmem<NX, NY, NZ, TC>::BYTES;
-    int64_t g = a.n_elem;
-    if (PERSIST && c.pgrid[stage] > 0 && c.pgrid[stage] < g) g = c.pgrid[stage];
-    const unsigned grid = (unsigned)g;
+template <int NX, int NY, int NZ, bool VISC, bool TC>
+int launch_stage_v(const StageArgs& a, int stage, cudaStream_t st) {
+    constexpr unsigned B = Geo<NX, NY, NZ>::BLOCK;
+    constexpr size_t SMEM = StageSmem<NX, NY, NZ, TC>::BYTES;
+    const unsigned grid = (unsigned)a.n_elem;
     switch (stage) {
-        case 0: k_mixed_stage<NX, NY, NZ, 0, VISC, TC, PERSIST><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-        case 1: k_mixed_stage<NX, NY, NZ, 1, VISC, TC, PERSIST><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-        case 2: k_mixed_stage<NX, NY, NZ, 2, VISC, TC, PERSIST><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-        default: k_mixed_stage<NX, NY, NZ, 3, VISC, TC, PERSIST><<<grid, G::BLOCK, SMEM, st>>>(a); break;
+        case 0: return nsem_launch_chained(k_mixed_stage<NX, NY, NZ, 0, VISC, TC>, grid, B, SMEM, st, a);
+        case 1: return nsem_launch_chained(k_mixed_stage<NX, NY, NZ, 1, VISC, TC>, grid, B, SMEM, st, a);
+        case 2: return nsem_launch_chained(k_mixed_stage<NX, NY, NZ, 2, VISC, TC>, grid, B, SMEM, st, a);
+        default: return nsem_launch_chained(k_mixed_stage<NX, NY, NZ, 3, VISC, TC>, grid, B, SMEM, st, a);
     }
 }
 
-/* the tensor-core line sums exist for order 7 only; persistent CTAs for the
- * inviscid kernels of up to 256 threads (order 7's 64 KB of shared memory
- * leaves no room for the staging area) */
+/* the tensor-core line sums exist for order 7 only */
 template <int NX, int NY, int NZ>
 constexpr bool tc_dims() {
     return NX == 8 && NY == 8 && NZ == 8;
 }
-template <int NX, int NY, int NZ>
-constexpr bool persist_dims() {
-    return Geo<NX, NY, NZ>::BLOCK <= 256;
-}
 
 template <int NX, int NY, int NZ, bool VISC>
-void launch_stage_tc(const StageArgs& a, int stage, cudaStream_t st, const LaunchCfg& c) {
+int launch_stage_tc(const StageArgs& a, int stage, cudaStream_t st, const LaunchCfg& c) {
     if constexpr (tc_dims<NX, NY, NZ>()) {
-        if (c.tc) {
-            launch_stage_v<NX, NY, NZ, VISC, true, false>(a, stage, st, c);
-            return;
-        }
+        if (c.tc) return launch_stage_v<NX, NY, NZ, VISC, true>(a, stage, st);
     }
-    if constexpr (!VISC && persist_dims<NX, NY, NZ>()) {
-        if (c.persist) {
-            launch_stage_v<NX, NY, NZ, false, false, true>(a, stage, st, c);
-            return;
-        }
-    }
-    launch_stage_v<NX, NY, NZ, VISC, false, false>(a, stage, st, c);
+    return launch_stage_v<NX, NY, NZ, VISC, false>(a, stage, st);
 }
 
 template <int NX, int NY, int NZ>
 int launch_stage(const StageArgs& a, int stage, cudaStream_t st, const LaunchCfg& c) {
-    if (c.visc) launch_stage_tc<NX, NY, NZ, true>(a, stage, st, c);
-    else launch_stage_tc<NX, NY, NZ, false>(a, stage, st, c);
-    return (int)cudaGetLastError();
+    return c.visc ? launch_stage_tc<NX, NY, NZ, true>(a, stage, st, c)
+                  : launch_stage_tc<NX, NY, NZ, false>(a, stage, st, c);
 }
 
 /* viscous runs: the gradients of the stage state, before the stage */
@@ -788,60 +711,34 @@ int launch_grad(const StageArgs& a, int stage, cudaStream_t st) {
     using G = Geo<NX, NY, NZ>;
     const unsigned grid = (unsigned)a.n_elem;
     constexpr size_t gs = grad_smem<NX, NY, NZ>();
-    if (stage <= 1) k_mixed_grad<NX, NY, NZ, 1><<<grid, G::BLOCK, gs, st>>>(a);
-    else k_mixed_grad<NX, NY, NZ, 2><<<grid, G::BLOCK, gs, st>>>(a);
-    return (int)cudaGetLastError();
+    constexpr unsigned B = G::BLOCK;
+    return stage <= 1 ? nsem_launch_chained(k_mixed_grad<NX, NY, NZ, 1>, grid, B, gs, st, a)
+                      : nsem_launch_chained(k_mixed_grad<NX, NY, NZ, 2>, grid, B, gs, st, a);
 }
 
-template <int NX, int NY, int NZ, bool VISC, bool TC, bool PERSIST>
+template <int NX, int NY, int NZ, bool VISC, bool TC>
 int set_smem(int stage) {
-    constexpr int SMEM = (int)(PERSIST ? StageSmem<NX, NY, NZ>::BYTES_P : StageSmem<NX, NY, NZ, TC>::BYTES);
+    constexpr int SMEM = (int)StageSmem<NX, NY, NZ, TC>::BYTES;
     if (SMEM <= 48 * 1024) return 0;
     const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
     switch (stage) {
-        case 0: return (int)cudaFuncSetAttribute(k_mixed_stage<NX, NY, NZ, 0, VISC, TC, PERSIST>, at, SMEM);
-        case 1: return (int)cudaFuncSetAttribute(k_mixed_stage<NX, NY, NZ, 1, VISC, TC, PERSIST>, at, SMEM);
-        case 2: return (int)cudaFuncSetAttribute(k_mixed_stage<NX, NY, NZ, 2, VISC, TC, PERSIST>, at, SMEM);
-        default: return (int)cudaFuncSetAttribute(k_mixed_stage<NX, NY, NZ, 3, VISC, TC, PERSIST>, at, SMEM);
+        case 0: return (int)cudaFuncSetAttribute(k_mixed_stage<NX, NY, NZ, 0, VISC, TC>, at, SMEM);
+        case 1: return (int)cudaFuncSetAttribute(k_mixed_stage<NX, NY, NZ, 1, VISC, TC>, at, SMEM);
+        case 2: return (int)cudaFuncSetAttribute(k_mixed_stage<NX, NY, NZ, 2, VISC, TC>, at, SMEM);
+        default: return (int)cudaFuncSetAttribute(k_mixed_stage<NX, NY, NZ, 3, VISC, TC>, at, SMEM);
     }
-}
-
-/* resident CTAs of a persistent stage kernel on the whole GPU */
-template <int NX, int NY, int NZ, int STAGE>
-int persist_grid() {
-    int per_sm = 0, dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, k_mixed_stage<NX, NY, NZ, STAGE, false, false, true>, Geo<NX, NY, NZ>::BLOCK,
-            StageSmem<NX, NY, NZ>::BYTES_P) != cudaSuccess)
-        return 0;
-    return per_sm * sms;
 }
 
 template <int NX, int NY, int NZ>
-int prepare_stage(LaunchCfg* c) {
+int prepare_stage() {
     int e = 0;
     for (int st = 0; st < 4 && !e; st++) {
-        e = set_smem<NX, NY, NZ, false, false, false>(st);
-        if (!e) e = set_smem<NX, NY, NZ, true, false, false>(st);
+        e = set_smem<NX, NY, NZ, false, false>(st);
+        if (!e) e = set_smem<NX, NY, NZ, true, false>(st);
         if constexpr (tc_dims<NX, NY, NZ>()) {
-            if (!e) e = set_smem<NX, NY, NZ, false, true, false>(st);
-            if (!e) e = set_smem<NX, NY, NZ, true, true, false>(st);
+            if (!e) e = set_smem<NX, NY, NZ, false, true>(st);
+            if (!e) e = set_smem<NX, NY, NZ, true, true>(st);
         }
-        if constexpr (persist_dims<NX, NY, NZ>()) {
-            if (!e) e = set_smem<NX, NY, NZ, false, false, true>(st);
-        }
-    }
-    if constexpr (persist_dims<NX, NY, NZ>()) {
-        c->pgrid[0] = persist_grid<NX, NY, NZ, 0>();
-        c->pgrid[1] = persist_grid<NX, NY, NZ, 1>();
-        c->pgrid[2] = persist_grid<NX, NY, NZ, 2>();
-        c->pgrid[3] = persist_grid<NX, NY, NZ, 3>();
-        if (!c->pgrid[0] || !c->pgrid[1] || !c->pgrid[2] || !c->pgrid[3]) c->persist = false;
-    } else {
-        c->persist = false;
     }
     constexpr size_t gs = grad_smem<NX, NY, NZ>();
     const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
@@ -856,8 +753,8 @@ int prepare_stage(LaunchCfg* c) {
 
 namespace nsem_mx {
 
-int prepare_aligned(int nx, int ny, int nz, LaunchCfg* c) {
-#define NSEM_PREP(A, B, C) if (nx == A && ny == B && nz == C) return prepare_stage<A, B, C>(c);
+int prepare_aligned(int nx, int ny, int nz) {
+#define NSEM_PREP(A, B, C) if (nx == A && ny == B && nz == C) return prepare_stage<A, B, C>();
     NSEM_MIXED_DIMS(NSEM_PREP)
 #undef NSEM_PREP
     return (int)cudaErrorNotSupported;
