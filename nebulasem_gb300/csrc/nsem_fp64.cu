@@ -28,6 +28,7 @@
 #include "nsem_gather.cuh"
 #include "nsem_internal.h"
 #include "nsem_mortar.cuh"
+#include "nsem_pdl.cuh"
 
 namespace {
 
@@ -103,6 +104,8 @@ __device__ __forceinline__ void prim_at(const NsemDev& m, const double* const* S
 
 __global__ void __launch_bounds__(256) k_prim(const NsemDev m, PrimArgs a) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    nsem_chain_wait();
+    nsem_chain_begin();
     if (i >= m.n_int) return;
     prim_at(m, a.S, a.prim, i);
 }
@@ -116,6 +119,7 @@ struct FaceArgs {
     double* mq[19];              /* the coarse side's interpolated quantities */
     double* mf[15];              /* face flux vectors (rho 3, momentum 9, theta 3) */
     double* dC[5];               /* projected, lifted coarse-side fluxes */
+    int early;                   /* the volume kernel's CTAs may start beside this kernel */
 };
 
 /* Non-conforming faces: the coarse side's node quantities of the stage
@@ -181,11 +185,13 @@ __global__ void __launch_bounds__(128) k_mortar_coupled_gather(const NsemDev m, 
 
 __global__ void __launch_bounds__(256) k_face(const NsemDev m, FaceArgs a) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= m.n_slot) return;
+    if (k >= m.n_slot) return;   /* a CTA has at least one slot */
     const int32_t c1 = m.c1[k], c2 = m.c2[k];
     const double n[3] = {m.fn[k], m.fn[m.n_slot + k], m.fn[2 * m.n_slot + k]};
     const double en[3] = {m.en[k], m.en[m.n_slot + k], m.en[2 * m.n_slot + k]};
     const double fi = m.fi[k], fo = 1 - fi;
+    nsem_chain_wait();
+    if (a.early) nsem_chain_begin();
 
     const double r1 = a.S0[c1];
     const double U1[3] = {a.prim[0][c1], a.prim[1][c1], a.prim[2][c1]};
@@ -370,6 +376,9 @@ __global__ void k_volume(const NsemDev m, const NsemTables tab, VolArgs a) {
     const bool active = t < NP;
     const int64_t node = e * NP + t;
     double rho = 0, U[3] = {0, 0, 0}, T = 0, pp = 0;
+    if (active)
+        for (int c = 0; c < 9; c++) sm[(size_t)t * SM_W + 15 + c] = m.jin[(int64_t)c * m.n_int + node];
+    nsem_chain_wait();
     if (active) {
         rho = a.S[0][node];
         U[0] = a.prim[0][node]; U[1] = a.prim[1][node]; U[2] = a.prim[2][node];
@@ -392,7 +401,6 @@ __global__ void k_volume(const NsemDev m, const NsemTables tab, VolArgs a) {
             for (int r = 0; r < 3; r++) my[5 * c + 1 + r] = fm[col[c][r]];
             my[5 * c + 4] = ft[c];
         }
-        for (int c = 0; c < 9; c++) my[15 + c] = m.jin[(int64_t)c * m.n_int + node];
     }
     const bool diag = __syncthreads_and(!active || nsem_node_diag<5>(sm + (size_t)t * SM_W));
     if (!active) return;
@@ -413,6 +421,7 @@ __global__ void k_volume(const NsemDev m, const NsemTables tab, VolArgs a) {
     /* weak volume term.  Source b adds -F_b . (Jin_b . dpsi(b->a)); sources
      * arrive in lexicographic order of b: X-line below, Y-line below, Z-line
      * below, self, Z above, Y above, X above. */
+    nsem_chain_begin();
     nsem_volume_gather<5, SM_W, SM_ROWS>(NPX, NPY, NPZ, sm, dps, t, diag, r);
 
     /* gravity source: Su -= ((rho - rho_ref) g) cV */
@@ -468,8 +477,7 @@ extern "C" int nsem_fp64_prim(const NsemDev* m, NsemBuf* b, int from_state, void
     for (int c = 0; c < 5; c++) a.S[c] = from_state ? b->u[c] : b->s[c];
     for (int c = 0; c < NSEM_NPRIM; c++) a.prim[c] = b->prim[c];
     const int64_t blocks = (m->n_int + 255) / 256;
-    k_prim<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(*m, a);
-    return launch_err();
+    return nsem_launch_chained(k_prim, (unsigned)blocks, 256, 0, (cudaStream_t)stream, *m, a);
 }
 
 extern "C" int nsem_fp64_face(const NsemDev* m, NsemBuf* b, int from_state, void* stream) {
@@ -481,11 +489,20 @@ extern "C" int nsem_fp64_face(const NsemDev* m, NsemBuf* b, int from_state, void
     for (int c = 0; c < 19; c++) a.mq[c] = b->mq[c];
     for (int c = 0; c < 15; c++) a.mf[c] = b->mf[c];
     for (int c = 0; c < 5; c++) a.dC[c] = b->dC[c];
+    /* a volume grid of less than a wave that fills the FP64 pipes (8 to 32 warps
+     * an SM) is started after this kernel: beside it, its CTAs gather on the
+     * SMs this grid leaves free (9 x 8 x 10 elements of order 4, forward and
+     * reverse: 9.2 against 7.8 ms); more waves even out (14 x 12 x 13: 6.14
+     * against 6.25 ms), fewer warps leave the pipes idle either way */
+    const int64_t warps = m->n_elem * ((m->np + 31) / 32) / 152;
+    a.early = warps < 8 || warps > 32;
     const int64_t blocks = (m->n_slot + 255) / 256;
     cudaStream_t st = (cudaStream_t)stream;
     const unsigned mb = (unsigned)((m->n_ms + 127) / 128);
     if (m->n_ms > 0) k_mortar_coupled<<<19 * mb, 128, 0, st>>>(*m, a);
-    k_face<<<(unsigned)blocks, 256, 0, st>>>(*m, a);
+    int e = launch_err();
+    if (!e) e = nsem_launch_chained(k_face, (unsigned)blocks, 256, 0, st, *m, a);
+    if (e) return e;
     if (m->n_ms > 0) k_mortar_coupled_gather<<<5 * mb, 128, 0, st>>>(*m, a);
     return launch_err();
 }
@@ -521,6 +538,6 @@ extern "C" int nsem_fp64_volume(const NsemDev* m, const NsemTables* t, NsemBuf* 
     for (int c = 0; c < 12; c++) a.G[c] = b->G[c];
     for (int c = 0; c < 5; c++) a.dC[c] = b->dC[c];
     const int threads = ((m->np + 31) / 32) * 32;
-    k_volume<<<(unsigned)m->n_elem, threads, vol_smem(m), (cudaStream_t)stream>>>(*m, *t, a);
-    return launch_err();
+    return nsem_launch_chained(k_volume, (unsigned)m->n_elem, (unsigned)threads, vol_smem(m),
+                               (cudaStream_t)stream, *m, *t, a);
 }

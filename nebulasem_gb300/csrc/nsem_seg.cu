@@ -43,6 +43,7 @@
 #include "nsem_ddpow.h"
 #include "nsem_gather.cuh"
 #include "nsem_mortar.cuh"
+#include "nsem_pdl.cuh"
 #include "nsem_seg.h"
 
 namespace {
@@ -213,6 +214,8 @@ __global__ void __launch_bounds__(128) k_seg_mortar_gather(const NsemDev m, SegA
 __global__ void __launch_bounds__(256) k_seg_prep(const NsemDev m, SegArgs a) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.n_int) return;
+    nsem_chain_wait();
+    nsem_chain_begin();
     const double r = a.rho_o[i];
     const double U[3] = {a.U[0][i], a.U[1][i], a.U[2][i]};
     const double Tf = a.Tp[i] + m.T0;
@@ -229,6 +232,8 @@ __global__ void __launch_bounds__(256) k_seg_face_rho(const NsemDev m, SegArgs a
     const double n[3] = {m.fn[k], m.fn[m.n_slot + k], m.fn[2 * m.n_slot + k]};
     const double en[3] = {m.en[k], m.en[m.n_slot + k], m.en[2 * m.n_slot + k]};
     const double fi = m.fi[k], fo = 1 - fi;
+    nsem_chain_wait();
+    nsem_chain_begin();
     const double r1 = a.rho_o[c1];
     const double U1[3] = {a.U[0][c1], a.U[1][c1], a.U[2][c1]};
     const double mu1 = a.mu[c1], cs1 = a.cs[c1];
@@ -338,6 +343,8 @@ __global__ void __launch_bounds__(256) k_seg_grad_face(const NsemDev m, GradArgs
     if (k >= m.n_slot) return;
     const int32_t c1 = m.c1[k], c2 = m.c2[k];
     const double fi = m.fi[k], fo = 1 - fi;
+    nsem_chain_wait();
+    nsem_chain_begin();
     const double U1[3] = {a.U[0][c1], a.U[1][c1], a.U[2][c1]};
     const double T1 = a.Tf[c1];
     double U2[3], T2;
@@ -364,11 +371,13 @@ __global__ void k_seg_grad_vol(const NsemDev m, const NsemTables tab, GradArgs a
     const int64_t e = blockIdx.x;
     const bool active = t < NP;
     const int64_t node = e * NP + t;
+    if (active)
+        for (int c = 0; c < 9; c++) sm[(size_t)t * W_GRAD + 4 + c] = m.jin[(int64_t)c * m.n_int + node];
+    nsem_chain_wait();
     if (active) {
         double* my = sm + (size_t)t * W_GRAD;
         for (int c = 0; c < 3; c++) my[c] = a.U[c][node];
         my[3] = a.Tf[node];
-        for (int c = 0; c < 9; c++) my[4 + c] = m.jin[(int64_t)c * m.n_int + node];
     }
     /* a diagonal metric (see nsem_volume_gather): only row r of the gradients
      * takes line r's terms, 1 + 4 products a source instead of 3 + 12 */
@@ -380,6 +389,7 @@ __global__ void k_seg_grad_vol(const NsemDev m, const NsemTables tab, GradArgs a
     }
     const bool diag = __syncthreads_and(ok);
     if (!active) return;
+    nsem_chain_begin();
     const double* me = sm + (size_t)t * W_GRAD;
     double gU[9], gT[3];
     for (int c = 0; c < 9; c++) gU[c] = 0.0;
@@ -515,11 +525,13 @@ __global__ void k_seg_vol_rho(const NsemDev m, const NsemTables tab, SegArgs a) 
     const bool active = t < NP;
     const int64_t node = e * NP + t;
     double rho = 0;
+    if (active)
+        for (int c = 0; c < 9; c++) sm[(size_t)t * W_RHO + 3 + c] = m.jin[(int64_t)c * m.n_int + node];
+    nsem_chain_wait();
     if (active) {
         rho = a.rho_o[node];
         double* my = sm + (size_t)t * W_RHO;
         for (int c = 0; c < 3; c++) my[c] = a.U[c][node] * rho;     /* U * rho */
-        for (int c = 0; c < 9; c++) my[3 + c] = m.jin[(int64_t)c * m.n_int + node];
     }
     const bool diag = __syncthreads_and(!active || nsem_node_diag<1>(sm + (size_t)t * W_RHO));
     if (!active) return;
@@ -532,6 +544,7 @@ __global__ void k_seg_vol_rho(const NsemDev m, const NsemTables tab, SegArgs a) 
         if (code & 1) r -= v;
         else r += v;
     }
+    nsem_chain_begin();
     nsem_volume_gather<1, W_RHO, 0>(m.npx, m.npy, m.npz, sm, dps, t, diag, &r);
     const double cv = m.cv[node];
     const double ap = a.c_dt * cv;
@@ -548,6 +561,8 @@ __global__ void __launch_bounds__(256) k_seg_face_ut(const NsemDev m, SegArgs a)
     const double n[3] = {m.fn[k], m.fn[m.n_slot + k], m.fn[2 * m.n_slot + k]};
     const double en[3] = {m.en[k], m.en[m.n_slot + k], m.en[2 * m.n_slot + k]};
     const double fi = m.fi[k], fo = 1 - fi;
+    nsem_chain_wait();
+    nsem_chain_begin();
     const double lam = a.lam[k];
     const double r1 = a.rho_n[c1];
     const double U1[3] = {a.U[0][c1], a.U[1][c1], a.U[2][c1]};
@@ -684,6 +699,9 @@ __global__ void k_seg_vol_ut(const NsemDev m, const NsemTables tab, SegArgs a) {
     const bool active = t < NP;
     const int64_t node = e * NP + t;
     double U[3] = {0, 0, 0}, Tf = 0;
+    if (active)
+        for (int c = 0; c < 9; c++) sm[(size_t)t * W_UT + 12 + c] = m.jin[(int64_t)c * m.n_int + node];
+    nsem_chain_wait();
     if (active) {
         double* my = sm + (size_t)t * W_UT;
         double Fc[3];
@@ -704,7 +722,6 @@ __global__ void k_seg_vol_ut(const NsemDev m, const NsemTables tab, SegArgs a) {
             for (int q = 0; q < 3; q++) my[4 * c + q] = fm[col[c][q]];
             my[4 * c + 3] = ft[c];
         }
-        for (int c = 0; c < 9; c++) my[12 + c] = m.jin[(int64_t)c * m.n_int + node];
     }
     const bool diag = __syncthreads_and(!active || nsem_node_diag<4>(sm + (size_t)t * W_UT));
     if (!active) return;
@@ -719,6 +736,7 @@ __global__ void k_seg_vol_ut(const NsemDev m, const NsemTables tab, SegArgs a) {
             r[v] += __hiloint2double(__double2hiint(x) ^ (code << 31), __double2loint(x));
         }
     }
+    nsem_chain_begin();
     nsem_volume_gather<4, W_UT, UT_ROWS>(m.npx, m.npy, m.npz, sm, dps, t, diag, r);
     const double cv = m.cv[node];
     const double rn = a.rho_n[node];
@@ -893,6 +911,8 @@ __global__ void __launch_bounds__(256) k_conv_face(const NsemDev m, AdvArgs a) {
     const double n[3] = {m.fn[k], m.fn[m.n_slot + k], m.fn[2 * m.n_slot + k]};
     const double en[3] = {m.en[k], m.en[m.n_slot + k], m.en[2 * m.n_slot + k]};
     const double fi = m.fi[k], fo = 1 - fi;
+    nsem_chain_wait();
+    nsem_chain_begin();
     const double U1[3] = {a.U[0][c1], a.U[1][c1], a.U[2][c1]};
     const double T1 = a.T_o[c1];
     double U2[3], T2;
@@ -952,11 +972,13 @@ __global__ void k_conv_vol(const NsemDev m, const NsemTables tab, AdvArgs a) {
     const bool active = t < NP;
     const int64_t node = e * NP + t;
     double T = 0;
+    if (active)
+        for (int c = 0; c < 9; c++) sm[(size_t)t * W_CONV + 3 + c] = m.jin[(int64_t)c * m.n_int + node];
+    nsem_chain_wait();
     if (active) {
         T = a.T_o[node];
         double* my = sm + (size_t)t * W_CONV;
         for (int c = 0; c < 3; c++) my[c] = a.U[c][node] * T;
-        for (int c = 0; c < 9; c++) my[3 + c] = m.jin[(int64_t)c * m.n_int + node];
     }
     const bool diag = __syncthreads_and(!active || nsem_node_diag<1>(sm + (size_t)t * W_CONV));
     if (!active) return;
@@ -969,6 +991,7 @@ __global__ void k_conv_vol(const NsemDev m, const NsemTables tab, AdvArgs a) {
         if (code & 1) r -= v;
         else r += v;
     }
+    nsem_chain_begin();
     nsem_volume_gather<1, W_CONV, 0>(m.npx, m.npy, m.npz, sm, dps, t, diag, &r);
     const double ap = a.c_dt * m.cv[node];
     double Tn;
@@ -1019,13 +1042,13 @@ int nsem_grad_ut_mortar(const NsemDev* m, const NsemTables* t, const double* con
     for (int c = 0; c < 4; c++) ga.gC[c] = gC ? gC[c] : nullptr;
     cudaStream_t st = (cudaStream_t)stream;
     const int threads = ((m->np + 31) / 32) * 32;
-    k_seg_grad_face<<<(unsigned)((m->n_slot + 255) / 256), 256, 0, st>>>(*m, ga);
+    nsem_launch_chained(k_seg_grad_face, (unsigned)((m->n_slot + 255) / 256), 256, 0, st, *m, ga);
     if (m->n_ms > 0 && gC) {
         const unsigned mb = (unsigned)((m->n_ms + 127) / 128);
         k_seg_mortar_gcds<<<mb, 128, 0, st>>>(*m, ga);
         k_seg_mortar_ggather<<<mb, 128, 0, st>>>(*m, ga);
     }
-    k_seg_grad_vol<<<(unsigned)m->n_elem, threads, smem_grad(m), st>>>(*m, *t, ga);
+    nsem_launch_chained(k_seg_grad_vol, (unsigned)m->n_elem, threads, smem_grad(m), st, *m, *t, ga);
     return (int)cudaGetLastError();
 }
 
@@ -1057,7 +1080,7 @@ int nsem_grad_vol(const NsemDev* m, const NsemTables* t, const double* const* U,
     for (int c = 0; c < 4; c++) ga.fF[c] = const_cast<double*>(fF[c]);
     for (int c = 0; c < 4; c++) ga.gC[c] = gC ? const_cast<double*>(gC[c]) : nullptr;
     const int threads = ((m->np + 31) / 32) * 32;
-    k_seg_grad_vol<<<(unsigned)m->n_elem, threads, smem_grad(m), (cudaStream_t)stream>>>(*m, *t, ga);
+    nsem_launch_chained(k_seg_grad_vol, (unsigned)m->n_elem, threads, smem_grad(m), (cudaStream_t)stream, *m, *t, ga);
     return (int)cudaGetLastError();
 }
 
@@ -1079,9 +1102,9 @@ int nsem_conv_steps(const NsemDev* m, const NsemTables* t, NsemConvBuf* b, int n
         const AdvArgs a = adv_args(b, cur, dt);
         const unsigned mb = (unsigned)((m->n_ms + 127) / 128);
         if (m->n_ms > 0) k_conv_mortar<1><<<4 * mb, 128, 0, st>>>(*m, a);
-        k_conv_face<<<sb, 256, 0, st>>>(*m, a);
+        nsem_launch_chained(k_conv_face, sb, 256, 0, st, *m, a);
         if (m->n_ms > 0) k_conv_mortar_gather<<<mb, 128, 0, st>>>(*m, a);
-        k_conv_vol<<<(unsigned)m->n_elem, threads, smem_conv(m), st>>>(*m, *t, a);
+        nsem_launch_chained(k_conv_vol, (unsigned)m->n_elem, threads, smem_conv(m), st, *m, *t, a);
         const int e = (int)cudaGetLastError();
         if (e) return e;
         cur ^= 1;
@@ -1111,9 +1134,9 @@ int nsem_conv_steps_wind(const NsemDev* m, const NsemTables* t, NsemConvBuf* b, 
         }
         const unsigned mb = (unsigned)((m->n_ms + 127) / 128);
         if (m->n_ms > 0) k_conv_mortar<1><<<4 * mb, 128, 0, st>>>(*m, a);
-        k_conv_face<<<sb, 256, 0, st>>>(*m, a);
+        nsem_launch_chained(k_conv_face, sb, 256, 0, st, *m, a);
         if (m->n_ms > 0) k_conv_mortar_gather<<<mb, 128, 0, st>>>(*m, a);
-        k_conv_vol<<<(unsigned)m->n_elem, threads, smem_conv(m), st>>>(*m, *t, a);
+        nsem_launch_chained(k_conv_vol, (unsigned)m->n_elem, threads, smem_conv(m), st, *m, *t, a);
         const int e = (int)cudaGetLastError();
         if (e) return e;
         b->cur ^= 1;
@@ -1155,7 +1178,7 @@ int nsem_seg_steps(const NsemDev* m, const NsemTables* t, NsemSegBuf* b, int nst
     int cur = b->cur;
     for (int s = 0; s < nsteps; s++) {
         const SegArgs a = seg_args(m, b, cur, dt);
-        k_seg_prep<<<nb, 256, 0, st>>>(*m, a);
+        nsem_launch_chained(k_seg_prep, nb, 256, 0, st, *m, a);
         if (a.visc) {
             GradArgs ga;
             for (int c = 0; c < 3; c++) ga.U[c] = a.U[c];
@@ -1163,21 +1186,21 @@ int nsem_seg_steps(const NsemDev* m, const NsemTables* t, NsemSegBuf* b, int nst
             for (int c = 0; c < 12; c++) ga.G[c] = a.G[c];
             for (int c = 0; c < 4; c++) ga.fF[c] = a.fF[c];
             for (int c = 0; c < 4; c++) ga.gC[c] = a.gC[c];
-            k_seg_grad_face<<<sb, 256, 0, st>>>(*m, ga);
+            nsem_launch_chained(k_seg_grad_face, sb, 256, 0, st, *m, ga);
             if (mort) {
                 k_seg_mortar_gcds<<<mb, 128, 0, st>>>(*m, ga);
                 k_seg_mortar_ggather<<<mb, 128, 0, st>>>(*m, ga);
             }
-            k_seg_grad_vol<<<(unsigned)m->n_elem, threads, smem_grad(m), st>>>(*m, *t, ga);
+            nsem_launch_chained(k_seg_grad_vol, (unsigned)m->n_elem, threads, smem_grad(m), st, *m, *t, ga);
         }
         if (mort) k_seg_mortar_rho<<<6 * mb, 128, 0, st>>>(*m, a);
-        k_seg_face_rho<<<sb, 256, 0, st>>>(*m, a);
+        nsem_launch_chained(k_seg_face_rho, sb, 256, 0, st, *m, a);
         if (mort) k_seg_mortar_gather<0><<<mb, 128, 0, st>>>(*m, a);
-        k_seg_vol_rho<<<(unsigned)m->n_elem, threads, smem_rho(m), st>>>(*m, *t, a);
+        nsem_launch_chained(k_seg_vol_rho, (unsigned)m->n_elem, threads, smem_rho(m), st, *m, *t, a);
         if (mort) k_seg_mortar_ut<<<16 * mb, 128, 0, st>>>(*m, a);
-        k_seg_face_ut<<<sb, 256, 0, st>>>(*m, a);
+        nsem_launch_chained(k_seg_face_ut, sb, 256, 0, st, *m, a);
         if (mort) k_seg_mortar_gather<1><<<4 * mb, 128, 0, st>>>(*m, a);
-        k_seg_vol_ut<<<(unsigned)m->n_elem, threads, smem_ut(m), st>>>(*m, *t, a);
+        nsem_launch_chained(k_seg_vol_ut, (unsigned)m->n_elem, threads, smem_ut(m), st, *m, *t, a);
         const int e = (int)cudaGetLastError();
         if (e) return e;
         cur ^= 1;
