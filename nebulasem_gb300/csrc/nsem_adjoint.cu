@@ -32,6 +32,7 @@
 #include "nsem_seg.h"
 #include "nsem_gather.cuh"
 #include "nsem_mortar.cuh"
+#include "nsem_pdl.cuh"
 
 namespace {
 
@@ -121,11 +122,15 @@ struct FaceAdjArgs {
 __global__ void __launch_bounds__(128) k_adj_face(const NsemDev m, FaceAdjArgs a) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= m.n_slot) return;
-    if (m.n_ms && m.ms_of[k] >= 0) return;   /* non-conforming: k_adj_face_mortar */
+    if (m.n_ms && m.ms_of[k] >= 0) {         /* non-conforming: k_adj_face_mortar */
+        nsem_chain_wait();
+        return;
+    }
     const int32_t c1 = m.c1[k], c2 = m.c2[k];
     const double n[3] = {m.fn[k], m.fn[m.n_slot + k], m.fn[2 * m.n_slot + k]};
     const double en[3] = {m.en[k], m.en[m.n_slot + k], m.en[2 * m.n_slot + k]};
     const double fi = m.fi[k], fo = 1 - fi;
+    nsem_chain_wait();
 
     const NodePrim P1 = node_prim<false>(m, a.S, c1);
     NodePrim P2;
@@ -350,6 +355,7 @@ struct VolAdjArgs {
      * mortar slot the fine side's viscous quantity adjoints */
     const double* qb[19];
     const double* mqv[12];
+    NsemAdjLin lin;          /* inviscid runs: written instead of G when out is set */
 };
 
 /* registers capped for the largest element: 736 threads (N+1 = 9) inviscid,
@@ -367,6 +373,7 @@ __global__ void __maxnreg__(VISC ? 128 : 88) k_adj_volume(const NsemDev m, const
     const int64_t e = blockIdx.x;
     const int64_t node = e * NP + t;
     const bool active = t < NP;
+    nsem_chain_wait();
     if (active) {
         const nsem_divisor dcv = nsem_make_divisor(m.cv[node]);
         for (int v = 0; v < 5; v++) rb[v * NP + t] = -nsem_div_by(a.W[v][node], dcv);
@@ -542,12 +549,21 @@ __global__ void __maxnreg__(VISC ? 128 : 88) k_adj_volume(const NsemDev m, const
     Tb += nsem_div(pg, P.T);
     /* U = m / rho, theta = E / rho */
     const double inv = nsem_div_by(1.0, dr);
-    double g0 = rbar - inv * vdot3(Ub, P.U) - inv * Tb * P.T;
-    a.G[0][node] = g0;
-    a.G[1][node] = Ub[0] * inv;
-    a.G[2][node] = Ub[1] * inv;
-    a.G[3][node] = Ub[2] * inv;
-    a.G[4][node] = Tb * inv;
+    const double g[5] = {rbar - inv * vdot3(Ub, P.U) - inv * Tb * P.T, Ub[0] * inv, Ub[1] * inv,
+                         Ub[2] * inv, Tb * inv};
+    if constexpr (!VISC) {
+        if (a.lin.out[0]) {
+            /* the reverse step's combination, without a pass of its own */
+            for (int v = 0; v < 5; v++) {
+                double x = a.lin.cx * a.lin.x[v][node];
+                if (a.lin.y[0]) x += a.lin.cy * a.lin.y[v][node];
+                if (a.lin.z[0]) x += a.lin.cz * a.lin.z[v][node];
+                a.lin.out[v][node] = x + a.lin.cg * g[v];
+            }
+            return;
+        }
+    }
+    for (int v = 0; v < 5; v++) a.G[v][node] = g[v];
 }
 
 /* ------------------------------------------------------------------------
@@ -1360,13 +1376,14 @@ __global__ void k_adj_grad_vol(const NsemDev m, const NsemTables tab, GradAdjArg
     a.G[4][node] += pb[3] * inv;
 }
 
-/* lam = c0 * lam + c1 * x + c2 * y (elementwise over 5 arrays) */
+/* out = cx x + cy y + cz z + cw w (elementwise over 5 arrays; y, z, w may be null) */
 struct Lin3Args {
     double* out[5];
     const double* x[5];
     const double* y[5];
     const double* z[5];
-    double cx, cy, cz;
+    const double* w[5];
+    double cx, cy, cz, cw;
     int64_t n;
 };
 
@@ -1377,6 +1394,7 @@ __global__ void k_lin3(Lin3Args a) {
             double s = a.cx * a.x[v][i];
             if (a.y[0]) s += a.cy * a.y[v][i];
             if (a.z[0]) s += a.cz * a.z[v][i];
+            if (a.w[0]) s += a.cw * a.w[v][i];
             a.out[v][i] = s;
         }
 }
@@ -1389,8 +1407,10 @@ int grid_for(int64_t n) {
 
 }  // namespace
 
-int nsem_adj_vjp(const NsemDev* m, const NsemTables* t, const double* const* S,
-                 const double* const* W, double* const* G, NsemAdjBuf* ab, void* stream) {
+/* the product into G, or (lin) its combination */
+static int adj_vjp(const NsemDev* m, const NsemTables* t, const double* const* S,
+                   const double* const* W, double* const* G, const NsemAdjLin* lin, NsemAdjBuf* ab,
+                   void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     FaceAdjArgs fa{};
     VolAdjArgs va{};
@@ -1411,7 +1431,7 @@ int nsem_adj_vjp(const NsemDev* m, const NsemTables* t, const double* const* S,
     for (int v = 0; v < 5; v++) { fa.S[v] = S[v]; fa.W[v] = W[v]; }
     for (int v = 0; v < NPA; v++) { fa.adjO[v] = ab->adjO[v]; fa.adjN[v] = ab->adjN[v]; }
     const int64_t fb = (m->n_slot + 127) / 128;
-    k_adj_face<<<(unsigned)fb, 128, 0, st>>>(*m, fa);
+    nsem_launch_chained(k_adj_face, (unsigned)fb, 128, 0, st, *m, fa);
     for (int c = 0; c < 19; c++) va.qb[c] = nullptr;
     if (m->n_ms > 0) {
         MortarArgs ma{};
@@ -1434,8 +1454,10 @@ int nsem_adj_vjp(const NsemDev* m, const NsemTables* t, const double* const* S,
     for (int v = 0; v < NPA; v++) { va.adjO[v] = ab->adjO[v]; va.adjN[v] = ab->adjN[v]; }
     const int threads = ((m->np + 31) / 32) * 32;
     const size_t smem = (5 * (size_t)m->np + 3 * NSEM_MAX_NPD * NSEM_MAX_NPD) * sizeof(double);
-    if (ab->visc) k_adj_volume<true><<<(unsigned)m->n_elem, threads, smem, st>>>(*m, *t, va);
-    else k_adj_volume<false><<<(unsigned)m->n_elem, threads, smem, st>>>(*m, *t, va);
+    if (lin && !ab->visc) va.lin = *lin;
+    const unsigned grid = (unsigned)m->n_elem;
+    if (ab->visc) nsem_launch_chained(k_adj_volume<true>, grid, (unsigned)threads, smem, st, *m, *t, va);
+    else nsem_launch_chained(k_adj_volume<false>, grid, (unsigned)threads, smem, st, *m, *t, va);
     if (ab->visc) {
         /* the gradients' transpose, added to the conserved adjoint */
         GradAdjArgs ga{};
@@ -1456,8 +1478,31 @@ int nsem_adj_vjp(const NsemDev* m, const NsemTables* t, const double* const* S,
         }
         const size_t gsm = ((size_t)m->np * GADJ_W + 3 * NSEM_MAX_NPD * NSEM_MAX_NPD) * sizeof(double);
         k_adj_grad_vol<<<(unsigned)m->n_elem, threads, gsm, st>>>(*m, *t, ga);
+        if (lin) {
+            Lin3Args la{};
+            for (int v = 0; v < 5; v++) {
+                la.out[v] = lin->out[v];
+                la.x[v] = lin->x[v];
+                la.y[v] = lin->y[v];
+                la.z[v] = lin->z[v];
+                la.w[v] = G[v];
+            }
+            la.cx = lin->cx; la.cy = lin->cy; la.cz = lin->cz; la.cw = lin->cg;
+            la.n = m->n_int;
+            k_lin3<<<grid_for(la.n), 256, 0, st>>>(la);
+        }
     }
     return (int)cudaGetLastError();
+}
+
+int nsem_adj_vjp(const NsemDev* m, const NsemTables* t, const double* const* S,
+                 const double* const* W, double* const* G, NsemAdjBuf* ab, void* stream) {
+    return adj_vjp(m, t, S, W, G, nullptr, ab, stream);
+}
+
+int nsem_adj_vjp_lin(const NsemDev* m, const NsemTables* t, const double* const* S,
+                     const double* const* W, const NsemAdjLin& lin, NsemAdjBuf* ab, void* stream) {
+    return adj_vjp(m, t, S, W, ab->g, &lin, ab, stream);
 }
 
 int nsem_adj_jvp(const NsemDev* m, const NsemTables* t, const double* const* S,
@@ -1516,7 +1561,7 @@ int nsem_adj_jvp(const NsemDev* m, const NsemTables* t, const double* const* S,
 
 int nsem_adj_lin3(double* const* out, const double* const* x, double cx, const double* const* y,
                   double cy, const double* const* z, double cz, int64_t n, void* stream) {
-    Lin3Args a;
+    Lin3Args a{};
     for (int v = 0; v < 5; v++) {
         a.out[v] = out[v];
         a.x[v] = x[v];

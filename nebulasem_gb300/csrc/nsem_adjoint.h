@@ -12,7 +12,6 @@ struct NsemAdjBuf {
     double* adjO[6] = {};   /* per slot: owner-side primitive adjoints   */
     double* adjN[6] = {};   /* per slot: neighbour-side primitive adjoints */
     double* lam[5] = {};    /* adjoint of the current step state          */
-    double* a3[5] = {};
     double* lu2[5] = {};
     double* lu1[5] = {};
     double* g[5] = {};      /* VJP output                                 */
@@ -20,6 +19,8 @@ struct NsemAdjBuf {
     double* ckpt = nullptr; /* [n_ckpt][5][n_int] states every k steps     */
     double* seg = nullptr;  /* [k][3][5][n_int] u^n, u1, u2 of a segment   */
     int64_t seg_slots = 0;  /* state slots allocated in seg                 */
+    int64_t ckpt_slots = 0; /* states allocated in ckpt                     */
+    int seg_of = -1;        /* the segment whose stage states seg holds (-1: none) */
     /* artificial viscosity (nu != 0): per node U, theta of the state and their
      * tangents / adjoints, gradients (9 + 3) and their tangents / adjoints;
      * per slot cds(U, theta) and its tangent, face adjoints */
@@ -64,10 +65,22 @@ struct NsemAdjBuf {
 /* g = J_L(S)^T W (all device pointers, 5 SoA arrays each) */
 int nsem_adj_vjp(const NsemDev* m, const NsemTables* t, const double* const* S,
                  const double* const* W, double* const* G, NsemAdjBuf* ab, void* stream);
+/* out = cx x + cy y + cz z + cg J_L(S)^T W (y, z may be null; out may be any of
+ * them: every node's operands are read by the thread that then writes it, and
+ * its element's W before that) */
+struct NsemAdjLin {
+    double* out[5] = {};
+    const double* x[5] = {};
+    const double* y[5] = {};
+    const double* z[5] = {};
+    double cx = 0, cy = 0, cz = 0, cg = 0;
+};
+int nsem_adj_vjp_lin(const NsemDev* m, const NsemTables* t, const double* const* S,
+                     const double* const* W, const NsemAdjLin& lin, NsemAdjBuf* ab, void* stream);
 /* out = J_L(S) dS (tangent-linear product; uses ab->adjO[0..4] as slot scratch) */
 int nsem_adj_jvp(const NsemDev* m, const NsemTables* t, const double* const* S,
                  const double* const* dS, double* const* out, NsemAdjBuf* ab, void* stream);
-/* out = cx x + cy y + cz z (y, z may be null) */
+/* out = cx x + cy y + cz z (y, z may be null), for the tangent-linear sweep */
 int nsem_adj_lin3(double* const* out, const double* const* x, double cx, const double* const* y,
                   double cy, const double* const* z, double cz, int64_t n, void* stream);
 int nsem_adj_prepare(const NsemDev* m);

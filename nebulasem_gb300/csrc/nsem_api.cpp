@@ -460,9 +460,9 @@ nsem_status materialise_conserved(nsem_ctx* ctx) {
     return ensure_rep(ctx, 0);
 }
 
-/* the FP64 face kernel of a stage, after the gradients of its state when the
- * run is viscous */
-int fp64_face(nsem_ctx* ctx, int from_state) {
+/* the FP64 face kernel of the state with density rho (and the primitives in
+ * buf.prim), after the gradients of that state when the run is viscous */
+int fp64_face(nsem_ctx* ctx, const double* rho) {
     NsemBuf* b = &ctx->buf;
     if (b->G[0]) {
         const double* U[3] = {b->prim[0], b->prim[1], b->prim[2]};
@@ -470,7 +470,33 @@ int fp64_face(nsem_ctx* ctx, int from_state) {
                                           ctx->dev.n_ms > 0 ? b->gC : nullptr, ctx->stream);
         if (e) return e;
     }
-    return nsem_fp64_face(&ctx->dev, b, from_state, ctx->stream);
+    return nsem_fp64_face(&ctx->dev, b, rho, ctx->stream);
+}
+
+/* stage 1..3 of an FP64 step from u^n = U0: stage state S (its primitives in
+ * buf.prim) -> out, whose primitives are left there */
+nsem_status fp64_stage(nsem_ctx* ctx, int stage, const double* const* S, const double* const* U0,
+                       double* const* out) {
+    int e = fp64_face(ctx, S[0]);
+    if (e) return cuda_fail(ctx, (cudaError_t)e, "face");
+    e = nsem_fp64_volume(&ctx->dev, &ctx->tab, &ctx->buf, stage, ctx->dt, S, U0, out, ctx->stream);
+    return e ? cuda_fail(ctx, (cudaError_t)e, "volume") : NSEM_OK;
+}
+
+/* one FP64 step U0 -> out with the stage states in u1 and u2 (which may be one
+ * set of arrays; out may be U0); out null: stages 1 and 2 only.  The
+ * primitives of U0 are in buf.prim, and those of the last state written after. */
+nsem_status fp64_step(nsem_ctx* ctx, double* const* U0, double* const* u1, double* const* u2,
+                      double* const* out) {
+    nsem_status s = fp64_stage(ctx, 1, U0, U0, u1);
+    if (s == NSEM_OK) s = fp64_stage(ctx, 2, u1, U0, u2);
+    if (s == NSEM_OK && out) s = fp64_stage(ctx, 3, u2, U0, out);
+    return s;
+}
+
+nsem_status fp64_prims(nsem_ctx* ctx, const double* const* S) {
+    const int e = nsem_fp64_prim(&ctx->dev, &ctx->buf, S, (void*)ctx->stream);
+    return e ? cuda_fail(ctx, (cudaError_t)e, "prim") : NSEM_OK;
 }
 
 /* launches of one nsem_step call (captured into a graph) */
@@ -480,15 +506,9 @@ nsem_status enqueue_steps(nsem_ctx* ctx, int nsteps, nsem_precision prec) {
     void* st = (void*)ctx->stream;
     int e;
     if (prec == NSEM_FP64) {
-        if ((e = nsem_fp64_prim(D, b, 1, st))) return cuda_fail(ctx, (cudaError_t)e, "prim");
-        for (int n = 0; n < nsteps; n++) {
-            for (int stage = 1; stage <= 3; stage++) {
-                if ((e = fp64_face(ctx, stage == 1)))
-                    return cuda_fail(ctx, (cudaError_t)e, "face");
-                if ((e = nsem_fp64_volume(D, &ctx->tab, b, stage, ctx->dt, st)))
-                    return cuda_fail(ctx, (cudaError_t)e, "volume");
-            }
-        }
+        nsem_status s = fp64_prims(ctx, b->u);
+        for (int n = 0; n < nsteps && s == NSEM_OK; n++) s = fp64_step(ctx, b->u, b->s, b->s, b->u);
+        if (s != NSEM_OK) return s;
     } else {
         if (!ctx->mixed_ready) return fail(ctx, NSEM_UNSUPPORTED, ctx->err);
         if ((e = nsem_mixed_steps(D, &ctx->mbuf, b, &ctx->tab, nsteps, ctx->dt, st)))
@@ -644,8 +664,7 @@ nsem_status nsem_get_pressure(nsem_ctx* ctx, double* p_prime) {
     }
     nsem_status rs = materialise_conserved(ctx);
     if (rs != NSEM_OK) return rs;
-    const int e = nsem_fp64_prim(&ctx->dev, &ctx->buf, 1, (void*)ctx->stream);
-    if (e) return cuda_fail(ctx, (cudaError_t)e, "prim");
+    if ((rs = fp64_prims(ctx, ctx->buf.u)) != NSEM_OK) return rs;
     NSEM_CUDA(cudaMemcpyAsync(p_prime, ctx->buf.prim[4], n * 8, cudaMemcpyDeviceToHost, ctx->stream));
     return check_status(ctx);
 }
@@ -689,10 +708,8 @@ nsem_status nsem_tendency(nsem_ctx* ctx, nsem_precision prec, double* const L[5]
     nsem_status rs = (prec == NSEM_MIXED) ? ensure_rep(ctx, 1) : materialise_conserved(ctx);
     if (rs != NSEM_OK) return rs;
     if (prec == NSEM_FP64) {
-        if ((e = nsem_fp64_prim(D, b, 1, st))) return cuda_fail(ctx, (cudaError_t)e, "prim");
-        if ((e = fp64_face(ctx, 1))) return cuda_fail(ctx, (cudaError_t)e, "face");
-        if ((e = nsem_fp64_volume(D, &ctx->tab, b, 0, ctx->dt, st)))
-            return cuda_fail(ctx, (cudaError_t)e, "volume");
+        if ((rs = fp64_prims(ctx, b->u)) != NSEM_OK) return rs;
+        if ((rs = fp64_stage(ctx, 0, b->u, b->u, b->L)) != NSEM_OK) return rs;
     } else if (prec == NSEM_MIXED) {
         if (!ctx->mixed_ready) return fail(ctx, NSEM_UNSUPPORTED, ctx->err);
         if ((e = nsem_mixed_tendency(D, &ctx->mbuf, b, &ctx->tab, st)))
@@ -786,7 +803,6 @@ static nsem_status adj_alloc(nsem_ctx* ctx) {
     for (int v = 0; v < 5; v++) {
         const size_t n = (size_t)ctx->dev.n_int;
         if ((s = dalloc(ctx, &A.lam[v], n)) != NSEM_OK) return s;
-        if ((s = dalloc(ctx, &A.a3[v], n)) != NSEM_OK) return s;
         if ((s = dalloc(ctx, &A.lu2[v], n)) != NSEM_OK) return s;
         if ((s = dalloc(ctx, &A.lu1[v], n)) != NSEM_OK) return s;
         if ((s = dalloc(ctx, &A.g[v], n)) != NSEM_OK) return s;
@@ -843,23 +859,33 @@ static void slots(double* block, int64_t j, int64_t n, double* out[5]) {
     for (int v = 0; v < 5; v++) out[v] = block + (j * 5 + v) * n;
 }
 
-/* one FP64 step; optionally keeps the two stage states */
-static nsem_status fp64_step(nsem_ctx* ctx, double* const* keep1, double* const* keep2) {
-    NsemDev* D = &ctx->dev;
-    NsemBuf* b = &ctx->buf;
-    void* st = (void*)ctx->stream;
-    int e;
-    if ((e = nsem_fp64_prim(D, b, 1, st))) return cuda_fail(ctx, (cudaError_t)e, "prim");
-    for (int stage = 1; stage <= 3; stage++) {
-        if ((e = fp64_face(ctx, stage == 1))) return cuda_fail(ctx, (cudaError_t)e, "face");
-        if ((e = nsem_fp64_volume(D, &ctx->tab, b, stage, ctx->dt, st)))
-            return cuda_fail(ctx, (cudaError_t)e, "volume");
-        nsem_status s = NSEM_OK;
-        if (stage == 1 && keep1) s = copy_state(ctx, keep1, b->s);
-        if (stage == 2 && keep2) s = copy_state(ctx, keep2, b->s);
-        if (s != NSEM_OK) return s;
+/* at least count state slots in *block (kept from call to call) */
+static nsem_status grow_states(nsem_ctx* ctx, double** block, int64_t* have, int64_t count) {
+    if (*block) cudaFree(*block);
+    *block = nullptr;
+    *have = 0;
+    if (cudaMalloc((void**)block, (size_t)count * 5 * ctx->dev.n_int * sizeof(double)) != cudaSuccess) {
+        *block = nullptr;
+        cudaGetLastError();   /* reported here, not by the next launch check */
+        return fail(ctx, NSEM_NO_MEMORY, "state storage allocation failed");
     }
+    *have = count;
     return NSEM_OK;
+}
+
+/* step j of segment sg: from its checkpoint (j = 0) or the state the step
+ * before left in the segment's storage; u1 and u2 into that storage, u^{n+1}
+ * into it too when another step follows, else into out (null: not formed) */
+static nsem_status segment_step(nsem_ctx* ctx, int sg, int j, bool more, double* const* out) {
+    NsemAdjBuf& A = ctx->abuf;
+    const int64_t n = ctx->dev.n_int;
+    double *u0[5], *u1[5], *u2[5], *next[5];
+    if (j == 0) slots(A.ckpt, sg, n, u0);
+    else slots(A.seg, 3 * j, n, u0);
+    slots(A.seg, 3 * j + 1, n, u1);
+    slots(A.seg, 3 * j + 2, n, u2);
+    slots(A.seg, 3 * (j + 1), n, next);
+    return fp64_step(ctx, u0, u1, u2, more ? next : out);
 }
 
 extern "C" nsem_status nsem_vjp(nsem_ctx* ctx, const double* const w[5], double* const g[5]) {
@@ -916,13 +942,9 @@ extern "C" nsem_status nsem_tlm(nsem_ctx* ctx, int nsteps, const double* const d
     NsemAdjBuf& A = ctx->abuf;
     const int64_t n = ctx->dev.n_int;
     const size_t bytes = (size_t)n * sizeof(double);
-    /* stage states of one step: u^n, u1, u2 */
-    if (!A.seg || A.seg_slots < 3) {
-        if (A.seg) { cudaFree(A.seg); A.seg = nullptr; }
-        if (cudaMalloc((void**)&A.seg, (size_t)3 * 5 * n * sizeof(double)) != cudaSuccess)
-            return fail(ctx, NSEM_NO_MEMORY, "stage-state allocation failed");
-        A.seg_slots = 3;
-    }
+    /* stage states of one step: u1, u2 */
+    A.seg_of = -1;
+    if (A.seg_slots < 2 && (s = grow_states(ctx, &A.seg, &A.seg_slots, 2)) != NSEM_OK) return s;
     for (int v = 0; v < 5; v++)
         NSEM_CUDA(cudaMemcpyAsync(A.lam[v], du0[v], bytes, cudaMemcpyHostToDevice, ctx->stream));
     const double dt = ctx->dt;
@@ -932,13 +954,12 @@ extern "C" nsem_status nsem_tlm(nsem_ctx* ctx, int nsteps, const double* const d
     NSEM_CUDA(cudaEventCreate(&e1));
     NSEM_CUDA(cudaEventRecord(e0, ctx->stream));
     int e = 0;
-    double *u0[5], *u1[5], *u2[5];
-    slots(A.seg, 0, n, u0);
-    slots(A.seg, 1, n, u1);
-    slots(A.seg, 2, n, u2);
+    double *const *u0 = ctx->buf.u, *u1[5], *u2[5];
+    slots(A.seg, 0, n, u1);
+    slots(A.seg, 1, n, u2);
+    s = fp64_prims(ctx, u0);
     for (int step = 0; step < nsteps && s == NSEM_OK && !e; step++) {
-        if ((s = copy_state(ctx, u0, ctx->buf.u)) != NSEM_OK) break;
-        if ((s = fp64_step(ctx, u1, u2)) != NSEM_OK) break;
+        if ((s = fp64_step(ctx, u0, u1, u2, nullptr)) != NSEM_OK) break;
         /* du1 = du + dt J(u^n) du */
         if ((e = nsem_adj_jvp(&ctx->dev, &ctx->tab, u0, A.lam, A.g, &A, st))) break;
         if ((e = nsem_adj_lin3(A.lu1, A.lam, 1.0, A.g, dt, nullptr, 0, n, st))) break;
@@ -948,6 +969,8 @@ extern "C" nsem_status nsem_tlm(nsem_ctx* ctx, int nsteps, const double* const d
         /* du^{n+1} = 1/3 du + 2/3 (du2 + dt J(u2) du2) */
         if ((e = nsem_adj_jvp(&ctx->dev, &ctx->tab, u2, A.lu2, A.g, &A, st))) break;
         if ((e = nsem_adj_lin3(A.lam, A.lam, 1.0 / 3.0, A.lu2, 2.0 / 3.0, A.g, 2.0 / 3.0 * dt, n, st))) break;
+        /* u^{n+1}, in place */
+        s = fp64_stage(ctx, 3, u2, u0, ctx->buf.u);
     }
     if (e) s = cuda_fail(ctx, (cudaError_t)e, "tangent-linear sweep");
     if (s != NSEM_OK) {
@@ -980,25 +1003,38 @@ extern "C" nsem_status nsem_forward_checkpointed(nsem_ctx* ctx, int nsteps, int 
     NsemAdjBuf& A = ctx->abuf;
     const int64_t n = ctx->dev.n_int;
     const int n_ckpt = (nsteps + ckpt_every - 1) / ckpt_every;
-    if (A.ckpt) { cudaFree(A.ckpt); A.ckpt = nullptr; }
-    if (A.seg) { cudaFree(A.seg); A.seg = nullptr; }
-    cudaError_t ce = cudaMalloc((void**)&A.ckpt, (size_t)n_ckpt * 5 * n * sizeof(double));
-    if (ce != cudaSuccess) return fail(ctx, NSEM_NO_MEMORY, "checkpoint allocation failed");
-    ce = cudaMalloc((void**)&A.seg, (size_t)ckpt_every * 3 * 5 * n * sizeof(double));
-    if (ce != cudaSuccess) return fail(ctx, NSEM_NO_MEMORY, "segment allocation failed");
-    A.seg_slots = 3 * (int64_t)ckpt_every;
+    A.nsteps = 0;   /* no run to differentiate until this one has ended */
+    A.seg_of = -1;
+    const int64_t n_seg = 3 * (int64_t)ckpt_every;
+    s = A.ckpt_slots < n_ckpt ? grow_states(ctx, &A.ckpt, &A.ckpt_slots, n_ckpt) : NSEM_OK;
+    if (s == NSEM_OK && A.seg_slots < n_seg) s = grow_states(ctx, &A.seg, &A.seg_slots, n_seg);
+    if (s != NSEM_OK) {
+        /* an earlier run's larger block may be what is in the way */
+        if (A.ckpt) cudaFree(A.ckpt);
+        if (A.seg) cudaFree(A.seg);
+        A.ckpt = A.seg = nullptr;
+        A.ckpt_slots = A.seg_slots = 0;
+        if ((s = grow_states(ctx, &A.ckpt, &A.ckpt_slots, n_ckpt)) != NSEM_OK) return s;
+        if ((s = grow_states(ctx, &A.seg, &A.seg_slots, n_seg)) != NSEM_OK) return s;
+    }
     cudaEvent_t e0, e1;
     NSEM_CUDA(cudaEventCreate(&e0));
     NSEM_CUDA(cudaEventCreate(&e1));
     NSEM_CUDA(cudaEventRecord(e0, ctx->stream));
-    for (int st = 0; st < nsteps; st++) {
+    s = fp64_prims(ctx, ctx->buf.u);
+    /* the last segment's steps write u^n, u1, u2 where the reverse sweep starts
+     * reading: it need not recompute that segment */
+    const int last = (n_ckpt - 1) * ckpt_every;
+    for (int st = 0; st < nsteps && s == NSEM_OK; st++) {
+        double* c[5];
         if (st % ckpt_every == 0) {
-            double* c[5];
             slots(A.ckpt, st / ckpt_every, n, c);
             if ((s = copy_state(ctx, c, ctx->buf.u)) != NSEM_OK) return s;
         }
-        if ((s = fp64_step(ctx, nullptr, nullptr)) != NSEM_OK) return s;
+        if (st < last) s = fp64_step(ctx, ctx->buf.u, ctx->buf.s, ctx->buf.s, ctx->buf.u);
+        else s = segment_step(ctx, n_ckpt - 1, st - last, st + 1 < nsteps, ctx->buf.u);
     }
+    if (s != NSEM_OK) return s;
     NSEM_CUDA(cudaEventRecord(e1, ctx->stream));
     if ((s = copy_state(ctx, A.fin, ctx->buf.u)) != NSEM_OK) return s;
     NSEM_CUDA(cudaMemcpyAsync(ctx->h_status, ctx->dev.status, sizeof(uint32_t),
@@ -1013,6 +1049,7 @@ extern "C" nsem_status nsem_forward_checkpointed(nsem_ctx* ctx, int nsteps, int 
     A.nsteps = nsteps;
     A.every = ckpt_every;
     A.n_ckpt = n_ckpt;
+    A.seg_of = n_ckpt - 1;
     ctx->adj_form = 0;
     return NSEM_OK;
 }
@@ -1127,6 +1164,21 @@ static nsem_status mixed_adjoint(nsem_ctx* ctx, const double* const lam_final[5]
     return NSEM_OK;
 }
 
+/* out = cx x + cy y + cz z + cg J_L(S)^T W */
+static int reverse_stage(nsem_ctx* ctx, double* const* S, double* const* W, double* const* out,
+                         double* const* x, double cx, double* const* y, double cy, double* const* z,
+                         double cz, double cg) {
+    NsemAdjLin l;
+    for (int v = 0; v < 5; v++) {
+        l.out[v] = out[v];
+        l.x[v] = x[v];
+        l.y[v] = y ? y[v] : nullptr;
+        l.z[v] = z ? z[v] : nullptr;
+    }
+    l.cx = cx; l.cy = cy; l.cz = cz; l.cg = cg;
+    return nsem_adj_vjp_lin(&ctx->dev, &ctx->tab, S, W, l, &ctx->abuf, ctx->stream);
+}
+
 extern "C" nsem_status nsem_adjoint(nsem_ctx* ctx, const double* const lam_final[5],
                                     double* const lam0[5], double* ms_adj) {
     if (!ctx) return NSEM_BAD_ARG;
@@ -1158,32 +1210,30 @@ extern "C" nsem_status nsem_adjoint(nsem_ctx* ctx, const double* const lam_final
         const int cnt = (A.nsteps - start < A.every) ? A.nsteps - start : A.every;
         double* c[5];
         slots(A.ckpt, sg, n, c);
-        if ((s = copy_state(ctx, ctx->buf.u, c)) != NSEM_OK) break;
-        for (int j = 0; j < cnt && s == NSEM_OK; j++) {
-            double *u0[5], *u1[5], *u2[5];
-            slots(A.seg, 3 * j, n, u0);
-            slots(A.seg, 3 * j + 1, n, u1);
-            slots(A.seg, 3 * j + 2, n, u2);
-            if ((s = copy_state(ctx, u0, ctx->buf.u)) != NSEM_OK) break;
-            s = fp64_step(ctx, u1, u2);
+        if (A.seg_of != sg) {
+            /* recompute the segment's stage states; its last step's result is
+             * not needed */
+            A.seg_of = -1;
+            if ((s = fp64_prims(ctx, c)) != NSEM_OK) break;
+            for (int j = 0; j < cnt && s == NSEM_OK; j++) s = segment_step(ctx, sg, j, j + 1 < cnt, nullptr);
+            if (s != NSEM_OK) break;
+            A.seg_of = sg;
         }
-        if (s != NSEM_OK) break;
         for (int j = cnt - 1; j >= 0; j--) {
             double *u0[5], *u1[5], *u2[5];
-            slots(A.seg, 3 * j, n, u0);
+            if (j == 0) slots(A.ckpt, sg, n, u0);
+            else slots(A.seg, 3 * j, n, u0);
             slots(A.seg, 3 * j + 1, n, u1);
             slots(A.seg, 3 * j + 2, n, u2);
             /* u3 = u/3 + 2/3 (u2 + dt L(u2)) */
-            if ((s = copy_state(ctx, A.a3, A.lam)) != NSEM_OK) break;
-            if ((e = nsem_adj_vjp(&ctx->dev, &ctx->tab, u2, A.a3, A.g, &A, st))) break;
-            if ((e = nsem_adj_lin3(A.lu2, A.a3, 2.0 / 3.0, A.g, 2.0 / 3.0 * dt, nullptr, 0, n, st))) break;
+            if ((e = reverse_stage(ctx, u2, A.lam, A.lu2, A.lam, 2.0 / 3.0, nullptr, 0, nullptr, 0,
+                                   2.0 / 3.0 * dt))) break;
             /* u2 = 3/4 u + 1/4 (u1 + dt L(u1)) */
-            if ((e = nsem_adj_vjp(&ctx->dev, &ctx->tab, u1, A.lu2, A.g, &A, st))) break;
-            if ((e = nsem_adj_lin3(A.lu1, A.lu2, 0.25, A.g, 0.25 * dt, nullptr, 0, n, st))) break;
+            if ((e = reverse_stage(ctx, u1, A.lu2, A.lu1, A.lu2, 0.25, nullptr, 0, nullptr, 0,
+                                   0.25 * dt))) break;
             /* u1 = u + dt L(u) */
-            if ((e = nsem_adj_vjp(&ctx->dev, &ctx->tab, u0, A.lu1, A.g, &A, st))) break;
-            if ((e = nsem_adj_lin3(A.lam, A.a3, 1.0 / 3.0, A.lu2, 0.75, A.lu1, 1.0, n, st))) break;
-            if ((e = nsem_adj_lin3(A.lam, A.lam, 1.0, A.g, dt, nullptr, 0, n, st))) break;
+            if ((e = reverse_stage(ctx, u0, A.lu1, A.lam, A.lam, 1.0 / 3.0, A.lu2, 0.75, A.lu1, 1.0, dt)))
+                break;
         }
     }
     if (e) s = cuda_fail(ctx, (cudaError_t)e, "adjoint sweep");
@@ -1372,12 +1422,16 @@ nsem_status nsem_profile(nsem_ctx* ctx, int nsteps, nsem_precision prec, double 
         std::strncpy(names + 0 * 32, "fp64_prim", 31);
         std::strncpy(names + 1 * 32, "fp64_face", 31);
         std::strncpy(names + 2 * 32, "fp64_volume", 31);
-        s = timed(0, [&] { return nsem_fp64_prim(D, b, 1, st); });
+        s = timed(0, [&] { return nsem_fp64_prim(D, b, b->u, st); });
         for (int n = 0; n < nsteps && s == NSEM_OK; n++)
             for (int stage = 1; stage <= 3 && s == NSEM_OK; stage++) {
-                s = timed(1, [&] { return fp64_face(ctx, stage == 1); });
+                double* const* S = stage == 1 ? b->u : b->s;
+                s = timed(1, [&] { return fp64_face(ctx, S[0]); });
                 if (s == NSEM_OK)
-                    s = timed(2, [&] { return nsem_fp64_volume(D, &ctx->tab, b, stage, ctx->dt, st); });
+                    s = timed(2, [&] {
+                        return nsem_fp64_volume(D, &ctx->tab, b, stage, ctx->dt, S, b->u,
+                                                stage == 3 ? b->u : b->s, st);
+                    });
             }
     } else if (prec == NSEM_MIXED) {
         if (!ctx->mixed_ready) return fail(ctx, NSEM_UNSUPPORTED, ctx->err);

@@ -83,15 +83,16 @@ struct PrimArgs {
     double* prim[NSEM_NPRIM];
 };
 
-__device__ __forceinline__ void prim_at(const NsemDev& m, const double* const* S,
-                                        double* const* prim, int64_t i) {
-    const double r = S[0][i];
+/* primitives of the state S at node i */
+__device__ __forceinline__ void prim_at(const NsemDev& m, const double* S, double* const* prim,
+                                        int64_t i) {
+    const double r = S[0];
     const nsem_divisor dr = nsem_make_divisor(r);
     double U[3];
-    U[0] = nsem_div_by(S[1][i], dr);
-    U[1] = nsem_div_by(S[2][i], dr);
-    U[2] = nsem_div_by(S[3][i], dr);
-    const double T = nsem_div_by(S[4][i], dr);
+    U[0] = nsem_div_by(S[1], dr);
+    U[1] = nsem_div_by(S[2], dr);
+    U[2] = nsem_div_by(S[3], dr);
+    const double T = nsem_div_by(S[4], dr);
     const double p = m.P0 * nsem_pow(nsem_div_by((r * T) * m.R, m.dP0), m.gamma);
     prim[0][i] = U[0];
     prim[1][i] = U[1];
@@ -107,7 +108,9 @@ __global__ void __launch_bounds__(256) k_prim(const NsemDev m, PrimArgs a) {
     nsem_chain_wait();
     nsem_chain_begin();
     if (i >= m.n_int) return;
-    prim_at(m, a.S, a.prim, i);
+    double S[5];
+    for (int c = 0; c < 5; c++) S[c] = a.S[c][i];
+    prim_at(m, S, a.prim, i);
 }
 
 struct FaceArgs {
@@ -464,25 +467,24 @@ __global__ void k_volume(const NsemDev m, const NsemTables tab, VolArgs a) {
     }
     if (!finite) atomicOr(m.status, NSEM_STATUS_NONFINITE);
     /* primitives of the new stage state for the next face kernel */
-    const double* const outc[5] = {a.out[0], a.out[1], a.out[2], a.out[3], a.out[4]};
-    prim_at(m, outc, a.prim, node);
+    prim_at(m, nu, a.prim, node);
 }
 
 inline int launch_err() { return (int)cudaGetLastError(); }
 
 }  // namespace
 
-extern "C" int nsem_fp64_prim(const NsemDev* m, NsemBuf* b, int from_state, void* stream) {
+extern "C" int nsem_fp64_prim(const NsemDev* m, NsemBuf* b, const double* const* S, void* stream) {
     PrimArgs a;
-    for (int c = 0; c < 5; c++) a.S[c] = from_state ? b->u[c] : b->s[c];
+    for (int c = 0; c < 5; c++) a.S[c] = S[c];
     for (int c = 0; c < NSEM_NPRIM; c++) a.prim[c] = b->prim[c];
     const int64_t blocks = (m->n_int + 255) / 256;
     return nsem_launch_chained(k_prim, (unsigned)blocks, 256, 0, (cudaStream_t)stream, *m, a);
 }
 
-extern "C" int nsem_fp64_face(const NsemDev* m, NsemBuf* b, int from_state, void* stream) {
+extern "C" int nsem_fp64_face(const NsemDev* m, NsemBuf* b, const double* rho, void* stream) {
     FaceArgs a;
-    a.S0 = from_state ? b->u[0] : b->s[0];
+    a.S0 = rho;
     for (int c = 0; c < NSEM_NPRIM; c++) a.prim[c] = b->prim[c];
     for (int c = 0; c < 5; c++) a.d[c] = b->d[c];
     for (int c = 0; c < 12; c++) a.G[c] = b->G[c];
@@ -522,17 +524,16 @@ extern "C" int nsem_fp64_check_smem(const NsemDev* m) {
 }
 
 extern "C" int nsem_fp64_volume(const NsemDev* m, const NsemTables* t, NsemBuf* b, int stage,
-                                double dt, void* stream) {
+                                double dt, const double* const* S, const double* const* U0,
+                                double* const* out, void* stream) {
     VolArgs a;
     a.stage = stage;
     a.dt = dt;
     for (int c = 0; c < 5; c++) {
         a.d[c] = b->d[c];
-        a.U0[c] = b->u[c];
-        if (stage == 0) { a.S[c] = b->u[c]; a.out[c] = b->L[c]; }
-        else if (stage == 1) { a.S[c] = b->u[c]; a.out[c] = b->s[c]; }
-        else if (stage == 2) { a.S[c] = b->s[c]; a.out[c] = b->s[c]; }
-        else { a.S[c] = b->s[c]; a.out[c] = b->u[c]; }
+        a.S[c] = S[c];
+        a.U0[c] = U0[c];
+        a.out[c] = out[c];
     }
     for (int c = 0; c < NSEM_NPRIM; c++) a.prim[c] = b->prim[c];
     for (int c = 0; c < 12; c++) a.G[c] = b->G[c];

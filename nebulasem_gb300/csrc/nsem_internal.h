@@ -91,12 +91,16 @@ struct NsemBuf {
 #ifdef __cplusplus
 extern "C" {
 #endif
-/* FP64 (plain) form launchers, nsem_fp64.cu.  stage: 0 = tendency only
- * (writes L), 1..3 = Shu-Osher stage. */
-int nsem_fp64_prim(const NsemDev* m, NsemBuf* b, int from_state, void* stream);
-int nsem_fp64_face(const NsemDev* m, NsemBuf* b, int from_state, void* stream);
-int nsem_fp64_volume(const NsemDev* m, const NsemTables* t, NsemBuf* b, int stage,
-                     double dt, void* stream);
+/* FP64 (plain) form launchers, nsem_fp64.cu: the primitives of a state (b->prim;
+ * a volume launch of stages 1-3 leaves its result's there), the face fluxes of
+ * the state whose primitives those are (rho: its density), the volume term and
+ * update.  stage: 0 = tendency only (out: L), 1..3 = Shu-Osher stage of the
+ * stage state S from u^n = U0 (out may be S or U0). */
+int nsem_fp64_prim(const NsemDev* m, NsemBuf* b, const double* const* S, void* stream);
+int nsem_fp64_face(const NsemDev* m, NsemBuf* b, const double* rho, void* stream);
+int nsem_fp64_volume(const NsemDev* m, const NsemTables* t, NsemBuf* b, int stage, double dt,
+                     const double* const* S, const double* const* U0, double* const* out,
+                     void* stream);
 int nsem_fp64_check_smem(const NsemDev* m);
 #ifdef __cplusplus
 }

@@ -1105,7 +1105,7 @@ int launch_args(const NsemMixedBuf* mb, const StageArgs& a, int stage, cudaStrea
 /* one SSP-RK3 step of the precision form with explicit buffers: shadow S of
  * u'^n (stage base), increments d1 and d2, FP64 state U -> Unew with shadow
  * Snew.  Used by the plain steps and by the checkpointed forward runs of the
- * adjoint, which keep S, d1, d2 of every step. */
+ * adjoint, which keep S, d1, d2 of every step; Unew null: stages 1 and 2 only. */
 int nsem_mixed_step_bufs(const NsemDev* dev, const NsemMixedBuf* mb, const double* U,
                          const float* S, float* d1, float* d2, double* Unew, float* Snew,
                          double dt, void* stream) {
@@ -1120,6 +1120,7 @@ int nsem_mixed_step_bufs(const NsemDev* dev, const NsemMixedBuf* mb, const doubl
     a.Din = d1;
     a.Dout = d2;
     if ((e = launch_args(mb, a, 2, st))) return e;
+    if (!Unew) return 0;
     a.Din = d2;
     a.Dout = nullptr;
     a.Unew = Unew;

@@ -71,6 +71,7 @@ struct NsemMixedBuf {
     double* ckpt = nullptr;       /* [n_ckpt][5 n_int] FP64 checkpoints of u'      */
     float* seg = nullptr;         /* [seg_steps][3][5 n_int] per step: shadow, d1, d2 */
     int64_t seg_steps = 0, ckpt_slots = 0;
+    int seg_of = -1;              /* the segment whose stage states seg holds (-1: none) */
     double* lam = nullptr;        /* [5 n_int] FP64 adjoint state             */
     double* fin = nullptr;        /* [5 n_int] FP64 final state of the forward */
     float* abar[3] = {};          /* FP32 stage adjoints: sbar, d2bar, d1bar  */

@@ -36,6 +36,7 @@
 #include <vector>
 
 #include "nsem_mixed_adj.cuh"
+#include "nsem_pdl.cuh"
 
 using namespace nsem_mx;
 using namespace nsem_mxa;
@@ -147,27 +148,13 @@ k_mixed_adj(AdjArgs a) {
     const int64_t e = blockIdx.x;
     constexpr bool has_din = RS == 3 || RS == 2;
 
+    /* what no kernel of the chain writes, before the wait for the previous
+     * kernel: background, neighbours, metric */
     float x[5], gb[5], bgs[4] = {0, 0, 0, 0};
     if (t < NP) {
-        const int64_t o = e * 5 * NP + t;
-#pragma unroll
-        for (int v = 0; v < 5; v++) x[v] = __ldg(a.S + o + v * NP);
-        if constexpr (has_din) {
-#pragma unroll
-            for (int v = 0; v < 5; v++) x[v] = __fadd_rn(x[v], __ldg(a.Din + o + v * NP));
-        }
-        load_gbar<RS>(a, o, NP, gb);
         const float* bg = a.bg + (int64_t)__ldg(a.layer + e) * 4 * NP + t;
 #pragma unroll
         for (int c = 0; c < 4; c++) bgs[c] = __ldg(bg + c * NP);
-    }
-    float gv[12];
-    if constexpr (VISC) {
-        if (t < NP) {
-            const float* gr = a.Gv + e * 12 * NP + t;
-#pragma unroll
-            for (int c = 0; c < 12; c++) gv[c] = __ldg(gr + c * NP);
-        }
     }
     FaceSlot fs{};
     int32_t nb = -1;
@@ -176,14 +163,6 @@ k_mixed_adj(AdjArgs a) {
         fs = face_slot<NX, NY, NZ>(t);
         nb = __ldg(a.nbr + (int64_t)fs.face * a.n_elem + e);
         if (nb >= 0) {
-            const int64_t o = (int64_t)nb * 5 * NP + fs.lo;
-#pragma unroll
-            for (int v = 0; v < 5; v++) xo[v] = __ldg(a.S + o + v * NP);
-            if constexpr (has_din) {
-#pragma unroll
-                for (int v = 0; v < 5; v++) xo[v] = __fadd_rn(xo[v], __ldg(a.Din + o + v * NP));
-            }
-            load_gbar<RS>(a, o, NP, go);
             const float* bg = a.bg + (int64_t)__ldg(a.layer + nb) * 4 * NP + fs.lo;
 #pragma unroll
             for (int c = 0; c < 4; c++) bgo[c] = __ldg(bg + c * NP);
@@ -191,6 +170,36 @@ k_mixed_adj(AdjArgs a) {
         }
     }
     if (t < 3) sMeta[t] = __ldg(a.J + (int64_t)t * a.n_elem + e);
+    nsem_chain_wait();
+
+    if (t < NP) {
+        const int64_t o = e * 5 * NP + t;
+#pragma unroll
+        for (int v = 0; v < 5; v++) x[v] = a.S[o + v * NP];
+        if constexpr (has_din) {
+#pragma unroll
+            for (int v = 0; v < 5; v++) x[v] = __fadd_rn(x[v], a.Din[o + v * NP]);
+        }
+        load_gbar<RS>(a, o, NP, gb);
+    }
+    float gv[12];
+    if constexpr (VISC) {
+        if (t < NP) {
+            const float* gr = a.Gv + e * 12 * NP + t;
+#pragma unroll
+            for (int c = 0; c < 12; c++) gv[c] = gr[c * NP];
+        }
+    }
+    if (t < NFS && nb >= 0) {
+        const int64_t o = (int64_t)nb * 5 * NP + fs.lo;
+#pragma unroll
+        for (int v = 0; v < 5; v++) xo[v] = a.S[o + v * NP];
+        if constexpr (has_din) {
+#pragma unroll
+            for (int v = 0; v < 5; v++) xo[v] = __fadd_rn(xo[v], a.Din[o + v * NP]);
+        }
+        load_gbar<RS>(a, o, NP, go);
+    }
 
     /* phase 1: gbar and the node's values for the face and pointwise transposes */
     float uu[3], th = 0.0f, pth = 0.0f, rho = 0.0f;
@@ -232,6 +241,7 @@ k_mixed_adj(AdjArgs a) {
     __syncthreads();
 
     /* phase 3: transposed line sums, pointwise transposes, face and source terms */
+    nsem_chain_begin();
     if (t >= NP) return;
     const int i = t / (NY * NZ), j = (t / NZ) % NY, k = t % NZ;
     float xb[5] = {0, 0, 0, 0, 0};
@@ -331,20 +341,30 @@ k_mixed_adj(AdjArgs a) {
             a.Bout[o + v * NP] = gb[v] + x3;
         }
     } else if constexpr (RS == 2) {
-        /* A += xbar2; C = B/4 + xbar2 (gb = B/4) */
+        /* A += xbar2; C = B/4 + xbar2 (gb = B/4); loads before stores, which
+         * could alias them */
+        float A[5];
+#pragma unroll
+        for (int v = 0; v < 5; v++) A[v] = a.A[o + v * NP];
 #pragma unroll
         for (int v = 0; v < 5; v++) {
             const float x2 = dt * xb[v];
-            a.A[o + v * NP] = __ldg(a.A + o + v * NP) + x2;
+            a.A[o + v * NP] = A[v] + x2;
             a.Bout[o + v * NP] = gb[v] + x2;
         }
     } else {
         /* lam <- lam + A + xbar1 (FP64) */
+        float A[5];
+        double l[5];
+#pragma unroll
+        for (int v = 0; v < 5; v++) {
+            A[v] = a.A[o + v * NP];
+            l[v] = a.lam[o + v * NP];
+        }
 #pragma unroll
         for (int v = 0; v < 5; v++) {
             const float x1 = dt * xb[v];
-            const double l = __ldg(a.lam + o + v * NP);
-            a.lam_out[o + v * NP] = l + (f2d(__ldg(a.A + o + v * NP)) + f2d(x1));
+            a.lam_out[o + v * NP] = l[v] + (f2d(A[v]) + f2d(x1));
         }
     }
 }
@@ -565,10 +585,10 @@ int launch_adj(const AdjArgs& a, int rs, cudaStream_t st, int passes) {
         return (int)cudaGetLastError();
     }
     switch (rs) {
-        case 0: k_mixed_adj<NX, NY, NZ, 0, false><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-        case 1: k_mixed_adj<NX, NY, NZ, 1, false><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-        case 2: k_mixed_adj<NX, NY, NZ, 2, false><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-        default: k_mixed_adj<NX, NY, NZ, 3, false><<<grid, G::BLOCK, SMEM, st>>>(a); break;
+        case 0: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 0, false>, grid, (unsigned)G::BLOCK, SMEM, st, a);
+        case 1: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 1, false>, grid, (unsigned)G::BLOCK, SMEM, st, a);
+        case 2: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 2, false>, grid, (unsigned)G::BLOCK, SMEM, st, a);
+        default: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 3, false>, grid, (unsigned)G::BLOCK, SMEM, st, a);
     }
     return (int)cudaGetLastError();
 }
@@ -1441,17 +1461,30 @@ int nsem_mixed_fwd_ckpt(const NsemDev* dev, NsemMixedBuf* mb, int nsteps, int ev
     int e = nsem_mixed_adj_alloc(mb);
     if (e) return e;
     int cur = mb->cur;
+    /* the last segment's steps write their stage states (S, d1, d2) where the
+     * reverse sweep starts reading: it need not recompute that segment */
+    mb->seg_of = -1;
+    const int last = (n_ckpt - 1) * every;
+    auto seg_S = [&](int s) { return mb->seg + (int64_t)(s - last) * 3 * n5; };
     for (int s = 0; s < nsteps; s++) {
         if (s % every == 0) {
             cudaError_t ce = cudaMemcpyAsync(mb->ckpt + (int64_t)(s / every) * n5, mb->U[cur],
                                              (size_t)n5 * sizeof(double), cudaMemcpyDeviceToDevice, st);
+            if (ce == cudaSuccess && s == last && s == 0)
+                ce = cudaMemcpyAsync(seg_S(0), mb->S[cur], (size_t)n5 * sizeof(float),
+                                     cudaMemcpyDeviceToDevice, st);
             if (ce != cudaSuccess) return (int)ce;
         }
-        if ((e = nsem_mixed_step_bufs(dev, mb, mb->U[cur], mb->S[cur], mb->D[0], mb->D[1],
-                                      mb->U[cur ^ 1], mb->S[cur ^ 1], dt, stream)))
+        const bool keep = s >= last, next = s + 1 >= last && s + 1 < nsteps;
+        const float* S = keep ? seg_S(s) : mb->S[cur];
+        float* d1 = keep ? seg_S(s) + n5 : mb->D[0];
+        float* d2 = keep ? seg_S(s) + 2 * n5 : mb->D[1];
+        if ((e = nsem_mixed_step_bufs(dev, mb, mb->U[cur], S, d1, d2, mb->U[cur ^ 1],
+                                      next ? seg_S(s + 1) : mb->S[cur ^ 1], dt, stream)))
             return e;
         cur ^= 1;
     }
+    mb->seg_of = n_ckpt - 1;
     mb->cur = cur;
     mb->nsteps = nsteps;
     mb->every = every;
@@ -1462,7 +1495,10 @@ int nsem_mixed_fwd_ckpt(const NsemDev* dev, NsemMixedBuf* mb, int nsteps, int ev
 /* Reverse sweep: lam (element-blocked FP64, mb->lam) holds dJ/du' at the
  * final state; on return it holds dJ/du' at the initial state.  Each segment
  * is recomputed from its checkpoint keeping S, d1, d2 of every step, then
- * swept backwards.  The forward's final state is restored afterwards. */
+ * swept backwards (the segment whose stage states the buffer holds already,
+ * after a forward run the last one, is not recomputed, and a segment's last
+ * step stops before stage 3, whose result no stage of the sweep reads).  The
+ * forward's final state is restored afterwards. */
 int nsem_mixed_adjoint_run(const NsemDev* dev, NsemMixedBuf* mb, double dt, void* stream) {
     const int64_t n5 = 5 * mb->n_int;
     cudaStream_t st = (cudaStream_t)stream;
@@ -1477,24 +1513,24 @@ int nsem_mixed_adjoint_run(const NsemDev* dev, NsemMixedBuf* mb, double dt, void
         const int start = sg * mb->every;
         const int cnt = (mb->nsteps - start < mb->every) ? mb->nsteps - start : mb->every;
         /* recompute the segment: step j reads U (FP64) and its shadow seg_S[j],
-         * writes d1, d2 into the segment and the next shadow into seg_S[j+1] */
-        const double* Uin = mb->ckpt + (int64_t)sg * n5;
-        float* S0 = mb->seg;
-        k_shadow<<<grid_for(n5), 256, 0, st>>>(Uin, S0, n5);
-        if ((e = (int)cudaGetLastError())) return e;
-        int pp = 0;
-        for (int j = 0; j < cnt; j++) {
-            float* Sj = mb->seg + (int64_t)j * 3 * n5;
-            float* d1 = Sj + n5;
-            float* d2 = Sj + 2 * n5;
-            /* the last step's next shadow is not needed: write it to the
-             * ping-pong shadow instead of past the segment */
-            float* Snext = (j + 1 < cnt) ? mb->seg + (int64_t)(j + 1) * 3 * n5 : mb->S[pp];
-            double* Unext = mb->U[pp];
-            if ((e = nsem_mixed_step_bufs(dev, mb, Uin, Sj, d1, d2, Unext, Snext, dt, stream)))
-                return e;
-            Uin = Unext;
-            pp ^= 1;
+         * writes d1, d2 into the segment and, but for the last step, the next
+         * shadow into seg_S[j+1] */
+        if (mb->seg_of != sg) {
+            mb->seg_of = -1;
+            const double* Uin = mb->ckpt + (int64_t)sg * n5;
+            k_shadow<<<grid_for(n5), 256, 0, st>>>(Uin, mb->seg, n5);
+            if ((e = (int)cudaGetLastError())) return e;
+            int pp = 0;
+            for (int j = 0; j < cnt; j++) {
+                float* Sj = mb->seg + (int64_t)j * 3 * n5;
+                double* Unext = j + 1 < cnt ? mb->U[pp] : nullptr;
+                if ((e = nsem_mixed_step_bufs(dev, mb, Uin, Sj, Sj + n5, Sj + 2 * n5, Unext,
+                                              Sj + 3 * n5, dt, stream)))
+                    return e;
+                Uin = Unext;
+                pp ^= 1;
+            }
+            mb->seg_of = sg;
         }
         for (int j = cnt - 1; j >= 0; j--) {
             const float* Sj = mb->seg + (int64_t)j * 3 * n5;

@@ -108,9 +108,9 @@ template <int RS>
 __device__ __forceinline__ void load_gbar(const AdjArgs& a, int64_t o, int np, float* gb) {
 #pragma unroll
     for (int v = 0; v < 5; v++) {
-        if constexpr (RS == 3) gb[v] = (2.0f / 3.0f) * d2f_rn(__ldg(a.lam + o + v * np));
-        else if constexpr (RS == 2) gb[v] = 0.25f * __ldg(a.Gin + o + v * np);
-        else gb[v] = __ldg(a.Gin + o + v * np);
+        if constexpr (RS == 3) gb[v] = (2.0f / 3.0f) * d2f_rn(a.lam[o + v * np]);
+        else if constexpr (RS == 2) gb[v] = 0.25f * a.Gin[o + v * np];
+        else gb[v] = a.Gin[o + v * np];
     }
 }
 
