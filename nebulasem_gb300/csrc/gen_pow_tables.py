@@ -10,11 +10,11 @@ Tables (values from their mathematical definitions, 200-bit mpmath):
   LOG_NLR[i]    -log(r_i) as an unevaluated sum hi + lo;
   EXP2[j]       2^(j/64) as hi + lo, j = 0..63;
   ILOG[i]       for the fixed-point phase, significands m in
-                [1 + i/128, 1 + (i+1)/128): k_i = ceil(1024 / (1 + i/128)), so
-                that 0 <= m k_i / 1024 - 1 < 2^-6.6, and the 96 fraction bits
-                of -log2(k_i / 1024) (three 32-bit words, high first);
-  IEXP2[j]      2^(j/128) as a 96-bit fixed-point number in [1, 2) (leading
-                bit 95), j = 0..127;
+                [1 + i/1024, 1 + (i+1)/1024): k_i = ceil(8192 / (1 + i/1024)),
+                so that 0 <= m k_i / 8192 - 1 < 2^-9.6, and the 96 fraction
+                bits of -log2(k_i / 8192) (three 32-bit words, high first);
+  IEXP2[j]      2^(j/1024) as a 96-bit fixed-point number in [1, 2) (leading
+                bit 95), j = 0..1023;
   ILOG_C[n]     1 / (n ln 2) and IEXP_D[n] = (ln 2)^n / n!, scaled by powers
                 of two as the Horner steps take them.
 """
@@ -77,23 +77,24 @@ def main():
         q = int(mpmath.nint(v * mpmath.mpf(2) ** (32 * n)))
         return [(q >> (32 * (n - 1 - w))) & 0xFFFFFFFF for w in range(n)]
 
-    print("NSEM_TABLE4 nsem_u4 nsem_ilog[128] = {")
-    for i in range(128):
-        k = -(-1024 * 128 // (128 + i))
-        w = words(-mpmath.log(mpmath.mpf(k) / 1024, 2), 3)
+    n = 1024
+    print(f"NSEM_TABLE4 nsem_u4 nsem_ilog[{n}] = {{")
+    for i in range(n):
+        k = -(-8 * n * n // (n + i))
+        w = words(-mpmath.log(mpmath.mpf(k) / (8 * n), 2), 3)
         print(f"  {{{k}u, {w[0]:#010x}u, {w[1]:#010x}u, {w[2]:#010x}u}},")
     print("};")
-    print("NSEM_TABLE4 nsem_u4 nsem_iexp2[128] = {")
-    for j in range(128):
-        w = words(mpmath.power(2, mpmath.mpf(j) / 128) / 2, 3)
+    print(f"NSEM_TABLE4 nsem_u4 nsem_iexp2[{n}] = {{")
+    for j in range(n):
+        w = words(mpmath.power(2, mpmath.mpf(j) / n) / 2, 3)
         print(f"  {{{w[0]:#010x}u, {w[1]:#010x}u, {w[2]:#010x}u, 0u}},")
     print("};")
-    for n in range(1, 11):
-        c = int(mpmath.nint(1 / (n * ln2) * mpmath.mpf(2) ** (69 - 6 * n)))
-        print(f"#define NSEM_ILOG_C{n} {c:#x}{'ull' if n < 6 else 'u'}")
-    for n in range(1, 8):
-        d = int(mpmath.nint(ln2 ** n / mpmath.factorial(n) * mpmath.mpf(2) ** (71 - 7 * n)))
-        print(f"#define NSEM_IEXP_D{n} {d:#x}{'ull' if n < 5 else 'u'}")
+    for q in range(1, 8):
+        c = int(mpmath.nint(1 / (q * ln2) * mpmath.mpf(2) ** (72 - 9 * q)))
+        print(f"#define NSEM_ILOG_C{q} {c:#x}{'ull' if q < 5 else 'u'}")
+    for q in range(1, 7):
+        d = int(mpmath.nint(ln2 ** q / mpmath.factorial(q) * mpmath.mpf(2) ** (74 - 10 * q)))
+        print(f"#define NSEM_IEXP_D{q} {d:#x}{'ull' if q < 4 else 'u'}")
     print("#endif")
 
 

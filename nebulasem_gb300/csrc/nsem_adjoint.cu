@@ -119,7 +119,10 @@ struct FaceAdjArgs {
     double* dbv[4];          /* viscous runs: momentum and theta flux adjoints (else null) */
 };
 
-__global__ void __launch_bounds__(128) k_adj_face(const NsemDev m, FaceAdjArgs a) {
+/* FACE threads a CTA, so that a small mesh's slots spread over the SMs */
+constexpr int FACE = 64;
+
+__global__ void __launch_bounds__(FACE) k_adj_face(const NsemDev m, FaceAdjArgs a) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= m.n_slot) return;
     if (m.n_ms && m.ms_of[k] >= 0) {         /* non-conforming: k_adj_face_mortar */
@@ -361,15 +364,13 @@ struct VolAdjArgs {
 /* registers capped for the largest element: 736 threads (N+1 = 9) inviscid,
  * 512 (N+1 = 8) with the viscous terms */
 template <bool VISC>
-__global__ void __maxnreg__(VISC ? 128 : 88) k_adj_volume(const NsemDev m, const NsemTables tab,
-                                                          VolAdjArgs a) {
+__global__ void __maxnreg__(VISC ? 128 : 88) k_adj_volume(const NsemDev m,                                                           VolAdjArgs a) {
     extern __shared__ double sm[];
     const int NPX = m.npx, NPY = m.npy, NPZ = m.npz, NP = m.np;
     double* rb = sm;                                 /* [5][NP] rbar of the element */
     double* dps = sm + 5 * NP;                       /* dpsi tables */
     const int t = threadIdx.x;
-    for (int q = t; q < 3 * NSEM_MAX_NPD * NSEM_MAX_NPD; q += blockDim.x)
-        dps[q] = (&tab.dpsi[0][0])[q];
+    nsem_load_tables(m, dps, t);
     const int64_t e = blockIdx.x;
     const int64_t node = e * NP + t;
     const bool active = t < NP;
@@ -978,7 +979,7 @@ __global__ void __launch_bounds__(256) k_tan_grad_face(const NsemDev m, GradFace
     a.dfF[3][k] = a.dpU[3][c1] * fi + dT2 * fo;
 }
 
-__global__ void __launch_bounds__(128) k_tan_face(const NsemDev m, FaceTanArgs a) {
+__global__ void __launch_bounds__(FACE) k_tan_face(const NsemDev m, FaceTanArgs a) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= m.n_slot) return;
     if (m.n_ms && m.ms_of[k] >= 0) return;   /* non-conforming: k_tan_face_mortar */
@@ -1079,13 +1080,12 @@ struct VolTanArgs {
  * in the forward kernel; then jin[9] */
 constexpr int TAN_W = 24;
 
-__global__ void k_tan_volume(const NsemDev m, const NsemTables tab, VolTanArgs a) {
+__global__ void __launch_bounds__(1024) k_tan_volume(const NsemDev m, VolTanArgs a) {
     extern __shared__ double sm[];
     const int NPX = m.npx, NPY = m.npy, NPZ = m.npz, NP = m.np;
     double* dps = sm + (size_t)NP * TAN_W;
     const int t = threadIdx.x;
-    for (int q = t; q < 3 * NSEM_MAX_NPD * NSEM_MAX_NPD; q += blockDim.x)
-        dps[q] = (&tab.dpsi[0][0])[q];
+    nsem_load_tables(m, dps, t);
     const int64_t e = blockIdx.x;
     const bool active = t < NP;
     const int64_t node = e * NP + t;
@@ -1116,7 +1116,7 @@ __global__ void k_tan_volume(const NsemDev m, const NsemTables tab, VolTanArgs a
         }
         for (int c = 0; c < 9; c++) my[15 + c] = m.jin[(int64_t)c * m.n_int + node];
     }
-    const bool diag = __syncthreads_and(!active || nsem_node_diag<5>(sm + (size_t)t * TAN_W));
+    const int kind = nsem_element_kind<5>(m, active, sm + (size_t)t * TAN_W);
     if (!active) return;
     double r[5] = {0, 0, 0, 0, 0};
     /* surface lift (a coarse side of a non-conforming face lifts the
@@ -1133,7 +1133,7 @@ __global__ void k_tan_volume(const NsemDev m, const NsemTables tab, VolTanArgs a
         }
     }
     /* volume term: r[a] -= dF_b . (Jin_b dpsi(b -> a)) over the lines through a */
-    nsem_volume_gather<5, TAN_W, 0xe>(NPX, NPY, NPZ, sm, dps, t, diag, r);
+    nsem_volume_gather<5, TAN_W, 0xe>(NPX, NPY, NPZ, sm, dps, t, kind, r);
     /* gravity source: r_m -= g (rho - rho_ref) cV */
     const double cv = m.cv[node];
     for (int c = 0; c < 3; c++) r[1 + c] -= m.g[c] * drho * cv;
@@ -1294,13 +1294,12 @@ __global__ void __launch_bounds__(128) k_adj_grad_mortar_b(const NsemDev m, Grad
 /* shared layout per node: Gbs[12] jin[9] */
 constexpr int GADJ_W = 21;
 
-__global__ void k_adj_grad_vol(const NsemDev m, const NsemTables tab, GradAdjArgs a) {
+__global__ void k_adj_grad_vol(const NsemDev m, GradAdjArgs a) {
     extern __shared__ double sm[];
     const int NPX = m.npx, NPY = m.npy, NPZ = m.npz, NP = m.np;
     double* dps = sm + (size_t)NP * GADJ_W;
     const int t = threadIdx.x;
-    for (int q = t; q < 3 * NSEM_MAX_NPD * NSEM_MAX_NPD; q += blockDim.x)
-        dps[q] = (&tab.dpsi[0][0])[q];
+    nsem_load_tables(m, dps, t);
     const int64_t e = blockIdx.x;
     const bool active = t < NP;
     const int64_t node = e * NP + t;
@@ -1408,7 +1407,7 @@ int grid_for(int64_t n) {
 }  // namespace
 
 /* the product into G, or (lin) its combination */
-static int adj_vjp(const NsemDev* m, const NsemTables* t, const double* const* S,
+static int adj_vjp(const NsemDev* m, const double* const* S,
                    const double* const* W, double* const* G, const NsemAdjLin* lin, NsemAdjBuf* ab,
                    void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
@@ -1420,7 +1419,7 @@ static int adj_vjp(const NsemDev* m, const NsemTables* t, const double* const* S
         for (int v = 0; v < 5; v++) { pa.S[v] = S[v]; pa.dS[v] = S[v]; }
         for (int c = 0; c < 4; c++) { pa.pU[c] = ab->pU[c]; pa.dpU[c] = ab->dpU[c]; }
         k_tan_prims<<<(unsigned)((m->n_int + 255) / 256), 256, 0, st>>>(*m, pa);
-        const int e = nsem_grad_ut_mortar(m, t, ab->pU, ab->pU[3], ab->Gv, ab->fF,
+        const int e = nsem_grad_ut_mortar(m, ab->pU, ab->pU[3], ab->Gv, ab->fF,
                                           m->n_ms > 0 ? ab->gC : nullptr, stream);
         if (e) return e;
         for (int c = 0; c < 4; c++) fa.dbv[c] = ab->dbv[c];
@@ -1430,8 +1429,8 @@ static int adj_vjp(const NsemDev* m, const NsemTables* t, const double* const* S
     }
     for (int v = 0; v < 5; v++) { fa.S[v] = S[v]; fa.W[v] = W[v]; }
     for (int v = 0; v < NPA; v++) { fa.adjO[v] = ab->adjO[v]; fa.adjN[v] = ab->adjN[v]; }
-    const int64_t fb = (m->n_slot + 127) / 128;
-    nsem_launch_chained(k_adj_face, (unsigned)fb, 128, 0, st, *m, fa);
+    const int64_t fb = (m->n_slot + FACE - 1) / FACE;
+    nsem_launch_chained(k_adj_face, (unsigned)fb, FACE, 0, st, *m, fa);
     for (int c = 0; c < 19; c++) va.qb[c] = nullptr;
     if (m->n_ms > 0) {
         MortarArgs ma{};
@@ -1456,8 +1455,8 @@ static int adj_vjp(const NsemDev* m, const NsemTables* t, const double* const* S
     const size_t smem = (5 * (size_t)m->np + 3 * NSEM_MAX_NPD * NSEM_MAX_NPD) * sizeof(double);
     if (lin && !ab->visc) va.lin = *lin;
     const unsigned grid = (unsigned)m->n_elem;
-    if (ab->visc) nsem_launch_chained(k_adj_volume<true>, grid, (unsigned)threads, smem, st, *m, *t, va);
-    else nsem_launch_chained(k_adj_volume<false>, grid, (unsigned)threads, smem, st, *m, *t, va);
+    if (ab->visc) nsem_launch_chained(k_adj_volume<true>, grid, (unsigned)threads, smem, st, *m, va);
+    else nsem_launch_chained(k_adj_volume<false>, grid, (unsigned)threads, smem, st, *m, va);
     if (ab->visc) {
         /* the gradients' transpose, added to the conserved adjoint */
         GradAdjArgs ga{};
@@ -1477,7 +1476,7 @@ static int adj_vjp(const NsemDev* m, const NsemTables* t, const double* const* S
             k_adj_grad_mortar_b<<<mb, 128, 0, st>>>(*m, ga);
         }
         const size_t gsm = ((size_t)m->np * GADJ_W + 3 * NSEM_MAX_NPD * NSEM_MAX_NPD) * sizeof(double);
-        k_adj_grad_vol<<<(unsigned)m->n_elem, threads, gsm, st>>>(*m, *t, ga);
+        k_adj_grad_vol<<<(unsigned)m->n_elem, threads, gsm, st>>>(*m, ga);
         if (lin) {
             Lin3Args la{};
             for (int v = 0; v < 5; v++) {
@@ -1495,17 +1494,17 @@ static int adj_vjp(const NsemDev* m, const NsemTables* t, const double* const* S
     return (int)cudaGetLastError();
 }
 
-int nsem_adj_vjp(const NsemDev* m, const NsemTables* t, const double* const* S,
+int nsem_adj_vjp(const NsemDev* m, const double* const* S,
                  const double* const* W, double* const* G, NsemAdjBuf* ab, void* stream) {
-    return adj_vjp(m, t, S, W, G, nullptr, ab, stream);
+    return adj_vjp(m, S, W, G, nullptr, ab, stream);
 }
 
-int nsem_adj_vjp_lin(const NsemDev* m, const NsemTables* t, const double* const* S,
+int nsem_adj_vjp_lin(const NsemDev* m, const double* const* S,
                      const double* const* W, const NsemAdjLin& lin, NsemAdjBuf* ab, void* stream) {
-    return adj_vjp(m, t, S, W, ab->g, &lin, ab, stream);
+    return adj_vjp(m, S, W, ab->g, &lin, ab, stream);
 }
 
-int nsem_adj_jvp(const NsemDev* m, const NsemTables* t, const double* const* S,
+int nsem_adj_jvp(const NsemDev* m, const double* const* S,
                  const double* const* dS, double* const* out, NsemAdjBuf* ab, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     FaceTanArgs fa{};
@@ -1518,7 +1517,7 @@ int nsem_adj_jvp(const NsemDev* m, const NsemTables* t, const double* const* S,
         for (int c = 0; c < 4; c++) { pa.pU[c] = ab->pU[c]; pa.dpU[c] = ab->dpU[c]; }
         k_tan_prims<<<(unsigned)((m->n_int + 255) / 256), 256, 0, st>>>(*m, pa);
         const bool mort = m->n_ms > 0;
-        int e = nsem_grad_ut_mortar(m, t, ab->pU, ab->pU[3], ab->Gv, ab->fF, mort ? ab->gC : nullptr, stream);
+        int e = nsem_grad_ut_mortar(m, ab->pU, ab->pU[3], ab->Gv, ab->fF, mort ? ab->gC : nullptr, stream);
         if (e) return e;
         GradFaceTanArgs ga;
         for (int c = 0; c < 4; c++) { ga.pU[c] = ab->pU[c]; ga.dpU[c] = ab->dpU[c]; ga.dfF[c] = ab->dfF[c]; }
@@ -1527,7 +1526,7 @@ int nsem_adj_jvp(const NsemDev* m, const NsemTables* t, const double* const* S,
          * face values of the tangents */
         if (mort && (e = nsem_grad_mortar_faces(m, ab->dpU, ab->dpU[3], ab->dfF, ab->dgC, stream)))
             return e;
-        e = nsem_grad_vol(m, t, ab->dpU, ab->dpU[3], ab->dGv, ab->dfF, mort ? ab->dgC : nullptr, stream);
+        e = nsem_grad_vol(m, ab->dpU, ab->dpU[3], ab->dGv, ab->dfF, mort ? ab->dgC : nullptr, stream);
         if (e) return e;
         for (int c = 0; c < 12; c++) {
             fa.G[c] = va.G[c] = ab->Gv[c];
@@ -1535,8 +1534,8 @@ int nsem_adj_jvp(const NsemDev* m, const NsemTables* t, const double* const* S,
         }
     }
     for (int v = 0; v < 5; v++) { fa.S[v] = S[v]; fa.dS[v] = dS[v]; fa.dd[v] = ab->adjO[v]; }
-    const int64_t fb = (m->n_slot + 127) / 128;
-    k_tan_face<<<(unsigned)fb, 128, 0, st>>>(*m, fa);
+    const int64_t fb = (m->n_slot + FACE - 1) / FACE;
+    k_tan_face<<<(unsigned)fb, FACE, 0, st>>>(*m, fa);
     for (int v = 0; v < 5; v++) va.ddC[v] = nullptr;
     if (m->n_ms > 0) {
         MortarArgs ma{};
@@ -1555,7 +1554,7 @@ int nsem_adj_jvp(const NsemDev* m, const NsemTables* t, const double* const* S,
     for (int v = 0; v < 5; v++) { va.S[v] = S[v]; va.dS[v] = dS[v]; va.dd[v] = ab->adjO[v]; va.out[v] = out[v]; }
     const int threads = ((m->np + 31) / 32) * 32;
     const size_t smem = ((size_t)m->np * TAN_W + 3 * NSEM_MAX_NPD * NSEM_MAX_NPD) * sizeof(double);
-    k_tan_volume<<<(unsigned)m->n_elem, threads, smem, st>>>(*m, *t, va);
+    k_tan_volume<<<(unsigned)m->n_elem, threads, smem, st>>>(*m, va);
     return (int)cudaGetLastError();
 }
 

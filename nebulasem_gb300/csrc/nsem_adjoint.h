@@ -63,7 +63,7 @@ struct NsemAdjBuf {
 };
 
 /* g = J_L(S)^T W (all device pointers, 5 SoA arrays each) */
-int nsem_adj_vjp(const NsemDev* m, const NsemTables* t, const double* const* S,
+int nsem_adj_vjp(const NsemDev* m, const double* const* S,
                  const double* const* W, double* const* G, NsemAdjBuf* ab, void* stream);
 /* out = cx x + cy y + cz z + cg J_L(S)^T W (y, z may be null; out may be any of
  * them: every node's operands are read by the thread that then writes it, and
@@ -75,10 +75,10 @@ struct NsemAdjLin {
     const double* z[5] = {};
     double cx = 0, cy = 0, cz = 0, cg = 0;
 };
-int nsem_adj_vjp_lin(const NsemDev* m, const NsemTables* t, const double* const* S,
+int nsem_adj_vjp_lin(const NsemDev* m, const double* const* S,
                      const double* const* W, const NsemAdjLin& lin, NsemAdjBuf* ab, void* stream);
 /* out = J_L(S) dS (tangent-linear product; uses ab->adjO[0..4] as slot scratch) */
-int nsem_adj_jvp(const NsemDev* m, const NsemTables* t, const double* const* S,
+int nsem_adj_jvp(const NsemDev* m, const double* const* S,
                  const double* const* dS, double* const* out, NsemAdjBuf* ab, void* stream);
 /* out = cx x + cy y + cz z (y, z may be null), for the tangent-linear sweep */
 int nsem_adj_lin3(double* const* out, const double* const* x, double cx, const double* const* y,

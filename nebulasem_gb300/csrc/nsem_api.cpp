@@ -28,7 +28,6 @@ struct nsem_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     NsemDev dev{};
-    NsemTables tab{};
     NsemBuf buf{};
     NsemMixedBuf mbuf{};
     NsemAdjBuf abuf{};
@@ -161,11 +160,16 @@ nsem_status build_device_mesh(nsem_ctx* ctx, const nsem_mesh_desc* m, const nsem
     ctx->dt = p->dt;
     ctx->T0 = p->T0;
 
-    /* tables: dpsi[d][s*npd + i] */
     const int npd[3] = {m->npx, m->npy, m->npz};
-    std::memset(&ctx->tab, 0, sizeof(ctx->tab));
+    std::vector<double> dpsi(3 * NSEM_MAX_NPD * NSEM_MAX_NPD, 0.0);
     for (int d = 0; d < 3; d++)
-        for (int q = 0; q < npd[d] * npd[d]; q++) ctx->tab.dpsi[d][q] = m->dpsi[d][q];
+        for (int q = 0; q < npd[d] * npd[d]; q++) dpsi[d * NSEM_MAX_NPD * NSEM_MAX_NPD + q] = m->dpsi[d][q];
+    auto tame = [](double x) { return x == 0.0 || (std::fabs(x) >= 0x1p-60 && std::fabs(x) < 0x1p60); };
+    D.tame_tables = 1;
+    for (int d = 0; d < 3; d++)
+        for (int q = 0; q < npd[d] * npd[d]; q++)
+            if (!tame(m->dpsi[d][q])) D.tame_tables = 0;
+    D.tame_const = tame(D.P0) && tame(D.R) && tame(D.gR) && tame(D.nu) && tame(D.iPr) && tame(D.T0);
 
     /* used slots in reference order */
     std::vector<int64_t> compact(n_slot_all, -1);
@@ -295,6 +299,7 @@ nsem_status build_device_mesh(nsem_ctx* ctx, const nsem_mesh_desc* m, const nsem
 
     nsem_status s;
 #define UP(ptr, vec) if ((s = upload(ctx, &(ptr), vec)) != NSEM_OK) return s
+    UP(D.dpsi, dpsi);
     UP(D.jin, jin);
     UP(D.cv, cv);
     UP(D.p_ref, pref);
@@ -466,7 +471,7 @@ int fp64_face(nsem_ctx* ctx, const double* rho) {
     NsemBuf* b = &ctx->buf;
     if (b->G[0]) {
         const double* U[3] = {b->prim[0], b->prim[1], b->prim[2]};
-        const int e = nsem_grad_ut_mortar(&ctx->dev, &ctx->tab, U, b->prim[3], b->G, b->fF,
+        const int e = nsem_grad_ut_mortar(&ctx->dev, U, b->prim[3], b->G, b->fF,
                                           ctx->dev.n_ms > 0 ? b->gC : nullptr, ctx->stream);
         if (e) return e;
     }
@@ -479,7 +484,7 @@ nsem_status fp64_stage(nsem_ctx* ctx, int stage, const double* const* S, const d
                        double* const* out) {
     int e = fp64_face(ctx, S[0]);
     if (e) return cuda_fail(ctx, (cudaError_t)e, "face");
-    e = nsem_fp64_volume(&ctx->dev, &ctx->tab, &ctx->buf, stage, ctx->dt, S, U0, out, ctx->stream);
+    e = nsem_fp64_volume(&ctx->dev, &ctx->buf, stage, ctx->dt, S, U0, out, ctx->stream);
     return e ? cuda_fail(ctx, (cudaError_t)e, "volume") : NSEM_OK;
 }
 
@@ -511,7 +516,7 @@ nsem_status enqueue_steps(nsem_ctx* ctx, int nsteps, nsem_precision prec) {
         if (s != NSEM_OK) return s;
     } else {
         if (!ctx->mixed_ready) return fail(ctx, NSEM_UNSUPPORTED, ctx->err);
-        if ((e = nsem_mixed_steps(D, &ctx->mbuf, b, &ctx->tab, nsteps, ctx->dt, st)))
+        if ((e = nsem_mixed_steps(D, &ctx->mbuf, b, nsteps, ctx->dt, st)))
             return cuda_fail(ctx, (cudaError_t)e, "mixed step");
     }
     return NSEM_OK;
@@ -712,7 +717,7 @@ nsem_status nsem_tendency(nsem_ctx* ctx, nsem_precision prec, double* const L[5]
         if ((rs = fp64_stage(ctx, 0, b->u, b->u, b->L)) != NSEM_OK) return rs;
     } else if (prec == NSEM_MIXED) {
         if (!ctx->mixed_ready) return fail(ctx, NSEM_UNSUPPORTED, ctx->err);
-        if ((e = nsem_mixed_tendency(D, &ctx->mbuf, b, &ctx->tab, st)))
+        if ((e = nsem_mixed_tendency(D, &ctx->mbuf, b, st)))
             return cuda_fail(ctx, (cudaError_t)e, "mixed tendency");
     } else {
         return fail(ctx, NSEM_BAD_ARG, "unknown precision");
@@ -748,7 +753,7 @@ nsem_status nsem_step(nsem_ctx* ctx, int nsteps, nsem_scheme scheme, nsem_precis
         NSEM_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
         nsem_status s;
         if (form == 2) {
-            const int e = nsem_seg_steps(&ctx->dev, &ctx->tab, &ctx->sbuf, nsteps, ctx->dt, ctx->stream);
+            const int e = nsem_seg_steps(&ctx->dev, &ctx->sbuf, nsteps, ctx->dt, ctx->stream);
             s = e ? cuda_fail(ctx, (cudaError_t)e, "segregated step") : NSEM_OK;
         } else {
             s = enqueue_steps(ctx, nsteps, prec);
@@ -901,7 +906,7 @@ extern "C" nsem_status nsem_vjp(nsem_ctx* ctx, const double* const w[5], double*
     const size_t bytes = (size_t)ctx->dev.n_int * sizeof(double);
     for (int v = 0; v < 5; v++)
         NSEM_CUDA(cudaMemcpyAsync(A.lam[v], w[v], bytes, cudaMemcpyHostToDevice, ctx->stream));
-    int e = nsem_adj_vjp(&ctx->dev, &ctx->tab, ctx->buf.u, A.lam, A.g, &A, ctx->stream);
+    int e = nsem_adj_vjp(&ctx->dev, ctx->buf.u, A.lam, A.g, &A, ctx->stream);
     if (e) return cuda_fail(ctx, (cudaError_t)e, "vjp");
     for (int v = 0; v < 5; v++)
         NSEM_CUDA(cudaMemcpyAsync(g[v], A.g[v], bytes, cudaMemcpyDeviceToHost, ctx->stream));
@@ -921,7 +926,7 @@ extern "C" nsem_status nsem_jvp(nsem_ctx* ctx, const double* const dv[5], double
     const size_t bytes = (size_t)ctx->dev.n_int * sizeof(double);
     for (int v = 0; v < 5; v++)
         NSEM_CUDA(cudaMemcpyAsync(A.lam[v], dv[v], bytes, cudaMemcpyHostToDevice, ctx->stream));
-    int e = nsem_adj_jvp(&ctx->dev, &ctx->tab, ctx->buf.u, A.lam, A.g, &A, ctx->stream);
+    int e = nsem_adj_jvp(&ctx->dev, ctx->buf.u, A.lam, A.g, &A, ctx->stream);
     if (e) return cuda_fail(ctx, (cudaError_t)e, "jvp");
     for (int v = 0; v < 5; v++)
         NSEM_CUDA(cudaMemcpyAsync(Ld[v], A.g[v], bytes, cudaMemcpyDeviceToHost, ctx->stream));
@@ -961,13 +966,13 @@ extern "C" nsem_status nsem_tlm(nsem_ctx* ctx, int nsteps, const double* const d
     for (int step = 0; step < nsteps && s == NSEM_OK && !e; step++) {
         if ((s = fp64_step(ctx, u0, u1, u2, nullptr)) != NSEM_OK) break;
         /* du1 = du + dt J(u^n) du */
-        if ((e = nsem_adj_jvp(&ctx->dev, &ctx->tab, u0, A.lam, A.g, &A, st))) break;
+        if ((e = nsem_adj_jvp(&ctx->dev, u0, A.lam, A.g, &A, st))) break;
         if ((e = nsem_adj_lin3(A.lu1, A.lam, 1.0, A.g, dt, nullptr, 0, n, st))) break;
         /* du2 = 3/4 du + 1/4 (du1 + dt J(u1) du1) */
-        if ((e = nsem_adj_jvp(&ctx->dev, &ctx->tab, u1, A.lu1, A.g, &A, st))) break;
+        if ((e = nsem_adj_jvp(&ctx->dev, u1, A.lu1, A.g, &A, st))) break;
         if ((e = nsem_adj_lin3(A.lu2, A.lam, 0.75, A.lu1, 0.25, A.g, 0.25 * dt, n, st))) break;
         /* du^{n+1} = 1/3 du + 2/3 (du2 + dt J(u2) du2) */
-        if ((e = nsem_adj_jvp(&ctx->dev, &ctx->tab, u2, A.lu2, A.g, &A, st))) break;
+        if ((e = nsem_adj_jvp(&ctx->dev, u2, A.lu2, A.g, &A, st))) break;
         if ((e = nsem_adj_lin3(A.lam, A.lam, 1.0 / 3.0, A.lu2, 2.0 / 3.0, A.g, 2.0 / 3.0 * dt, n, st))) break;
         /* u^{n+1}, in place */
         s = fp64_stage(ctx, 3, u2, u0, ctx->buf.u);
@@ -1176,7 +1181,7 @@ static int reverse_stage(nsem_ctx* ctx, double* const* S, double* const* W, doub
         l.z[v] = z ? z[v] : nullptr;
     }
     l.cx = cx; l.cy = cy; l.cz = cz; l.cg = cg;
-    return nsem_adj_vjp_lin(&ctx->dev, &ctx->tab, S, W, l, &ctx->abuf, ctx->stream);
+    return nsem_adj_vjp_lin(&ctx->dev, S, W, l, &ctx->abuf, ctx->stream);
 }
 
 extern "C" nsem_status nsem_adjoint(nsem_ctx* ctx, const double* const lam_final[5],
@@ -1305,7 +1310,7 @@ extern "C" nsem_status nsem_convection_step(nsem_ctx* ctx, int nsteps) {
     if (it == ctx->graphs.end()) {
         cudaGraph_t g;
         NSEM_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-        const int e = nsem_conv_steps(&ctx->dev, &ctx->tab, &C, nsteps, ctx->dt, ctx->stream);
+        const int e = nsem_conv_steps(&ctx->dev, &C, nsteps, ctx->dt, ctx->stream);
         cudaError_t ce = cudaStreamEndCapture(ctx->stream, &g);
         if (e) {
             if (ce == cudaSuccess) cudaGraphDestroy(g);
@@ -1367,7 +1372,7 @@ extern "C" nsem_status nsem_convection_step_scaled(nsem_ctx* ctx, int nsteps, co
     if (!C.ready) return fail(ctx, NSEM_BAD_ARG, "nsem_convection_set was not called");
     if (nsteps == 0) return NSEM_OK;
     NSEM_CUDA(cudaSetDevice(ctx->device));
-    const int e = nsem_conv_steps_wind(&ctx->dev, &ctx->tab, &C, nsteps, ctx->dt, scale, ctx->stream);
+    const int e = nsem_conv_steps_wind(&ctx->dev, &C, nsteps, ctx->dt, scale, ctx->stream);
     if (e) return cuda_fail(ctx, (cudaError_t)e, "convection step");
     NSEM_CUDA(cudaMemcpyAsync(ctx->h_status, ctx->dev.status, sizeof(uint32_t),
                               cudaMemcpyDeviceToHost, ctx->stream));
@@ -1429,7 +1434,7 @@ nsem_status nsem_profile(nsem_ctx* ctx, int nsteps, nsem_precision prec, double 
                 s = timed(1, [&] { return fp64_face(ctx, S[0]); });
                 if (s == NSEM_OK)
                     s = timed(2, [&] {
-                        return nsem_fp64_volume(D, &ctx->tab, b, stage, ctx->dt, S, b->u,
+                        return nsem_fp64_volume(D, b, stage, ctx->dt, S, b->u,
                                                 stage == 3 ? b->u : b->s, st);
                     });
             }
@@ -1441,7 +1446,7 @@ nsem_status nsem_profile(nsem_ctx* ctx, int nsteps, nsem_precision prec, double 
             for (int k = 0; k < nsem_mixed_launches_per_step() && s == NSEM_OK; k++) {
                 int cls = nsem_mixed_launch_class(k);
                 s = timed(cls, [&] {
-                    return nsem_mixed_launch(D, &ctx->mbuf, b, &ctx->tab, k, n == 0, ctx->dt, st);
+                    return nsem_mixed_launch(D, &ctx->mbuf, b, k, n == 0, ctx->dt, st);
                 });
             }
         }

@@ -18,9 +18,9 @@
  * Tables come from nsem_pow_tables.h (gen_pow_tables.py, 200-bit mpmath).
  *
  * Evaluation order (Ziv's strategy, A. Ziv, ACM TOMS 17(3), 1991): a first
- * phase evaluates x^y to about 2^-66 relative and tests whether every value
+ * phase evaluates x^y to about 2^-70 relative and tests whether every value
  * within the phase's error bound rounds to the same double; only when it does
- * not (about one call in 2^11) does the accurate double-double phase above
+ * not (about one call in 2^14) does the accurate double-double phase above
  * run.  For exponents in [2^-11, 8) the first phase is nsem_pow_int, in 64- and
  * 96-bit fixed point on the integer pipes (the FP64 pipe, which bounds the
  * callers, issues 1.6 instructions per clock and SM, and a call of the
@@ -398,18 +398,20 @@ NSEM_HD nsem_u4 nsem_row(const nsem_u4* p) {
 /* Fixed-point phase of x^y for normal x > 0 and y in [2^-11, 8), correctly
  * rounded, or 0 when its rounding test cannot decide (or out of domain).
  *
- *   x = 2^e m, m k_i / 1024 = 1 + z, 0 <= z < 2^-6.6 exact (62 bits),
- *   log2 m = -log2(k_i / 1024) + z (c1 - z (c2 - z (.. - z c10))),
- *     c_n = 1 / (n ln 2); the tail is below 2^-74, the sum within 2^-67.5;
+ *   x = 2^e m, m k_i / 8192 = 1 + z, 0 <= z < 2^-9.6 exact (65 bits),
+ *   log2 m = -log2(k_i / 8192) + z (c1 - z (c2 - z (.. - z c7))),
+ *     c_n = 1 / (n ln 2); the tail is below 2^-79, the sum within 2^-70.4;
  *   y log2 x = n + phi, phi in [0, 1) to 96 bits, from the integer and the
  *     fraction of y;
- *   2^phi = 2^(j/128) (1 + rho (d1 + rho (.. + rho d7))), rho < 2^-7,
- *     d_n = (ln 2)^n / n!; the tail is below 2^-75, the sum within 2^-69.
+ *   2^phi = 2^(j/1024) (1 + rho (d1 + rho (.. + rho d6))), rho < 2^-10,
+ *     d_n = (ln 2)^n / n!; the tail is below 2^-86, the sum within 2^-72.
  * Every step truncates; a multiplication by z (or rho) moves the scale of the
- * next coefficient by 6 (7) bits, so all steps err by about a unit at the
+ * next coefficient by 9 (10) bits, so all steps err by about a unit at the
  * final scale, and the high-order ones fit 32 bits.  In units of the 96-bit
- * result (2^-95) the error is below (floor(y) + 1) 2^28.3 + 2^27.2; the test
- * uses (floor(y) + 2) 2^29. */
+ * result (2^-95) the error is below (floor(y) + 1) 2^25.2 + 2^24; the test
+ * uses (floor(y) + 2) 2^26.  (Tables of 128 rows leave eight times as many
+ * calls undecided; a small grid then nearly always waits for one warp in the
+ * accurate phase, some ten microseconds.) */
 NSEM_HD int nsem_pow_int(double x, double y, double* out) {
     const uint64_t ux = nsem_bits(x), uy = nsem_bits(y);
     const uint32_t ex = (uint32_t)(ux >> 52), ey = (uint32_t)(uy >> 52);
@@ -419,23 +421,20 @@ NSEM_HD int nsem_pow_int(double x, double y, double* out) {
     const uint32_t yi = (uint32_t)(Y >> (1075u - ey));
     const uint64_t G = Y << (ey - 1011u);                  /* fraction of y, 2^-64 */
     /* log2 of the significand */
-    const nsem_u4 t = nsem_row(&NSEM_ILOG[(uint32_t)(M >> 45) & 127u]);
-    const uint64_t Z = (M * t.a - 0x4000000000000000ull) << 8;     /* z, 2^-70 */
+    const nsem_u4 t = nsem_row(&NSEM_ILOG[(uint32_t)(M >> 42) & 1023u]);
+    const uint64_t Z = (M * t.a) << 8;                     /* z, 2^-73 (m k_i = 2^65 (1 + z)) */
     const uint32_t z32 = (uint32_t)(Z >> 32);
-    uint32_t q = NSEM_ILOG_C9 - nsem_mulhi32(z32, NSEM_ILOG_C10);
-    q = NSEM_ILOG_C8 - nsem_mulhi32(z32, q);
-    q = NSEM_ILOG_C7 - nsem_mulhi32(z32, q);
-    q = NSEM_ILOG_C6 - nsem_mulhi32(z32, q);
-    uint64_t p = NSEM_ILOG_C5 - nsem_mulhi32(z32, q);
-    p = NSEM_ILOG_C4 - nsem_mulhi64(Z, p);
+    uint32_t q = NSEM_ILOG_C6 - nsem_mulhi32(z32, NSEM_ILOG_C7);
+    q = NSEM_ILOG_C5 - nsem_mulhi32(z32, q);
+    uint64_t p = NSEM_ILOG_C4 - nsem_mulhi32(z32, q);
     p = NSEM_ILOG_C3 - nsem_mulhi64(Z, p);
     p = NSEM_ILOG_C2 - nsem_mulhi64(Z, p);
     p = NSEM_ILOG_C1 - nsem_mulhi64(Z, p);
-    const uint64_t l = nsem_mulhi64(Z, p);                         /* log2(1 + z), 2^-69 */
+    const uint64_t l = nsem_mulhi64(Z, p);                         /* log2(1 + z), 2^-72 */
     /* F = log2 m in 96 bits; log2 x = e + F */
-    const uint64_t f0 = (uint64_t)t.d + ((uint32_t)l << 27);
+    const uint64_t f0 = (uint64_t)t.d + ((uint32_t)l << 24);
     const uint64_t T = (uint64_t)t.b << 32 | t.c;
-    const uint64_t Fh1 = T + (l >> 5);
+    const uint64_t Fh1 = T + (l >> 8);
     const uint64_t Fh = Fh1 + (f0 >> 32);
     const uint32_t Fl = (uint32_t)f0;
     const int32_t e = (int32_t)ex - 1023 + (int32_t)((Fh1 < T) | (Fh < Fh1));
@@ -453,24 +452,23 @@ NSEM_HD int nsem_pow_int(double x, double y, double* out) {
     if (!(n > -1022 && n < 1023)) return 0;
     /* 2^phi */
     const uint32_t ph = (uint32_t)s2, pm = (uint32_t)s1, pl = (uint32_t)s0;
-    const nsem_u4 w = nsem_row(&NSEM_IEXP2[ph >> 25]);
-    const uint64_t r = ((uint64_t)ph << 32 | pm) << 7 | pl >> 25;  /* rho, 2^-71 */
+    const nsem_u4 w = nsem_row(&NSEM_IEXP2[ph >> 22]);
+    const uint64_t r = ((uint64_t)ph << 32 | pm) << 10 | pl >> 22; /* rho, 2^-74 */
     const uint32_t r32 = (uint32_t)(r >> 32);
-    uint32_t d = NSEM_IEXP_D6 + nsem_mulhi32(r32, NSEM_IEXP_D7);
-    d = NSEM_IEXP_D5 + nsem_mulhi32(r32, d);
-    uint64_t c = NSEM_IEXP_D4 + nsem_mulhi32(r32, d);
-    c = NSEM_IEXP_D3 + nsem_mulhi64(r, c);
+    uint32_t d = NSEM_IEXP_D5 + nsem_mulhi32(r32, NSEM_IEXP_D6);
+    d = NSEM_IEXP_D4 + nsem_mulhi32(r32, d);
+    uint64_t c = NSEM_IEXP_D3 + nsem_mulhi32(r32, d);
     c = NSEM_IEXP_D2 + nsem_mulhi64(r, c);
     c = NSEM_IEXP_D1 + nsem_mulhi64(r, c);
-    const uint64_t E = nsem_mulhi64(r, c);                         /* 2^rho - 1, 2^-71 */
+    const uint64_t E = nsem_mulhi64(r, c);                         /* 2^rho - 1, 2^-74 */
     const uint64_t W = (uint64_t)w.a << 32 | w.b;
-    const uint64_t TE = nsem_mulhi64(W, E);                        /* 2^-70 */
-    const uint64_t r0 = (uint64_t)w.c + ((uint32_t)TE << 25);
-    const uint64_t Rh = W + (TE >> 7) + (r0 >> 32);
+    const uint64_t TE = nsem_mulhi64(W, E);                        /* 2^-73 */
+    const uint64_t r0 = (uint64_t)w.c + ((uint32_t)TE << 22);
+    const uint64_t Rh = W + (TE >> 10) + (r0 >> 32);
     if (!(Rh >> 63)) return 0;                                     /* carried past 2 */
     /* rounding test on the 43 bits below the significand */
     const int64_t rem = (int64_t)((Rh & 0x7ffu) << 32 | (uint32_t)r0) - ((int64_t)1 << 42);
-    const int64_t lim = (int64_t)(yi + 2u) << 29;
+    const int64_t lim = (int64_t)(yi + 2u) << 26;
     if (rem <= lim && rem >= -lim) return 0;
     const uint64_t m = (Rh >> 11) + (rem > 0) + ((uint64_t)(n + 1022) << 52);
     *out = nsem_from_bits((uint32_t)(m >> 32), (uint32_t)m);

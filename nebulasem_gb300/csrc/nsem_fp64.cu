@@ -20,7 +20,8 @@
  *           L = -Su/cV, Shu-Osher combination, primitives of the new state.
  * Roofline: FP64-pipe bound (hundreds of FP64 instructions per node-stage
  * against 40-80 bytes of traffic); products with the zeros of a diagonal
- * metric or an axis normal are left out (nsem_gather.cuh).
+ * metric or an axis normal are left out and the other products, divisions,
+ * roots and the power run on the integer pipes (nsem_gather.cuh, nsem_intfp.h).
  */
 #include <cuda_runtime.h>
 
@@ -83,6 +84,26 @@ struct PrimArgs {
     double* prim[NSEM_NPRIM];
 };
 
+/* p', |U| and c of (r, U, T); INT: all mild, and the fluid's constants
+ * (tame_const) */
+template <bool INT>
+__device__ __forceinline__ void prim_rest(const NsemDev& m, double r, const double* U, double T,
+                                          double* const* prim, int64_t i) {
+    const double x = nsem_div_by(nsem_x<INT>(m.R, nsem_x<INT>(r, T)), m.dP0);
+    const double y = nsem_pow(x, m.gamma);
+    /* the power of a mild argument can leave that range */
+    const double p = nsem_mild(y) ? nsem_x<INT>(m.P0, y) : m.P0 * y;
+    /* the sum of squares' trailing + 0.0 changes no square */
+    const double uu = nsem_x<INT>(U[0], U[0]) + (nsem_x<INT>(U[1], U[1]) + nsem_x<INT>(U[2], U[2]));
+    prim[0][i] = U[0];
+    prim[1][i] = U[1];
+    prim[2][i] = U[2];
+    prim[3][i] = T;
+    prim[4][i] = p - m.p_ref[i];
+    prim[5][i] = nsem_sqrt(uu);
+    prim[6][i] = nsem_sqrt(nsem_x<INT>(m.gR, T));
+}
+
 /* primitives of the state S at node i */
 __device__ __forceinline__ void prim_at(const NsemDev& m, const double* S, double* const* prim,
                                         int64_t i) {
@@ -93,14 +114,10 @@ __device__ __forceinline__ void prim_at(const NsemDev& m, const double* S, doubl
     U[1] = nsem_div_by(S[2], dr);
     U[2] = nsem_div_by(S[3], dr);
     const double T = nsem_div_by(S[4], dr);
-    const double p = m.P0 * nsem_pow(nsem_div_by((r * T) * m.R, m.dP0), m.gamma);
-    prim[0][i] = U[0];
-    prim[1][i] = U[1];
-    prim[2][i] = U[2];
-    prim[3][i] = T;
-    prim[4][i] = p - m.p_ref[i];
-    prim[5][i] = nsem_sqrt(vdot3(U, U));
-    prim[6][i] = nsem_sqrt(m.gR * T);
+    if (m.tame_const && nsem_mild(r) && nsem_mild(U[0]) && nsem_mild(U[1]) && nsem_mild(U[2]) && nsem_mild(T))
+        prim_rest<true>(m, r, U, T, prim, i);
+    else
+        prim_rest<false>(m, r, U, T, prim, i);
 }
 
 __global__ void __launch_bounds__(256) k_prim(const NsemDev m, PrimArgs a) {
@@ -186,7 +203,55 @@ __global__ void __launch_bounds__(128) k_mortar_coupled_gather(const NsemDev m, 
     }
 }
 
-__global__ void __launch_bounds__(256) k_face(const NsemDev m, FaceArgs a) {
+/* the five lifted values of a slot whose normal lies along axis ax (FP64-pipe
+ * bound: about 60 operations instead of 190, with INT 20 and the products on
+ * the integer pipes; 14 x 12 x 13 elements of order 4: 92 -> 38 -> 25 us) */
+template <bool INT>
+__device__ __forceinline__ void face_axis(const NsemDev& m, const FaceArgs& a, int64_t k, int ax,
+                                          const double* n, const double* en, double fi, double fo,
+                                          double lam, double r1, const double* U1, double T1, double p1,
+                                          double r2, const double* U2, double T2, double p2,
+                                          int32_t c1, int32_t c2) {
+    const double na = nsem_pick(ax, n[0], n[1], n[2]), ea = nsem_pick(ax, en[0], en[1], en[2]);
+    const double Ua1 = nsem_pick(ax, U1[0], U1[1], U1[2]), Ua2 = nsem_pick(ax, U2[0], U2[1], U2[2]);
+    double Fc1[3], Fc2[3];
+    for (int c = 0; c < 3; c++) {
+        Fc1[c] = nsem_x<INT>(r1, U1[c]);
+        Fc2[c] = nsem_x<INT>(r2, U2[c]);
+    }
+    const double Fa1 = nsem_pick(ax, Fc1[0], Fc1[1], Fc1[2]);
+    const double Fa2 = nsem_pick(ax, Fc2[0], Fc2[1], Fc2[2]);
+    /* artificial viscosity: mu = rho nu */
+    const double mu1 = a.G[0] ? nsem_x<INT>(m.nu, r1) : 0.0, mu2 = a.G[0] ? nsem_x<INT>(m.nu, r2) : 0.0;
+    auto avg = [&](double x, double y) { return nsem_x<INT>(fi, x) + nsem_x<INT>(fo, y); };
+    a.d[0][k] = nsem_x<INT>(na, avg(Fa1, Fa2) - nsem_signed(ea, nsem_x<INT>(lam, r2 - r1)));
+    const double dq = nsem_signed(ea, nsem_x<INT>(lam, Fa2 - Fa1));
+    for (int r = 0; r < 3; r++) {
+        double A = nsem_x<INT>(Ua1, Fc1[r]), B = nsem_x<INT>(Ua2, Fc2[r]);
+        /* the pressure sits on the diagonal: p added there, 0 elsewhere */
+        if (r == ax) { A += p1; B += p2; }
+        if (a.G[0]) {
+            const double* g = r == ax ? a.G[r] : a.G[r == 0 ? (ax == 1 ? XY : XZ)
+                                                     : r == 1 ? (ax == 2 ? YZ : YX) : (ax == 0 ? ZX : ZY)];
+            A = A - nsem_x<INT>(mu1, g[c1]);
+            B = B - nsem_x<INT>(mu2, c2 >= 0 ? g[c2] : 0.0);
+        }
+        double F = avg(A, B);
+        if (r == ax) F -= dq;
+        a.d[1 + r][k] = nsem_x<INT>(na, F);
+    }
+    double x = nsem_x<INT>(T1, Fa1), y = nsem_x<INT>(T2, Fa2);
+    if (a.G[0]) {
+        x = x - nsem_x<INT>(nsem_x<INT>(m.iPr, mu1), a.G[9 + ax][c1]);
+        y = y - nsem_x<INT>(nsem_x<INT>(m.iPr, mu2), c2 >= 0 ? a.G[9 + ax][c2] : 0.0);
+    }
+    a.d[4][k] = nsem_x<INT>(na, avg(x, y) - nsem_signed(ea, nsem_x<INT>(lam, nsem_x<INT>(r2, T2) - nsem_x<INT>(r1, T1))));
+}
+
+/* FACE threads a CTA, so that a small mesh's slots spread over the SMs */
+constexpr int FACE = 64;
+
+__global__ void __launch_bounds__(FACE) k_face(const NsemDev m, FaceArgs a) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= m.n_slot) return;   /* a CTA has at least one slot */
     const int32_t c1 = m.c1[k], c2 = m.c2[k];
@@ -227,51 +292,32 @@ __global__ void __launch_bounds__(256) k_face(const NsemDev m, FaceArgs a) {
     if (side == 2) { mu2 = a.mq[0][ms]; cs2 = a.mq[1][ms]; r2v = a.mq[5][ms]; }
     const double lam = ((mu1v * fi + mu2 * fo) + (cs1v * fi + cs2 * fo)) / 2;
 
-    /* a normal along one axis (FP64-pipe bound: about 60 operations instead of
-     * 190): only the flux tensor's column of that axis meets a nonzero
-     * normal component; the products left out are zeros that change no sum
-     * (the lift starts at +0), provided nothing can overflow */
+    /* a normal along one axis: only the flux tensor's column of that axis meets
+     * a nonzero normal component; the products left out are zeros that change
+     * no sum (the lift starts at +0), provided nothing can overflow */
     const int ax = side == 0 ? nsem_axis_of(n, en) : -1;
-    bool gok = true;
-    if (ax >= 0 && a.G[0])
-        for (int c = 0; c < 12; c++)
-            gok = gok && nsem_bounded(a.G[c][c1]) && (c2 < 0 || nsem_bounded(a.G[c][c2]));
-    if (ax >= 0 && gok && nsem_bounded(r1) && nsem_bounded(r2) && nsem_bounded(T1) && nsem_bounded(T2) &&
-        nsem_bounded(p1) && nsem_bounded(p2) && nsem_bounded(lam) && nsem_bounded(U1[0]) &&
-        nsem_bounded(U1[1]) && nsem_bounded(U1[2]) && nsem_bounded(U2[0]) && nsem_bounded(U2[1]) &&
-        nsem_bounded(U2[2])) {
-        const double na = nsem_pick(ax, n[0], n[1], n[2]), ea = nsem_pick(ax, en[0], en[1], en[2]);
-        const double Ua1 = nsem_pick(ax, U1[0], U1[1], U1[2]), Ua2 = nsem_pick(ax, U2[0], U2[1], U2[2]);
-        const double Fc1[3] = {U1[0] * r1, U1[1] * r1, U1[2] * r1};
-        const double Fc2[3] = {U2[0] * r2, U2[1] * r2, U2[2] * r2};
-        const double Fa1 = nsem_pick(ax, Fc1[0], Fc1[1], Fc1[2]);
-        const double Fa2 = nsem_pick(ax, Fc2[0], Fc2[1], Fc2[2]);
-        /* artificial viscosity: mu = rho nu */
-        const double mu1 = a.G[0] ? r1 * m.nu : 0.0, mu2 = a.G[0] ? r2 * m.nu : 0.0;
-        a.d[0][k] = ((Fa1 * fi + Fa2 * fo) - nsem_signed(ea, lam * (r2 - r1))) * na;
-        const double dq = nsem_signed(ea, (Fa2 - Fa1) * lam);
-        for (int r = 0; r < 3; r++) {
-            double A = Fc1[r] * Ua1, B = Fc2[r] * Ua2;
-            /* the pressure sits on the diagonal: p added there, 0 elsewhere */
-            const double A1 = A + p1, B1 = B + p2;
-            if (r == ax) { A = A1; B = B1; }
-            if (a.G[0]) {
-                const double* g = r == ax ? a.G[r] : a.G[r == 0 ? (ax == 1 ? XY : XZ)
-                                                         : r == 1 ? (ax == 2 ? YZ : YX) : (ax == 0 ? ZX : ZY)];
-                A = A - mu1 * g[c1];
-                B = B - mu2 * (c2 >= 0 ? g[c2] : 0.0);
-            }
-            const double F = A * fi + B * fo;
-            const double Fj = F - dq;
-            a.d[1 + r][k] = (r == ax ? Fj : F) * na;
-        }
-        double x = Fa1 * T1, y = Fa2 * T2;
+    if (ax >= 0) {
+        bool bounded = true, mild = true;
+        auto look = [&](double x) {
+            bounded = bounded && nsem_bounded(x);
+            mild = mild && nsem_mild(x);
+        };
+        look(r1); look(r2); look(T1); look(T2); look(p1); look(p2); look(lam);
+        look(fi); look(fo);
+        for (int c = 0; c < 3; c++) { look(U1[c]); look(U2[c]); look(n[c]); }
         if (a.G[0]) {
-            x = x - (mu1 * m.iPr) * a.G[9 + ax][c1];
-            y = y - (mu2 * m.iPr) * (c2 >= 0 ? a.G[9 + ax][c2] : 0.0);
+            look(m.nu);
+            look(m.iPr);
+            for (int c = 0; c < 12; c++) {
+                look(a.G[c][c1]);
+                if (c2 >= 0) look(a.G[c][c2]);
+            }
         }
-        a.d[4][k] = ((x * fi + y * fo) - nsem_signed(ea, lam * (r2 * T2 - r1 * T1))) * na;
-        return;
+        if (bounded) {
+            if (mild) face_axis<true>(m, a, k, ax, n, en, fi, fo, lam, r1, U1, T1, p1, r2, U2, T2, p2, c1, c2);
+            else face_axis<false>(m, a, k, ax, n, en, fi, fo, lam, r1, U1, T1, p1, r2, U2, T2, p2, c1, c2);
+            return;
+        }
     }
 
     /* continuity: flux U rho, state rho */
@@ -367,13 +413,26 @@ struct VolArgs {
 constexpr int SM_W = 24;
 constexpr unsigned SM_ROWS = 0xe;   /* the momentum equations are tensor rows */
 
-__global__ void k_volume(const NsemDev m, const NsemTables tab, VolArgs a) {
+/* the Shu-Osher combination of a stage; INT: operands mild (a sum that is not
+ * mild takes its product in FP64) */
+template <bool INT>
+__device__ __forceinline__ void update(int stage, double dt, const double* S, const double* U0,
+                                       const double* L, double* nu) {
+    const double cu = stage == 2 ? 0.75 : 1.0 / 3.0, cs = stage == 2 ? 0.25 : 2.0 / 3.0;
+    for (int c = 0; c < 5; c++) {
+        const double s = S[c] + nsem_x<INT>(dt, L[c]);
+        nu[c] = stage == 1 ? s
+                           : nsem_x<INT>(cu, U0[c]) + (!INT || nsem_mild(s) ? nsem_x<INT>(cs, s) : cs * s);
+    }
+}
+
+/* registers for the largest element (1000 nodes, N+1 = 10) */
+__global__ void __launch_bounds__(1024) k_volume(const NsemDev m, VolArgs a) {
     extern __shared__ double sm[];
     const int NPX = m.npx, NPY = m.npy, NPZ = m.npz, NP = m.np;
     double* dps = sm + (size_t)NP * SM_W;           /* 3 * npd^2 tables */
     const int t = threadIdx.x;
-    for (int q = t; q < 3 * NSEM_MAX_NPD * NSEM_MAX_NPD; q += blockDim.x)
-        dps[q] = (&tab.dpsi[0][0])[q];
+    nsem_load_tables(m, dps, t);
 
     const int64_t e = blockIdx.x;
     const bool active = t < NP;
@@ -388,24 +447,24 @@ __global__ void k_volume(const NsemDev m, const NsemTables tab, VolArgs a) {
         T = a.prim[3][node];
         pp = a.prim[4][node];
         double* my = sm + (size_t)t * SM_W;
-        const double Fc[3] = {U[0] * rho, U[1] * rho, U[2] * rho};
-        double fm[9];
-        outer(Fc, U, fm);                                     /* U*rho == rho*U */
-        for (int c = 0; c < 9; c++) fm[c] = fm[c] + ((c < 3) ? 1.0 : 0.0) * pp;
-        double ft[3] = {Fc[0] * T, Fc[1] * T, Fc[2] * T};
+        const bool mild = nsem_mild(rho) && nsem_mild(U[0]) && nsem_mild(U[1]) && nsem_mild(U[2]) &&
+                          nsem_mild(T) && nsem_bounded(pp);
+        double Fc[3];
+        for (int c = 0; c < 3; c++) Fc[c] = mild ? nsem_x<true>(rho, U[c]) : rho * U[c];
+        if (mild) nsem_flux_columns<5, 1, true>(my, Fc, U, T, pp);
+        else nsem_flux_columns<5, 1, false>(my, Fc, U, T, pp);
+        for (int c = 0; c < 3; c++) my[5 * c] = Fc[c];        /* U*rho == rho*U */
         if (a.G[0]) {
             const double mu = rho * m.nu;
-            for (int c = 0; c < 9; c++) fm[c] = fm[c] - mu * a.G[c][node];
-            for (int c = 0; c < 3; c++) ft[c] = ft[c] - (mu * m.iPr) * a.G[9 + c][node];
-        }
-        const int col[3][3] = {{XX, YX, ZX}, {XY, YY, ZY}, {XZ, YZ, ZZ}};
-        for (int c = 0; c < 3; c++) {
-            my[5 * c] = Fc[c];
-            for (int r = 0; r < 3; r++) my[5 * c + 1 + r] = fm[col[c][r]];
-            my[5 * c + 4] = ft[c];
+            for (int c = 0; c < 3; c++) {
+                const int row[3] = {c == 0 ? XX : c == 1 ? XY : XZ, c == 0 ? YX : c == 1 ? YY : YZ,
+                                    c == 0 ? ZX : c == 1 ? ZY : ZZ};
+                for (int r = 0; r < 3; r++) my[5 * c + 1 + r] -= mu * a.G[row[r]][node];
+                my[5 * c + 4] -= (mu * m.iPr) * a.G[9 + c][node];
+            }
         }
     }
-    const bool diag = __syncthreads_and(!active || nsem_node_diag<5>(sm + (size_t)t * SM_W));
+    const int kind = nsem_element_kind<5>(m, active, sm + (size_t)t * SM_W);
     if (!active) return;
 
     /* surface lift, in the order div_flux visits the element's faces */
@@ -425,16 +484,13 @@ __global__ void k_volume(const NsemDev m, const NsemTables tab, VolArgs a) {
      * arrive in lexicographic order of b: X-line below, Y-line below, Z-line
      * below, self, Z above, Y above, X above. */
     nsem_chain_begin();
-    nsem_volume_gather<5, SM_W, SM_ROWS>(NPX, NPY, NPZ, sm, dps, t, diag, r);
+    nsem_volume_gather<5, SM_W, SM_ROWS>(NPX, NPY, NPZ, sm, dps, t, kind, r);
 
     /* gravity source: Su -= ((rho - rho_ref) g) cV */
     const double cv = m.cv[node];
     {
         const double s = rho - m.rho_ref[node];
-        const double sc0 = 0.0 + m.g[0] * s, sc1 = 0.0 + m.g[1] * s, sc2 = 0.0 + m.g[2] * s;
-        r[1] = r[1] - sc0 * cv;
-        r[2] = r[2] - sc1 * cv;
-        r[3] = r[3] - sc2 * cv;
+        for (int c = 0; c < 3; c++) r[1 + c] = nsem_sub_source(r[1 + c], m.g[c], s, cv);
     }
     const nsem_divisor dcv = nsem_make_divisor(cv);
     double L[5];
@@ -445,25 +501,22 @@ __global__ void k_volume(const NsemDev m, const NsemTables tab, VolArgs a) {
         return;
     }
     double nu[5];
-    const double dt = a.dt;
-    if (a.stage == 1) {
-        for (int c = 0; c < 5; c++) nu[c] = a.S[c][node] + dt * L[c];
-    } else if (a.stage == 2) {
-        for (int c = 0; c < 5; c++) {
-            const double s = a.S[c][node] + dt * L[c];
-            nu[c] = 0.75 * a.U0[c][node] + 0.25 * s;
-        }
-    } else {
-        const double a3 = 1.0 / 3.0, b3 = 2.0 / 3.0;
-        for (int c = 0; c < 5; c++) {
-            const double s = a.S[c][node] + dt * L[c];
-            nu[c] = a3 * a.U0[c][node] + b3 * s;
-        }
+    bool finite = true, mild = nsem_mild(a.dt);
+    double S[5], U0[5];
+    for (int c = 0; c < 5; c++) {
+        S[c] = a.S[c][node];
+        mild = mild && nsem_mild(L[c]) && nsem_mild(S[c]);
     }
-    bool finite = true;
+    if (a.stage > 1)
+        for (int c = 0; c < 5; c++) {
+            U0[c] = a.U0[c][node];
+            mild = mild && nsem_mild(U0[c]);
+        }
+    if (mild) update<true>(a.stage, a.dt, S, U0, L, nu);
+    else update<false>(a.stage, a.dt, S, U0, L, nu);
     for (int c = 0; c < 5; c++) {
         a.out[c][node] = nu[c];
-        finite = finite && isfinite(nu[c]);
+        finite = finite && nsem_finite(nu[c]);
     }
     if (!finite) atomicOr(m.status, NSEM_STATUS_NONFINITE);
     /* primitives of the new stage state for the next face kernel */
@@ -498,12 +551,12 @@ extern "C" int nsem_fp64_face(const NsemDev* m, NsemBuf* b, const double* rho, v
      * against 6.25 ms), fewer warps leave the pipes idle either way */
     const int64_t warps = m->n_elem * ((m->np + 31) / 32) / 152;
     a.early = warps < 8 || warps > 32;
-    const int64_t blocks = (m->n_slot + 255) / 256;
+    const int64_t blocks = (m->n_slot + FACE - 1) / FACE;
     cudaStream_t st = (cudaStream_t)stream;
     const unsigned mb = (unsigned)((m->n_ms + 127) / 128);
     if (m->n_ms > 0) k_mortar_coupled<<<19 * mb, 128, 0, st>>>(*m, a);
     int e = launch_err();
-    if (!e) e = nsem_launch_chained(k_face, (unsigned)blocks, 256, 0, st, *m, a);
+    if (!e) e = nsem_launch_chained(k_face, (unsigned)blocks, FACE, 0, st, *m, a);
     if (e) return e;
     if (m->n_ms > 0) k_mortar_coupled_gather<<<5 * mb, 128, 0, st>>>(*m, a);
     return launch_err();
@@ -523,7 +576,7 @@ extern "C" int nsem_fp64_check_smem(const NsemDev* m) {
     return 0;
 }
 
-extern "C" int nsem_fp64_volume(const NsemDev* m, const NsemTables* t, NsemBuf* b, int stage,
+extern "C" int nsem_fp64_volume(const NsemDev* m, NsemBuf* b, int stage,
                                 double dt, const double* const* S, const double* const* U0,
                                 double* const* out, void* stream) {
     VolArgs a;
@@ -540,5 +593,5 @@ extern "C" int nsem_fp64_volume(const NsemDev* m, const NsemTables* t, NsemBuf* 
     for (int c = 0; c < 5; c++) a.dC[c] = b->dC[c];
     const int threads = ((m->np + 31) / 32) * 32;
     return nsem_launch_chained(k_volume, (unsigned)m->n_elem, (unsigned)threads, vol_smem(m),
-                               (cudaStream_t)stream, *m, *t, a);
+                               (cudaStream_t)stream, *m, a);
 }

@@ -13,30 +13,46 @@
  * sm: W doubles per node in shared memory: the NC flux values of each
  * direction, [3][NC] (value v of direction c at c NC + v), then the metric
  * Jinv cV at offset 3 NC (components XX,YY,ZZ,XY,YZ,XZ,YX,ZY,ZX); dps: the
- * three dpsi tables (dpsi[d][s * npd + i], NSEM_MAX_NPD^2 apart).  A source on
+ * three dpsi tables (nsem_load_tables).  A source on
  * a line contributes its own metric column times one derivative (J[col] D),
  * the node itself the product Jinv . (Dx_ii, Dy_jj, Dz_kk) -- the reference's
  * products, evaluated in its operand order.  r[v] -= the contribution.
  *
  * Bound by the FP64 pipe (about 1.6 instructions per clock and SM), so the
- * operation count is the time.  On an element whose metric is diagonal
- * (`diag`: every off-diagonal component of every node is zero) a line source
- * has dj = (0, .., J_cc D, .., 0), and the products with the zeros are zeros
- * that change no sum: r starts at +0 and is never -0, so subtracting either
- * zero leaves it, and x + (+-0) is x for x != 0.  Such an element takes
- * J_cc D times the direction's own NC values, 1 + 2 NC operations a source
- * instead of 3 + 6 NC, with the same bits; the node's own term is formed in
- * full once, before the loop.  Zero times infinity is NaN and not zero, hence
- * `diag` also asks for values bounded so that no skipped product can overflow
- * (nsem_bounded); any other element takes the full products.  Measured
- * on 14 x 12 x 13 elements of order 4: an SSP-RK3 stage 552 -> 338 us (with
- * the faces' counterpart), a convection step of order 5 on 12 x 14 x 10
- * 196 -> 97 us.
+ * FP64 operation count is the time:
+ *   - products run on the integer pipes (nsem_mul_normal: the same correctly
+ *     rounded product), beside the FP64 pipe's additions, on an element whose
+ *     values are zero or of a size at which every product is normal (`tame`);
+ *   - on an element whose metric is also diagonal (every off-diagonal component
+ *     of every node is zero) a line source has dj = (0, .., J_cc D, .., 0), and
+ *     the products with the zeros are zeros that change no sum: r starts at +0
+ *     and is never -0, so subtracting either zero leaves it, and x + (+-0) is x
+ *     for x != 0.  Such an element takes J_cc D times the direction's own NC
+ *     values, 1 + NC products and NC additions a source instead of 3 + 3 NC and
+ *     3 NC; the node's own term is formed in full once, before the loop.
+ * Zero times infinity is NaN and not zero, hence the bounds; any other element
+ * takes the full products in FP64.  Same bits on every path.  Measured on 14 x
+ * 12 x 13 elements of order 4, whole volume kernel: 453 us with the full
+ * products, 168 us with the zeros left out and the integer divisions and power
+ * (nsem_intfp.h, nsem_ddpow.h), 106 us with the integer products; a full metric
+ * (12^3 elements tilted by 30 degrees, 5 SSP-RK3 steps) 6.7 -> 3.1 ms.
  */
 #ifndef NSEM_GATHER_CUH
 #define NSEM_GATHER_CUH
 
 #include "nsem_internal.h"
+
+/* the derivative tables into shared memory (their used entries), coalesced;
+ * as a kernel parameter read per thread they serialise on the constant port,
+ * about two microseconds of a one-warp CTA */
+__device__ __forceinline__ void nsem_load_tables(const NsemDev& m, double* dps, int t) {
+    const int npd[3] = {m.npx, m.npy, m.npz};
+    for (int d = 0; d < 3; d++)
+        for (int q = t; q < npd[d] * npd[d]; q += blockDim.x) {
+            const int i = d * NSEM_MAX_NPD * NSEM_MAX_NPD + q;
+            dps[i] = m.dpsi[i];
+        }
+}
 
 /* |x| < 2^200 (false for infinities and NaN): products of up to five such
  * factors stay finite */
@@ -49,66 +65,94 @@ __device__ __forceinline__ bool nsem_is_zero(double x) {
     return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) == 0;
 }
 
-/* this node's part of `diag`: my = its record in the layout above */
+/* zero, or 2^-400 <= |x| < 2^200 */
+__device__ __forceinline__ bool nsem_tame(double x) {
+    const uint32_t h = (uint32_t)__double2hiint(x) & 0x7fffffffu;
+    return h - ((1023u - 400u) << 20) < (600u << 20) || (h | (uint32_t)__double2loint(x)) == 0u;
+}
+/* zero, or 2^-200 <= |x| < 2^200: a product with a tame value is normal or zero */
+__device__ __forceinline__ bool nsem_mild(double x) {
+    const uint32_t h = (uint32_t)__double2hiint(x) & 0x7fffffffu;
+    return h - ((1023u - 200u) << 20) < (400u << 20) || (h | (uint32_t)__double2loint(x)) == 0u;
+}
+
+/* zero, or within 2^+-140: a metric component whose product with a derivative
+ * (host-checked to be zero or within 2^+-60) is mild */
+__device__ __forceinline__ bool nsem_metric_tame(double J) {
+    const uint32_t h = (uint32_t)__double2hiint(J) & 0x7fffffffu;
+    return h - ((1023u - 140u) << 20) < (280u << 20) || (h | (uint32_t)__double2loint(J)) == 0u;
+}
+
+/* what nsem_volume_gather may do on an element: bit 0 every value tame, bit 1
+ * the metric diagonal too */
+enum { NSEM_EL_TAME = 1, NSEM_EL_DIAG = 2 };
+
+/* this node's part of it: my = its record in the layout above.  */
 template <int NC>
-__device__ __forceinline__ bool nsem_node_diag(const double* my) {
-    bool ok = true;
+__device__ __forceinline__ int nsem_node_kind(const double* my) {
+    bool tame = true, diag = true;
 #pragma unroll
-    for (int c = 0; c < 3 * NC + 3; c++) ok = ok && nsem_bounded(my[c]);
+    for (int c = 0; c < 3 * NC; c++) tame = tame && nsem_tame(my[c]);
 #pragma unroll
-    for (int c = 3; c < 9; c++) ok = ok && nsem_is_zero(my[3 * NC + c]);
-    return ok;
+    for (int c = 0; c < 9; c++) {
+        const double J = my[3 * NC + c];
+        tame = tame && nsem_metric_tame(J);
+        if (c >= 3) diag = diag && nsem_is_zero(J);
+    }
+    return (tame ? NSEM_EL_TAME : 0) | (tame && diag ? NSEM_EL_DIAG : 0);
+}
+
+/* the element's kind from its nodes' (barriers of the whole CTA) */
+template <int NC>
+__device__ __forceinline__ int nsem_element_kind(const NsemDev& m, bool active, const double* my) {
+    const int k = active ? nsem_node_kind<NC>(my) : NSEM_EL_TAME | NSEM_EL_DIAG;
+    const bool tame = __syncthreads_and(k & NSEM_EL_TAME), diag = __syncthreads_and(k & NSEM_EL_DIAG);
+    return !(tame && m.tame_tables) ? 0 : diag ? NSEM_EL_TAME | NSEM_EL_DIAG : NSEM_EL_TAME;
+}
+
+struct NsemMulFp64 {
+    double f;
+    __device__ __forceinline__ explicit NsemMulFp64(double x) : f(x) {}
+    __device__ __forceinline__ double operator()(double b) const { return f * b; }
+};
+struct NsemMulInt {
+    nsem_factor f;
+    __device__ __forceinline__ explicit NsemMulInt(double x) : f(nsem_make_factor(x)) {}
+    __device__ __forceinline__ double operator()(double b) const { return nsem_mul_normal(f, b); }
+};
+
+/* a b, on the integer pipes (INT: operands mild, see nsem_mild) or in FP64 */
+template <bool INT>
+__device__ __forceinline__ double nsem_x(double a, double b) {
+    if constexpr (INT) return nsem_mul_normal(nsem_make_factor(a), b);
+    else return a * b;
+}
+/* x finite, by its bits */
+__device__ __forceinline__ bool nsem_finite(double x) {
+    return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
 }
 
 /* x . dj as the reference sums it: vectors (rho, theta) from the last
  * component (its + 0.0 only turns -0 into +0, which no sum here shows), tensor
  * rows (ROW) from the first */
-template <bool ROW>
-__device__ __forceinline__ double nsem_dj_dot(double x0, double x1, double x2, const double* dj) {
-    return ROW ? x0 * dj[0] + x1 * dj[1] + x2 * dj[2] : x0 * dj[0] + (x1 * dj[1] + x2 * dj[2]);
+template <bool ROW, typename Mul>
+__device__ __forceinline__ double nsem_dj_dot(double x0, double x1, double x2, const Mul* dj) {
+    return ROW ? (dj[0](x0) + dj[1](x1)) + dj[2](x2) : dj[0](x0) + (dj[1](x1) + dj[2](x2));
 }
 
-/* r[v] -= volume term of the NC equations; ROWS: bit v set where equation v is
- * a tensor row.  JOFF = 3 NC, W >= 3 NC + 9. */
-template <int NC, int W, unsigned ROWS>
-__device__ __forceinline__ void nsem_volume_gather(int npx, int npy, int npz, const double* sm,
-                                                   const double* dps, int t, bool diag, double* r) {
-    constexpr int M2 = NSEM_MAX_NPD * NSEM_MAX_NPD, JOFF = 3 * NC;
-    static_assert(W >= JOFF + 9, "record: 3 NC flux values and the metric");
-    /* metric columns of the X, Y and Z derivatives: (XX,YX,ZX), (XY,YY,ZY),
-     * (XZ,YZ,ZZ), four bits per component index */
-    constexpr int COLS_X = 0 | (6 << 4) | (8 << 8);
-    constexpr int COLS_Y = 3 | (1 << 4) | (7 << 8);
-    constexpr int COLS_Z = 5 | (4 << 4) | (2 << 8);
-    const int ia = t / (npy * npz), ja = (t / npz) % npy, ka = t % npz;
-    const int sx = npy * npz, sy = npz;
-    auto full = [&](const double* s, const double* dj, double* out) {
-#pragma unroll
-        for (int v = 0; v < NC; v++)
-            out[v] = (ROWS >> v & 1) ? nsem_dj_dot<true>(s[v], s[NC + v], s[2 * NC + v], dj)
-                                     : nsem_dj_dot<false>(s[v], s[NC + v], s[2 * NC + v], dj);
-    };
-    double dj_self[3];
-    {
-        const double* J = sm + (size_t)t * W + JOFF;
-        const double d0 = dps[ia * npx + ia], d1 = dps[M2 + ja * npy + ja],
-                     d2 = dps[2 * M2 + ka * npz + ka];
-        if (diag) {
-            dj_self[0] = J[0] * d0;
-            dj_self[1] = J[1] * d1;
-            dj_self[2] = J[2] * d2;
-        } else {
-            dj_self[0] = J[0] * d0 + J[3] * d1 + J[5] * d2;
-            dj_self[1] = J[6] * d0 + J[1] * d1 + J[4] * d2;
-            dj_self[2] = J[8] * d0 + J[7] * d1 + J[2] * d2;
-        }
+/* the direction of source position p of the node (ia, ja, ka) = t, the
+ * source's node and its derivative */
+struct NsemSource {
+    int npx, npy, npz, t, ia, ja, ka, xb, yb, zb, za, ya;
+    __device__ __forceinline__ NsemSource(int nx, int ny, int nz, int t_)
+        : npx(nx), npy(ny), npz(nz), t(t_), ia(t_ / (ny * nz)), ja((t_ / nz) % ny), ka(t_ % nz) {
+        xb = ia; yb = ia + ja; zb = ia + ja + ka;   /* ends of X<, Y<, Z< */
+        za = ia + ja + npz;                         /* end of Z> */
+        ya = ia + npy + npz - 1;                    /* end of Y> */
     }
-    const int L = npx + npy + npz - 2;
-    const int xb = ia, yb = ia + ja, zb = ia + ja + ka;   /* ends of X<, Y<, Z< */
-    const int za = ia + ja + npz;                         /* end of Z> */
-    const int ya = ia + npy + npz - 1;                    /* end of Y> */
-    /* direction of position p, the source's node and its derivative */
-    auto source = [&](int p, int& dir, int& lb, double& D) {
+    __device__ __forceinline__ int count() const { return npx + npy + npz - 2; }
+    __device__ __forceinline__ void at(int p, const double* dps, int& dir, int& lb, double& D) const {
+        constexpr int M2 = NSEM_MAX_NPD * NSEM_MAX_NPD;
         const bool on_x = p < xb || p >= ya;
         const bool on_y = !on_x && (p < yb || p >= za);
         const int q = on_x ? (p < xb ? p : p - npy - npz + 2)
@@ -116,47 +160,129 @@ __device__ __forceinline__ void nsem_volume_gather(int npx, int npy, int npz, co
                            : p - ia - ja;               /* Z line; q == ka at the node itself */
         const int da = on_x ? ia : on_y ? ja : ka;
         const int dn = on_x ? npx : on_y ? npy : npz;
-        const int st = on_x ? sx : on_y ? sy : 1;
+        const int st = on_x ? npy * npz : on_y ? npz : 1;
         dir = on_x ? 0 : on_y ? 1 : 2;
         lb = t + (q - da) * st;
         D = dps[dir * M2 + q * dn + da];
-    };
-    if (diag) {
-        double own[NC];
-        full(sm + (size_t)t * W, dj_self, own);
-#pragma unroll 1
-        for (int p = 0; p < L; p++) {
-            int dir, lb;
-            double D;
-            source(p, dir, lb, D);
-            const double* s = sm + (size_t)lb * W;
-            const double x = s[JOFF + dir] * D;
-            const bool self = p == zb;
-            s += dir * NC;
-#pragma unroll
-            for (int v = 0; v < NC; v++) {
-                const double y = s[v] * x;
-                r[v] -= self ? own[v] : y;
-            }
-        }
-        return;
     }
+};
+
+/* the three components of Jinv . (d0, d1, d2) */
+template <typename Mul>
+__device__ __forceinline__ void nsem_dj_self(const double* J, const NsemSource& s, const double* dps,
+                                             double* dj) {
+    constexpr int M2 = NSEM_MAX_NPD * NSEM_MAX_NPD;
+    const Mul d0(dps[s.ia * s.npx + s.ia]), d1(dps[M2 + s.ja * s.npy + s.ja]),
+        d2(dps[2 * M2 + s.ka * s.npz + s.ka]);
+    dj[0] = (d0(J[0]) + d1(J[3])) + d2(J[5]);
+    dj[1] = (d0(J[6]) + d1(J[1])) + d2(J[4]);
+    dj[2] = (d0(J[8]) + d1(J[7])) + d2(J[2]);
+}
+
+/* y[v] = value v's contribution F . dj of a node's record s */
+template <int NC, unsigned ROWS, typename Mul>
+__device__ __forceinline__ void nsem_dj_all(const double* s, const Mul* dj, double* y) {
+#pragma unroll
+    for (int v = 0; v < NC; v++)
+        y[v] = (ROWS >> v & 1) ? nsem_dj_dot<true>(s[v], s[NC + v], s[2 * NC + v], dj)
+                               : nsem_dj_dot<false>(s[v], s[NC + v], s[2 * NC + v], dj);
+}
+
+/* the full products, whatever the metric */
+template <int NC, int W, unsigned ROWS, typename Mul>
+__device__ __forceinline__ void nsem_gather_full(const NsemSource& src, const double* sm,
+                                                 const double* dps, double* r) {
+    constexpr int JOFF = 3 * NC;
+    /* metric columns of the X, Y and Z derivatives: (XX,YX,ZX), (XY,YY,ZY),
+     * (XZ,YZ,ZZ), four bits per component index */
+    constexpr int COLS_X = 0 | (6 << 4) | (8 << 8);
+    constexpr int COLS_Y = 3 | (1 << 4) | (7 << 8);
+    constexpr int COLS_Z = 5 | (4 << 4) | (2 << 8);
+    double dj_self[3];
+    nsem_dj_self<Mul>(sm + (size_t)src.t * W + JOFF, src, dps, dj_self);
+    const int L = src.count();
 #pragma unroll 1
     for (int p = 0; p < L; p++) {
         int dir, lb;
         double D;
-        source(p, dir, lb, D);
+        src.at(p, dps, dir, lb, D);
         const int cols = dir == 0 ? COLS_X : dir == 1 ? COLS_Y : COLS_Z;
-        const bool self = p == zb;
+        const bool self = p == src.zb;
         const double* s = sm + (size_t)lb * W;
         const double* J = s + JOFF;
-        const double l0 = J[cols & 15] * D, l1 = J[(cols >> 4) & 15] * D, l2 = J[cols >> 8] * D;
-        const double dj[3] = {self ? dj_self[0] : l0, self ? dj_self[1] : l1, self ? dj_self[2] : l2};
+        const Mul d(D);
+        const double l0 = d(J[cols & 15]), l1 = d(J[(cols >> 4) & 15]), l2 = d(J[cols >> 8]);
+        const Mul dj[3] = {Mul(self ? dj_self[0] : l0), Mul(self ? dj_self[1] : l1),
+                           Mul(self ? dj_self[2] : l2)};
         double y[NC];
-        full(s, dj, y);
+        nsem_dj_all<NC, ROWS>(s, dj, y);
 #pragma unroll
         for (int v = 0; v < NC; v++) r[v] -= y[v];
     }
+}
+
+/* r[v] -= volume term of the NC equations; ROWS: bit v set where equation v is
+ * a tensor row; kind: nsem_element_kind.  JOFF = 3 NC, W >= 3 NC + 9. */
+template <int NC, int W, unsigned ROWS>
+__device__ __forceinline__ void nsem_volume_gather(int npx, int npy, int npz, const double* sm,
+                                                   const double* dps, int t, int kind, double* r) {
+    static_assert(W >= 3 * NC + 9, "record: 3 NC flux values and the metric");
+    const NsemSource src(npx, npy, npz, t);
+    if (!(kind & NSEM_EL_TAME)) {
+        nsem_gather_full<NC, W, ROWS, NsemMulFp64>(src, sm, dps, r);
+        return;
+    }
+    if (!(kind & NSEM_EL_DIAG)) {
+        nsem_gather_full<NC, W, ROWS, NsemMulInt>(src, sm, dps, r);
+        return;
+    }
+    constexpr int JOFF = 3 * NC;
+    double own[NC];
+    {
+        double dj[3];
+        nsem_dj_self<NsemMulInt>(sm + (size_t)t * W + JOFF, src, dps, dj);
+        const NsemMulInt f[3] = {NsemMulInt(dj[0]), NsemMulInt(dj[1]), NsemMulInt(dj[2])};
+        nsem_dj_all<NC, ROWS>(sm + (size_t)t * W, f, own);
+    }
+    const int L = src.count();
+#pragma unroll 1
+    for (int p = 0; p < L; p++) {
+        int dir, lb;
+        double D;
+        src.at(p, dps, dir, lb, D);
+        const double* s = sm + (size_t)lb * W;
+        const NsemMulInt x(NsemMulInt(D)(s[JOFF + dir]));
+        const bool self = p == src.zb;
+        s += dir * NC;
+#pragma unroll
+        for (int v = 0; v < NC; v++) {
+            const double y = x(s[v]);
+            r[v] -= self ? own[v] : y;
+        }
+    }
+}
+
+/* the momentum and theta flux columns of a node in the record of NC values per
+ * direction, Fc (x) U + p' I from value R0 on and Fc theta after it; INT: U and
+ * T mild, Fc tame and below 2^400, p' bounded, so that the products run on the
+ * integer pipes and the off-diagonal components' 0 p' is a zero that changes
+ * nothing */
+template <int NC, int R0, bool INT>
+__device__ __forceinline__ void nsem_flux_columns(double* my, const double* Fc, const double* U, double T,
+                                                  double pp) {
+    for (int r = 0; r < 3; r++)
+        for (int c = 0; c < 3; c++) {
+            const double x = nsem_x<INT>(Fc[r], U[c]);
+            my[NC * c + R0 + r] = r == c ? x + 1.0 * pp : INT ? x : x + 0.0 * pp;
+        }
+    for (int c = 0; c < 3; c++) my[NC * c + R0 + 3] = nsem_x<INT>(Fc[c], T);
+}
+
+/* r - (g s) cv */
+__device__ __forceinline__ double nsem_sub_source(double r, double g, double s, double cv) {
+    /* no gravity along the axis: 0 s cv is a zero that changes no sum */
+    if (nsem_is_zero(g) && nsem_bounded(s) && nsem_bounded(cv)) return r;
+    return r - (0.0 + g * s) * cv;
 }
 
 /* the axis a face slot's normal n lies along, with en its unit normal +-1 on

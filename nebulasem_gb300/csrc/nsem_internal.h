@@ -26,10 +26,6 @@
 #define NSEM_NPRIM 7
 #define NSEM_STATUS_NONFINITE 1u
 
-struct NsemTables {
-    double dpsi[3][NSEM_MAX_NPD * NSEM_MAX_NPD]; /* dpsi[d][s*npd + i] = l_i'(x_s) */
-};
-
 /* per mortar slot (ms_i rows): its used slot, the coarse side (1: c1, 2: c2),
  * the coarse face's node (0, 0), node strides and node counts along the face's
  * two in-plane axes, their 2:1 table ids (axis * 2 + half), the slot's position
@@ -40,11 +36,14 @@ enum { NSEM_MS_K, NSEM_MS_SIDE, NSEM_MS_BASE, NSEM_MS_SA, NSEM_MS_SB, NSEM_MS_NA
 struct NsemDev {
     int32_t npx, npy, npz, np;
     int64_t n_elem, n_int, n_slot;
+    int32_t tame_tables; /* every dpsi entry zero or within 2^+-60 */
+    int32_t tame_const;  /* P0, R, gamma R, nu, 1/Pr and T0 zero or within 2^+-60 */
     /* physical constants */
     double P0, R, gamma, gR, cv_heat, cp, T0;
     nsem_divisor dP0;  /* P0 prepared for nsem_div_by */
     double nu, iPr;    /* artificial viscosity (segregated scheme), 1 / Pr */
     double g[3];
+    double* dpsi;      /* [3][NSEM_MAX_NPD^2] derivative tables: dpsi[d][s*npd + i] = l_i'(x_s) */
     /* node arrays */
     double* jin;       /* [9][n_int] */
     double* cv;
@@ -98,7 +97,7 @@ extern "C" {
  * stage state S from u^n = U0 (out may be S or U0). */
 int nsem_fp64_prim(const NsemDev* m, NsemBuf* b, const double* const* S, void* stream);
 int nsem_fp64_face(const NsemDev* m, NsemBuf* b, const double* rho, void* stream);
-int nsem_fp64_volume(const NsemDev* m, const NsemTables* t, NsemBuf* b, int stage, double dt,
+int nsem_fp64_volume(const NsemDev* m, NsemBuf* b, int stage, double dt,
                      const double* const* S, const double* const* U0, double* const* out,
                      void* stream);
 int nsem_fp64_check_smem(const NsemDev* m);

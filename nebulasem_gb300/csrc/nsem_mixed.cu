@@ -1190,7 +1190,7 @@ int nsem_mixed_host_layout(const NsemDev* dev, NsemMixedBuf* mb, int to_pert, do
     return (int)cudaErrorNotSupported;
 }
 
-int nsem_mixed_steps(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf*, const NsemTables*,
+int nsem_mixed_steps(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf*, 
                      int nsteps, double dt, void* stream) {
     int cur = mb->cur;
     for (int n = 0; n < nsteps; n++) {
@@ -1202,7 +1202,7 @@ int nsem_mixed_steps(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf*, const NsemT
     return 0;
 }
 
-int nsem_mixed_tendency(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf* b, const NsemTables*,
+int nsem_mixed_tendency(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf* b, 
                         void* stream) {
     StageArgs a = base_args(dev, mb, 0.0);
     a.U = mb->U[mb->cur];
@@ -1216,7 +1216,7 @@ const char* const* nsem_mixed_kernel_names() { return k_names; }
 int nsem_mixed_launches_per_step() { return 3; }
 int nsem_mixed_launch_class(int k) { return k; }
 
-int nsem_mixed_launch(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf*, const NsemTables*, int k,
+int nsem_mixed_launch(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf*, int k,
                       int, double dt, void* stream) {
     const int cur = mb->cur;
     StageArgs a = base_args(dev, mb, dt);

@@ -108,9 +108,9 @@ int nsem_mixed_host_layout(const NsemDev* dev, NsemMixedBuf* mb, int to_pert, do
 
 nsem_status nsem_mixed_setup(const NsemDev& dev, const nsem_mesh_desc* m, NsemMixedBuf* mb,
                              std::vector<void*>* allocs, std::string& err);
-int nsem_mixed_steps(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf* b, const NsemTables* t,
+int nsem_mixed_steps(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf* b,
                      int nsteps, double dt, void* stream);
-int nsem_mixed_tendency(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf* b, const NsemTables* t,
+int nsem_mixed_tendency(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf* b,
                         void* stream);
 
 bool nsem_mixed_supported(int nx, int ny, int nz);
@@ -140,7 +140,7 @@ int nsem_mixed_adjoint_run(const NsemDev* dev, NsemMixedBuf* mb, double dt, void
 const char* const* nsem_mixed_kernel_names();
 int nsem_mixed_launches_per_step();
 int nsem_mixed_launch_class(int k);
-int nsem_mixed_launch(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf* b, const NsemTables* t, int k,
+int nsem_mixed_launch(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf* b, int k,
                       int first_step, double dt, void* stream);
 
 /* auxiliary kernels (nsem_aux.cu) */

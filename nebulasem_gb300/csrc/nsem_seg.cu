@@ -220,12 +220,28 @@ __global__ void __launch_bounds__(256) k_seg_prep(const NsemDev m, SegArgs a) {
     const double U[3] = {a.U[0][i], a.U[1][i], a.U[2][i]};
     const double Tf = a.Tp[i] + m.T0;
     a.Tf[i] = Tf;
+    if (m.tame_const && nsem_mild(r) && nsem_mild(Tf) && nsem_mild(U[0]) && nsem_mild(U[1]) && nsem_mild(U[2])) {
+        for (int c = 0; c < 3; c++) a.Fc[c][i] = nsem_x<true>(r, U[c]);
+        a.mu[i] = nsem_sqrt(nsem_x<true>(U[0], U[0]) + (nsem_x<true>(U[1], U[1]) + nsem_x<true>(U[2], U[2])));
+        a.cs[i] = nsem_sqrt(nsem_x<true>(m.gR, Tf));
+        return;
+    }
     for (int c = 0; c < 3; c++) a.Fc[c][i] = r * U[c];
     a.mu[i] = nsem_sqrt(vdot3(U, U));
     a.cs[i] = nsem_sqrt(m.gR * Tf);
 }
 
-__global__ void __launch_bounds__(256) k_seg_face_rho(const NsemDev m, SegArgs a) {
+/* Face kernels: FACE threads a CTA, so that a small mesh's slots spread over
+ * the SMs (32 x 24 elements of order 4 in 2D have 8 k slots, 32 CTAs of 256) */
+constexpr int FACE = 64;
+
+/* all values mild (nsem_mild) */
+template <typename... X>
+__device__ __forceinline__ bool all_mild(X... x) {
+    return (nsem_mild(x) && ...);
+}
+
+__global__ void __launch_bounds__(FACE) k_seg_face_rho(const NsemDev m, SegArgs a) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= m.n_slot) return;
     const int32_t c1 = m.c1[k], c2 = m.c2[k];
@@ -247,6 +263,21 @@ __global__ void __launch_bounds__(256) k_seg_face_rho(const NsemDev m, SegArgs a
         ghost_U(m, k, U1, U2);
         mu2 = nsem_sqrt(vdot3(U2, U2));
         cs2 = cs1;   /* sqrt(gamma R theta) of the same theta */
+    }
+    /* a normal along one axis meets one component of the flux (the others'
+     * products are zeros that change no sum); products on the integer pipes */
+    const int ax = m.n_ms && m.ms_of[k] >= 0 ? -1 : nsem_axis_of(n, en);
+    if (ax >= 0 && all_mild(r1, r2, mu1, mu2, cs1, cs2, fi, fo, nsem_pick(ax, n[0], n[1], n[2])) &&
+        all_mild(U1[0], U1[1], U1[2], U2[0], U2[1], U2[2])) {
+        auto avg = [&](double x, double y) { return nsem_x<true>(fi, x) + nsem_x<true>(fo, y); };
+        const double lam = (avg(mu1, mu2) + avg(cs1, cs2)) * 0.5;
+        a.lam[k] = lam;
+        const double jump = nsem_x<true>(lam, r2 - r1);
+        a.d[0][k] = nsem_x<true>(nsem_pick(ax, n[0], n[1], n[2]),
+                                 avg(nsem_x<true>(r1, nsem_pick(ax, U1[0], U1[1], U1[2])),
+                                     nsem_x<true>(r2, nsem_pick(ax, U2[0], U2[1], U2[2]))) -
+                                     nsem_signed(nsem_pick(ax, en[0], en[1], en[2]), jump));
+        return;
     }
     double X1[3], X2[3];
     for (int c = 0; c < 3; c++) {
@@ -272,16 +303,6 @@ __global__ void __launch_bounds__(256) k_seg_face_rho(const NsemDev m, SegArgs a
     const double lam = ((mu1v * fi + mu2 * fo) + (cs1v * fi + cs2 * fo)) / 2;
     a.lam[k] = lam;
     const double jump = lam * (r2 - r1v);
-    /* a normal along one axis meets one component of the flux (the others'
-     * products are zeros that change no sum) */
-    const int ax = ms < 0 ? nsem_axis_of(n, en) : -1;
-    if (ax >= 0 && nsem_bounded(jump) && nsem_bounded(X1[0]) && nsem_bounded(X1[1]) &&
-        nsem_bounded(X1[2]) && nsem_bounded(X2[0]) && nsem_bounded(X2[1]) && nsem_bounded(X2[2])) {
-        a.d[0][k] = ((nsem_pick(ax, X1[0], X1[1], X1[2]) * fi + nsem_pick(ax, X2[0], X2[1], X2[2]) * fo) -
-                     nsem_signed(nsem_pick(ax, en[0], en[1], en[2]), jump)) *
-                    nsem_pick(ax, n[0], n[1], n[2]);
-        return;
-    }
     double F[3];
     for (int c = 0; c < 3; c++) F[c] = (X1[c] * fi + X2[c] * fo) - en[c] * jump;
     a.d[0][k] = vdot3(F, n);
@@ -338,7 +359,7 @@ __global__ void __launch_bounds__(128) k_seg_mortar_ggather(const NsemDev m, Gra
 }
 
 /* cds(U), cds(theta) per slot for the gradients */
-__global__ void __launch_bounds__(256) k_seg_grad_face(const NsemDev m, GradArgs a) {
+__global__ void __launch_bounds__(FACE) k_seg_grad_face(const NsemDev m, GradArgs a) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= m.n_slot) return;
     const int32_t c1 = m.c1[k], c2 = m.c2[k];
@@ -355,19 +376,23 @@ __global__ void __launch_bounds__(256) k_seg_grad_face(const NsemDev m, GradArgs
         ghost_U(m, k, U1, U2);
         T2 = T1 + 0.0;
     }
+    if (all_mild(fi, fo, T1, T2, U1[0], U1[1], U1[2], U2[0], U2[1], U2[2])) {
+        for (int c = 0; c < 3; c++) a.fF[c][k] = nsem_x<true>(fi, U1[c]) + nsem_x<true>(fo, U2[c]);
+        a.fF[3][k] = nsem_x<true>(fi, T1) + nsem_x<true>(fo, T2);
+        return;
+    }
     for (int c = 0; c < 3; c++) a.fF[c][k] = (U1[c] * fi) + (U2[c] * fo);
     a.fF[3][k] = (T1 * fi) + (T2 * fo);
 }
 
 constexpr int W_GRAD = 13;   /* U[3] theta jin[9] */
 
-__global__ void k_seg_grad_vol(const NsemDev m, const NsemTables tab, GradArgs a) {
+__global__ void k_seg_grad_vol(const NsemDev m, GradArgs a) {
     extern __shared__ double sm[];
     const int NP = m.np, NPX = m.npx, NPY = m.npy, NPZ = m.npz;
     double* dps = sm + (size_t)NP * W_GRAD;
     const int t = threadIdx.x;
-    for (int q = t; q < 3 * NSEM_MAX_NPD * NSEM_MAX_NPD; q += blockDim.x)
-        dps[q] = (&tab.dpsi[0][0])[q];
+    nsem_load_tables(m, dps, t);
     const int64_t e = blockIdx.x;
     const bool active = t < NP;
     const int64_t node = e * NP + t;
@@ -379,12 +404,14 @@ __global__ void k_seg_grad_vol(const NsemDev m, const NsemTables tab, GradArgs a
         for (int c = 0; c < 3; c++) my[c] = a.U[c][node];
         my[3] = a.Tf[node];
     }
-    /* a diagonal metric (see nsem_volume_gather): only row r of the gradients
-     * takes line r's terms, 1 + 4 products a source instead of 3 + 12 */
-    bool ok = true;
+    /* a diagonal metric and values of ordinary size (see nsem_volume_gather):
+     * only row r of the gradients takes line r's terms, 1 + 4 products a source
+     * instead of 3 + 12, on the integer pipes */
+    bool ok = m.tame_tables;
     if (active) {
         const double* my = sm + (size_t)t * W_GRAD;
-        for (int c = 0; c < 7; c++) ok = ok && nsem_bounded(my[c]);
+        ok = ok && all_mild(my[0], my[1], my[2], my[3]);
+        for (int c = 4; c < 7; c++) ok = ok && nsem_metric_tame(my[c]);
         for (int c = 7; c < 13; c++) ok = ok && nsem_is_zero(my[c]);
     }
     const bool diag = __syncthreads_and(ok);
@@ -415,7 +442,15 @@ __global__ void k_seg_grad_vol(const NsemDev m, const NsemTables tab, GradArgs a
             /* r - x is r + (-x): the sign goes into the normal's bits */
             const double na = nsem_pick(ax, n[0], n[1], n[2]);
             const double ns = __hiloint2double(__double2hiint(na) ^ (code << 31), __double2loint(na));
-            const double x[4] = {ns * dU[0], ns * dU[1], ns * dU[2], ns * dT};
+            double x[4];
+            /* differences of mild values are zero or above 2^-253 */
+            if (diag && !coarse && all_mild(na, f4[0], f4[1], f4[2], f4[3])) {
+                for (int c = 0; c < 3; c++) x[c] = nsem_x<true>(ns, dU[c]);
+                x[3] = nsem_x<true>(ns, dT);
+            } else {
+                for (int c = 0; c < 3; c++) x[c] = ns * dU[c];
+                x[3] = ns * dT;
+            }
             if (ax == 0) {
                 gU[XX] += x[0]; gU[XY] += x[1]; gU[XZ] += x[2]; gT[0] += x[3];
             } else if (ax == 1) {
@@ -453,24 +488,25 @@ __global__ void k_seg_grad_vol(const NsemDev m, const NsemTables tab, GradArgs a
     if (diag) {
         /* row r: the node's own term, which the x line's order puts first in
          * rows y and z, then line r's sources in order */
-        auto row = [&](int lb, double dj, double& g0, double& g1, double& g2, double& gt) {
+        auto row = [&](int lb, double dj_, double& g0, double& g1, double& g2, double& gt) {
             const double* sb = sm + (size_t)lb * W_GRAD;
-            g0 += dj * sb[0];
-            g1 += dj * sb[1];
-            g2 += dj * sb[2];
-            gt += dj * sb[3];
+            const NsemMulInt dj(dj_);
+            g0 += dj(sb[0]);
+            g1 += dj(sb[1]);
+            g2 += dj(sb[2]);
+            gt += dj(sb[3]);
         };
         for (int ii = 0; ii < NPX; ii++)
-            row(t + (ii - ia) * sx, J[XX] * Dx[ia * NPX + ii], gU[XX], gU[XY], gU[XZ], gT[0]);
-        row(t, J[YY] * Dy[ja * NPY + ja], gU[YX], gU[YY], gU[YZ], gT[1]);
+            row(t + (ii - ia) * sx, nsem_x<true>(J[XX], Dx[ia * NPX + ii]), gU[XX], gU[XY], gU[XZ], gT[0]);
+        row(t, nsem_x<true>(J[YY], Dy[ja * NPY + ja]), gU[YX], gU[YY], gU[YZ], gT[1]);
         for (int q = 0; q + 1 < NPY; q++) {
             const int jj = q < ja ? q : q + 1;
-            row(t + (jj - ja) * sy, J[YY] * Dy[ja * NPY + jj], gU[YX], gU[YY], gU[YZ], gT[1]);
+            row(t + (jj - ja) * sy, nsem_x<true>(J[YY], Dy[ja * NPY + jj]), gU[YX], gU[YY], gU[YZ], gT[1]);
         }
-        row(t, J[ZZ] * Dz[ka * NPZ + ka], gU[ZX], gU[ZY], gU[ZZ], gT[2]);
+        row(t, nsem_x<true>(J[ZZ], Dz[ka * NPZ + ka]), gU[ZX], gU[ZY], gU[ZZ], gT[2]);
         for (int q = 0; q + 1 < NPZ; q++) {
             const int kk = q < ka ? q : q + 1;
-            row(t + (kk - ka), J[ZZ] * Dz[ka * NPZ + kk], gU[ZX], gU[ZY], gU[ZZ], gT[2]);
+            row(t + (kk - ka), nsem_x<true>(J[ZZ], Dz[ka * NPZ + kk]), gU[ZX], gU[ZY], gU[ZZ], gT[2]);
         }
         const double cv = m.cv[node];
         const nsem_divisor dcv = nsem_make_divisor(cv);
@@ -514,13 +550,12 @@ constexpr int W_RHO = 12;   /* fr[3] jin[9] */
 constexpr int W_UT = 21;    /* per direction: momentum tensor column [3], ft; then jin[9] */
 constexpr unsigned UT_ROWS = 0x7;   /* the U equations are tensor rows */
 
-__global__ void k_seg_vol_rho(const NsemDev m, const NsemTables tab, SegArgs a) {
+__global__ void __launch_bounds__(1024) k_seg_vol_rho(const NsemDev m, SegArgs a) {
     extern __shared__ double sm[];
     const int NP = m.np;
     double* dps = sm + (size_t)NP * W_RHO;
     const int t = threadIdx.x;
-    for (int q = t; q < 3 * NSEM_MAX_NPD * NSEM_MAX_NPD; q += blockDim.x)
-        dps[q] = (&tab.dpsi[0][0])[q];
+    nsem_load_tables(m, dps, t);
     const int64_t e = blockIdx.x;
     const bool active = t < NP;
     const int64_t node = e * NP + t;
@@ -531,9 +566,12 @@ __global__ void k_seg_vol_rho(const NsemDev m, const NsemTables tab, SegArgs a) 
     if (active) {
         rho = a.rho_o[node];
         double* my = sm + (size_t)t * W_RHO;
-        for (int c = 0; c < 3; c++) my[c] = a.U[c][node] * rho;     /* U * rho */
+        for (int c = 0; c < 3; c++) {
+            const double U = a.U[c][node];
+            my[c] = all_mild(U, rho) ? nsem_x<true>(rho, U) : U * rho;
+        }
     }
-    const bool diag = __syncthreads_and(!active || nsem_node_diag<1>(sm + (size_t)t * W_RHO));
+    const int kind = nsem_element_kind<1>(m, active, sm + (size_t)t * W_RHO);
     if (!active) return;
     double r = 0.0;
     for (int j = 0; j < m.n_lift; j++) {
@@ -545,7 +583,7 @@ __global__ void k_seg_vol_rho(const NsemDev m, const NsemTables tab, SegArgs a) 
         else r += v;
     }
     nsem_chain_begin();
-    nsem_volume_gather<1, W_RHO, 0>(m.npx, m.npy, m.npz, sm, dps, t, diag, &r);
+    nsem_volume_gather<1, W_RHO, 0>(m.npx, m.npy, m.npz, sm, dps, t, kind, &r);
     const double cv = m.cv[node];
     const double ap = a.c_dt * cv;
     const double rn = nsem_div(r + rho * ap, 0.0 + ap);
@@ -554,7 +592,43 @@ __global__ void k_seg_vol_rho(const NsemDev m, const NsemTables tab, SegArgs a) 
     a.pp[node] = p - m.p_ref[node];
 }
 
-__global__ void __launch_bounds__(256) k_seg_face_ut(const NsemDev m, SegArgs a) {
+/* the four lifted values of a slot whose normal lies along axis ax (about 45
+ * operations instead of 160, with INT 14 and the products on the integer
+ * pipes) */
+template <bool INT>
+__device__ __forceinline__ void face_ut_axis(const NsemDev& m, const SegArgs& a, int64_t k, int ax,
+                                             const double* n, const double* en, double fi, double fo,
+                                             double lam, double r1, const double* U1, const double* Fc1,
+                                             double T1, double p1, double mu1, double r2,
+                                             const double* U2, const double* Fc2, double T2, double p2,
+                                             double mu2, int32_t c1, int32_t c2) {
+    const double na = nsem_pick(ax, n[0], n[1], n[2]), ea = nsem_pick(ax, en[0], en[1], en[2]);
+    const double Ua1 = nsem_pick(ax, U1[0], U1[1], U1[2]), Ua2 = nsem_pick(ax, U2[0], U2[1], U2[2]);
+    auto avg = [&](double x, double y) { return nsem_x<INT>(fi, x) + nsem_x<INT>(fo, y); };
+    const double dq = nsem_signed(ea, nsem_x<INT>(lam, nsem_x<INT>(r2, Ua2) - nsem_x<INT>(r1, Ua1)));
+    for (int r = 0; r < 3; r++) {
+        double A = nsem_x<INT>(Ua1, Fc1[r]), B = nsem_x<INT>(Ua2, Fc2[r]);
+        if (r == ax) { A += p1; B += p2; }
+        if (a.visc) {
+            const double* g = r == ax ? a.G[r] : a.G[r == 0 ? (ax == 1 ? XY : XZ)
+                                                     : r == 1 ? (ax == 2 ? YZ : YX) : (ax == 0 ? ZX : ZY)];
+            A = A - nsem_x<INT>(mu1, g[c1]);
+            B = B - nsem_x<INT>(mu2, c2 >= 0 ? g[c2] : 0.0);
+        }
+        double F = avg(A, B);
+        if (r == ax) F -= dq;
+        a.d[1 + r][k] = nsem_x<INT>(na, F);
+    }
+    double x = nsem_x<INT>(T1, nsem_pick(ax, Fc1[0], Fc1[1], Fc1[2]));
+    double y = nsem_x<INT>(T2, nsem_pick(ax, Fc2[0], Fc2[1], Fc2[2]));
+    if (a.visc) {
+        x = x - nsem_x<INT>(nsem_x<INT>(m.iPr, mu1), a.G[9 + ax][c1]);
+        y = y - nsem_x<INT>(nsem_x<INT>(m.iPr, mu2), c2 >= 0 ? a.G[9 + ax][c2] : 0.0);
+    }
+    a.d[4][k] = nsem_x<INT>(na, avg(x, y) - nsem_signed(ea, nsem_x<INT>(lam, nsem_x<INT>(r2, T2) - nsem_x<INT>(r1, T1))));
+}
+
+__global__ void __launch_bounds__(FACE) k_seg_face_ut(const NsemDev m, SegArgs a) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= m.n_slot) return;
     const int32_t c1 = m.c1[k], c2 = m.c2[k];
@@ -589,41 +663,34 @@ __global__ void __launch_bounds__(256) k_seg_face_ut(const NsemDev m, SegArgs a)
     const int32_t ms = m.n_ms ? m.ms_of[k] : -1;
     const int mside = ms >= 0 ? ms_field(m, NSEM_MS_SIDE, ms) : 0;
     /* a normal along one axis: only the flux tensor's column of that axis
-     * meets a nonzero normal component (about 45 operations instead of 160);
-     * the products left out are zeros that change no sum */
+     * meets a nonzero normal component; the products left out are zeros that
+     * change no sum */
     const int ax = mside == 0 ? nsem_axis_of(n, en) : -1;
-    bool ok = ax >= 0 && nsem_bounded(lam) && nsem_bounded(r1) && nsem_bounded(r2) &&
-              nsem_bounded(T1) && nsem_bounded(T2) && nsem_bounded(p1) && nsem_bounded(p2);
-    for (int c = 0; c < 3; c++)
-        ok = ok && nsem_bounded(U1[c]) && nsem_bounded(U2[c]) && nsem_bounded(Fc1[c]) && nsem_bounded(Fc2[c]);
-    if (a.visc && ok)
-        for (int c = 0; c < 12; c++)
-            ok = ok && nsem_bounded(a.G[c][c1]) && (c2 < 0 || nsem_bounded(a.G[c][c2]));
-    if (ok) {
-        const double na = nsem_pick(ax, n[0], n[1], n[2]), ea = nsem_pick(ax, en[0], en[1], en[2]);
-        const double Ua1 = nsem_pick(ax, U1[0], U1[1], U1[2]), Ua2 = nsem_pick(ax, U2[0], U2[1], U2[2]);
-        const double dq = nsem_signed(ea, (r2 * Ua2 - r1 * Ua1) * lam);
-        for (int r = 0; r < 3; r++) {
-            double A = Fc1[r] * Ua1, B = Fc2[r] * Ua2;
-            const double A1 = A + p1, B1 = B + p2;
-            if (r == ax) { A = A1; B = B1; }
-            if (a.visc) {
-                const double* g = r == ax ? a.G[r] : a.G[r == 0 ? (ax == 1 ? XY : XZ)
-                                                         : r == 1 ? (ax == 2 ? YZ : YX) : (ax == 0 ? ZX : ZY)];
-                A = A - mu1 * g[c1];
-                B = B - mu2 * (c2 >= 0 ? g[c2] : 0.0);
-            }
-            const double F = A * fi + B * fo;
-            const double Fj = F - dq;
-            a.d[1 + r][k] = (r == ax ? Fj : F) * na;
+    if (ax >= 0) {
+        bool bounded = true, mild = m.tame_const;
+        auto look = [&](double x) {
+            bounded = bounded && nsem_bounded(x);
+            mild = mild && nsem_mild(x);
+        };
+        look(lam); look(r1); look(r2); look(T1); look(T2); look(p1); look(p2); look(fi); look(fo);
+        for (int c = 0; c < 3; c++) {
+            look(U1[c]); look(U2[c]); look(n[c]);
+            bounded = bounded && nsem_bounded(Fc1[c]) && nsem_bounded(Fc2[c]);
+            mild = mild && nsem_tame(Fc1[c]) && nsem_tame(Fc2[c]);
         }
-        double x = nsem_pick(ax, Fc1[0], Fc1[1], Fc1[2]) * T1, y = nsem_pick(ax, Fc2[0], Fc2[1], Fc2[2]) * T2;
         if (a.visc) {
-            x = x - (mu1 * m.iPr) * a.G[9 + ax][c1];
-            y = y - (mu2 * m.iPr) * (c2 >= 0 ? a.G[9 + ax][c2] : 0.0);
+            look(mu1);
+            look(mu2);
+            for (int c = 0; c < 12; c++) {
+                look(a.G[c][c1]);
+                if (c2 >= 0) look(a.G[c][c2]);
+            }
         }
-        a.d[4][k] = ((x * fi + y * fo) - nsem_signed(ea, lam * (r2 * T2 - r1 * T1))) * na;
-        return;
+        if (bounded) {
+            if (mild) face_ut_axis<true>(m, a, k, ax, n, en, fi, fo, lam, r1, U1, Fc1, T1, p1, mu1, r2, U2, Fc2, T2, p2, mu2, c1, c2);
+            else face_ut_axis<false>(m, a, k, ax, n, en, fi, fo, lam, r1, U1, Fc1, T1, p1, mu1, r2, U2, Fc2, T2, p2, mu2, c1, c2);
+            return;
+        }
     }
     /* U equation: flux Fc (x) U + p' I - mu grad U, state rho U */
     {
@@ -688,13 +755,12 @@ __global__ void __launch_bounds__(256) k_seg_face_ut(const NsemDev m, SegArgs a)
     }
 }
 
-__global__ void k_seg_vol_ut(const NsemDev m, const NsemTables tab, SegArgs a) {
+__global__ void __launch_bounds__(1024) k_seg_vol_ut(const NsemDev m, SegArgs a) {
     extern __shared__ double sm[];
     const int NP = m.np;
     double* dps = sm + (size_t)NP * W_UT;
     const int t = threadIdx.x;
-    for (int q = t; q < 3 * NSEM_MAX_NPD * NSEM_MAX_NPD; q += blockDim.x)
-        dps[q] = (&tab.dpsi[0][0])[q];
+    nsem_load_tables(m, dps, t);
     const int64_t e = blockIdx.x;
     const bool active = t < NP;
     const int64_t node = e * NP + t;
@@ -708,22 +774,24 @@ __global__ void k_seg_vol_ut(const NsemDev m, const NsemTables tab, SegArgs a) {
         for (int c = 0; c < 3; c++) { U[c] = a.U[c][node]; Fc[c] = a.Fc[c][node]; }
         Tf = a.Tf[node];
         const double p = a.pp[node];
-        double fm[9], ft[3];
-        outer(Fc, U, fm);
-        for (int c = 0; c < 9; c++) fm[c] = fm[c] + ((c < 3) ? 1.0 : 0.0) * p;
-        for (int c = 0; c < 3; c++) ft[c] = Fc[c] * Tf;
+        /* Fc: a product of two values, or what the caller's fields hold */
+        const bool mild = all_mild(U[0], U[1], U[2], Tf) && nsem_tame(Fc[0]) && nsem_tame(Fc[1]) &&
+                          nsem_tame(Fc[2]) && nsem_bounded(p);
+        if (mild) nsem_flux_columns<4, 0, true>(my, Fc, U, Tf, p);
+        else nsem_flux_columns<4, 0, false>(my, Fc, U, Tf, p);
         if (a.visc) {
+            /* these products in FP64: on the integer pipes they are code that a
+             * small grid's warps, which run it once, wait for (2.94 against
+             * 2.87 ms for 40 steps of 32 x 24 elements of order 4) */
             const double mu = a.rho_o[node] * m.nu;
-            for (int c = 0; c < 9; c++) fm[c] = fm[c] - mu * a.G[c][node];
-            for (int c = 0; c < 3; c++) ft[c] = ft[c] - (mu * m.iPr) * a.G[9 + c][node];
-        }
-        const int col[3][3] = {{XX, YX, ZX}, {XY, YY, ZY}, {XZ, YZ, ZZ}};
-        for (int c = 0; c < 3; c++) {
-            for (int q = 0; q < 3; q++) my[4 * c + q] = fm[col[c][q]];
-            my[4 * c + 3] = ft[c];
+            const int col[3][3] = {{XX, YX, ZX}, {XY, YY, ZY}, {XZ, YZ, ZZ}};
+            for (int c = 0; c < 3; c++) {
+                for (int q = 0; q < 3; q++) my[4 * c + q] -= mu * a.G[col[c][q]][node];
+                my[4 * c + 3] -= (mu * m.iPr) * a.G[9 + c][node];
+            }
         }
     }
-    const bool diag = __syncthreads_and(!active || nsem_node_diag<4>(sm + (size_t)t * W_UT));
+    const int kind = nsem_element_kind<4>(m, active, sm + (size_t)t * W_UT);
     if (!active) return;
     double r[4] = {0.0, 0.0, 0.0, 0.0};
     for (int j = 0; j < m.n_lift; j++) {
@@ -737,25 +805,27 @@ __global__ void k_seg_vol_ut(const NsemDev m, const NsemTables tab, SegArgs a) {
         }
     }
     nsem_chain_begin();
-    nsem_volume_gather<4, W_UT, UT_ROWS>(m.npx, m.npy, m.npz, sm, dps, t, diag, r);
+    nsem_volume_gather<4, W_UT, UT_ROWS>(m.npx, m.npy, m.npz, sm, dps, t, kind, r);
     const double cv = m.cv[node];
     const double rn = a.rho_n[node];
     const double ro = a.rho_o[node];
     const double s = rn - m.rho_ref[node];
-    const double ap0 = a.c_dt * cv;
-    const double ap = ap0 * rn;
+    const bool mild = all_mild(a.c_dt, cv, rn, ro, U[0], U[1], U[2], Tf);
+    const double ap0 = mild ? nsem_x<true>(a.c_dt, cv) : a.c_dt * cv;
+    const double ap = mild ? nsem_x<true>(ap0, rn) : ap0 * rn;
     const nsem_divisor dap = nsem_make_divisor(0.0 + ap);
-    bool finite = isfinite(rn);
+    bool finite = nsem_finite(rn);
+    /* (q rho^n) ap0 of a field q */
+    auto old = [&](double q) { return mild ? nsem_x<true>(ap0, nsem_x<true>(ro, q)) : (q * ro) * ap0; };
     for (int c = 0; c < 3; c++) {
-        const double sc = 0.0 + m.g[c] * s;
-        const double su = r[c] - sc * cv;
-        const double un = nsem_div_by(su + (U[c] * ro) * ap0, dap);
+        const double su = nsem_sub_source(r[c], m.g[c], s, cv);
+        const double un = nsem_div_by(su + old(U[c]), dap);
         a.U[c][node] = un;
-        finite = finite && isfinite(un);
+        finite = finite && nsem_finite(un);
     }
-    const double Tn = nsem_div_by(r[3] + (Tf * ro) * ap0, dap);
+    const double Tn = nsem_div_by(r[3] + old(Tf), dap);
     a.Tp[node] = Tn - m.T0;
-    finite = finite && isfinite(Tn);
+    finite = finite && nsem_finite(Tn);
     if (!finite) atomicOr(m.status, NSEM_STATUS_NONFINITE);
 }
 
@@ -881,7 +951,7 @@ __global__ void __launch_bounds__(128) k_conv_mortar_gather(const NsemDev m, Adv
     a.dC[ms] = vdot3(F, n);
 }
 
-__global__ void __launch_bounds__(256) k_conv_lambda(const NsemDev m, AdvArgs a) {
+__global__ void __launch_bounds__(FACE) k_conv_lambda(const NsemDev m, AdvArgs a) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= m.n_slot) return;
     const int32_t c1 = m.c1[k], c2 = m.c2[k];
@@ -904,7 +974,7 @@ __global__ void __launch_bounds__(256) k_conv_lambda(const NsemDev m, AdvArgs a)
     a.lam[k] = (u1 * fi + u2 * fo) / 2;
 }
 
-__global__ void __launch_bounds__(256) k_conv_face(const NsemDev m, AdvArgs a) {
+__global__ void __launch_bounds__(FACE) k_conv_face(const NsemDev m, AdvArgs a) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= m.n_slot) return;
     const int32_t c1 = m.c1[k], c2 = m.c2[k];
@@ -927,6 +997,18 @@ __global__ void __launch_bounds__(256) k_conv_face(const NsemDev m, AdvArgs a) {
         }
         T2 = T1 + 0.0;
     }
+    /* a normal along one axis: one flux component (as k_seg_face_rho) */
+    const double lam = a.lam[k];
+    const int ax = m.n_ms && m.ms_of[k] >= 0 ? -1 : nsem_axis_of(n, en);
+    if (ax >= 0 && all_mild(lam, T1, T2, fi, fo, nsem_pick(ax, n[0], n[1], n[2])) &&
+        all_mild(U1[0], U1[1], U1[2], U2[0], U2[1], U2[2])) {
+        const double x = nsem_x<true>(T1, nsem_pick(ax, U1[0], U1[1], U1[2]));
+        const double y = nsem_x<true>(T2, nsem_pick(ax, U2[0], U2[1], U2[2]));
+        const double jump = nsem_signed(nsem_pick(ax, en[0], en[1], en[2]), nsem_x<true>(lam, T2 - T1));
+        a.d[k] = nsem_x<true>(nsem_pick(ax, n[0], n[1], n[2]),
+                              (nsem_x<true>(fi, x) + nsem_x<true>(fo, y)) - jump);
+        return;
+    }
     double X1[3], X2[3];
     for (int c = 0; c < 3; c++) {
         X1[c] = U1[c] * T1;
@@ -942,16 +1024,7 @@ __global__ void __launch_bounds__(256) k_conv_face(const NsemDev m, AdvArgs a) {
         for (int c = 0; c < 3; c++) X2[c] = a.mq[c][ms];
         T2v = a.mq[3][ms];
     }
-    const double jump = a.lam[k] * (T2v - T1v);
-    /* a normal along one axis: one flux component (as k_seg_face_rho) */
-    const int ax = side == 0 ? nsem_axis_of(n, en) : -1;
-    if (ax >= 0 && nsem_bounded(jump) && nsem_bounded(X1[0]) && nsem_bounded(X1[1]) &&
-        nsem_bounded(X1[2]) && nsem_bounded(X2[0]) && nsem_bounded(X2[1]) && nsem_bounded(X2[2])) {
-        a.d[k] = ((nsem_pick(ax, X1[0], X1[1], X1[2]) * fi + nsem_pick(ax, X2[0], X2[1], X2[2]) * fo) -
-                  nsem_signed(nsem_pick(ax, en[0], en[1], en[2]), jump)) *
-                 nsem_pick(ax, n[0], n[1], n[2]);
-        return;
-    }
+    const double jump = lam * (T2v - T1v);
     double F[3];
     for (int c = 0; c < 3; c++) F[c] = (X1[c] * fi + X2[c] * fo) - en[c] * jump;
     a.d[k] = vdot3(F, n);
@@ -961,13 +1034,12 @@ __global__ void __launch_bounds__(256) k_conv_face(const NsemDev m, AdvArgs a) {
 
 constexpr int W_CONV = 12;   /* fv[3] jin[9] */
 
-__global__ void k_conv_vol(const NsemDev m, const NsemTables tab, AdvArgs a) {
+__global__ void __launch_bounds__(1024) k_conv_vol(const NsemDev m, AdvArgs a) {
     extern __shared__ double sm[];
     const int NP = m.np;
     double* dps = sm + (size_t)NP * W_CONV;
     const int t = threadIdx.x;
-    for (int q = t; q < 3 * NSEM_MAX_NPD * NSEM_MAX_NPD; q += blockDim.x)
-        dps[q] = (&tab.dpsi[0][0])[q];
+    nsem_load_tables(m, dps, t);
     const int64_t e = blockIdx.x;
     const bool active = t < NP;
     const int64_t node = e * NP + t;
@@ -978,9 +1050,12 @@ __global__ void k_conv_vol(const NsemDev m, const NsemTables tab, AdvArgs a) {
     if (active) {
         T = a.T_o[node];
         double* my = sm + (size_t)t * W_CONV;
-        for (int c = 0; c < 3; c++) my[c] = a.U[c][node] * T;
+        for (int c = 0; c < 3; c++) {
+            const double U = a.U[c][node];
+            my[c] = all_mild(U, T) ? nsem_x<true>(T, U) : U * T;
+        }
     }
-    const bool diag = __syncthreads_and(!active || nsem_node_diag<1>(sm + (size_t)t * W_CONV));
+    const int kind = nsem_element_kind<1>(m, active, sm + (size_t)t * W_CONV);
     if (!active) return;
     double r = 0.0;
     for (int j = 0; j < m.n_lift; j++) {
@@ -992,7 +1067,7 @@ __global__ void k_conv_vol(const NsemDev m, const NsemTables tab, AdvArgs a) {
         else r += v;
     }
     nsem_chain_begin();
-    nsem_volume_gather<1, W_CONV, 0>(m.npx, m.npy, m.npz, sm, dps, t, diag, &r);
+    nsem_volume_gather<1, W_CONV, 0>(m.npx, m.npy, m.npz, sm, dps, t, kind, &r);
     const double ap = a.c_dt * m.cv[node];
     double Tn;
     if (a.ab2) {
@@ -1004,7 +1079,7 @@ __global__ void k_conv_vol(const NsemDev m, const NsemTables tab, AdvArgs a) {
     }
     if (a.R_n) a.R_n[node] = r;
     a.T_n[node] = Tn;
-    if (!isfinite(Tn)) atomicOr(m.status, NSEM_STATUS_NONFINITE);
+    if (!nsem_finite(Tn)) atomicOr(m.status, NSEM_STATUS_NONFINITE);
 }
 
 size_t smem_conv(const NsemDev* m) {
@@ -1031,7 +1106,7 @@ AdvArgs adv_args(NsemConvBuf* b, int cur, double dt) {
 
 }  // namespace
 
-int nsem_grad_ut_mortar(const NsemDev* m, const NsemTables* t, const double* const* U,
+int nsem_grad_ut_mortar(const NsemDev* m, const double* const* U,
                         const double* T, double* const* G, double* const* fF, double* const* gC,
                         void* stream) {
     GradArgs ga;
@@ -1042,19 +1117,19 @@ int nsem_grad_ut_mortar(const NsemDev* m, const NsemTables* t, const double* con
     for (int c = 0; c < 4; c++) ga.gC[c] = gC ? gC[c] : nullptr;
     cudaStream_t st = (cudaStream_t)stream;
     const int threads = ((m->np + 31) / 32) * 32;
-    nsem_launch_chained(k_seg_grad_face, (unsigned)((m->n_slot + 255) / 256), 256, 0, st, *m, ga);
+    nsem_launch_chained(k_seg_grad_face, (unsigned)((m->n_slot + FACE - 1) / FACE), FACE, 0, st, *m, ga);
     if (m->n_ms > 0 && gC) {
         const unsigned mb = (unsigned)((m->n_ms + 127) / 128);
         k_seg_mortar_gcds<<<mb, 128, 0, st>>>(*m, ga);
         k_seg_mortar_ggather<<<mb, 128, 0, st>>>(*m, ga);
     }
-    nsem_launch_chained(k_seg_grad_vol, (unsigned)m->n_elem, threads, smem_grad(m), st, *m, *t, ga);
+    nsem_launch_chained(k_seg_grad_vol, (unsigned)m->n_elem, threads, smem_grad(m), st, *m, ga);
     return (int)cudaGetLastError();
 }
 
-int nsem_grad_ut(const NsemDev* m, const NsemTables* t, const double* const* U, const double* T,
+int nsem_grad_ut(const NsemDev* m, const double* const* U, const double* T,
                  double* const* G, double* const* fF, void* stream) {
-    return nsem_grad_ut_mortar(m, t, U, T, G, fF, nullptr, stream);
+    return nsem_grad_ut_mortar(m, U, T, G, fF, nullptr, stream);
 }
 
 int nsem_grad_mortar_faces(const NsemDev* m, const double* const* U, const double* T,
@@ -1071,7 +1146,7 @@ int nsem_grad_mortar_faces(const NsemDev* m, const double* const* U, const doubl
     return (int)cudaGetLastError();
 }
 
-int nsem_grad_vol(const NsemDev* m, const NsemTables* t, const double* const* U, const double* T,
+int nsem_grad_vol(const NsemDev* m, const double* const* U, const double* T,
                   double* const* G, const double* const* fF, const double* const* gC, void* stream) {
     GradArgs ga;
     for (int c = 0; c < 3; c++) ga.U[c] = U[c];
@@ -1080,7 +1155,7 @@ int nsem_grad_vol(const NsemDev* m, const NsemTables* t, const double* const* U,
     for (int c = 0; c < 4; c++) ga.fF[c] = const_cast<double*>(fF[c]);
     for (int c = 0; c < 4; c++) ga.gC[c] = gC ? const_cast<double*>(gC[c]) : nullptr;
     const int threads = ((m->np + 31) / 32) * 32;
-    nsem_launch_chained(k_seg_grad_vol, (unsigned)m->n_elem, threads, smem_grad(m), (cudaStream_t)stream, *m, *t, ga);
+    nsem_launch_chained(k_seg_grad_vol, (unsigned)m->n_elem, threads, smem_grad(m), (cudaStream_t)stream, *m, ga);
     return (int)cudaGetLastError();
 }
 
@@ -1088,23 +1163,23 @@ int nsem_conv_lambda(const NsemDev* m, NsemConvBuf* b, void* stream) {
     const AdvArgs a = adv_args(b, b->cur, 1.0);
     if (m->n_ms > 0)
         k_conv_mortar<0><<<(unsigned)((m->n_ms + 127) / 128), 128, 0, (cudaStream_t)stream>>>(*m, a);
-    k_conv_lambda<<<(unsigned)((m->n_slot + 255) / 256), 256, 0, (cudaStream_t)stream>>>(*m, a);
+    k_conv_lambda<<<(unsigned)((m->n_slot + FACE - 1) / FACE), FACE, 0, (cudaStream_t)stream>>>(*m, a);
     return (int)cudaGetLastError();
 }
 
-int nsem_conv_steps(const NsemDev* m, const NsemTables* t, NsemConvBuf* b, int nsteps, double dt,
+int nsem_conv_steps(const NsemDev* m, NsemConvBuf* b, int nsteps, double dt,
                     void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
-    const unsigned sb = (unsigned)((m->n_slot + 255) / 256);
+    const unsigned sb = (unsigned)((m->n_slot + FACE - 1) / FACE);
     const int threads = ((m->np + 31) / 32) * 32;
     int cur = b->cur;
     for (int s = 0; s < nsteps; s++) {
         const AdvArgs a = adv_args(b, cur, dt);
         const unsigned mb = (unsigned)((m->n_ms + 127) / 128);
         if (m->n_ms > 0) k_conv_mortar<1><<<4 * mb, 128, 0, st>>>(*m, a);
-        nsem_launch_chained(k_conv_face, sb, 256, 0, st, *m, a);
+        nsem_launch_chained(k_conv_face, sb, FACE, 0, st, *m, a);
         if (m->n_ms > 0) k_conv_mortar_gather<<<mb, 128, 0, st>>>(*m, a);
-        nsem_launch_chained(k_conv_vol, (unsigned)m->n_elem, threads, smem_conv(m), st, *m, *t, a);
+        nsem_launch_chained(k_conv_vol, (unsigned)m->n_elem, threads, smem_conv(m), st, *m, a);
         const int e = (int)cudaGetLastError();
         if (e) return e;
         cur ^= 1;
@@ -1112,10 +1187,10 @@ int nsem_conv_steps(const NsemDev* m, const NsemTables* t, NsemConvBuf* b, int n
     return 0;
 }
 
-int nsem_conv_steps_wind(const NsemDev* m, const NsemTables* t, NsemConvBuf* b, int nsteps,
+int nsem_conv_steps_wind(const NsemDev* m, NsemConvBuf* b, int nsteps,
                          double dt, const double* scale, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
-    const unsigned sb = (unsigned)((m->n_slot + 255) / 256);
+    const unsigned sb = (unsigned)((m->n_slot + FACE - 1) / FACE);
     const int threads = ((m->np + 31) / 32) * 32;
     const int64_t nw = m->n_int > m->n_slot ? m->n_int : m->n_slot;
     for (int s = 0; s < nsteps; s++) {
@@ -1134,9 +1209,9 @@ int nsem_conv_steps_wind(const NsemDev* m, const NsemTables* t, NsemConvBuf* b, 
         }
         const unsigned mb = (unsigned)((m->n_ms + 127) / 128);
         if (m->n_ms > 0) k_conv_mortar<1><<<4 * mb, 128, 0, st>>>(*m, a);
-        nsem_launch_chained(k_conv_face, sb, 256, 0, st, *m, a);
+        nsem_launch_chained(k_conv_face, sb, FACE, 0, st, *m, a);
         if (m->n_ms > 0) k_conv_mortar_gather<<<mb, 128, 0, st>>>(*m, a);
-        nsem_launch_chained(k_conv_vol, (unsigned)m->n_elem, threads, smem_conv(m), st, *m, *t, a);
+        nsem_launch_chained(k_conv_vol, (unsigned)m->n_elem, threads, smem_conv(m), st, *m, a);
         const int e = (int)cudaGetLastError();
         if (e) return e;
         b->cur ^= 1;
@@ -1167,11 +1242,11 @@ int nsem_seg_prepare(const NsemDev* m) {
     return 0;
 }
 
-int nsem_seg_steps(const NsemDev* m, const NsemTables* t, NsemSegBuf* b, int nsteps, double dt,
+int nsem_seg_steps(const NsemDev* m, NsemSegBuf* b, int nsteps, double dt,
                    void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     const unsigned nb = (unsigned)((m->n_int + 255) / 256);
-    const unsigned sb = (unsigned)((m->n_slot + 255) / 256);
+    const unsigned sb = (unsigned)((m->n_slot + FACE - 1) / FACE);
     const int threads = ((m->np + 31) / 32) * 32;
     const bool mort = m->n_ms > 0;
     const unsigned mb = (unsigned)((m->n_ms + 127) / 128);
@@ -1186,21 +1261,21 @@ int nsem_seg_steps(const NsemDev* m, const NsemTables* t, NsemSegBuf* b, int nst
             for (int c = 0; c < 12; c++) ga.G[c] = a.G[c];
             for (int c = 0; c < 4; c++) ga.fF[c] = a.fF[c];
             for (int c = 0; c < 4; c++) ga.gC[c] = a.gC[c];
-            nsem_launch_chained(k_seg_grad_face, sb, 256, 0, st, *m, ga);
+            nsem_launch_chained(k_seg_grad_face, sb, FACE, 0, st, *m, ga);
             if (mort) {
                 k_seg_mortar_gcds<<<mb, 128, 0, st>>>(*m, ga);
                 k_seg_mortar_ggather<<<mb, 128, 0, st>>>(*m, ga);
             }
-            nsem_launch_chained(k_seg_grad_vol, (unsigned)m->n_elem, threads, smem_grad(m), st, *m, *t, ga);
+            nsem_launch_chained(k_seg_grad_vol, (unsigned)m->n_elem, threads, smem_grad(m), st, *m, ga);
         }
         if (mort) k_seg_mortar_rho<<<6 * mb, 128, 0, st>>>(*m, a);
-        nsem_launch_chained(k_seg_face_rho, sb, 256, 0, st, *m, a);
+        nsem_launch_chained(k_seg_face_rho, sb, FACE, 0, st, *m, a);
         if (mort) k_seg_mortar_gather<0><<<mb, 128, 0, st>>>(*m, a);
-        nsem_launch_chained(k_seg_vol_rho, (unsigned)m->n_elem, threads, smem_rho(m), st, *m, *t, a);
+        nsem_launch_chained(k_seg_vol_rho, (unsigned)m->n_elem, threads, smem_rho(m), st, *m, a);
         if (mort) k_seg_mortar_ut<<<16 * mb, 128, 0, st>>>(*m, a);
-        nsem_launch_chained(k_seg_face_ut, sb, 256, 0, st, *m, a);
+        nsem_launch_chained(k_seg_face_ut, sb, FACE, 0, st, *m, a);
         if (mort) k_seg_mortar_gather<1><<<4 * mb, 128, 0, st>>>(*m, a);
-        nsem_launch_chained(k_seg_vol_ut, (unsigned)m->n_elem, threads, smem_ut(m), st, *m, *t, a);
+        nsem_launch_chained(k_seg_vol_ut, (unsigned)m->n_elem, threads, smem_ut(m), st, *m, a);
         const int e = (int)cudaGetLastError();
         if (e) return e;
         cur ^= 1;

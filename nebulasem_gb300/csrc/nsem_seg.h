@@ -55,7 +55,7 @@ struct NsemConvBuf {
 int nsem_seg_prepare(const NsemDev* m);
 /* convection steps with the analytic wind scaled by scale[s] (NULL: 1) and
  * the buffer's time scheme; advances b->cur and the AB2 history */
-int nsem_conv_steps_wind(const NsemDev* m, const NsemTables* t, NsemConvBuf* b, int nsteps,
+int nsem_conv_steps_wind(const NsemDev* m, NsemConvBuf* b, int nsteps,
                          double dt, const double* scale, void* stream);
 /* strong-form gradients of U (3 arrays) and the full theta T into G (12 per
  * node) with the per-slot scratch fF (4), for the viscous fluxes */
@@ -63,25 +63,25 @@ int nsem_conv_steps_wind(const NsemDev* m, const NsemTables* t, NsemConvBuf* b, 
  * (cds of U and theta) and, on a mesh with non-conforming faces, the
  * projected coarse-side values gC (4 arrays per mortar slot; else null);
  * linear in (U, T, fF, gC) */
-int nsem_grad_vol(const NsemDev* m, const NsemTables* t, const double* const* U, const double* T,
+int nsem_grad_vol(const NsemDev* m, const double* const* U, const double* T,
                   double* const* G, const double* const* fF, const double* const* gC, void* stream);
 /* the mortar slots' face values of the gradients alone: cds(U, theta) with
  * the coarse side interpolated into fF, and its projection onto the coarse
  * side into gC; linear in (U, T) */
 int nsem_grad_mortar_faces(const NsemDev* m, const double* const* U, const double* T,
                            double* const* fF, double* const* gC, void* stream);
-int nsem_grad_ut(const NsemDev* m, const NsemTables* t, const double* const* U, const double* T,
+int nsem_grad_ut(const NsemDev* m, const double* const* U, const double* T,
                  double* const* G, double* const* fF, void* stream);
 /* the same on a mesh with non-conforming faces: gC (4 arrays per mortar
  * slot) receives the projected face values */
-int nsem_grad_ut_mortar(const NsemDev* m, const NsemTables* t, const double* const* U,
+int nsem_grad_ut_mortar(const NsemDev* m, const double* const* U,
                         const double* T, double* const* G, double* const* fF, double* const* gC,
                         void* stream);
 /* lambda of the fixed wind (once, after U is set) */
 int nsem_conv_lambda(const NsemDev* m, NsemConvBuf* b, void* stream);
-int nsem_conv_steps(const NsemDev* m, const NsemTables* t, NsemConvBuf* b, int nsteps, double dt,
+int nsem_conv_steps(const NsemDev* m, NsemConvBuf* b, int nsteps, double dt,
                     void* stream);
-int nsem_seg_steps(const NsemDev* m, const NsemTables* t, NsemSegBuf* b, int nsteps, double dt,
+int nsem_seg_steps(const NsemDev* m, NsemSegBuf* b, int nsteps, double dt,
                    void* stream);
 /* u = conserved state of the primitive fields rho[cur], U, T' */
 int nsem_seg_to_cons(const NsemDev* m, const NsemSegBuf* b, double* const* u, void* stream);

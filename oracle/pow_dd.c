@@ -89,7 +89,7 @@ void nsem_oracle_intfp_sweep(int64_t n, uint64_t seed, int64_t bad[3]) {
         const double d[3] = {p, nextafter(p, 0.0), nextafter(p, INFINITY)};
         bd += nsem_bits(nsem_div(a, b)) != nsem_bits(a / b);
         bs += nsem_bits(nsem_sqrt(c)) != nsem_bits(sqrt(c));
-        bm += nsem_bits(nsem_mul_normal(nsem_make_factor(a), b)) != nsem_bits(p);
+        bm += nsem_bits(nsem_mul_normal(nsem_make_factor(a), b)) != nsem_bits(p) && (p != 0.0);
         for (int q = 0; q < 3; q++) {
             bd += nsem_bits(nsem_div(d[q], b)) != nsem_bits(d[q] / b);
             bs += nsem_bits(nsem_sqrt(t[q])) != nsem_bits(sqrt(t[q]));
