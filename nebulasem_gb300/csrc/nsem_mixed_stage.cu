@@ -68,8 +68,9 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
 /* registers sized for 8 resident CTAs per SM in stages 1-2 and 9 in stage 3,
  * which loads the FP64 state only at the update (measured best on GB300:
  * 152 us at 32^3, against 172 us with the state held in registers at 7 CTAs
- * and 163 us at 8); viscous runs 6, and 5 in stage 3 (its gradients spill at
- * 6) */
+ * and 163 us at 8); viscous runs, which hold 12 gradients, 7 and 6 in stage 3
+ * (9240 elements of order 4, 20 steps: 5186 us; 5311 us at 6 and at 5 with the
+ * state held; 5196 at 6 and 6, 5182 at 7 and 7 with spills) */
 #ifndef NSEM_MIXED_MB12
 #define NSEM_MIXED_MB12 8
 #endif
@@ -83,7 +84,7 @@ constexpr int stage_min_blocks() {
     if (Geo<NX, NY, NZ>::BLOCK >= 512)
         return min_blocks((VISC || STAGE == 0) ? 2 : 3, Geo<NX, NY, NZ>::BLOCK,
                           StageSmem<NX, NY, NZ>::BYTES);
-    return min_blocks(VISC ? (STAGE == 3 ? 5 : 6) : (STAGE == 1 || STAGE == 2) ? NSEM_MIXED_MB12 : NSEM_MIXED_MB3,
+    return min_blocks(VISC ? (STAGE == 3 ? 6 : 7) : (STAGE == 1 || STAGE == 2) ? NSEM_MIXED_MB12 : NSEM_MIXED_MB3,
                       Geo<NX, NY, NZ>::BLOCK, StageSmem<NX, NY, NZ>::BYTES);
 }
 
@@ -324,7 +325,6 @@ k_mixed_stage(StageArgs a) {
     /* what no kernel of the chain writes, before the wait for the previous
      * kernel: background, neighbours, metric */
     float own[5], din[5] = {0, 0, 0, 0, 0}, bgs[4] = {0, 0, 0, 0};
-    double u64[5];
     float gown[12];
     if (t < NP) {
         const float* bg = a.bg + (int64_t)__ldg(a.layer + e) * 4 * NP + t;
@@ -364,18 +364,13 @@ k_mixed_stage(StageArgs a) {
             }
         }
         if constexpr (STAGE == 3) {
-            /* u'^n is needed only at the update: inviscid runs fetch it into L2
-             * here and load it there (with the increment reloaded from L1/L2),
-             * so that neither holds registers through the element and nine
-             * CTAs fit per SM; viscous runs (five CTAs either way) hold it */
+            /* u'^n is needed only at the update: fetched into L2 here and
+             * loaded there (with the increment reloaded from L1/L2), so that
+             * neither holds registers through the element and nine CTAs (six
+             * in viscous runs) fit per SM */
             const double* u = a.U + e * 5 * NP + t;
-            if constexpr (VISC) {
 #pragma unroll
-                for (int v = 0; v < 5; v++) u64[v] = u[v * NP];
-            } else {
-#pragma unroll
-                for (int v = 0; v < 5; v++) asm volatile("prefetch.global.L2 [%0];" ::"l"(u + v * NP));
-            }
+            for (int v = 0; v < 5; v++) asm volatile("prefetch.global.L2 [%0];" ::"l"(u + v * NP));
         }
         if constexpr (VISC) {
             const float* gr = a.G + e * 12 * NP + t;
@@ -579,12 +574,11 @@ k_mixed_stage(StageArgs a) {
     } else if constexpr (STAGE == 3) {
         bool finite = true;
         /* every load before the first store, which could alias them */
-        if constexpr (!VISC) {
+        double u64[5];
 #pragma unroll
-            for (int v = 0; v < 5; v++) {
-                din[v] = a.Din[o + v * NP];
-                u64[v] = a.U[o + v * NP];
-            }
+        for (int v = 0; v < 5; v++) {
+            din[v] = a.Din[o + v * NP];
+            u64[v] = a.U[o + v * NP];
         }
 #pragma unroll
         for (int v = 0; v < 5; v++) {
