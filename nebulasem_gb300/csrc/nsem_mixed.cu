@@ -501,9 +501,12 @@ int dispatch_stage(int nx, int ny, int nz, const StageArgs& a, int stage, cudaSt
     return launch_stage_aligned(nx, ny, nz, a, stage, st, c);
 }
 
-int dispatch_grad(int nx, int ny, int nz, const StageArgs& a, int stage, cudaStream_t st,
-                  const LaunchCfg& c) {
-    if (c.gen) return launch_grad_general(nx, ny, nz, a, stage, st);
+/* the gradient kernels take the derivative tables in place of the weights */
+int dispatch_grad(const NsemMixedBuf* mb, const StageArgs& s, int stage, cudaStream_t st) {
+    StageArgs a = s;
+    std::memcpy(a.qc, mb->dc, sizeof(a.qc));
+    const int nx = mb->npd[0], ny = mb->npd[1], nz = mb->npd[2];
+    if (mb->gen) return launch_grad_general(nx, ny, nz, a, stage, st);
     return launch_grad_aligned(nx, ny, nz, a, stage, st);
 }
 
@@ -699,7 +702,7 @@ nsem_status nsem_mixed_setup(const NsemDev& dev, const nsem_mesh_desc* m, NsemMi
         }
         for (int q = 0; q < n; q++) wdir[d][q] = 2.0 * wdir[d][q] / sum;
     }
-    std::vector<float> qtab(QTAB, 0.0f), dtab(QTAB, 0.0f);
+    std::vector<float> qtab(QTAB, 0.0f);
     for (int d = 0; d < 3; d++) {
         const int n = npd[d];
         const std::vector<double>& w = wdir[d];
@@ -709,14 +712,13 @@ nsem_status nsem_mixed_setup(const NsemDev& dev, const nsem_mesh_desc* m, NsemMi
                  * weights sit in Jinv cV and 1/cV */
                 qtab[d * MAXN * QS + aa * QS + mm] =
                     gen ? (float)m->dpsi[d][mm * n + aa] : (float)(m->dpsi[d][mm * n + aa] * w[mm] / w[aa]);
-                /* D_d[a][m] = l_m'(x_a) = dpsi[a * n + m] for the gradient kernel */
-                dtab[d * MAXN * QS + aa * QS + mm] = (float)m->dpsi[d][aa * n + mm];
             }
         mb->lift[d] = (float)(1.0 / w[0]);
         for (int aa = 0; aa < n && aa < 8; aa++)
             for (int mm = 0; mm < n && mm < 8; mm++) {
                 mb->qc[d][aa][mm] = qtab[d * MAXN * QS + aa * QS + mm];
-                mb->dc[d][aa][mm] = dtab[d * MAXN * QS + aa * QS + mm];
+                /* D_d[a][m] = l_m'(x_a) = dpsi[a * n + m] for the gradient kernels */
+                mb->dc[d][aa][mm] = (float)m->dpsi[d][aa * n + mm];
             }
     }
     /* order 7: the tensor-core line sums' B fragments, Q_d^T split into TF32
@@ -910,7 +912,7 @@ nsem_status nsem_mixed_setup(const NsemDev& dev, const nsem_mesh_desc* m, NsemMi
         return cudaMemcpy(*ptr, vec.data(), bytes, cudaMemcpyHostToDevice) == cudaSuccess;
     };
     if (!up(&mb->nbr, nbr) || !up(&mb->J, J) || !up(&mb->layer, layer) || !up(&mb->bg, bg) ||
-        !up(&mb->Qg, qtab) || !up(&mb->Dg, dtab) || (gen && (!up(&mb->Jg, Jg) || !up(&mb->Fn, Fn)))) {
+        !up(&mb->Qg, qtab) || (gen && (!up(&mb->Jg, Jg) || !up(&mb->Fn, Fn)))) {
         err = "precision form: device allocation failed";
         return NSEM_NO_MEMORY;
     }
@@ -989,7 +991,6 @@ StageArgs base_args(const NsemDev* dev, const NsemMixedBuf* mb, double dt) {
     a.J = mb->J;
     a.layer = mb->layer;
     a.Qg = mb->Qg;
-    a.Dg = mb->Dg;
     a.G = mb->G;
     a.Gout = mb->G;
     a.nu = mb->nu;
@@ -1087,7 +1088,7 @@ int launch_args(const NsemMixedBuf* mb, const StageArgs& a, int stage, cudaStrea
             const int e = launch_mortar_grads(mb, a, stage, st);
             if (e) return e;
         }
-        const int e = dispatch_grad(mb->npd[0], mb->npd[1], mb->npd[2], a, stage, st, c);
+        const int e = dispatch_grad(mb, a, stage, st);
         if (e) return e;
     }
     if (mb->n_ms > 0) {
@@ -1133,15 +1134,12 @@ int nsem_mixed_grad_at(const NsemDev* dev, const NsemMixedBuf* mb, const float* 
     StageArgs a = base_args(dev, mb, 0.0);
     a.S = S;
     a.Din = Din;
-    LaunchCfg c{};
-    c.visc = true;
-    c.gen = mb->gen;
     /* the gradients' face values on mortars first */
     if (mb->n_ms > 0) {
         const int e = launch_mortar_grads(mb, a, Din ? 2 : 1, (cudaStream_t)stream);
         if (e) return e;
     }
-    return dispatch_grad(mb->npd[0], mb->npd[1], mb->npd[2], a, Din ? 2 : 1, (cudaStream_t)stream, c);
+    return dispatch_grad(mb, a, Din ? 2 : 1, (cudaStream_t)stream);
 }
 
 int nsem_mixed_convert(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf* b, int to_pert,

@@ -29,10 +29,9 @@ struct NsemMixedBuf {
     float* J = nullptr;           /* [3][n_elem] metric diagonal 2/h        */
     int32_t* layer = nullptr;     /* [n_elem] background layer              */
     float qc[3][8][8] = {};       /* host copy of the line-sum weights      */
-    float dc[3][8][8] = {};       /* host copy of the derivative tables D_d[a][m] */
+    float dc[3][8][8] = {};       /* derivative tables D_d[a][m] = l_m'(x_a) */
     float* bg = nullptr;          /* [layers][4][NP] rho_ref, Theta_ref, 1/Theta_ref, p_ref */
     float* Qg = nullptr;          /* line-sum weights Q_d[a][m], row stride MAXN+1 */
-    float* Dg = nullptr;          /* derivative tables D_d[a][m] = l_m'(x_a), same layout */
     float* G = nullptr;           /* viscous runs: [n_elem][12][NP] gradients of the stage state */
     bool visc = false;            /* artificial viscosity (diffusion YES)   */
     bool tc = false;              /* order-7 line sums on the tensor cores  */

@@ -391,9 +391,8 @@ k_mixed_grad_gen(StageArgs a) {
     constexpr int NFS = G::NFS;
     constexpr bool has_din = SIN >= 2;
     extern __shared__ float4 ggsm4[];
-    float4* sV = ggsm4;                                             /* [NP]  U, theta - T0 */
-    float4* sD = ggsm4 + NP;                                        /* [NFS] cds - own */
-    float* sDg = reinterpret_cast<float*>(ggsm4 + NP + NFS);       /* line tables */
+    using GL = GradLay<NX, NY, NZ>;
+    float4* sD = ggsm4 + GL::OFF_D;                                 /* [NFS] cds - own */
     const int t = threadIdx.x;
     const int64_t e = blockIdx.x;
 
@@ -415,7 +414,6 @@ k_mixed_grad_gen(StageArgs a) {
         for (int c = 0; c < 3; c++) fno[c] = __ldg(a.Fn + (e * 3 + c) * NFS + t);
         if (nb >= 0) bgo0 = __ldg(a.bg + (int64_t)__ldg(a.layer + nb) * 4 * NP + fs.lo);
     }
-    for (int q = t; q < QTAB; q += G::BLOCK) sDg[q] = __ldg(a.Dg + q);
     nsem_chain_wait();
     if (t < NP) {
         const float* s = a.S + e * 5 * NP + t;
@@ -444,11 +442,11 @@ k_mixed_grad_gen(StageArgs a) {
         return make_float4(__fmul_rn(s[1], inv), __fmul_rn(s[2], inv), __fmul_rn(s[3], inv),
                            __fmul_rn(__fmaf_rn(-T0, s[0], s[4]), inv));
     };
-    if (t < NP) sV[t] = prim_ut(own, bgs0);
+    if (t < NP) ggsm4[GL::at(t)] = prim_ut(own, bgs0);
     __syncthreads();
 
     if (t < NFS && nb > -2) {
-        const float4 S = sV[fs.la];
+        const float4 S = ggsm4[GL::at(fs.la)];
         float4 c;
         if (nb >= 0) {
             const float4 O = prim_ut(oth, bgo0);
@@ -474,39 +472,15 @@ k_mixed_grad_gen(StageArgs a) {
     __syncthreads();
 
     nsem_chain_begin();
+    /* derivatives along the reference directions */
+    grad_lines<NX, NY, NZ, false>(ggsm4, a, t, nullptr);
+    __syncthreads();
     if (t >= NP) return;
     const int i = t / (NY * NZ), j = (t / NZ) % NY, k = t % NZ;
-    /* derivatives along the reference directions */
     float4 d[3];
 #pragma unroll
-    for (int r = 0; r < 3; r++) d[r] = make_float4(0, 0, 0, 0);
-    {
-        const float* q = sDg + i * QS;
-#pragma unroll
-        for (int m = 0; m < NX; m++) {
-            const float4 v = sV[(m * NY + j) * NZ + k];
-            d[0].x = fmaf(q[m], v.x, d[0].x); d[0].y = fmaf(q[m], v.y, d[0].y);
-            d[0].z = fmaf(q[m], v.z, d[0].z); d[0].w = fmaf(q[m], v.w, d[0].w);
-        }
-    }
-    if constexpr (G::HAS_Y) {
-        const float* q = sDg + MAXN * QS + j * QS;
-#pragma unroll
-        for (int m = 0; m < NY; m++) {
-            const float4 v = sV[(i * NY + m) * NZ + k];
-            d[1].x = fmaf(q[m], v.x, d[1].x); d[1].y = fmaf(q[m], v.y, d[1].y);
-            d[1].z = fmaf(q[m], v.z, d[1].z); d[1].w = fmaf(q[m], v.w, d[1].w);
-        }
-    }
-    {
-        const float* q = sDg + 2 * MAXN * QS + k * QS;
-#pragma unroll
-        for (int m = 0; m < NZ; m++) {
-            const float4 v = sV[(i * NY + j) * NZ + m];
-            d[2].x = fmaf(q[m], v.x, d[2].x); d[2].y = fmaf(q[m], v.y, d[2].y);
-            d[2].z = fmaf(q[m], v.z, d[2].z); d[2].w = fmaf(q[m], v.w, d[2].w);
-        }
-    }
+    for (int r = 0; r < 3; r++)
+        d[r] = r == 1 && !G::HAS_Y ? make_float4(0, 0, 0, 0) : ggsm4[GL::w(r) + GL::at(t)];
     /* physical components: sum_d (Jinv cV)[r][d] d_d, then the face terms */
     float4 g[3];
 #pragma unroll
@@ -588,7 +562,7 @@ template <int NX, int NY, int NZ>
 int launch_grad_gen(const StageArgs& a, int stage, cudaStream_t st) {
     using G = Geo<NX, NY, NZ>;
     const unsigned grid = (unsigned)a.n_elem;
-    constexpr size_t gs = grad_smem<NX, NY, NZ>();
+    constexpr size_t gs = GradLay<NX, NY, NZ>::BYTES;
     constexpr unsigned B = G::BLOCK;
     return stage <= 1 ? nsem_launch_chained(k_mixed_grad_gen<NX, NY, NZ, 1>, grid, B, gs, st, a)
                       : nsem_launch_chained(k_mixed_grad_gen<NX, NY, NZ, 2>, grid, B, gs, st, a);
@@ -612,7 +586,7 @@ int prepare_gen() {
         if (!e) e = (int)cudaFuncSetAttribute(k_mixed_stage_gen<NX, NY, NZ, 2, true>, at, GSV);
         if (!e) e = (int)cudaFuncSetAttribute(k_mixed_stage_gen<NX, NY, NZ, 3, true>, at, GSV);
     }
-    constexpr size_t gs = grad_smem<NX, NY, NZ>();
+    constexpr size_t gs = GradLay<NX, NY, NZ>::BYTES;
     if (!e && gs > 48 * 1024) {
         e = (int)cudaFuncSetAttribute(k_mixed_grad_gen<NX, NY, NZ, 1>, at, (int)gs);
         if (!e) e = (int)cudaFuncSetAttribute(k_mixed_grad_gen<NX, NY, NZ, 2>, at, (int)gs);

@@ -28,7 +28,6 @@ struct StageArgs {
     const float* J;            /* [3][n_elem]                             */
     const int32_t* layer;      /* [n_elem]                                */
     const float* Qg;           /* line-sum weights                        */
-    const float* Dg;           /* derivative tables (gradient kernel)     */
     const float* G;            /* viscous runs: [e][12][NP] gradients      */
     float* Gout;               /* gradient kernel output                   */
     const float* bg;           /* [layers][4][NP]                          */
@@ -43,8 +42,9 @@ struct StageArgs {
     float lift[3];             /* 1 / w_end per direction                  */
     float eos[6];              /* binomial coefficients C(gamma, k), k = 1..6 */
     uint32_t* status;
-    /* line-sum weights Q_d[a][m] as kernel parameters: read with
-     * compile-time indices they are constant-bank operands of the FMAs */
+    /* line-sum weights Q_d[a][m] (gradient kernels: the derivative tables
+     * D_d[a][m]) as kernel parameters: read with compile-time indices they
+     * are constant-bank operands of the FMAs */
     float qc[3][8][8];
 };
 
@@ -97,12 +97,89 @@ __device__ __forceinline__ int face_local(int t) {
     return (t - G::OFF_Z) % G::NFZ;
 }
 
-/* dynamic shared memory of the gradient kernels: the nodes' U and theta,
- * the face values, the derivative tables */
+/* The gradient kernels' shared memory, in float4 (U, theta - T0): the nodes'
+ * values V, the face terms cds - own, and per direction the derivatives at
+ * the nodes.  Rows of nodes along z have an odd pitch: a quarter warp's
+ * 16-byte accesses down z lines are then conflict-free at even node counts. */
 template <int NX, int NY, int NZ>
-constexpr size_t grad_smem() {
+struct GradLay {
     using G = Geo<NX, NY, NZ>;
-    return sizeof(float4) * (G::NP + G::NFS) + sizeof(float) * (QTAB + 4);
+    static constexpr int PZ = NZ | 1;
+    static constexpr int NV = NX * NY * PZ;
+    static constexpr int OFF_D = NV;
+    static constexpr int OFF_W = OFF_D + G::NFS;
+    static constexpr size_t BYTES = sizeof(float4) * (OFF_W + (G::HAS_Y ? 3 : 2) * NV);
+    /* first position of direction D's derivatives */
+    __host__ __device__ static constexpr int w(int D) { return OFF_W + (D == 0 ? 0 : D == 1 ? NV : (G::HAS_Y ? 2 : 1) * NV); }
+    __device__ static __forceinline__ int at(int i, int j, int k) { return (i * NY + j) * PZ + k; }
+    /* node t of the element's own numbering */
+    __device__ static __forceinline__ int at(int t) { return NZ == PZ ? t : t / NZ * PZ + t % NZ; }
+};
+
+/* derivatives along line l of direction D: W_a = sum_m D_D[a][m] V_m.  With
+ * ALIGNED the metric and the face terms at the line's two ends join here:
+ * J_D W_a - / + (J_D / w_end) (cds - own). */
+template <int NX, int NY, int NZ, int D, bool ALIGNED>
+__device__ __forceinline__ void grad_line(float4* sm, const StageArgs& a, int l, float Jd) {
+    using G = Geo<NX, NY, NZ>;
+    using L = GradLay<NX, NY, NZ>;
+    constexpr int n = D == 0 ? NX : D == 1 ? NY : NZ;
+    constexpr int STEP = D == 0 ? NY * L::PZ : D == 1 ? L::PZ : 1;
+    constexpr int OFF = D == 0 ? G::OFF_X : D == 1 ? G::OFF_Y : G::OFF_Z;
+    constexpr int NF = D == 0 ? G::NFX : D == 1 ? G::NFY : G::NFZ;
+    /* lines in the order of the face's nodes: x (j, k), y (i, k), z (i, j) */
+    const int n0 = D == 0 ? L::at(0, l / NZ, l % NZ) : D == 1 ? L::at(l / NZ, 0, l % NZ) : l * L::PZ;
+    float4 in[n];
+#pragma unroll
+    for (int m = 0; m < n; m++) in[m] = sm[n0 + m * STEP];
+#pragma unroll
+    for (int q = 0; q < n; q++) {
+        float4 acc = make_float4(0, 0, 0, 0);
+#pragma unroll
+        for (int m = 0; m < n; m++) {
+            const float d = a.qc[D][q][m];
+            acc.x = __fmaf_rn(d, in[m].x, acc.x); acc.y = __fmaf_rn(d, in[m].y, acc.y);
+            acc.z = __fmaf_rn(d, in[m].z, acc.z); acc.w = __fmaf_rn(d, in[m].w, acc.w);
+        }
+        if constexpr (ALIGNED) {
+            acc.x = __fmul_rn(acc.x, Jd); acc.y = __fmul_rn(acc.y, Jd);
+            acc.z = __fmul_rn(acc.z, Jd); acc.w = __fmul_rn(acc.w, Jd);
+            if (q == 0 || q == n - 1) {
+                const float c = __fmul_rn(Jd, a.lift[D]);
+                const float coef = q == 0 ? -c : c;
+                const float4 f = sm[L::OFF_D + OFF + (q == 0 ? 0 : NF) + l];
+                acc.x = __fmaf_rn(coef, f.x, acc.x); acc.y = __fmaf_rn(coef, f.y, acc.y);
+                acc.z = __fmaf_rn(coef, f.z, acc.z); acc.w = __fmaf_rn(coef, f.w, acc.w);
+            }
+        }
+        sm[L::w(D) + n0 + q * STEP] = acc;
+    }
+}
+
+/* all lines of the element, one per thread, each direction's in warps of its
+ * own.  The kernels are bound by shared-memory wavefronts: a line's values are
+ * read once and shared by its sums, 10 float4 accesses per line of 5 nodes
+ * where a thread per node makes 25 and 25 table reads (viscous step with its
+ * stage kernels, 9240 elements of order 4, 20 steps: 4960 us against 5185;
+ * 1716 of order 7: 3650 against 3884; 400 in 2D, order 3, 40 steps: 632
+ * against 849; with the full metric 7280 against 7486, order 3 alone 1.5 %
+ * slower, 3708 against 3652) */
+template <int NX, int NY, int NZ, bool ALIGNED>
+__device__ __forceinline__ void grad_lines(float4* sm, const StageArgs& a, int t, const float* sJ) {
+    using G = Geo<NX, NY, NZ>;
+    constexpr int WX = (G::NFX + 31) / 32 * 32, WY = G::HAS_Y ? (G::NFY + 31) / 32 * 32 : 0,
+                  WZ = (G::NFZ + 31) / 32 * 32;
+    for (int r = t; r < WX + WY + WZ; r += G::BLOCK) {
+        if (r < WX) {
+            if (r < G::NFX) grad_line<NX, NY, NZ, 0, ALIGNED>(sm, a, r, ALIGNED ? sJ[0] : 1.0f);
+        } else if (r < WX + WY) {
+            if constexpr (G::HAS_Y) {
+                if (r - WX < G::NFY) grad_line<NX, NY, NZ, 1, ALIGNED>(sm, a, r - WX, ALIGNED ? sJ[1] : 1.0f);
+            }
+        } else if (r - WX - WY < G::NFZ) {
+            grad_line<NX, NY, NZ, 2, ALIGNED>(sm, a, r - WX - WY, ALIGNED ? sJ[2] : 1.0f);
+        }
+    }
 }
 
 struct LaunchCfg {

@@ -135,80 +135,6 @@ __device__ __forceinline__ float4 cds_minus_own(const float4 S, const float4* O,
                        __fsub_rn(c.w, S.w));
 }
 
-/* the gradients of node (i, j, k) from the element's values sV [NP], the
- * face terms sD [NFS] and the derivative tables sDg; out in the 12-entry
- * layout */
-template <int NX, int NY, int NZ>
-__device__ __forceinline__ void grad_node(int i, int j, int k, const float4* sV, const float4* sD,
-                                          const float* sDg, const float* Jd, const float* lift,
-                                          float* out) {
-    using G = Geo<NX, NY, NZ>;
-    float4 d[3];
-    {
-        float4 acc = make_float4(0, 0, 0, 0);
-        const float* q = sDg + i * QS;
-#pragma unroll
-        for (int m = 0; m < NX; m++) {
-            const float4 v = sV[(m * NY + j) * NZ + k];
-            acc.x = __fmaf_rn(q[m], v.x, acc.x); acc.y = __fmaf_rn(q[m], v.y, acc.y);
-            acc.z = __fmaf_rn(q[m], v.z, acc.z); acc.w = __fmaf_rn(q[m], v.w, acc.w);
-        }
-        d[0] = acc;
-    }
-    {
-        float4 acc = make_float4(0, 0, 0, 0);
-        if (NY > 1) {
-            const float* q = sDg + MAXN * QS + j * QS;
-#pragma unroll
-            for (int m = 0; m < NY; m++) {
-                const float4 v = sV[(i * NY + m) * NZ + k];
-                acc.x = __fmaf_rn(q[m], v.x, acc.x); acc.y = __fmaf_rn(q[m], v.y, acc.y);
-                acc.z = __fmaf_rn(q[m], v.z, acc.z); acc.w = __fmaf_rn(q[m], v.w, acc.w);
-            }
-        }
-        d[1] = acc;
-    }
-    {
-        float4 acc = make_float4(0, 0, 0, 0);
-        const float* q = sDg + 2 * MAXN * QS + k * QS;
-#pragma unroll
-        for (int m = 0; m < NZ; m++) {
-            const float4 v = sV[(i * NY + j) * NZ + m];
-            acc.x = __fmaf_rn(q[m], v.x, acc.x); acc.y = __fmaf_rn(q[m], v.y, acc.y);
-            acc.z = __fmaf_rn(q[m], v.z, acc.z); acc.w = __fmaf_rn(q[m], v.w, acc.w);
-        }
-        d[2] = acc;
-    }
-#pragma unroll
-    for (int r = 0; r < 3; r++) {
-        d[r].x = __fmul_rn(d[r].x, Jd[r]); d[r].y = __fmul_rn(d[r].y, Jd[r]);
-        d[r].z = __fmul_rn(d[r].z, Jd[r]); d[r].w = __fmul_rn(d[r].w, Jd[r]);
-    }
-    /* face terms: + (J_r / w_end) (cds - own) on the upper face, - on the lower */
-    auto lf = [&](int r, int slot, float coef) {
-        const float4 f = sD[slot];
-        d[r].x = __fmaf_rn(coef, f.x, d[r].x); d[r].y = __fmaf_rn(coef, f.y, d[r].y);
-        d[r].z = __fmaf_rn(coef, f.z, d[r].z); d[r].w = __fmaf_rn(coef, f.w, d[r].w);
-    };
-    const float cx = __fmul_rn(Jd[0], lift[0]), cy = __fmul_rn(Jd[1], lift[1]),
-                cz = __fmul_rn(Jd[2], lift[2]);
-    if (i == 0) lf(0, G::OFF_X + j * NZ + k, -cx);
-    if (i == NX - 1) lf(0, G::OFF_X + G::NFX + j * NZ + k, cx);
-    if (NY > 1) {
-        if (j == 0) lf(1, G::OFF_Y + i * NZ + k, -cy);
-        if (j == NY - 1) lf(1, G::OFF_Y + G::NFY + i * NZ + k, cy);
-    }
-    if (k == 0) lf(2, G::OFF_Z + i * NY + j, -cz);
-    if (k == NZ - 1) lf(2, G::OFF_Z + G::NFZ + i * NY + j, cz);
-#pragma unroll
-    for (int r = 0; r < 3; r++) {
-        out[tidx(r, 0)] = d[r].x;
-        out[tidx(r, 1)] = d[r].y;
-        out[tidx(r, 2)] = d[r].z;
-        out[9 + r] = d[r].w;
-    }
-}
-
 /* phase 2: flux through face node t, seen from the element.  The face's
  * axis is a run-time value (selects, no branches), so a warp whose face
  * nodes lie on faces of two axes runs one instruction stream; the operations
@@ -601,11 +527,10 @@ k_mixed_grad(StageArgs a) {
     constexpr int NP = G::NP;
     constexpr int NFS = G::NFS;
     constexpr bool has_din = SIN >= 2;
+    using GL = GradLay<NX, NY, NZ>;
     extern __shared__ float4 gsm4[];
-    float4* sV = gsm4;                                              /* [NP]  U, theta */
-    float4* sD = gsm4 + NP;                                         /* [NFS] cds - own */
-    float* sDg = reinterpret_cast<float*>(gsm4 + NP + NFS);        /* line tables */
-    float* sJ = sDg + QTAB;                                         /* [3] */
+    __shared__ float sJ[3];
+    float4* sD = gsm4 + GL::OFF_D;                                  /* [NFS] cds - own */
     const int t = threadIdx.x;
     const int64_t e = blockIdx.x;
 
@@ -619,7 +544,6 @@ k_mixed_grad(StageArgs a) {
         nb = __ldg(a.nbr + (int64_t)fs.face * a.n_elem + e);
         if (nb >= 0) bgo0 = __ldg(a.bg + (int64_t)__ldg(a.layer + nb) * 4 * NP + fs.lo);
     }
-    for (int q = t; q < QTAB; q += G::BLOCK) sDg[q] = __ldg(a.Dg + q);
     if (t < 3) sJ[t] = __ldg(a.J + (int64_t)t * a.n_elem + e);
     nsem_chain_wait();
     if (t < NP) {
@@ -643,7 +567,7 @@ k_mixed_grad(StageArgs a) {
         }
     }
 
-    if (t < NP) sV[t] = prim_ut(own, bgs0, a.T0);
+    if (t < NP) gsm4[GL::at(t)] = prim_ut(own, bgs0, a.T0);
     __syncthreads();
 
     if (t < NFS && nb <= -2) {
@@ -652,18 +576,23 @@ k_mixed_grad(StageArgs a) {
         sD[t] = make_float4(gf[0], gf[a.nfmax], gf[2 * a.nfmax], gf[3 * a.nfmax]);
     } else if (t < NFS) {
         const float4 O = nb >= 0 ? prim_ut(oth, bgo0, a.T0) : make_float4(0, 0, 0, 0);
-        sD[t] = cds_minus_own(sV[fs.la], nb >= 0 ? &O : nullptr, fs.dir);
+        sD[t] = cds_minus_own(gsm4[GL::at(fs.la)], nb >= 0 ? &O : nullptr, fs.dir);
     }
     __syncthreads();
 
     nsem_chain_begin();
+    grad_lines<NX, NY, NZ, true>(gsm4, a, t, sJ);
+    __syncthreads();
     if (t >= NP) return;
-    const int i = t / (NY * NZ), j = (t / NZ) % NY, k = t % NZ;
-    float g12[12];
-    grad_node<NX, NY, NZ>(i, j, k, sV, sD, sDg, sJ, a.lift, g12);
     float* out = a.Gout + e * 12 * NP + t;
 #pragma unroll
-    for (int c = 0; c < 12; c++) out[c * NP] = g12[c];
+    for (int r = 0; r < 3; r++) {
+        const float4 d = r == 1 && !G::HAS_Y ? make_float4(0, 0, 0, 0) : gsm4[GL::w(r) + GL::at(t)];
+        out[tidx(r, 0) * NP] = d.x;
+        out[tidx(r, 1) * NP] = d.y;
+        out[tidx(r, 2) * NP] = d.z;
+        out[(9 + r) * NP] = d.w;
+    }
 }
 
 template <int NX, int NY, int NZ, bool VISC, bool TC>
@@ -704,7 +633,7 @@ template <int NX, int NY, int NZ>
 int launch_grad(const StageArgs& a, int stage, cudaStream_t st) {
     using G = Geo<NX, NY, NZ>;
     const unsigned grid = (unsigned)a.n_elem;
-    constexpr size_t gs = grad_smem<NX, NY, NZ>();
+    constexpr size_t gs = GradLay<NX, NY, NZ>::BYTES;
     constexpr unsigned B = G::BLOCK;
     return stage <= 1 ? nsem_launch_chained(k_mixed_grad<NX, NY, NZ, 1>, grid, B, gs, st, a)
                       : nsem_launch_chained(k_mixed_grad<NX, NY, NZ, 2>, grid, B, gs, st, a);
@@ -734,7 +663,7 @@ int prepare_stage() {
             if (!e) e = set_smem<NX, NY, NZ, true, true>(st);
         }
     }
-    constexpr size_t gs = grad_smem<NX, NY, NZ>();
+    constexpr size_t gs = GradLay<NX, NY, NZ>::BYTES;
     const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
     if (!e && gs > 48 * 1024) {
         e = (int)cudaFuncSetAttribute(k_mixed_grad<NX, NY, NZ, 1>, at, (int)gs);
