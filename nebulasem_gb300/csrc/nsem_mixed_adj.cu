@@ -126,14 +126,14 @@ __device__ __forceinline__ void face_adj(const FaceSlot& fs, int32_t nb, const f
 }
 
 template <int NX, int NY, int NZ, int RS, bool VISC>
-__global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK, (adj_min_blocks<NX, NY, NZ>()))
+__global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK * Geo<NX, NY, NZ>::EPB, (adj_min_blocks<NX, NY, NZ>()))
 k_mixed_adj(AdjArgs a) {
     using G = Geo<NX, NY, NZ>;
     using SM = AdjSmem<NX, NY, NZ>;
     constexpr int NP = G::NP;
     constexpr int NFS = G::NFS;
     extern __shared__ float4 asm4[];
-    float* smem = reinterpret_cast<float*>(asm4);
+    float* smem = reinterpret_cast<float*>(G::template smem_of<SM::BYTES>(asm4));
     float* sGb = smem;                                          /* [5][NP] */
     float* sR = smem + SM::OFF_R;
     float4* sP = reinterpret_cast<float4*>(smem + SM::OFF_P);
@@ -145,7 +145,8 @@ k_mixed_adj(AdjArgs a) {
     float* sMeta = smem + SM::OFF_META;
 
     const int t = threadIdx.x;
-    const int64_t e = blockIdx.x;
+    const int64_t e = G::element();
+    if (G::EPB > 1 && e >= a.n_elem) return;
     constexpr bool has_din = RS == 3 || RS == 2;
 
     /* what no kernel of the chain writes, before the wait for the previous
@@ -218,7 +219,7 @@ k_mixed_adj(AdjArgs a) {
         sP[2 * NP + t] = make_float4(p.u[0], p.u[1], p.u[2], pth);
         sT[t] = x[4];
     }
-    __syncthreads();
+    G::sync();
 
     /* phase 2: face adjoints */
     if (t < NFS) {
@@ -238,7 +239,7 @@ k_mixed_adj(AdjArgs a) {
     line_transform_t<NX, NY, NZ, 0>(sGb, sR, a, t);
     if constexpr (G::HAS_Y) line_transform_t<NX, NY, NZ, 1>(sGb, sR, a, t);
     line_transform_t<NX, NY, NZ, 2>(sGb, sR, a, t);
-    __syncthreads();
+    G::sync();
 
     /* phase 3: transposed line sums, pointwise transposes, face and source terms */
     nsem_chain_begin();
@@ -370,20 +371,21 @@ k_mixed_adj(AdjArgs a) {
 }
 
 template <int NX, int NY, int NZ, int RS>
-__global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK)
+__global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK * Geo<NX, NY, NZ>::EPB)
 k_mixed_adj_grad(AdjArgs a) {
     using G = Geo<NX, NY, NZ>;
     using SM = AdjGradSmem<NX, NY, NZ>;
     constexpr int NP = G::NP;
     constexpr int NFS = G::NFS;
     extern __shared__ float4 agm4[];
-    float* smem = reinterpret_cast<float*>(agm4);
+    float* smem = reinterpret_cast<float*>(G::template smem_of<SM::BYTES>(agm4));
     float* sR = smem;
     float4* sV = reinterpret_cast<float4*>(smem + SM::OFF_V);
     float4* sF = reinterpret_cast<float4*>(smem + SM::OFF_F);
     float* sMeta = smem + SM::OFF_META;
     const int t = threadIdx.x;
-    const int64_t e = blockIdx.x;
+    const int64_t e = G::element();
+    if (G::EPB > 1 && e >= a.n_elem) return;
     constexpr bool has_din = RS == 3 || RS == 2;
 
     float x[5], rref = 0.0f, gbv[12], xbp[5], gb[5];
@@ -436,7 +438,7 @@ k_mixed_adj_grad(AdjArgs a) {
         if constexpr (G::HAS_Y) put(sR + LineLay<NX, NY, NZ, 1>::at(i, j, k), LineLay<NX, NY, NZ, 1>::NL, 1);
         put(sR + LineLay<NX, NY, NZ, 2>::at(i, j, k), LineLay<NX, NY, NZ, 2>::NL, 2);
     }
-    __syncthreads();
+    G::sync();
 
     /* phase 2: per face node the face terms' adjoints for the node */
     if (t < NFS) {
@@ -486,13 +488,13 @@ k_mixed_adj_grad(AdjArgs a) {
         }
         sF[t] = out;
     }
-    __syncthreads();
+    G::sync();
 
     /* phase 3: transposed line sums */
     grad_transform_t<NX, NY, NZ, 0>(sR, a, t);
     if constexpr (G::HAS_Y) grad_transform_t<NX, NY, NZ, 1>(sR, a, t);
     grad_transform_t<NX, NY, NZ, 2>(sR, a, t);
-    __syncthreads();
+    G::sync();
     if (t >= NP) return;
     const int i = t / (NY * NZ), j = (t / NZ) % NY, k = t % NZ;
     float vb[4] = {0, 0, 0, 0};
@@ -560,35 +562,35 @@ k_mixed_adj_grad(AdjArgs a) {
 template <int NX, int NY, int NZ>
 int launch_adj(const AdjArgs& a, int rs, cudaStream_t st, int passes) {
     using G = Geo<NX, NY, NZ>;
-    constexpr int SMEM = (int)AdjSmem<NX, NY, NZ>::BYTES;
-    const unsigned grid = (unsigned)a.n_elem;
+    constexpr int SMEM = G::EPB * (int)AdjSmem<NX, NY, NZ>::BYTES;
+    const unsigned grid = G::grid(a.n_elem);
     if (a.GB) {
         /* viscous: pass 1 the flux transposes, pass 2 the gradients'
          * transpose and the stage combination */
-        constexpr int GS = (int)AdjGradSmem<NX, NY, NZ>::BYTES;
+        constexpr int GS = G::EPB * (int)AdjGradSmem<NX, NY, NZ>::BYTES;
         if (passes & 1) {
             switch (rs) {
-                case 0: k_mixed_adj<NX, NY, NZ, 0, true><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-                case 1: k_mixed_adj<NX, NY, NZ, 1, true><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-                case 2: k_mixed_adj<NX, NY, NZ, 2, true><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-                default: k_mixed_adj<NX, NY, NZ, 3, true><<<grid, G::BLOCK, SMEM, st>>>(a); break;
+                case 0: k_mixed_adj<NX, NY, NZ, 0, true><<<grid, G::block(), SMEM, st>>>(a); break;
+                case 1: k_mixed_adj<NX, NY, NZ, 1, true><<<grid, G::block(), SMEM, st>>>(a); break;
+                case 2: k_mixed_adj<NX, NY, NZ, 2, true><<<grid, G::block(), SMEM, st>>>(a); break;
+                default: k_mixed_adj<NX, NY, NZ, 3, true><<<grid, G::block(), SMEM, st>>>(a); break;
             }
         }
         if (passes & 2) {
             switch (rs) {
-                case 0: k_mixed_adj_grad<NX, NY, NZ, 0><<<grid, G::BLOCK, GS, st>>>(a); break;
-                case 1: k_mixed_adj_grad<NX, NY, NZ, 1><<<grid, G::BLOCK, GS, st>>>(a); break;
-                case 2: k_mixed_adj_grad<NX, NY, NZ, 2><<<grid, G::BLOCK, GS, st>>>(a); break;
-                default: k_mixed_adj_grad<NX, NY, NZ, 3><<<grid, G::BLOCK, GS, st>>>(a); break;
+                case 0: k_mixed_adj_grad<NX, NY, NZ, 0><<<grid, G::block(), GS, st>>>(a); break;
+                case 1: k_mixed_adj_grad<NX, NY, NZ, 1><<<grid, G::block(), GS, st>>>(a); break;
+                case 2: k_mixed_adj_grad<NX, NY, NZ, 2><<<grid, G::block(), GS, st>>>(a); break;
+                default: k_mixed_adj_grad<NX, NY, NZ, 3><<<grid, G::block(), GS, st>>>(a); break;
             }
         }
         return (int)cudaGetLastError();
     }
     switch (rs) {
-        case 0: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 0, false>, grid, (unsigned)G::BLOCK, SMEM, st, a);
-        case 1: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 1, false>, grid, (unsigned)G::BLOCK, SMEM, st, a);
-        case 2: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 2, false>, grid, (unsigned)G::BLOCK, SMEM, st, a);
-        default: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 3, false>, grid, (unsigned)G::BLOCK, SMEM, st, a);
+        case 0: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 0, false>, grid, G::block(), SMEM, st, a);
+        case 1: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 1, false>, grid, G::block(), SMEM, st, a);
+        case 2: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 2, false>, grid, G::block(), SMEM, st, a);
+        default: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 3, false>, grid, G::block(), SMEM, st, a);
     }
     return (int)cudaGetLastError();
 }

@@ -64,7 +64,7 @@ struct AdjSmem {
     static constexpr int OFF_XD4 = (OFF_FA1 + NFS + 3) / 4 * 4;
     static constexpr int OFF_XD1 = OFF_XD4 + 4 * NFS;
     static constexpr int OFF_META = OFF_XD1 + NFS;
-    static constexpr size_t BYTES = sizeof(float) * (OFF_META + 4);
+    static constexpr size_t BYTES = sizeof(float) * ((OFF_META + 4 + 3) / 4 * 4);
 };
 
 template <int NX, int NY, int NZ>
@@ -167,7 +167,7 @@ struct AdjGradSmem {
     static constexpr int OFF_V = (line_floats<NX, NY, NZ>() + 3) / 4 * 4;
     static constexpr int OFF_F = OFF_V + 4 * NP;
     static constexpr int OFF_META = OFF_F + 4 * NFS;
-    static constexpr size_t BYTES = sizeof(float) * (OFF_META + 4);
+    static constexpr size_t BYTES = sizeof(float) * ((OFF_META + 4 + 3) / 4 * 4);
 };
 
 /* the transposed line sums of the gradient rows of axis D (4 quantities) */

@@ -39,18 +39,18 @@ struct AdjGenSmem {
     static constexpr int OFF_FA1 = OFF_FA4 + 4 * NFS;
     static constexpr int OFF_XD4 = (OFF_FA1 + NFS + 3) / 4 * 4;
     static constexpr int OFF_XD1 = OFF_XD4 + 4 * NFS;
-    static constexpr size_t BYTES = sizeof(float) * (OFF_XD1 + NFS);
+    static constexpr size_t BYTES = sizeof(float) * ((OFF_XD1 + NFS + 3) / 4 * 4);
 };
 
 template <int NX, int NY, int NZ, int RS, bool VISC>
-__global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK, (adj_min_blocks<NX, NY, NZ>()))
+__global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK * Geo<NX, NY, NZ>::EPB, (adj_min_blocks<NX, NY, NZ>()))
 k_mixed_adj_gen(AdjArgs a) {
     using G = Geo<NX, NY, NZ>;
     using SM = AdjGenSmem<NX, NY, NZ>;
     constexpr int NP = G::NP;
     constexpr int NFS = G::NFS;
     extern __shared__ float4 agen4[];
-    float* smem = reinterpret_cast<float*>(agen4);
+    float* smem = reinterpret_cast<float*>(G::template smem_of<SM::BYTES>(agen4));
     float* sVb = smem;                                            /* [5][NP] */
     float* sR = smem + SM::OFF_R;
     float4* sP = reinterpret_cast<float4*>(smem + SM::OFF_P);
@@ -61,7 +61,8 @@ k_mixed_adj_gen(AdjArgs a) {
     float* sXd1 = smem + SM::OFF_XD1;
 
     const int t = threadIdx.x;
-    const int64_t e = blockIdx.x;
+    const int64_t e = G::element();
+    if (G::EPB > 1 && e >= a.n_elem) return;
     constexpr bool has_din = RS == 3 || RS == 2;
 
     float x[5], gb[5], bgs[4] = {0, 0, 0, 0}, jin[9], icv = 0.0f;
@@ -134,7 +135,7 @@ k_mixed_adj_gen(AdjArgs a) {
         sP[2 * NP + t] = make_float4(p.u[0], p.u[1], p.u[2], pth);
         sT[t] = x[4];
     }
-    __syncthreads();
+    G::sync();
 
     /* phase 2: face adjoints, per face node */
     if (t < NFS) {
@@ -200,7 +201,7 @@ k_mixed_adj_gen(AdjArgs a) {
     line_transform_t<NX, NY, NZ, 0>(sVb, sR, a, t);
     if constexpr (G::HAS_Y) line_transform_t<NX, NY, NZ, 1>(sVb, sR, a, t);
     line_transform_t<NX, NY, NZ, 2>(sVb, sR, a, t);
-    __syncthreads();
+    G::sync();
 
     /* phase 3: Cartesian flux adjoints, transposes, face terms, update */
     if (t >= NP) return;
@@ -317,19 +318,20 @@ k_mixed_adj_gen(AdjArgs a) {
  * its 1/cV) from the neighbour's side; on a wall the SYMMETRY ghost along the
  * unit normal is transposed. */
 template <int NX, int NY, int NZ, int RS>
-__global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK)
+__global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK * Geo<NX, NY, NZ>::EPB)
 k_mixed_adj_grad_gen(AdjArgs a) {
     using G = Geo<NX, NY, NZ>;
     using SM = AdjGradSmem<NX, NY, NZ>;
     constexpr int NP = G::NP;
     constexpr int NFS = G::NFS;
     extern __shared__ float4 aggm4[];
-    float* smem = reinterpret_cast<float*>(aggm4);
+    float* smem = reinterpret_cast<float*>(G::template smem_of<SM::BYTES>(aggm4));
     float* sR = smem;
     float4* sV = reinterpret_cast<float4*>(smem + SM::OFF_V);
     float4* sF = reinterpret_cast<float4*>(smem + SM::OFF_F);
     const int t = threadIdx.x;
-    const int64_t e = blockIdx.x;
+    const int64_t e = G::element();
+    if (G::EPB > 1 && e >= a.n_elem) return;
     constexpr bool has_din = RS == 3 || RS == 2;
 
     float x[5], rref = 0.0f, gbv[12], xbp[5], gb[5], jin[9], icv = 0.0f;
@@ -407,7 +409,7 @@ k_mixed_adj_grad_gen(AdjArgs a) {
         if constexpr (G::HAS_Y) put(sR + LineLay<NX, NY, NZ, 1>::at(i, j, k), LineLay<NX, NY, NZ, 1>::NL, 1);
         put(sR + LineLay<NX, NY, NZ, 2>::at(i, j, k), LineLay<NX, NY, NZ, 2>::NL, 2);
     }
-    __syncthreads();
+    G::sync();
 
     /* phase 2: the face terms' adjoints for each face node */
     if (t < NFS) {
@@ -446,13 +448,13 @@ k_mixed_adj_grad_gen(AdjArgs a) {
         }
         sF[t] = out;
     }
-    __syncthreads();
+    G::sync();
 
     /* phase 3: transposed line sums, face terms, back to the state, combination */
     grad_transform_t<NX, NY, NZ, 0>(sR, a, t);
     if constexpr (G::HAS_Y) grad_transform_t<NX, NY, NZ, 1>(sR, a, t);
     grad_transform_t<NX, NY, NZ, 2>(sR, a, t);
-    __syncthreads();
+    G::sync();
     if (t >= NP) return;
     const int i = t / (NY * NZ), j = (t / NZ) % NY, k = t % NZ;
     float vb[4] = {0, 0, 0, 0};
@@ -519,35 +521,35 @@ k_mixed_adj_grad_gen(AdjArgs a) {
 template <int NX, int NY, int NZ>
 int launch_adj_gen(const AdjArgs& a, int rs, cudaStream_t st, int passes) {
     using G = Geo<NX, NY, NZ>;
-    constexpr int SMEM = (int)AdjGenSmem<NX, NY, NZ>::BYTES;
-    constexpr int GS = (int)AdjGradSmem<NX, NY, NZ>::BYTES;
-    const unsigned grid = (unsigned)a.n_elem;
+    constexpr int SMEM = G::EPB * (int)AdjGenSmem<NX, NY, NZ>::BYTES;
+    constexpr int GS = G::EPB * (int)AdjGradSmem<NX, NY, NZ>::BYTES;
+    const unsigned grid = G::grid(a.n_elem);
     if (a.GB) {
         /* viscous: pass 1 the flux transposes, pass 2 the gradients'
          * transpose and the stage combination */
         if (passes & 1) {
             switch (rs) {
-                case 0: k_mixed_adj_gen<NX, NY, NZ, 0, true><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-                case 1: k_mixed_adj_gen<NX, NY, NZ, 1, true><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-                case 2: k_mixed_adj_gen<NX, NY, NZ, 2, true><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-                default: k_mixed_adj_gen<NX, NY, NZ, 3, true><<<grid, G::BLOCK, SMEM, st>>>(a); break;
+                case 0: k_mixed_adj_gen<NX, NY, NZ, 0, true><<<grid, G::block(), SMEM, st>>>(a); break;
+                case 1: k_mixed_adj_gen<NX, NY, NZ, 1, true><<<grid, G::block(), SMEM, st>>>(a); break;
+                case 2: k_mixed_adj_gen<NX, NY, NZ, 2, true><<<grid, G::block(), SMEM, st>>>(a); break;
+                default: k_mixed_adj_gen<NX, NY, NZ, 3, true><<<grid, G::block(), SMEM, st>>>(a); break;
             }
         }
         if (passes & 2) {
             switch (rs) {
-                case 0: k_mixed_adj_grad_gen<NX, NY, NZ, 0><<<grid, G::BLOCK, GS, st>>>(a); break;
-                case 1: k_mixed_adj_grad_gen<NX, NY, NZ, 1><<<grid, G::BLOCK, GS, st>>>(a); break;
-                case 2: k_mixed_adj_grad_gen<NX, NY, NZ, 2><<<grid, G::BLOCK, GS, st>>>(a); break;
-                default: k_mixed_adj_grad_gen<NX, NY, NZ, 3><<<grid, G::BLOCK, GS, st>>>(a); break;
+                case 0: k_mixed_adj_grad_gen<NX, NY, NZ, 0><<<grid, G::block(), GS, st>>>(a); break;
+                case 1: k_mixed_adj_grad_gen<NX, NY, NZ, 1><<<grid, G::block(), GS, st>>>(a); break;
+                case 2: k_mixed_adj_grad_gen<NX, NY, NZ, 2><<<grid, G::block(), GS, st>>>(a); break;
+                default: k_mixed_adj_grad_gen<NX, NY, NZ, 3><<<grid, G::block(), GS, st>>>(a); break;
             }
         }
         return (int)cudaGetLastError();
     }
     switch (rs) {
-        case 0: k_mixed_adj_gen<NX, NY, NZ, 0, false><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-        case 1: k_mixed_adj_gen<NX, NY, NZ, 1, false><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-        case 2: k_mixed_adj_gen<NX, NY, NZ, 2, false><<<grid, G::BLOCK, SMEM, st>>>(a); break;
-        default: k_mixed_adj_gen<NX, NY, NZ, 3, false><<<grid, G::BLOCK, SMEM, st>>>(a); break;
+        case 0: k_mixed_adj_gen<NX, NY, NZ, 0, false><<<grid, G::block(), SMEM, st>>>(a); break;
+        case 1: k_mixed_adj_gen<NX, NY, NZ, 1, false><<<grid, G::block(), SMEM, st>>>(a); break;
+        case 2: k_mixed_adj_gen<NX, NY, NZ, 2, false><<<grid, G::block(), SMEM, st>>>(a); break;
+        default: k_mixed_adj_gen<NX, NY, NZ, 3, false><<<grid, G::block(), SMEM, st>>>(a); break;
     }
     return (int)cudaGetLastError();
 }

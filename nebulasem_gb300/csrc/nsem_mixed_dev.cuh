@@ -49,6 +49,30 @@ struct Geo {
     static constexpr int OFF_Z = 2 * NFX + (HAS_Y ? 2 * NFY : 0);
     static constexpr int NFS = OFF_Z + 2 * NFZ;
     static constexpr int BLOCK = ((NP > NFS ? NP : NFS) + 31) / 32 * 32;
+    /* Elements of one warp (2D) share a CTA, four at a time: alone they are
+     * held to 32 warps per SM by the CTA limit, and while a chained kernel's
+     * CTAs wait, to fewer.  30 steps of order 4 in 2D, one, two, four, eight
+     * elements per CTA: 7920 elements 1067, 796, 798, 814 us; 3000: 552, 448,
+     * 441, 455; 1600: 396, 358, 362, 379; 100: 293, 293, 292, 302; order 3,
+     * viscous, 7920 elements: 1895, 1294, 1214, 1262 */
+    static constexpr int EPB = BLOCK == 32 ? 4 : 1;
+    /* the thread's element (to be compared with the number of elements) */
+    __device__ static __forceinline__ int64_t element() {
+        return EPB > 1 ? (int64_t)blockIdx.x * EPB + threadIdx.y : (int64_t)blockIdx.x;
+    }
+    /* the element's part of the CTA's dynamic shared memory */
+    template <size_t BYTES>
+    __device__ static __forceinline__ float4* smem_of(float4* base) {
+        static_assert(EPB == 1 || (BYTES % 16 == 0 && EPB * BYTES <= 48 * 1024), "elements side by side");
+        return EPB > 1 ? base + threadIdx.y * (BYTES / 16) : base;
+    }
+    /* orders the element's threads */
+    __device__ static __forceinline__ void sync() {
+        if constexpr (EPB > 1) __syncwarp();
+        else __syncthreads();
+    }
+    static dim3 block() { return dim3(BLOCK, EPB); }
+    static unsigned grid(int64_t n_elem) { return (unsigned)((n_elem + EPB - 1) / EPB); }
 };
 
 /* resident CTAs per SM asked of the register allocator: the wanted count,

@@ -38,7 +38,7 @@ struct GenSmem {
     static constexpr int OFF_FF4 = (OFF_P + (VISC ? 13 : 12) * NP + 3) / 4 * 4;
     static constexpr int OFF_FF1 = OFF_FF4 + 4 * NFS;
     static constexpr int OFF_GV = OFF_FF1 + NFS;
-    static constexpr size_t BYTES = sizeof(float) * (OFF_GV + (VISC ? 12 * NP : 0));
+    static constexpr size_t BYTES = sizeof(float) * ((OFF_GV + (VISC ? 12 * NP : 0) + 3) / 4 * 4);
 };
 
 /* normal flux F(x).fN of one side */
@@ -65,8 +65,8 @@ __device__ __forceinline__ void normal_flux(const float* m, const float* u, floa
 #endif
 
 template <int NX, int NY, int NZ, int STAGE, bool VISC>
-__global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK,
-                                  (min_blocks(NX == 8 ? 2 : (VISC ? 4 : (STAGE == 1 || STAGE == 2) ? NSEM_GEN_MB12 : NSEM_GEN_MB3), Geo<NX, NY, NZ>::BLOCK,
+__global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK * Geo<NX, NY, NZ>::EPB,
+                                  (min_blocks(NX == 8 ? 2 : Geo<NX, NY, NZ>::EPB > 1 ? 1 : (VISC ? 4 : (STAGE == 1 || STAGE == 2) ? NSEM_GEN_MB12 : NSEM_GEN_MB3), Geo<NX, NY, NZ>::BLOCK,
                                               GenSmem<NX, NY, NZ, VISC>::BYTES)))
 k_mixed_stage_gen(StageArgs a) {
     using G = Geo<NX, NY, NZ>;
@@ -74,13 +74,14 @@ k_mixed_stage_gen(StageArgs a) {
     constexpr int NP = G::NP;
     constexpr int NFS = G::NFS;
     extern __shared__ float4 gen4[];
-    float* smem = reinterpret_cast<float*>(gen4);
+    float* smem = reinterpret_cast<float*>(G::template smem_of<SM::BYTES>(gen4));
     float* sP = smem + SM::OFF_P;       /* [12 or 13][NP] */
     float4* sFF4 = reinterpret_cast<float4*>(smem + SM::OFF_FF4);
     float* sFF1 = smem + SM::OFF_FF1;
     float* sGV = smem + SM::OFF_GV;     /* viscous runs: [12][NP] */
     const int t = threadIdx.x;
-    const int64_t e = blockIdx.x;
+    const int64_t e = G::element();
+    if (G::EPB > 1 && e >= a.n_elem) return;
     constexpr bool has_din = STAGE >= 2;
 
     /* what no kernel of the chain writes, before the wait for the previous
@@ -218,7 +219,7 @@ k_mixed_stage_gen(StageArgs a) {
             f[0] = g4.x; f[nl] = g4.y; f[2 * nl] = g4.z; f[3 * nl] = g4.w; f[4 * nl] = g1;
         }
     }
-    __syncthreads();
+    G::sync();
 
     /* phase 2: Rusanov flux through every face node, dotted with its normal */
     if (t < NFS) {
@@ -297,7 +298,7 @@ k_mixed_stage_gen(StageArgs a) {
         sFF4[t] = o4;
         sFF1[t] = o1;
     }
-    __syncthreads();
+    G::sync();
 
     nsem_chain_begin();   /* here: see k_mixed_stage */
     /* phase 3: line sums l_a'(x_m) G_d(m) (in-place line transform), lift,
@@ -305,7 +306,7 @@ k_mixed_stage_gen(StageArgs a) {
     line_transform<NX, NY, NZ, 0>(smem, a, t);
     if constexpr (G::HAS_Y) line_transform<NX, NY, NZ, 1>(smem, a, t);
     line_transform<NX, NY, NZ, 2>(smem, a, t);
-    __syncthreads();
+    G::sync();
     if (t >= NP) return;
     const int i = t / (NY * NZ), j = (t / NZ) % NY, k = t % NZ;
     float4 acc;
@@ -384,17 +385,19 @@ k_mixed_stage_gen(StageArgs a) {
  *                    + sum_faces fN_out[r] (cds(q) - q) ],
  * the SYMMETRY ghost velocity along the face node's unit normal on walls. */
 template <int NX, int NY, int NZ, int SIN>
-__global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK)
+__global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK * Geo<NX, NY, NZ>::EPB)
 k_mixed_grad_gen(StageArgs a) {
     using G = Geo<NX, NY, NZ>;
     constexpr int NP = G::NP;
     constexpr int NFS = G::NFS;
     constexpr bool has_din = SIN >= 2;
-    extern __shared__ float4 ggsm4[];
     using GL = GradLay<NX, NY, NZ>;
+    extern __shared__ float4 ggsm[];
+    float4* ggsm4 = G::template smem_of<GL::BYTES>(ggsm);
     float4* sD = ggsm4 + GL::OFF_D;                                 /* [NFS] cds - own */
     const int t = threadIdx.x;
-    const int64_t e = blockIdx.x;
+    const int64_t e = G::element();
+    if (G::EPB > 1 && e >= a.n_elem) return;
 
     float own[5], bgs0 = 0.0f, jin[9], icv = 0.0f;
     if (t < NP) {
@@ -443,7 +446,7 @@ k_mixed_grad_gen(StageArgs a) {
                            __fmul_rn(__fmaf_rn(-T0, s[0], s[4]), inv));
     };
     if (t < NP) ggsm4[GL::at(t)] = prim_ut(own, bgs0);
-    __syncthreads();
+    G::sync();
 
     if (t < NFS && nb > -2) {
         const float4 S = ggsm4[GL::at(fs.la)];
@@ -469,12 +472,12 @@ k_mixed_grad_gen(StageArgs a) {
         }
         sD[t] = make_float4(c.x - S.x, c.y - S.y, c.z - S.z, c.w - S.w);
     }
-    __syncthreads();
+    G::sync();
 
     nsem_chain_begin();
     /* derivatives along the reference directions */
     grad_lines<NX, NY, NZ, false>(ggsm4, a, t, nullptr);
-    __syncthreads();
+    G::sync();
     if (t >= NP) return;
     const int i = t / (NY * NZ), j = (t / NZ) % NY, k = t % NZ;
     float4 d[3];
@@ -538,10 +541,10 @@ k_mixed_grad_gen(StageArgs a) {
 
 template <int NX, int NY, int NZ>
 int launch_gen(const StageArgs& a, int stage, cudaStream_t st, bool visc) {
-    constexpr unsigned B = Geo<NX, NY, NZ>::BLOCK;
-    const unsigned grid = (unsigned)a.n_elem;
+    const dim3 B = Geo<NX, NY, NZ>::block();
+    const unsigned grid = Geo<NX, NY, NZ>::grid(a.n_elem);
     if (visc) {
-        constexpr size_t SMEM = GenSmem<NX, NY, NZ, true>::BYTES;
+        constexpr size_t SMEM = Geo<NX, NY, NZ>::EPB * GenSmem<NX, NY, NZ, true>::BYTES;
         switch (stage) {
             case 0: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 0, true>, grid, B, SMEM, st, a);
             case 1: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 1, true>, grid, B, SMEM, st, a);
@@ -549,7 +552,7 @@ int launch_gen(const StageArgs& a, int stage, cudaStream_t st, bool visc) {
             default: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 3, true>, grid, B, SMEM, st, a);
         }
     }
-    constexpr size_t SMEM = GenSmem<NX, NY, NZ>::BYTES;
+    constexpr size_t SMEM = Geo<NX, NY, NZ>::EPB * GenSmem<NX, NY, NZ>::BYTES;
     switch (stage) {
         case 0: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 0, false>, grid, B, SMEM, st, a);
         case 1: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 1, false>, grid, B, SMEM, st, a);
@@ -561,9 +564,9 @@ int launch_gen(const StageArgs& a, int stage, cudaStream_t st, bool visc) {
 template <int NX, int NY, int NZ>
 int launch_grad_gen(const StageArgs& a, int stage, cudaStream_t st) {
     using G = Geo<NX, NY, NZ>;
-    const unsigned grid = (unsigned)a.n_elem;
-    constexpr size_t gs = GradLay<NX, NY, NZ>::BYTES;
-    constexpr unsigned B = G::BLOCK;
+    const unsigned grid = Geo<NX, NY, NZ>::grid(a.n_elem);
+    constexpr size_t gs = G::EPB * GradLay<NX, NY, NZ>::BYTES;
+    const dim3 B = G::block();
     return stage <= 1 ? nsem_launch_chained(k_mixed_grad_gen<NX, NY, NZ, 1>, grid, B, gs, st, a)
                       : nsem_launch_chained(k_mixed_grad_gen<NX, NY, NZ, 2>, grid, B, gs, st, a);
 }

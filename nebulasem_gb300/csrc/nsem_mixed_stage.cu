@@ -29,7 +29,7 @@ struct StageSmem {
     /* tensor-core line sums: the B fragments of Q_d^T pre-split into TF32
      * high and low parts, [3][2][8][8] words after the metric */
     static constexpr int OFF_QTC = OFF_META + 4;
-    static constexpr size_t BYTES = sizeof(float) * (OFF_QTC + (TC ? TC_QTAB : 0));
+    static constexpr size_t BYTES = sizeof(float) * ((OFF_QTC + (TC ? TC_QTAB : 0) + 3) / 4 * 4);
 };
 
 /* Tensor-core line sums (order 7, 8 nodes per direction).  The volume term
@@ -84,6 +84,7 @@ constexpr int stage_min_blocks() {
     if (Geo<NX, NY, NZ>::BLOCK >= 512)
         return min_blocks((VISC || STAGE == 0) ? 2 : 3, Geo<NX, NY, NZ>::BLOCK,
                           StageSmem<NX, NY, NZ>::BYTES);
+    if (Geo<NX, NY, NZ>::EPB > 1) return 1;   /* 2D: 40 registers, for 12 CTAs, spill */
     return min_blocks(VISC ? (STAGE == 3 ? 6 : 7) : (STAGE == 1 || STAGE == 2) ? NSEM_MIXED_MB12 : NSEM_MIXED_MB3,
                       Geo<NX, NY, NZ>::BLOCK, StageSmem<NX, NY, NZ>::BYTES);
 }
@@ -226,7 +227,7 @@ __device__ __forceinline__ void face_flux(const FaceSlot& fs, int32_t nb, const 
 
 /* one kernel per stage (0: tendency only): the stage's own loads and update */
 template <int NX, int NY, int NZ, int STAGE, bool VISC, bool TC>
-__global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK, (stage_min_blocks<NX, NY, NZ, STAGE, VISC>()))
+__global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK * Geo<NX, NY, NZ>::EPB, (stage_min_blocks<NX, NY, NZ, STAGE, VISC>()))
 k_mixed_stage(StageArgs a) {
     static_assert(!TC || (NX == 8 && NY == 8 && NZ == 8), "tensor-core line sums: order 7");
     using G = Geo<NX, NY, NZ>;
@@ -234,14 +235,15 @@ k_mixed_stage(StageArgs a) {
     constexpr int NP = G::NP;
     constexpr int NFS = G::NFS;
     extern __shared__ float4 smem4[];
-    float* smem = reinterpret_cast<float*>(smem4);
+    float* smem = reinterpret_cast<float*>(G::template smem_of<SM::BYTES>(smem4));
     float4* sP = reinterpret_cast<float4*>(smem + SM::OFF_P);     /* [NP] */
     float4* sFF4 = reinterpret_cast<float4*>(smem + SM::OFF_FF4); /* [NFS] */
     float* sFF1 = smem + SM::OFF_FF1;                             /* [NFS] */
     float* sMeta = smem + SM::OFF_META;
 
     const int t = threadIdx.x;
-    const int64_t e = blockIdx.x;
+    const int64_t e = G::element();
+    if (G::EPB > 1 && e >= a.n_elem) return;
     constexpr bool has_din = STAGE >= 2;
     if constexpr (TC) {
         float* sQtc = smem + SM::OFF_QTC;
@@ -367,7 +369,7 @@ k_mixed_stage(StageArgs a) {
             put(smem + LineLay<NX, NY, NZ, 2>::at(i, j, k), LineLay<NX, NY, NZ, 2>::NL, f4, f1);
         }
     }
-    __syncthreads();
+    G::sync();
     /* phase 2: Rusanov flux on every face node */
     if (t < NFS) {
         float4 o4;
@@ -381,7 +383,7 @@ k_mixed_stage(StageArgs a) {
         sFF4[t] = o4;
         sFF1[t] = o1;
     }
-    __syncthreads();
+    G::sync();
 
     /* the next stage's CTAs may start: launched earlier (at the start, or after
      * the wait) they take the slots of a grid below one wave unevenly
@@ -420,12 +422,12 @@ k_mixed_stage(StageArgs a) {
             base[TC_SA + oc0] = c[2];
             base[TC_SA + oc1] = c[3];
         }
-        __syncthreads();
+        G::sync();
     } else {
         line_transform<NX, NY, NZ, 0>(smem, a, t);
         if constexpr (G::HAS_Y) line_transform<NX, NY, NZ, 1>(smem, a, t);
         line_transform<NX, NY, NZ, 2>(smem, a, t);
-        __syncthreads();
+        G::sync();
     }
     if (t < NP) {
     const int i = t / (NY * NZ), j = (t / NZ) % NY, k = t % NZ;
@@ -521,18 +523,21 @@ k_mixed_stage(StageArgs a) {
 }
 
 template <int NX, int NY, int NZ, int SIN>
-__global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK)
+__global__ void __launch_bounds__(Geo<NX, NY, NZ>::BLOCK * Geo<NX, NY, NZ>::EPB)
 k_mixed_grad(StageArgs a) {
     using G = Geo<NX, NY, NZ>;
     constexpr int NP = G::NP;
     constexpr int NFS = G::NFS;
     constexpr bool has_din = SIN >= 2;
     using GL = GradLay<NX, NY, NZ>;
-    extern __shared__ float4 gsm4[];
-    __shared__ float sJ[3];
+    extern __shared__ float4 gsm[];
+    __shared__ float sJ_of[G::EPB][3];
+    float4* gsm4 = G::template smem_of<GL::BYTES>(gsm);
+    float* sJ = sJ_of[G::EPB > 1 ? threadIdx.y : 0];
     float4* sD = gsm4 + GL::OFF_D;                                  /* [NFS] cds - own */
     const int t = threadIdx.x;
-    const int64_t e = blockIdx.x;
+    const int64_t e = G::element();
+    if (G::EPB > 1 && e >= a.n_elem) return;
 
     float own[5], bgs0 = 0.0f;
     if (t < NP) bgs0 = __ldg(a.bg + (int64_t)__ldg(a.layer + e) * 4 * NP + t);
@@ -568,7 +573,7 @@ k_mixed_grad(StageArgs a) {
     }
 
     if (t < NP) gsm4[GL::at(t)] = prim_ut(own, bgs0, a.T0);
-    __syncthreads();
+    G::sync();
 
     if (t < NFS && nb <= -2) {
         /* a face on a 2:1 mortar: the projected values from the mortar kernels */
@@ -578,11 +583,11 @@ k_mixed_grad(StageArgs a) {
         const float4 O = nb >= 0 ? prim_ut(oth, bgo0, a.T0) : make_float4(0, 0, 0, 0);
         sD[t] = cds_minus_own(gsm4[GL::at(fs.la)], nb >= 0 ? &O : nullptr, fs.dir);
     }
-    __syncthreads();
+    G::sync();
 
     nsem_chain_begin();
     grad_lines<NX, NY, NZ, true>(gsm4, a, t, sJ);
-    __syncthreads();
+    G::sync();
     if (t >= NP) return;
     float* out = a.Gout + e * 12 * NP + t;
 #pragma unroll
@@ -597,9 +602,9 @@ k_mixed_grad(StageArgs a) {
 
 template <int NX, int NY, int NZ, bool VISC, bool TC>
 int launch_stage_v(const StageArgs& a, int stage, cudaStream_t st) {
-    constexpr unsigned B = Geo<NX, NY, NZ>::BLOCK;
-    constexpr size_t SMEM = StageSmem<NX, NY, NZ, TC>::BYTES;
-    const unsigned grid = (unsigned)a.n_elem;
+    const dim3 B = Geo<NX, NY, NZ>::block();
+    constexpr size_t SMEM = Geo<NX, NY, NZ>::EPB * StageSmem<NX, NY, NZ, TC>::BYTES;
+    const unsigned grid = Geo<NX, NY, NZ>::grid(a.n_elem);
     switch (stage) {
         case 0: return nsem_launch_chained(k_mixed_stage<NX, NY, NZ, 0, VISC, TC>, grid, B, SMEM, st, a);
         case 1: return nsem_launch_chained(k_mixed_stage<NX, NY, NZ, 1, VISC, TC>, grid, B, SMEM, st, a);
@@ -632,9 +637,9 @@ int launch_stage(const StageArgs& a, int stage, cudaStream_t st, const LaunchCfg
 template <int NX, int NY, int NZ>
 int launch_grad(const StageArgs& a, int stage, cudaStream_t st) {
     using G = Geo<NX, NY, NZ>;
-    const unsigned grid = (unsigned)a.n_elem;
-    constexpr size_t gs = GradLay<NX, NY, NZ>::BYTES;
-    constexpr unsigned B = G::BLOCK;
+    const unsigned grid = Geo<NX, NY, NZ>::grid(a.n_elem);
+    constexpr size_t gs = G::EPB * GradLay<NX, NY, NZ>::BYTES;
+    const dim3 B = G::block();
     return stage <= 1 ? nsem_launch_chained(k_mixed_grad<NX, NY, NZ, 1>, grid, B, gs, st, a)
                       : nsem_launch_chained(k_mixed_grad<NX, NY, NZ, 2>, grid, B, gs, st, a);
 }

@@ -32,14 +32,14 @@ __device__ __forceinline__ void nsem_chain_wait() {
 }
 
 template <typename... P, typename... A>
-inline int nsem_launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+inline int nsem_launch_chained(void (*kernel)(P...), unsigned grid, dim3 block, size_t smem,
                                cudaStream_t st, A... args) {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t c{};
     c.gridDim = dim3(grid);
-    c.blockDim = dim3(block);
+    c.blockDim = block;
     c.dynamicSmemBytes = smem;
     c.stream = st;
     c.attrs = &at;
