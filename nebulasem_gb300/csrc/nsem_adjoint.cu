@@ -1430,7 +1430,7 @@ static int adj_vjp(const NsemDev* m, const double* const* S,
     for (int v = 0; v < 5; v++) { fa.S[v] = S[v]; fa.W[v] = W[v]; }
     for (int v = 0; v < NPA; v++) { fa.adjO[v] = ab->adjO[v]; fa.adjN[v] = ab->adjN[v]; }
     const int64_t fb = (m->n_slot + FACE - 1) / FACE;
-    nsem_launch_chained(k_adj_face, (unsigned)fb, FACE, 0, st, *m, fa);
+    nsem_launch_chained(k_adj_face, (unsigned)fb, FACE, 0, st, m->split, *m, fa);
     for (int c = 0; c < 19; c++) va.qb[c] = nullptr;
     if (m->n_ms > 0) {
         MortarArgs ma{};
@@ -1455,8 +1455,8 @@ static int adj_vjp(const NsemDev* m, const double* const* S,
     const size_t smem = (5 * (size_t)m->np + 3 * NSEM_MAX_NPD * NSEM_MAX_NPD) * sizeof(double);
     if (lin && !ab->visc) va.lin = *lin;
     const unsigned grid = (unsigned)m->n_elem;
-    if (ab->visc) nsem_launch_chained(k_adj_volume<true>, grid, (unsigned)threads, smem, st, *m, va);
-    else nsem_launch_chained(k_adj_volume<false>, grid, (unsigned)threads, smem, st, *m, va);
+    if (ab->visc) nsem_launch_chained(k_adj_volume<true>, grid, (unsigned)threads, smem, st, m->split, *m, va);
+    else nsem_launch_chained(k_adj_volume<false>, grid, (unsigned)threads, smem, st, m->split, *m, va);
     if (ab->visc) {
         /* the gradients' transpose, added to the conserved adjoint */
         GradAdjArgs ga{};

@@ -554,7 +554,7 @@ nsem_status nsem_create(const nsem_mesh_desc* mesh, const nsem_params* params, n
     NSEM_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     s = build_device_mesh(ctx, mesh, params);
     if (s != NSEM_OK) return s;
-    int e = nsem_fp64_check_smem(&ctx->dev);
+    int e = nsem_fp64_prepare(&ctx->dev);
     if (e) return cuda_fail(ctx, (cudaError_t)e, "volume kernel shared memory");
     if (ctx->dev.nu != 0.0) {
         /* viscous runs: gradient buffers shared by the coupled and the

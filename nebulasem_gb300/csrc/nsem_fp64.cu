@@ -532,7 +532,7 @@ extern "C" int nsem_fp64_prim(const NsemDev* m, NsemBuf* b, const double* const*
     for (int c = 0; c < 5; c++) a.S[c] = S[c];
     for (int c = 0; c < NSEM_NPRIM; c++) a.prim[c] = b->prim[c];
     const int64_t blocks = (m->n_int + 255) / 256;
-    return nsem_launch_chained(k_prim, (unsigned)blocks, 256, 0, (cudaStream_t)stream, *m, a);
+    return nsem_launch_chained(k_prim, (unsigned)blocks, 256, 0, (cudaStream_t)stream, m->split, *m, a);
 }
 
 extern "C" int nsem_fp64_face(const NsemDev* m, NsemBuf* b, const double* rho, void* stream) {
@@ -556,7 +556,7 @@ extern "C" int nsem_fp64_face(const NsemDev* m, NsemBuf* b, const double* rho, v
     const unsigned mb = (unsigned)((m->n_ms + 127) / 128);
     if (m->n_ms > 0) k_mortar_coupled<<<19 * mb, 128, 0, st>>>(*m, a);
     int e = launch_err();
-    if (!e) e = nsem_launch_chained(k_face, (unsigned)blocks, FACE, 0, st, *m, a);
+    if (!e) e = nsem_launch_chained(k_face, (unsigned)blocks, FACE, 0, st, m->split, *m, a);
     if (e) return e;
     if (m->n_ms > 0) k_mortar_coupled_gather<<<5 * mb, 128, 0, st>>>(*m, a);
     return launch_err();
@@ -566,13 +566,14 @@ static size_t vol_smem(const NsemDev* m) {
     return ((size_t)m->np * SM_W + 3 * NSEM_MAX_NPD * NSEM_MAX_NPD) * sizeof(double);
 }
 
-extern "C" int nsem_fp64_check_smem(const NsemDev* m) {
+extern "C" int nsem_fp64_prepare(NsemDev* m) {
     const size_t smem = vol_smem(m);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(k_volume, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
+    m->split = nsem_chain_split(NSEM_SPLIT, k_volume, (unsigned)m->n_elem, ((m->np + 31) / 32) * 32, smem);
     return 0;
 }
 
@@ -593,5 +594,5 @@ extern "C" int nsem_fp64_volume(const NsemDev* m, NsemBuf* b, int stage,
     for (int c = 0; c < 5; c++) a.dC[c] = b->dC[c];
     const int threads = ((m->np + 31) / 32) * 32;
     return nsem_launch_chained(k_volume, (unsigned)m->n_elem, (unsigned)threads, vol_smem(m),
-                               (cudaStream_t)stream, *m, a);
+                               (cudaStream_t)stream, m->split, *m, a);
 }

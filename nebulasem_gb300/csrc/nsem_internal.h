@@ -37,6 +37,7 @@ struct NsemDev {
     int32_t npx, npy, npz, np;
     int64_t n_elem, n_int, n_slot;
     int32_t tame_tables; /* every dpsi entry zero or within 2^+-60 */
+    int32_t split;       /* shared-memory split of the coupled form's launches */
     int32_t tame_const;  /* P0, R, gamma R, nu, 1/Pr and T0 zero or within 2^+-60 */
     /* physical constants */
     double P0, R, gamma, gR, cv_heat, cp, T0;
@@ -100,7 +101,7 @@ int nsem_fp64_face(const NsemDev* m, NsemBuf* b, const double* rho, void* stream
 int nsem_fp64_volume(const NsemDev* m, NsemBuf* b, int stage, double dt,
                      const double* const* S, const double* const* U0, double* const* out,
                      void* stream);
-int nsem_fp64_check_smem(const NsemDev* m);
+int nsem_fp64_prepare(NsemDev* m);
 #ifdef __cplusplus
 }
 #endif

@@ -973,6 +973,7 @@ nsem_status nsem_mixed_setup(const NsemDev& dev, const nsem_mesh_desc* m, NsemMi
         const char* lines = std::getenv("NSEM_MIXED_LINES");
         mb->tc = NX == 8 && NY == 8 && NZ == 8 && lines && std::string(lines) == "tensor";
     }
+    mb->split = gen ? split_general(NX, NY, NZ, ne, mb->visc) : split_aligned(NX, NY, NZ, ne, mb->visc);
     mb->n_elem = ne;
     mb->n_int = n_int;
     mb->npd[0] = NX; mb->npd[1] = NY; mb->npd[2] = NZ;
@@ -991,6 +992,7 @@ StageArgs base_args(const NsemDev* dev, const NsemMixedBuf* mb, double dt) {
     a.J = mb->J;
     a.layer = mb->layer;
     a.Qg = mb->Qg;
+    a.split = mb->split;
     a.G = mb->G;
     a.Gout = mb->G;
     a.nu = mb->nu;

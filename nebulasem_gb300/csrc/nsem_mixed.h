@@ -33,6 +33,7 @@ struct NsemMixedBuf {
     float* bg = nullptr;          /* [layers][4][NP] rho_ref, Theta_ref, 1/Theta_ref, p_ref */
     float* Qg = nullptr;          /* line-sum weights Q_d[a][m], row stride MAXN+1 */
     float* G = nullptr;           /* viscous runs: [n_elem][12][NP] gradients of the stage state */
+    int split = 0;                /* shared-memory split of the chain's launches */
     bool visc = false;            /* artificial viscosity (diffusion YES)   */
     bool tc = false;              /* order-7 line sums on the tensor cores  */
     bool gen = false;             /* general geometry (inclined, curved)    */

@@ -587,10 +587,10 @@ int launch_adj(const AdjArgs& a, int rs, cudaStream_t st, int passes) {
         return (int)cudaGetLastError();
     }
     switch (rs) {
-        case 0: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 0, false>, grid, G::block(), SMEM, st, a);
-        case 1: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 1, false>, grid, G::block(), SMEM, st, a);
-        case 2: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 2, false>, grid, G::block(), SMEM, st, a);
-        default: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 3, false>, grid, G::block(), SMEM, st, a);
+        case 0: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 0, false>, grid, G::block(), SMEM, st, a.split, a);
+        case 1: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 1, false>, grid, G::block(), SMEM, st, a.split, a);
+        case 2: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 2, false>, grid, G::block(), SMEM, st, a.split, a);
+        default: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 3, false>, grid, G::block(), SMEM, st, a.split, a);
     }
     return (int)cudaGetLastError();
 }
@@ -1245,6 +1245,7 @@ AdjArgs adj_args(const NsemDev* dev, const NsemMixedBuf* mb, double dt) {
     a.Qg = mb->Qg;
     a.bg = mb->bg;
     a.n_elem = mb->n_elem;
+    a.split = mb->split;
     if (mb->visc) {
         a.Gv = mb->G;
         a.GB = mb->GB;

@@ -29,6 +29,7 @@ struct AdjArgs {
     const float* Qg;
     const float* bg;
     int64_t n_elem;
+    int split;                 /* shared-memory split of the launches */
     float dt, gamma, gR, g[3];
     float lift[3];
     float eos[6];

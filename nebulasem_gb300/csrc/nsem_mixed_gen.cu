@@ -546,18 +546,18 @@ int launch_gen(const StageArgs& a, int stage, cudaStream_t st, bool visc) {
     if (visc) {
         constexpr size_t SMEM = Geo<NX, NY, NZ>::EPB * GenSmem<NX, NY, NZ, true>::BYTES;
         switch (stage) {
-            case 0: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 0, true>, grid, B, SMEM, st, a);
-            case 1: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 1, true>, grid, B, SMEM, st, a);
-            case 2: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 2, true>, grid, B, SMEM, st, a);
-            default: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 3, true>, grid, B, SMEM, st, a);
+            case 0: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 0, true>, grid, B, SMEM, st, a.split, a);
+            case 1: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 1, true>, grid, B, SMEM, st, a.split, a);
+            case 2: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 2, true>, grid, B, SMEM, st, a.split, a);
+            default: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 3, true>, grid, B, SMEM, st, a.split, a);
         }
     }
     constexpr size_t SMEM = Geo<NX, NY, NZ>::EPB * GenSmem<NX, NY, NZ>::BYTES;
     switch (stage) {
-        case 0: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 0, false>, grid, B, SMEM, st, a);
-        case 1: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 1, false>, grid, B, SMEM, st, a);
-        case 2: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 2, false>, grid, B, SMEM, st, a);
-        default: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 3, false>, grid, B, SMEM, st, a);
+        case 0: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 0, false>, grid, B, SMEM, st, a.split, a);
+        case 1: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 1, false>, grid, B, SMEM, st, a.split, a);
+        case 2: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 2, false>, grid, B, SMEM, st, a.split, a);
+        default: return nsem_launch_chained(k_mixed_stage_gen<NX, NY, NZ, 3, false>, grid, B, SMEM, st, a.split, a);
     }
 }
 
@@ -567,8 +567,8 @@ int launch_grad_gen(const StageArgs& a, int stage, cudaStream_t st) {
     const unsigned grid = Geo<NX, NY, NZ>::grid(a.n_elem);
     constexpr size_t gs = G::EPB * GradLay<NX, NY, NZ>::BYTES;
     const dim3 B = G::block();
-    return stage <= 1 ? nsem_launch_chained(k_mixed_grad_gen<NX, NY, NZ, 1>, grid, B, gs, st, a)
-                      : nsem_launch_chained(k_mixed_grad_gen<NX, NY, NZ, 2>, grid, B, gs, st, a);
+    return stage <= 1 ? nsem_launch_chained(k_mixed_grad_gen<NX, NY, NZ, 1>, grid, B, gs, st, a.split, a)
+                      : nsem_launch_chained(k_mixed_grad_gen<NX, NY, NZ, 2>, grid, B, gs, st, a.split, a);
 }
 
 template <int NX, int NY, int NZ>
@@ -597,9 +597,28 @@ int prepare_gen() {
     return e;
 }
 
+template <int NX, int NY, int NZ>
+int chain_split(int64_t n_elem) {
+    using G = Geo<NX, NY, NZ>;
+    return nsem_chain_split(MIXED_SPLIT, k_mixed_stage_gen<NX, NY, NZ, 1, false>, G::grid(n_elem), G::block(),
+                            G::EPB * GenSmem<NX, NY, NZ>::BYTES);
+}
+
 }  // namespace
 
 namespace nsem_mx {
+
+/* viscous runs keep the driver's choice: gradient and stage CTAs side by side
+ * are spread less evenly than one after the other (30 steps of 24 x 24
+ * elements in 2D, order 3: 615 us and 742 with one split; 9 x 7 x 11, 20
+ * steps: 620 and 680) */
+int split_general(int nx, int ny, int nz, int64_t n_elem, bool visc) {
+    if (visc) return 0;
+#define NSEM_SPLIT_OF(A, B, C) if (nx == A && ny == B && nz == C) return chain_split<A, B, C>(n_elem);
+    NSEM_MIXED_DIMS(NSEM_SPLIT_OF)
+#undef NSEM_SPLIT_OF
+    return 0;
+}
 
 int prepare_general(int nx, int ny, int nz) {
 #define NSEM_PREPG(A, B, C) if (nx == A && ny == B && nz == C) return prepare_gen<A, B, C>();

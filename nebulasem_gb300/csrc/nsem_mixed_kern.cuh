@@ -42,6 +42,7 @@ struct StageArgs {
     float lift[3];             /* 1 / w_end per direction                  */
     float eos[6];              /* binomial coefficients C(gamma, k), k = 1..6 */
     uint32_t* status;
+    int split;                 /* shared-memory split of the launches */
     /* line-sum weights Q_d[a][m] (gradient kernels: the derivative tables
      * D_d[a][m]) as kernel parameters: read with compile-time indices they
      * are constant-bank operands of the FMAs */
@@ -191,6 +192,14 @@ struct LaunchCfg {
  * node counts per direction */
 int prepare_aligned(int nx, int ny, int nz);
 int prepare_general(int nx, int ny, int nz);
+/* the shared-memory split of the stage (and gradient) launches (NSEM_SPLIT
+ * explains it): what the stage kernels' resident CTAs fill.  20 steps of 693
+ * elements: order 4 384 to 370 us, tilted 409 to 394, order 3 viscous 460 to
+ * 425; 30 of 1600 in 2D, tilted 425 to 376; at 72 viscous runs of order 4 lose
+ * 2 % */
+constexpr int MIXED_SPLIT = 58;
+int split_aligned(int nx, int ny, int nz, int64_t n_elem, bool visc);
+int split_general(int nx, int ny, int nz, int64_t n_elem, bool visc);
 int launch_stage_aligned(int nx, int ny, int nz, const StageArgs& a, int stage, cudaStream_t st,
                          const LaunchCfg& c);
 int launch_stage_general(int nx, int ny, int nz, const StageArgs& a, int stage, cudaStream_t st,

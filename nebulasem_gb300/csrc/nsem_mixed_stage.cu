@@ -606,10 +606,10 @@ int launch_stage_v(const StageArgs& a, int stage, cudaStream_t st) {
     constexpr size_t SMEM = Geo<NX, NY, NZ>::EPB * StageSmem<NX, NY, NZ, TC>::BYTES;
     const unsigned grid = Geo<NX, NY, NZ>::grid(a.n_elem);
     switch (stage) {
-        case 0: return nsem_launch_chained(k_mixed_stage<NX, NY, NZ, 0, VISC, TC>, grid, B, SMEM, st, a);
-        case 1: return nsem_launch_chained(k_mixed_stage<NX, NY, NZ, 1, VISC, TC>, grid, B, SMEM, st, a);
-        case 2: return nsem_launch_chained(k_mixed_stage<NX, NY, NZ, 2, VISC, TC>, grid, B, SMEM, st, a);
-        default: return nsem_launch_chained(k_mixed_stage<NX, NY, NZ, 3, VISC, TC>, grid, B, SMEM, st, a);
+        case 0: return nsem_launch_chained(k_mixed_stage<NX, NY, NZ, 0, VISC, TC>, grid, B, SMEM, st, a.split, a);
+        case 1: return nsem_launch_chained(k_mixed_stage<NX, NY, NZ, 1, VISC, TC>, grid, B, SMEM, st, a.split, a);
+        case 2: return nsem_launch_chained(k_mixed_stage<NX, NY, NZ, 2, VISC, TC>, grid, B, SMEM, st, a.split, a);
+        default: return nsem_launch_chained(k_mixed_stage<NX, NY, NZ, 3, VISC, TC>, grid, B, SMEM, st, a.split, a);
     }
 }
 
@@ -640,8 +640,8 @@ int launch_grad(const StageArgs& a, int stage, cudaStream_t st) {
     const unsigned grid = Geo<NX, NY, NZ>::grid(a.n_elem);
     constexpr size_t gs = G::EPB * GradLay<NX, NY, NZ>::BYTES;
     const dim3 B = G::block();
-    return stage <= 1 ? nsem_launch_chained(k_mixed_grad<NX, NY, NZ, 1>, grid, B, gs, st, a)
-                      : nsem_launch_chained(k_mixed_grad<NX, NY, NZ, 2>, grid, B, gs, st, a);
+    return stage <= 1 ? nsem_launch_chained(k_mixed_grad<NX, NY, NZ, 1>, grid, B, gs, st, a.split, a)
+                      : nsem_launch_chained(k_mixed_grad<NX, NY, NZ, 2>, grid, B, gs, st, a.split, a);
 }
 
 template <int NX, int NY, int NZ, bool VISC, bool TC>
@@ -677,9 +677,26 @@ int prepare_stage() {
     return e;
 }
 
+template <int NX, int NY, int NZ, bool VISC>
+int chain_split(int64_t n_elem) {
+    using G = Geo<NX, NY, NZ>;
+    if (NX == 4 && !VISC) return 0;   /* order 3, the driver's choice: 267 us, 275 with one split */
+    return nsem_chain_split(MIXED_SPLIT, k_mixed_stage<NX, NY, NZ, 1, VISC, false>, G::grid(n_elem), G::block(),
+                            G::EPB * StageSmem<NX, NY, NZ>::BYTES);
+}
+
 }  // namespace
 
 namespace nsem_mx {
+
+int split_aligned(int nx, int ny, int nz, int64_t n_elem, bool visc) {
+#define NSEM_SPLIT_OF(A, B, C)           \
+    if (nx == A && ny == B && nz == C)   \
+        return visc ? chain_split<A, B, C, true>(n_elem) : chain_split<A, B, C, false>(n_elem);
+    NSEM_MIXED_DIMS(NSEM_SPLIT_OF)
+#undef NSEM_SPLIT_OF
+    return 0;
+}
 
 int prepare_aligned(int nx, int ny, int nz) {
 #define NSEM_PREP(A, B, C) if (nx == A && ny == B && nz == C) return prepare_stage<A, B, C>();

@@ -31,19 +31,47 @@ __device__ __forceinline__ void nsem_chain_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+/* The split of an SM's storage into L1 and shared memory is the driver's
+ * choice per kernel, and an SM changes it only when it is empty: between
+ * kernels of different splits the next one's CTAs wait for the last of this
+ * one.  A chain's launches therefore name one split, the shared memory in
+ * percent of the most there can be (0: the driver's choice).  FP64 form and
+ * its adjoint, 150 elements of order 4: 1030 to 665 us for 5 steps, 1888 to
+ * 1513; 576 of order 3: 885 to 702; convection of 336 elements of order 3, 15
+ * steps: 355 to 248.  44, 58, 82 and 100 are each 3 to 6 % slower than 72
+ * at some size. */
+constexpr int NSEM_SPLIT = 72;
+
+/* Grids of more than one wave keep the driver's choice: their own kernels
+ * fill the SMs, and the best split of each counts for more (2184 elements of
+ * order 3: 1323 us and 1358 with one split, of order 4 2151 and 2195). */
+template <typename... P>
+inline int nsem_chain_split(int split, void (*kernel)(P...), unsigned grid, dim3 block, size_t smem) {
+    int n = 0, dev = 0, sms = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, (int)(block.x * block.y), smem) != cudaSuccess ||
+        cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    return grid <= (unsigned)n * (unsigned)sms ? split : 0;
+}
+
 template <typename... P, typename... A>
 inline int nsem_launch_chained(void (*kernel)(P...), unsigned grid, dim3 block, size_t smem,
-                               cudaStream_t st, A... args) {
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
+                               cudaStream_t st, int split, A... args) {
+    cudaLaunchAttribute at[2] = {};
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at[1].val.sharedMemCarveout = (unsigned)split;
     cudaLaunchConfig_t c{};
     c.gridDim = dim3(grid);
     c.blockDim = block;
     c.dynamicSmemBytes = smem;
     c.stream = st;
-    c.attrs = &at;
-    c.numAttrs = 1;
+    c.attrs = at;
+    c.numAttrs = split > 0 ? 2 : 1;
     return (int)cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
 

@@ -234,6 +234,12 @@ __global__ void __launch_bounds__(256) k_seg_prep(const NsemDev m, SegArgs a) {
 /* Face kernels: FACE threads a CTA, so that a small mesh's slots spread over
  * the SMs (32 x 24 elements of order 4 in 2D have 8 k slots, 32 CTAs of 256) */
 constexpr int FACE = 64;
+/* shared-memory split of the segregated step's launches (NSEM_SPLIT explains
+ * it): less than the other chains', whose face kernels gather less through
+ * L1.  8 steps of 336 elements of order 4: 582 us, 590 at 72, 695 with the
+ * driver's choice per kernel; viscous, 2D, 1600 of order 3: 663, 690, 835;
+ * 2184 of order 4: 1428, 1420, 1420 */
+constexpr int SEG_SPLIT = 58;
 
 /* all values mild (nsem_mild) */
 template <typename... X>
@@ -1117,13 +1123,13 @@ int nsem_grad_ut_mortar(const NsemDev* m, const double* const* U,
     for (int c = 0; c < 4; c++) ga.gC[c] = gC ? gC[c] : nullptr;
     cudaStream_t st = (cudaStream_t)stream;
     const int threads = ((m->np + 31) / 32) * 32;
-    nsem_launch_chained(k_seg_grad_face, (unsigned)((m->n_slot + FACE - 1) / FACE), FACE, 0, st, *m, ga);
+    nsem_launch_chained(k_seg_grad_face, (unsigned)((m->n_slot + FACE - 1) / FACE), FACE, 0, st, m->split, *m, ga);
     if (m->n_ms > 0 && gC) {
         const unsigned mb = (unsigned)((m->n_ms + 127) / 128);
         k_seg_mortar_gcds<<<mb, 128, 0, st>>>(*m, ga);
         k_seg_mortar_ggather<<<mb, 128, 0, st>>>(*m, ga);
     }
-    nsem_launch_chained(k_seg_grad_vol, (unsigned)m->n_elem, threads, smem_grad(m), st, *m, ga);
+    nsem_launch_chained(k_seg_grad_vol, (unsigned)m->n_elem, threads, smem_grad(m), st, m->split, *m, ga);
     return (int)cudaGetLastError();
 }
 
@@ -1155,7 +1161,7 @@ int nsem_grad_vol(const NsemDev* m, const double* const* U, const double* T,
     for (int c = 0; c < 4; c++) ga.fF[c] = const_cast<double*>(fF[c]);
     for (int c = 0; c < 4; c++) ga.gC[c] = gC ? const_cast<double*>(gC[c]) : nullptr;
     const int threads = ((m->np + 31) / 32) * 32;
-    nsem_launch_chained(k_seg_grad_vol, (unsigned)m->n_elem, threads, smem_grad(m), (cudaStream_t)stream, *m, ga);
+    nsem_launch_chained(k_seg_grad_vol, (unsigned)m->n_elem, threads, smem_grad(m), (cudaStream_t)stream, m->split, *m, ga);
     return (int)cudaGetLastError();
 }
 
@@ -1177,9 +1183,9 @@ int nsem_conv_steps(const NsemDev* m, NsemConvBuf* b, int nsteps, double dt,
         const AdvArgs a = adv_args(b, cur, dt);
         const unsigned mb = (unsigned)((m->n_ms + 127) / 128);
         if (m->n_ms > 0) k_conv_mortar<1><<<4 * mb, 128, 0, st>>>(*m, a);
-        nsem_launch_chained(k_conv_face, sb, FACE, 0, st, *m, a);
+        nsem_launch_chained(k_conv_face, sb, FACE, 0, st, NSEM_SPLIT, *m, a);
         if (m->n_ms > 0) k_conv_mortar_gather<<<mb, 128, 0, st>>>(*m, a);
-        nsem_launch_chained(k_conv_vol, (unsigned)m->n_elem, threads, smem_conv(m), st, *m, a);
+        nsem_launch_chained(k_conv_vol, (unsigned)m->n_elem, threads, smem_conv(m), st, NSEM_SPLIT, *m, a);
         const int e = (int)cudaGetLastError();
         if (e) return e;
         cur ^= 1;
@@ -1209,9 +1215,9 @@ int nsem_conv_steps_wind(const NsemDev* m, NsemConvBuf* b, int nsteps,
         }
         const unsigned mb = (unsigned)((m->n_ms + 127) / 128);
         if (m->n_ms > 0) k_conv_mortar<1><<<4 * mb, 128, 0, st>>>(*m, a);
-        nsem_launch_chained(k_conv_face, sb, FACE, 0, st, *m, a);
+        nsem_launch_chained(k_conv_face, sb, FACE, 0, st, NSEM_SPLIT, *m, a);
         if (m->n_ms > 0) k_conv_mortar_gather<<<mb, 128, 0, st>>>(*m, a);
-        nsem_launch_chained(k_conv_vol, (unsigned)m->n_elem, threads, smem_conv(m), st, *m, a);
+        nsem_launch_chained(k_conv_vol, (unsigned)m->n_elem, threads, smem_conv(m), st, NSEM_SPLIT, *m, a);
         const int e = (int)cudaGetLastError();
         if (e) return e;
         b->cur ^= 1;
@@ -1253,7 +1259,7 @@ int nsem_seg_steps(const NsemDev* m, NsemSegBuf* b, int nsteps, double dt,
     int cur = b->cur;
     for (int s = 0; s < nsteps; s++) {
         const SegArgs a = seg_args(m, b, cur, dt);
-        nsem_launch_chained(k_seg_prep, nb, 256, 0, st, *m, a);
+        nsem_launch_chained(k_seg_prep, nb, 256, 0, st, SEG_SPLIT, *m, a);
         if (a.visc) {
             GradArgs ga;
             for (int c = 0; c < 3; c++) ga.U[c] = a.U[c];
@@ -1261,21 +1267,21 @@ int nsem_seg_steps(const NsemDev* m, NsemSegBuf* b, int nsteps, double dt,
             for (int c = 0; c < 12; c++) ga.G[c] = a.G[c];
             for (int c = 0; c < 4; c++) ga.fF[c] = a.fF[c];
             for (int c = 0; c < 4; c++) ga.gC[c] = a.gC[c];
-            nsem_launch_chained(k_seg_grad_face, sb, FACE, 0, st, *m, ga);
+            nsem_launch_chained(k_seg_grad_face, sb, FACE, 0, st, SEG_SPLIT, *m, ga);
             if (mort) {
                 k_seg_mortar_gcds<<<mb, 128, 0, st>>>(*m, ga);
                 k_seg_mortar_ggather<<<mb, 128, 0, st>>>(*m, ga);
             }
-            nsem_launch_chained(k_seg_grad_vol, (unsigned)m->n_elem, threads, smem_grad(m), st, *m, ga);
+            nsem_launch_chained(k_seg_grad_vol, (unsigned)m->n_elem, threads, smem_grad(m), st, SEG_SPLIT, *m, ga);
         }
         if (mort) k_seg_mortar_rho<<<6 * mb, 128, 0, st>>>(*m, a);
-        nsem_launch_chained(k_seg_face_rho, sb, FACE, 0, st, *m, a);
+        nsem_launch_chained(k_seg_face_rho, sb, FACE, 0, st, SEG_SPLIT, *m, a);
         if (mort) k_seg_mortar_gather<0><<<mb, 128, 0, st>>>(*m, a);
-        nsem_launch_chained(k_seg_vol_rho, (unsigned)m->n_elem, threads, smem_rho(m), st, *m, a);
+        nsem_launch_chained(k_seg_vol_rho, (unsigned)m->n_elem, threads, smem_rho(m), st, SEG_SPLIT, *m, a);
         if (mort) k_seg_mortar_ut<<<16 * mb, 128, 0, st>>>(*m, a);
-        nsem_launch_chained(k_seg_face_ut, sb, FACE, 0, st, *m, a);
+        nsem_launch_chained(k_seg_face_ut, sb, FACE, 0, st, SEG_SPLIT, *m, a);
         if (mort) k_seg_mortar_gather<1><<<4 * mb, 128, 0, st>>>(*m, a);
-        nsem_launch_chained(k_seg_vol_ut, (unsigned)m->n_elem, threads, smem_ut(m), st, *m, a);
+        nsem_launch_chained(k_seg_vol_ut, (unsigned)m->n_elem, threads, smem_ut(m), st, SEG_SPLIT, *m, a);
         const int e = (int)cudaGetLastError();
         if (e) return e;
         cur ^= 1;
