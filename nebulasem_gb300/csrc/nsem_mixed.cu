@@ -904,6 +904,28 @@ nsem_status nsem_mixed_setup(const NsemDev& dev, const nsem_mesh_desc* m, NsemMi
         }
     }
 
+    /* the packed background rows (packed_bg) */
+    const bool pack = !gen && packed_bg(NX);
+    std::vector<float4> bgp;
+    if (pack) {
+        const int n[3] = {NX, NY, NZ}, st[3] = {NY * NZ, NZ, 1};
+        std::vector<int> lo;   /* per face slot: the node across, in its element */
+        for (int d = 0; d < 3; d++) {
+            if (d == 1 && NY == 1) continue;
+            const int p = d == 0 ? 1 : 0, q = d == 2 ? 1 : 2;
+            for (int side = 0; side < 2; side++)
+                for (int i = 0; i < n[p]; i++)
+                    for (int j = 0; j < n[q]; j++)
+                        lo.push_back((side ? 0 : n[d] - 1) * st[d] + i * st[p] + j * st[q]);
+        }
+        for (size_t l = 0; l < seen.size(); l++) {
+            const float* b = bg.data() + l * 4 * NP;
+            auto put = [&](int64_t a) { bgp.push_back({b[a], b[NP + a], b[2 * NP + a], b[3 * NP + a]}); };
+            for (int64_t a = 0; a < NP; a++) put(a);
+            for (int a : lo) put(a);
+        }
+    }
+
     auto up = [&](auto** ptr, const auto& vec) -> bool {
         using T = typename std::remove_reference<decltype(vec[0])>::type;
         size_t bytes = vec.size() * sizeof(T);
@@ -911,7 +933,7 @@ nsem_status nsem_mixed_setup(const NsemDev& dev, const nsem_mesh_desc* m, NsemMi
         allocs->push_back((void*)*ptr);
         return cudaMemcpy(*ptr, vec.data(), bytes, cudaMemcpyHostToDevice) == cudaSuccess;
     };
-    if (!up(&mb->nbr, nbr) || !up(&mb->J, J) || !up(&mb->layer, layer) || !up(&mb->bg, bg) ||
+    if (!up(&mb->nbr, nbr) || !up(&mb->J, J) || !up(&mb->layer, layer) || !up(&mb->bg, bg) || (pack && !up(&mb->bgp, bgp)) ||
         !up(&mb->Qg, qtab) || (gen && (!up(&mb->Jg, Jg) || !up(&mb->Fn, Fn)))) {
         err = "precision form: device allocation failed";
         return NSEM_NO_MEMORY;
@@ -999,6 +1021,7 @@ StageArgs base_args(const NsemDev* dev, const NsemMixedBuf* mb, double dt) {
     a.nu_pr = mb->nu_pr;
     a.T0 = (float)dev->T0;
     a.bg = mb->bg;
+    a.bgp = mb->bgp;
     a.Jg = mb->Jg;
     a.Fn = mb->Fn;
     a.MF = mb->MF;

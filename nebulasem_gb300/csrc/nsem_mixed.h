@@ -31,6 +31,8 @@ struct NsemMixedBuf {
     float qc[3][8][8] = {};       /* host copy of the line-sum weights      */
     float dc[3][8][8] = {};       /* derivative tables D_d[a][m] = l_m'(x_a) */
     float* bg = nullptr;          /* [layers][4][NP] rho_ref, Theta_ref, 1/Theta_ref, p_ref */
+    float4* bgp = nullptr;        /* axis-aligned, order 7: [layers][NP + NFS], packed: of the nodes,
+                                     of the node across each face slot */
     float* Qg = nullptr;          /* line-sum weights Q_d[a][m], row stride MAXN+1 */
     float* G = nullptr;           /* viscous runs: [n_elem][12][NP] gradients of the stage state */
     int split = 0;                /* shared-memory split of the chain's launches */

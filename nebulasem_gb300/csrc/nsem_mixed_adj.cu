@@ -152,11 +152,7 @@ k_mixed_adj(AdjArgs a) {
     /* what no kernel of the chain writes, before the wait for the previous
      * kernel: background, neighbours, metric */
     float x[5], gb[5], bgs[4] = {0, 0, 0, 0};
-    if (t < NP) {
-        const float* bg = a.bg + (int64_t)__ldg(a.layer + e) * 4 * NP + t;
-#pragma unroll
-        for (int c = 0; c < 4; c++) bgs[c] = __ldg(bg + c * NP);
-    }
+    if (t < NP) load_bg<NX, NY, NZ>(a, __ldg(a.layer + e), -1, t, bgs);
     FaceSlot fs{};
     int32_t nb = -1;
     float xo[5], bgo[4], go[5], cn = 0.0f;
@@ -164,9 +160,7 @@ k_mixed_adj(AdjArgs a) {
         fs = face_slot<NX, NY, NZ>(t);
         nb = __ldg(a.nbr + (int64_t)fs.face * a.n_elem + e);
         if (nb >= 0) {
-            const float* bg = a.bg + (int64_t)__ldg(a.layer + nb) * 4 * NP + fs.lo;
-#pragma unroll
-            for (int c = 0; c < 4; c++) bgo[c] = __ldg(bg + c * NP);
+            load_bg<NX, NY, NZ>(a, __ldg(a.layer + nb), t, fs.lo, bgo);
             cn = __ldg(a.J + (int64_t)fs.dir * a.n_elem + nb) * a.lift[fs.dir];
         }
     }
@@ -1244,6 +1238,7 @@ AdjArgs adj_args(const NsemDev* dev, const NsemMixedBuf* mb, double dt) {
     a.layer = mb->layer;
     a.Qg = mb->Qg;
     a.bg = mb->bg;
+    a.bgp = mb->bgp;
     a.n_elem = mb->n_elem;
     a.split = mb->split;
     if (mb->visc) {

@@ -28,6 +28,7 @@ struct AdjArgs {
     const int32_t* layer;
     const float* Qg;
     const float* bg;
+    const float4* bgp;
     int64_t n_elem;
     int split;                 /* shared-memory split of the launches */
     float dt, gamma, gR, g[3];

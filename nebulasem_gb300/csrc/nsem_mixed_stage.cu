@@ -254,11 +254,7 @@ k_mixed_stage(StageArgs a) {
      * kernel: background, neighbours, metric */
     float own[5], din[5] = {0, 0, 0, 0, 0}, bgs[4] = {0, 0, 0, 0};
     float gown[12];
-    if (t < NP) {
-        const float* bg = a.bg + (int64_t)__ldg(a.layer + e) * 4 * NP + t;
-#pragma unroll
-        for (int c = 0; c < 4; c++) bgs[c] = __ldg(bg + c * NP);
-    }
+    if (t < NP) load_bg<NX, NY, NZ>(a, __ldg(a.layer + e), -1, t, bgs);
     FaceSlot fs{};
     int32_t nb = -1;
     /* the other side's node; a wall's flux is formed from the own trace */
@@ -271,9 +267,7 @@ k_mixed_stage(StageArgs a) {
         nb = __ldg(a.nbr + (int64_t)fs.face * a.n_elem + e);
         lo = fs.la;
         if (nb >= 0) { eo = nb; lo = fs.lo; }
-        const float* bg = a.bg + (int64_t)__ldg(a.layer + eo) * 4 * NP + lo;
-#pragma unroll
-        for (int c = 0; c < 4; c++) bgo[c] = __ldg(bg + c * NP);
+        load_bg<NX, NY, NZ>(a, __ldg(a.layer + eo), nb >= 0 ? t : -1, lo, bgo);
     }
     if (t < 3) sMeta[t] = __ldg(a.J + (int64_t)t * a.n_elem + e);
     nsem_chain_wait();
