@@ -10,6 +10,7 @@
  */
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -23,6 +24,13 @@
 #include "nsem_adjoint.h"
 #include "nsem_mixed.h"
 #include "nsem_seg.h"
+
+/* results staged together (copy_out): the device writes a pinned buffer and
+ * pageable memory equally fast here, and each copy into the latter costs 5 us
+ * of its own, but the host's second copy costs 30 us per MB of fresh pages.
+ * Precision-form tendency (five arrays), one by one and staged: 2500
+ * nodes 84 and 53 us, 8000 nodes 86 and 69, 27000 nodes (1 MB) 92 and 122 */
+constexpr size_t OUT_BYTES = 384 << 10;
 
 struct nsem_ctx {
     int device = 0;
@@ -50,6 +58,8 @@ struct nsem_ctx {
     double* red = nullptr;           /* reduction partials */
     double* h_red = nullptr;         /* pinned host copy of the reduction result */
     uint32_t* h_status = nullptr;    /* pinned host copy of the status word */
+    char* h_out = nullptr;           /* pinned buffer of results for pageable arrays */
+    size_t h_out_bytes = 0;
     std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  /* key: (form*2 + cur, nsteps) */
     std::string err;
 };
@@ -345,8 +355,10 @@ nsem_status build_device_mesh(nsem_ctx* ctx, const nsem_mesh_desc* m, const nsem
         if ((s = dalloc(ctx, &b.u[c], n_int)) != NSEM_OK) return s;
         if ((s = dalloc(ctx, &b.s[c], n_int)) != NSEM_OK) return s;
         if ((s = dalloc(ctx, &b.d[c], D.n_slot)) != NSEM_OK) return s;
-        if ((s = dalloc(ctx, &b.L[c], n_int)) != NSEM_OK) return s;
     }
+    /* one block: staged results leave it in one copy */
+    if ((s = dalloc(ctx, &b.L[0], 5 * n_int)) != NSEM_OK) return s;
+    for (int c = 1; c < 5; c++) b.L[c] = b.L[0] + c * n_int;
     for (int c = 0; c < NSEM_NPRIM; c++)
         if ((s = dalloc(ctx, &b.prim[c], n_int)) != NSEM_OK) return s;
     if ((s = dalloc(ctx, &ctx->scratch_aos, 3 * n_int)) != NSEM_OK) return s;
@@ -354,6 +366,13 @@ nsem_status build_device_mesh(nsem_ctx* ctx, const nsem_mesh_desc* m, const nsem
     NSEM_CUDA(cudaMallocHost((void**)&ctx->h_red, 8 * sizeof(double)));
     NSEM_CUDA(cudaMallocHost((void**)&ctx->h_status, sizeof(uint32_t)));
     *ctx->h_status = 0;
+    /* without it results are copied straight to the caller's arrays */
+    ctx->h_out_bytes = std::min<size_t>(6 * (size_t)ctx->dev.n_int * sizeof(double), OUT_BYTES);
+    if (cudaMallocHost((void**)&ctx->h_out, ctx->h_out_bytes) != cudaSuccess) {
+        (void)cudaGetLastError();
+        ctx->h_out = nullptr;
+        ctx->h_out_bytes = 0;
+    }
 
     /* mixed form: per-element affine data, FP32 */
     if ((s = nsem_mixed_setup(ctx->dev, m, &ctx->mbuf, &ctx->allocations, ctx->err)) != NSEM_OK) {
@@ -374,6 +393,43 @@ nsem_status check_status(nsem_ctx* ctx) {
         return fail(ctx, NSEM_NONFINITE, "non-finite value in the state");
     }
     return NSEM_OK;
+}
+
+/* Results to the caller's arrays, then the status.  A copy into pageable memory
+ * is waited for on its own; several small ones share the context's pinned
+ * buffer and one wait. */
+struct HostCopy { double* dst; const double* src; size_t n; };
+
+nsem_status copy_out(nsem_ctx* ctx, const std::vector<HostCopy>& out) {
+    size_t total = 0;
+    for (const HostCopy& c : out) total += c.n * sizeof(double);
+    cudaPointerAttributes at{};
+    const bool stage = out.size() > 1 && total <= ctx->h_out_bytes &&
+                       cudaPointerGetAttributes(&at, out[0].dst) == cudaSuccess &&
+                       at.type == cudaMemoryTypeUnregistered;
+    char* h = ctx->h_out;
+    for (size_t i = 0, k; i < out.size(); i = k) {
+        /* staged results that lie side by side on the device: one copy */
+        size_t n = out[i].n;
+        for (k = i + 1; stage && k < out.size() && out[k].src == out[i].src + n; k++) n += out[k].n;
+        NSEM_CUDA(cudaMemcpyAsync(stage ? (void*)h : (void*)out[i].dst, out[i].src, n * sizeof(double),
+                                  cudaMemcpyDeviceToHost, ctx->stream));
+        h += n * sizeof(double);
+    }
+    const nsem_status s = check_status(ctx);
+    if (!stage || (s != NSEM_OK && s != NSEM_NONFINITE)) return s;
+    h = ctx->h_out;
+    for (const HostCopy& c : out) {
+        std::memcpy(c.dst, h, c.n * sizeof(double));
+        h += c.n * sizeof(double);
+    }
+    return s;
+}
+
+nsem_status copy_out(nsem_ctx* ctx, double* const dst[5], double* const src[5]) {
+    const size_t n = (size_t)ctx->dev.n_int;
+    return copy_out(ctx, {{dst[0], src[0], n}, {dst[1], src[1], n}, {dst[2], src[2], n},
+                          {dst[3], src[3], n}, {dst[4], src[4], n}});
 }
 
 /* move the current state to the representation a form needs */
@@ -592,6 +648,7 @@ void nsem_destroy(nsem_ctx* ctx) {
     }
     if (ctx->h_red) cudaFreeHost(ctx->h_red);
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
+    if (ctx->h_out) cudaFreeHost(ctx->h_out);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -621,20 +678,16 @@ nsem_status nsem_get_state(nsem_ctx* ctx, double* rho, double* rhoU, double* rho
         int e = nsem_mixed_host_layout(&ctx->dev, &ctx->mbuf, 0, ctx->buf.u[0], ctx->scratch_aos,
                                        ctx->buf.u[4], ctx->stream);
         if (e) return cuda_fail(ctx, (cudaError_t)e, "state conversion");
-        NSEM_CUDA(cudaMemcpyAsync(rho, ctx->buf.u[0], n * 8, cudaMemcpyDeviceToHost, ctx->stream));
-        NSEM_CUDA(cudaMemcpyAsync(rhoTheta, ctx->buf.u[4], n * 8, cudaMemcpyDeviceToHost, ctx->stream));
-        NSEM_CUDA(cudaMemcpyAsync(rhoU, ctx->scratch_aos, 3 * n * 8, cudaMemcpyDeviceToHost, ctx->stream));
-        return check_status(ctx);
+        return copy_out(ctx, {{rho, ctx->buf.u[0], n}, {rhoTheta, ctx->buf.u[4], n},
+                              {rhoU, ctx->scratch_aos, 3 * n}});
     }
     nsem_status rs = materialise_conserved(ctx);
     if (rs != NSEM_OK) return rs;
     int e = nsem_soa_to_aos(ctx->buf.u[1], ctx->buf.u[2], ctx->buf.u[3], ctx->scratch_aos,
                             ctx->dev.n_int, ctx->stream);
     if (e) return cuda_fail(ctx, (cudaError_t)e, "soa_to_aos");
-    NSEM_CUDA(cudaMemcpyAsync(rho, ctx->buf.u[0], n * 8, cudaMemcpyDeviceToHost, ctx->stream));
-    NSEM_CUDA(cudaMemcpyAsync(rhoTheta, ctx->buf.u[4], n * 8, cudaMemcpyDeviceToHost, ctx->stream));
-    NSEM_CUDA(cudaMemcpyAsync(rhoU, ctx->scratch_aos, 3 * n * 8, cudaMemcpyDeviceToHost, ctx->stream));
-    return check_status(ctx);
+    return copy_out(ctx, {{rho, ctx->buf.u[0], n}, {rhoTheta, ctx->buf.u[4], n},
+                          {rhoU, ctx->scratch_aos, 3 * n}});
 }
 
 nsem_status nsem_set_fields(nsem_ctx* ctx, const double* rho, const double* U, const double* T) {
@@ -664,14 +717,12 @@ nsem_status nsem_get_pressure(nsem_ctx* ctx, double* p_prime) {
     NSEM_CUDA(cudaSetDevice(ctx->device));
     const size_t n = (size_t)ctx->dev.n_int;
     if (ctx->rep == 2 && ctx->seg_pp_valid) {
-        NSEM_CUDA(cudaMemcpyAsync(p_prime, ctx->sbuf.pp, n * 8, cudaMemcpyDeviceToHost, ctx->stream));
-        return check_status(ctx);
+        return copy_out(ctx, {{p_prime, ctx->sbuf.pp, n}});
     }
     nsem_status rs = materialise_conserved(ctx);
     if (rs != NSEM_OK) return rs;
     if ((rs = fp64_prims(ctx, ctx->buf.u)) != NSEM_OK) return rs;
-    NSEM_CUDA(cudaMemcpyAsync(p_prime, ctx->buf.prim[4], n * 8, cudaMemcpyDeviceToHost, ctx->stream));
-    return check_status(ctx);
+    return copy_out(ctx, {{p_prime, ctx->buf.prim[4], n}});
 }
 
 nsem_status nsem_get_fields(nsem_ctx* ctx, double* rho, double* U, double* T) {
@@ -683,10 +734,8 @@ nsem_status nsem_get_fields(nsem_ctx* ctx, double* rho, double* U, double* T) {
         NsemSegBuf& S = ctx->sbuf;
         int e = nsem_soa_to_aos(S.U[0], S.U[1], S.U[2], ctx->scratch_aos, n, ctx->stream);
         if (e) return cuda_fail(ctx, (cudaError_t)e, "soa_to_aos");
-        NSEM_CUDA(cudaMemcpyAsync(rho, S.rho[S.cur], n * 8, cudaMemcpyDeviceToHost, ctx->stream));
-        NSEM_CUDA(cudaMemcpyAsync(T, S.Tp, n * 8, cudaMemcpyDeviceToHost, ctx->stream));
-        NSEM_CUDA(cudaMemcpyAsync(U, ctx->scratch_aos, 3 * n * 8, cudaMemcpyDeviceToHost, ctx->stream));
-        return check_status(ctx);
+        const size_t nn = (size_t)n;
+        return copy_out(ctx, {{rho, S.rho[S.cur], nn}, {T, S.Tp, nn}, {U, ctx->scratch_aos, 3 * nn}});
     }
     std::vector<double> ru(3 * n), rt(n);
     nsem_status s = nsem_get_state(ctx, rho, ru.data(), rt.data());
@@ -723,11 +772,10 @@ nsem_status nsem_tendency(nsem_ctx* ctx, nsem_precision prec, double* const L[5]
         return fail(ctx, NSEM_BAD_ARG, "unknown precision");
     }
     const size_t n = (size_t)D->n_int;
-    for (int c = 0; c < 5; c++)
-        NSEM_CUDA(cudaMemcpyAsync(L[c], b->L[c], n * 8, cudaMemcpyDeviceToHost, ctx->stream));
-    if (p_prime && prec == NSEM_FP64)
-        NSEM_CUDA(cudaMemcpyAsync(p_prime, b->prim[4], n * 8, cudaMemcpyDeviceToHost, ctx->stream));
-    return check_status(ctx);
+    std::vector<HostCopy> out;
+    for (int c = 0; c < 5; c++) out.push_back({L[c], b->L[c], n});
+    if (p_prime && prec == NSEM_FP64) out.push_back({p_prime, b->prim[4], n});
+    return copy_out(ctx, out);
 }
 
 nsem_status nsem_step(nsem_ctx* ctx, int nsteps, nsem_scheme scheme, nsem_precision prec) {
@@ -908,9 +956,7 @@ extern "C" nsem_status nsem_vjp(nsem_ctx* ctx, const double* const w[5], double*
         NSEM_CUDA(cudaMemcpyAsync(A.lam[v], w[v], bytes, cudaMemcpyHostToDevice, ctx->stream));
     int e = nsem_adj_vjp(&ctx->dev, ctx->buf.u, A.lam, A.g, &A, ctx->stream);
     if (e) return cuda_fail(ctx, (cudaError_t)e, "vjp");
-    for (int v = 0; v < 5; v++)
-        NSEM_CUDA(cudaMemcpyAsync(g[v], A.g[v], bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    return check_status(ctx);
+    return copy_out(ctx, g, A.g);
 }
 
 extern "C" nsem_status nsem_jvp(nsem_ctx* ctx, const double* const dv[5], double* const Ld[5]) {
@@ -928,9 +974,7 @@ extern "C" nsem_status nsem_jvp(nsem_ctx* ctx, const double* const dv[5], double
         NSEM_CUDA(cudaMemcpyAsync(A.lam[v], dv[v], bytes, cudaMemcpyHostToDevice, ctx->stream));
     int e = nsem_adj_jvp(&ctx->dev, ctx->buf.u, A.lam, A.g, &A, ctx->stream);
     if (e) return cuda_fail(ctx, (cudaError_t)e, "jvp");
-    for (int v = 0; v < 5; v++)
-        NSEM_CUDA(cudaMemcpyAsync(Ld[v], A.g[v], bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    return check_status(ctx);
+    return copy_out(ctx, Ld, A.g);
 }
 
 extern "C" nsem_status nsem_tlm(nsem_ctx* ctx, int nsteps, const double* const du0[5],
@@ -984,10 +1028,8 @@ extern "C" nsem_status nsem_tlm(nsem_ctx* ctx, int nsteps, const double* const d
         return s;
     }
     NSEM_CUDA(cudaEventRecord(e1, ctx->stream));
-    for (int v = 0; v < 5; v++)
-        NSEM_CUDA(cudaMemcpyAsync(du_final[v], A.lam[v], bytes, cudaMemcpyDeviceToHost, ctx->stream));
     ctx->rep = 0;
-    s = check_status(ctx);
+    s = copy_out(ctx, du_final, A.lam);
     float ms = 0;
     cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
@@ -1123,9 +1165,7 @@ extern "C" nsem_status nsem_vjp_prec(nsem_ctx* ctx, nsem_precision prec, const d
     e = nsem_mixed_vjp(&ctx->dev, &ctx->mbuf, b->L, b->L, ctx->mbuf.abar[0], ctx->mbuf.abar[1],
                        ctx->stream);
     if (e) return cuda_fail(ctx, (cudaError_t)e, "precision-form vjp");
-    for (int v = 0; v < 5; v++)
-        NSEM_CUDA(cudaMemcpyAsync(g[v], b->L[v], bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    return check_status(ctx);
+    return copy_out(ctx, g, b->L);
 }
 
 /* the precision form's reverse sweep of the last checkpointed run */
@@ -1157,9 +1197,7 @@ static nsem_status mixed_adjoint(nsem_ctx* ctx, const double* const lam_final[5]
     NSEM_CUDA(cudaEventRecord(e1, ctx->stream));
     e = nsem_mixed_layout(&M, 1, nullptr, M.lam, b->L, ctx->stream);
     if (e) return cuda_fail(ctx, (cudaError_t)e, "adjoint layout");
-    for (int v = 0; v < 5; v++)
-        NSEM_CUDA(cudaMemcpyAsync(lam0[v], b->L[v], bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    s = check_status(ctx);
+    s = copy_out(ctx, lam0, b->L);
     float ms = 0;
     cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
@@ -1244,11 +1282,9 @@ extern "C" nsem_status nsem_adjoint(nsem_ctx* ctx, const double* const lam_final
     if (e) s = cuda_fail(ctx, (cudaError_t)e, "adjoint sweep");
     if (s != NSEM_OK) return s;
     NSEM_CUDA(cudaEventRecord(e1, ctx->stream));
-    for (int v = 0; v < 5; v++)
-        NSEM_CUDA(cudaMemcpyAsync(lam0[v], A.lam[v], bytes, cudaMemcpyDeviceToHost, ctx->stream));
     if ((s = copy_state(ctx, ctx->buf.u, A.fin)) != NSEM_OK) return s;
     ctx->rep = 0;
-    s = check_status(ctx);
+    s = copy_out(ctx, lam0, A.lam);
     float ms = 0;
     cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
@@ -1385,9 +1421,7 @@ extern "C" nsem_status nsem_convection_get(nsem_ctx* ctx, double* T) {
     NsemConvBuf& C = ctx->cbuf;
     if (!C.ready) return fail(ctx, NSEM_BAD_ARG, "nsem_convection_set was not called");
     NSEM_CUDA(cudaSetDevice(ctx->device));
-    NSEM_CUDA(cudaMemcpyAsync(T, C.T[C.cur], (size_t)ctx->dev.n_int * 8, cudaMemcpyDeviceToHost,
-                              ctx->stream));
-    return check_status(ctx);
+    return copy_out(ctx, {{T, C.T[C.cur], (size_t)ctx->dev.n_int}});
 }
 
 nsem_status nsem_profile(nsem_ctx* ctx, int nsteps, nsem_precision prec, double ms[8],
