@@ -110,6 +110,29 @@ __device__ __forceinline__ double f2d(float f) {
     return __hiloint2double((int)(hi | sgn), (int)lo);
 }
 
+/* The same for values known to be in range, which leaves out the rest of the
+ * tests: f finite; |x| below in_float_range's bound. */
+__device__ __forceinline__ double f2d_finite(float f) {
+    const unsigned int u = __float_as_uint(f);
+    const bool tiny = (u & 0x7f800000u) == 0u;                             /* zero, subnormal */
+    const unsigned int hi = (((unsigned int)((int)u >> 3)) & 0x8fffffffu) + (896u << 20);
+    return __hiloint2double((int)(tiny ? u & 0x80000000u : hi), (int)(tiny ? 0u : u << 29));
+}
+/* below the largest float with its low 20 mantissa bits cleared; false for inf
+ * and nan */
+__device__ __forceinline__ bool in_float_range(double x) {
+    return ((unsigned int)__double2hiint(x) & 0x7fffffffu) < 0x47efffffu;
+}
+__device__ __forceinline__ float d2f_in_range(double x) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    /* the sign, bit 63, and the two bits below it are shifted out */
+    const unsigned long long r = b + (0x0fffffffull + ((b >> 29) & 1ull));
+    const unsigned int h = (unsigned int)(b >> 32);
+    unsigned int f = (unsigned int)(r >> 29) - (896u << 23);
+    f = (h & 0x7fffffffu) < 0x38100000u ? 0u : f;
+    return __uint_as_float(f | (h & 0x80000000u));
+}
+
 /* reciprocal: hardware approximation refined by one Newton step (within an
  * ulp; deterministic, so every element evaluating it on the same bits gets
  * the same result) */

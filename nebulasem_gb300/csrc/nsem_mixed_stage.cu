@@ -494,24 +494,7 @@ k_mixed_stage(StageArgs a) {
 #pragma unroll
         for (int v = 0; v < 5; v++) a.Dout[o + v * NP] = 0.25f * fmaf(dt, Lv[v], din[v]);
     } else if constexpr (STAGE == 3) {
-        bool finite = true;
-        /* every load before the first store, which could alias them */
-        double u64[5];
-#pragma unroll
-        for (int v = 0; v < 5; v++) {
-            din[v] = a.Din[o + v * NP];
-            u64[v] = a.U[o + v * NP];
-        }
-#pragma unroll
-        for (int v = 0; v < 5; v++) {
-            const float D = (2.0f / 3.0f) * fmaf(dt, Lv[v], din[v]);
-            const double un = u64[v] + f2d(D);
-            a.Unew[o + v * NP] = un;
-            a.Snew[o + v * NP] = d2f_rn(un);
-            /* exponent field all ones = inf or nan (integer test, no FP64 op) */
-            finite = finite && ((__double2hiint(un) & 0x7ff00000) != 0x7ff00000);
-        }
-        if (!finite) atomicOr(a.status, NSEM_STATUS_NONFINITE);
+        update_state<NP>(a, o, Lv);
     }
     }  /* t < NP */
 }
