@@ -403,10 +403,12 @@ struct HostCopy { double* dst; const double* src; size_t n; };
 nsem_status copy_out(nsem_ctx* ctx, const std::vector<HostCopy>& out) {
     size_t total = 0;
     for (const HostCopy& c : out) total += c.n * sizeof(double);
-    cudaPointerAttributes at{};
-    const bool stage = out.size() > 1 && total <= ctx->h_out_bytes &&
-                       cudaPointerGetAttributes(&at, out[0].dst) == cudaSuccess &&
-                       at.type == cudaMemoryTypeUnregistered;
+    bool stage = out.size() > 1 && total <= ctx->h_out_bytes;
+    if (stage) {
+        cudaPointerAttributes at{};
+        if (cudaPointerGetAttributes(&at, out[0].dst) != cudaSuccess) (void)cudaGetLastError();
+        else stage = at.type == cudaMemoryTypeUnregistered;
+    }
     char* h = ctx->h_out;
     for (size_t i = 0, k; i < out.size(); i = k) {
         /* staged results that lie side by side on the device: one copy */
