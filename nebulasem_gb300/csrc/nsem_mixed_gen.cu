@@ -358,7 +358,8 @@ k_mixed_stage_gen(StageArgs a) {
 #pragma unroll
         for (int v = 0; v < 5; v++) a.Dout[o + v * NP] = 0.25f * fmaf(dt, Lv[v], din[v]);
     } else {
-        update_state<NP>(a, o, Lv);
+        double u64[5];
+        update_state<NP, false>(a, o, Lv, din, u64);
     }
 }
 

@@ -192,15 +192,17 @@ __device__ __forceinline__ void grad_lines(float4* sm, const StageArgs& a, int t
  * steps: 6979 to 6916 us; 693 elements 628 to 603; 4096 in 2D, 50 steps: 784
  * to 719; with the hardware's float-to-double conversion, which runs on the
  * FP64 pipe, 6950, 626 and 779) */
-template <int NP>
-__device__ __forceinline__ void update_state(const StageArgs& a, int64_t o, const float* Lv) {
-    float D[5];
-    double un[5];
-    /* every load before the first store, which could alias them */
+template <int NP, bool LOADED>
+__device__ __forceinline__ void update_state(const StageArgs& a, int64_t o, const float* Lv, float* D,
+                                             double* un) {
+    /* LOADED: D and un hold the increment d2 and u'^n already */
+    if constexpr (!LOADED) {
+        /* every load before the first store, which could alias them */
 #pragma unroll
-    for (int v = 0; v < 5; v++) {
-        D[v] = a.Din[o + v * NP];
-        un[v] = a.U[o + v * NP];
+        for (int v = 0; v < 5; v++) {
+            D[v] = a.Din[o + v * NP];
+            un[v] = a.U[o + v * NP];
+        }
     }
     bool ok = true;
 #pragma unroll

@@ -254,6 +254,11 @@ k_mixed_stage(StageArgs a) {
      * kernel: background, neighbours, metric */
     float own[5], din[5] = {0, 0, 0, 0, 0}, bgs[4] = {0, 0, 0, 0};
     float gown[12];
+    /* 30 steps in 2D, at the update and here: 24 x 24 elements of order 4 303
+     * and 295 us, 40 x 40 347 and 338, 88 x 90 748 and 741; viscous, whose 74
+     * registers cost CTAs, 88 x 90 1381 and 1408 */
+    constexpr bool EARLY_U = STAGE == 3 && G::EPB > 1 && !VISC;
+    double u64[5];
     if (t < NP) load_bg<NX, NY, NZ>(a, __ldg(a.layer + e), -1, t, bgs);
     FaceSlot fs{};
     int32_t nb = -1;
@@ -289,10 +294,14 @@ k_mixed_stage(StageArgs a) {
             /* u'^n is needed only at the update: fetched into L2 here and
              * loaded there (with the increment reloaded from L1/L2), so that
              * neither holds registers through the element and nine CTAs (six
-             * in viscous runs) fit per SM */
+             * in viscous runs) fit per SM.  Inviscid runs in 2D load it here:
+             * their registers suffice, and the wait at the update is gone */
             const double* u = a.U + e * 5 * NP + t;
 #pragma unroll
-            for (int v = 0; v < 5; v++) asm volatile("prefetch.global.L2 [%0];" ::"l"(u + v * NP));
+            for (int v = 0; v < 5; v++) {
+                if constexpr (EARLY_U) u64[v] = u[v * NP];
+                else asm volatile("prefetch.global.L2 [%0];" ::"l"(u + v * NP));
+            }
         }
         if constexpr (VISC) {
             const float* gr = a.G + e * 12 * NP + t;
@@ -494,7 +503,7 @@ k_mixed_stage(StageArgs a) {
 #pragma unroll
         for (int v = 0; v < 5; v++) a.Dout[o + v * NP] = 0.25f * fmaf(dt, Lv[v], din[v]);
     } else if constexpr (STAGE == 3) {
-        update_state<NP>(a, o, Lv);
+        update_state<NP, EARLY_U>(a, o, Lv, din, u64);
     }
     }  /* t < NP */
 }
