@@ -49,7 +49,7 @@ struct nsem_ctx {
      * into the form that steps it */
     int rep = 0;
     bool seg_pp_valid = false;   /* sbuf.pp holds the p' of the last segregated step */
-    int adj_form = -1;           /* form of the last checkpointed forward run (-1: none) */
+    int adj_form = -1;           /* form of the last checkpointed forward run (-1: none, or it failed) */
     double dt = 0, T0 = 0;
     int64_t n_all = 0;
     std::vector<void*> allocations;
@@ -1052,7 +1052,7 @@ extern "C" nsem_status nsem_forward_checkpointed(nsem_ctx* ctx, int nsteps, int 
     NsemAdjBuf& A = ctx->abuf;
     const int64_t n = ctx->dev.n_int;
     const int n_ckpt = (nsteps + ckpt_every - 1) / ckpt_every;
-    A.nsteps = 0;   /* no run to differentiate until this one has ended */
+    ctx->adj_form = -1;   /* no run of either form to differentiate until this one has ended */
     A.seg_of = -1;
     const int64_t n_seg = 3 * (int64_t)ckpt_every;
     s = A.ckpt_slots < n_ckpt ? grow_states(ctx, &A.ckpt, &A.ckpt_slots, n_ckpt) : NSEM_OK;
@@ -1109,7 +1109,7 @@ static nsem_status mixed_forward_checkpointed(nsem_ctx* ctx, int nsteps, int ckp
     if (!ctx->mixed_ready) return fail(ctx, NSEM_UNSUPPORTED, ctx->err);
     nsem_status s = ensure_rep(ctx, 1);
     if (s != NSEM_OK) return s;
-    ctx->adj_form = -1;
+    ctx->adj_form = -1;   /* as in the FP64 form's run */
     cudaEvent_t e0, e1;
     NSEM_CUDA(cudaEventCreate(&e0));
     NSEM_CUDA(cudaEventCreate(&e1));
@@ -1232,9 +1232,9 @@ extern "C" nsem_status nsem_adjoint(nsem_ctx* ctx, const double* const lam_final
         NSEM_CUDA(cudaSetDevice(ctx->device));
         return mixed_adjoint(ctx, lam_final, lam0, ms_adj);
     }
-    NsemAdjBuf& A = ctx->abuf;
-    if (!A.ready || !A.ckpt || A.nsteps < 1)
+    if (ctx->adj_form != 0)
         return fail(ctx, NSEM_BAD_ARG, "no checkpointed forward run to differentiate");
+    NsemAdjBuf& A = ctx->abuf;
     NSEM_CUDA(cudaSetDevice(ctx->device));
     const int64_t n = ctx->dev.n_int;
     const size_t bytes = (size_t)n * sizeof(double);
