@@ -294,20 +294,20 @@ __global__ void __launch_bounds__(FACE) k_face(const NsemDev m, FaceArgs a) {
 
     /* a normal along one axis: only the flux tensor's column of that axis meets
      * a nonzero normal component; the products left out are zeros that change
-     * no sum (the lift starts at +0), provided nothing can overflow */
+     * no sum (the lift starts at +0), provided the flux components that meet a
+     * zero stay finite: they have up to five factors, the normal not among them */
     const int ax = side == 0 ? nsem_axis_of(n, en) : -1;
     if (ax >= 0) {
-        bool bounded = true, mild = true;
+        bool bounded = true, mild = !a.G[0] || m.tame_const;
         auto look = [&](double x) {
             bounded = bounded && nsem_bounded(x);
-            mild = mild && nsem_mild(x);
+            mild = mild && nsem_flux_mild(x);
         };
         look(r1); look(r2); look(T1); look(T2); look(p1); look(p2); look(lam);
         look(fi); look(fo);
         for (int c = 0; c < 3; c++) { look(U1[c]); look(U2[c]); look(n[c]); }
         if (a.G[0]) {
-            look(m.nu);
-            look(m.iPr);
+            bounded = bounded && nsem_bounded(m.nu) && nsem_bounded(m.iPr);
             for (int c = 0; c < 12; c++) {
                 look(a.G[c][c1]);
                 if (c2 >= 0) look(a.G[c][c2]);

@@ -70,18 +70,31 @@ __device__ __forceinline__ bool nsem_tame(double x) {
     const uint32_t h = (uint32_t)__double2hiint(x) & 0x7fffffffu;
     return h - ((1023u - 400u) << 20) < (600u << 20) || (h | (uint32_t)__double2loint(x)) == 0u;
 }
-/* zero, or 2^-200 <= |x| < 2^200: a product with a tame value is normal or zero */
-__device__ __forceinline__ bool nsem_mild(double x) {
+/* zero, or 2^-K <= |x| < 2^K */
+template <unsigned K>
+__device__ __forceinline__ bool nsem_within(double x) {
     const uint32_t h = (uint32_t)__double2hiint(x) & 0x7fffffffu;
-    return h - ((1023u - 200u) << 20) < (400u << 20) || (h | (uint32_t)__double2loint(x)) == 0u;
+    return h - ((1023u - K) << 20) < (2u * K << 20) || (h | (uint32_t)__double2loint(x)) == 0u;
 }
+/* zero, or within 2^+-200: a product with a tame value is normal or zero */
+__device__ __forceinline__ bool nsem_mild(double x) { return nsem_within<200>(x); }
+/* a metric component whose product with a derivative (host-checked to be zero
+ * or within 2^+-60) is mild */
+__device__ __forceinline__ bool nsem_metric_tame(double J) { return nsem_within<140>(J); }
 
-/* zero, or within 2^+-140: a metric component whose product with a derivative
- * (host-checked to be zero or within 2^+-60) is mild */
-__device__ __forceinline__ bool nsem_metric_tame(double J) {
-    const uint32_t h = (uint32_t)__double2hiint(J) & 0x7fffffffu;
-    return h - ((1023u - 140u) << 20) < (280u << 20) || (h | (uint32_t)__double2loint(J)) == 0u;
-}
+/* An axis flux multiplies up to five values and takes differences on the way,
+ * which can cancel down to the last place of their terms, so mild values do not
+ * suffice for its integer products.  With density, velocity, theta, pressure,
+ * gradients, lambda, weights and normal within 2^+-180, the mass flux density
+ * (rho U) within 2^+-360 and nu and 1 / Pr within 2^+-60 (tame_const), each
+ * value is zero or, with its last place 52 bits below,
+ *   U (rho U) + p' - mu g, theta (rho U) - (mu / Pr) g    2^-592 .. 2^542
+ *   their weighted averages                               2^-772 .. 2^723
+ *   averages less lambda (rho U), lambda (rho theta)      2^-824 .. 2^724
+ *   that times the normal                                 2^-1004 .. 2^904
+ * and no product leaves the normal range. */
+__device__ __forceinline__ bool nsem_flux_mild(double x) { return nsem_within<180>(x); }
+__device__ __forceinline__ bool nsem_mass_flux_mild(double x) { return nsem_within<360>(x); }
 
 /* what nsem_volume_gather may do on an element: bit 0 every value tame, bit 1
  * the metric diagonal too */

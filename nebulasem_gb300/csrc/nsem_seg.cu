@@ -676,13 +676,13 @@ __global__ void __launch_bounds__(FACE) k_seg_face_ut(const NsemDev m, SegArgs a
         bool bounded = true, mild = m.tame_const;
         auto look = [&](double x) {
             bounded = bounded && nsem_bounded(x);
-            mild = mild && nsem_mild(x);
+            mild = mild && nsem_flux_mild(x);
         };
         look(lam); look(r1); look(r2); look(T1); look(T2); look(p1); look(p2); look(fi); look(fo);
         for (int c = 0; c < 3; c++) {
             look(U1[c]); look(U2[c]); look(n[c]);
             bounded = bounded && nsem_bounded(Fc1[c]) && nsem_bounded(Fc2[c]);
-            mild = mild && nsem_tame(Fc1[c]) && nsem_tame(Fc2[c]);
+            mild = mild && nsem_mass_flux_mild(Fc1[c]) && nsem_mass_flux_mild(Fc2[c]);
         }
         if (a.visc) {
             look(mu1);
