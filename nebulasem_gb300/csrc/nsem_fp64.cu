@@ -414,15 +414,16 @@ constexpr int SM_W = 24;
 constexpr unsigned SM_ROWS = 0xe;   /* the momentum equations are tensor rows */
 
 /* the Shu-Osher combination of a stage; INT: operands mild (a sum that is not
- * mild takes its product in FP64) */
+ * mild takes its product in FP64).  A zero product keeps its sign: a momentum
+ * of -0 without a tendency, L = -0, stays -0. */
 template <bool INT>
 __device__ __forceinline__ void update(int stage, double dt, const double* S, const double* U0,
                                        const double* L, double* nu) {
     const double cu = stage == 2 ? 0.75 : 1.0 / 3.0, cs = stage == 2 ? 0.25 : 2.0 / 3.0;
+    auto mul = [](double a, double b) { return INT ? nsem_mul_signed(nsem_make_factor(a), b) : a * b; };
     for (int c = 0; c < 5; c++) {
-        const double s = S[c] + nsem_x<INT>(dt, L[c]);
-        nu[c] = stage == 1 ? s
-                           : nsem_x<INT>(cu, U0[c]) + (!INT || nsem_mild(s) ? nsem_x<INT>(cs, s) : cs * s);
+        const double s = S[c] + mul(dt, L[c]);
+        nu[c] = stage == 1 ? s : mul(cu, U0[c]) + (!INT || nsem_mild(s) ? mul(cs, s) : cs * s);
     }
 }
 

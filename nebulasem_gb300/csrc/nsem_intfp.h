@@ -200,9 +200,9 @@ NSEM_IHD nsem_factor nsem_make_factor(double a) {
 }
 
 /* the product for operands that are zero or normal with a normal result (the
- * caller has bounded their exponents); a zero product is +0.  About 32
- * instructions, four of them 32 x 32 + 64-bit multiply-adds. */
-NSEM_IHD double nsem_mul_normal(nsem_factor f, double b) {
+ * caller has bounded their exponents); zero_hi: the high word of a zero product.
+ * About 32 instructions, four of them 32 x 32 + 64-bit multiply-adds. */
+NSEM_IHD double nsem_mul_bits(nsem_factor f, double b, uint32_t zero_hi) {
     const uint64_t ub = nsem_bits(b);
     const uint32_t bh = (uint32_t)(ub >> 32), b0 = (uint32_t)ub;
     const uint32_t b1 = (bh & 0xfffffu) | 0x100000u;
@@ -234,7 +234,15 @@ NSEM_IHD double nsem_mul_normal(nsem_factor f, double b) {
     hi = (uint32_t)(m >> 32);
 #endif
     const int zero = ((f.h & 0x7ff00000u) == 0u) | ((bh & 0x7ff00000u) == 0u);
-    return nsem_from_bits(zero ? 0u : hi, zero ? 0u : lo);
+    return nsem_from_bits(zero ? zero_hi : hi, zero ? 0u : lo);
+}
+
+/* a zero product is +0: for sums that start at +0, which show no zero's sign */
+NSEM_IHD double nsem_mul_normal(nsem_factor f, double b) { return nsem_mul_bits(f, b, 0u); }
+
+/* a zero product has the sign of its factors */
+NSEM_IHD double nsem_mul_signed(nsem_factor f, double b) {
+    return nsem_mul_bits(f, b, (f.h ^ (uint32_t)(nsem_bits(b) >> 32)) & 0x80000000u);
 }
 
 #endif
