@@ -22,6 +22,7 @@
 #include "nsem.h"
 #include "nsem_internal.h"
 #include "nsem_adjoint.h"
+#include "nsem_copy.h"
 #include "nsem_mixed.h"
 #include "nsem_seg.h"
 
@@ -397,33 +398,25 @@ nsem_status check_status(nsem_ctx* ctx) {
 
 /* Results to the caller's arrays, then the status.  A copy into pageable memory
  * is waited for on its own; several small ones share the context's pinned
- * buffer and one wait. */
-struct HostCopy { double* dst; const double* src; size_t n; };
-
-nsem_status copy_out(nsem_ctx* ctx, const std::vector<HostCopy>& out) {
-    size_t total = 0;
-    for (const HostCopy& c : out) total += c.n * sizeof(double);
-    bool stage = out.size() > 1 && total <= ctx->h_out_bytes;
-    if (stage) {
+ * buffer and one wait (nsem_copy.h). */
+nsem_status copy_out(nsem_ctx* ctx, const std::vector<NsemHostCopy>& out) {
+    const int n = (int)out.size();
+    const bool stage = nsem_stage_results(out.data(), n, ctx->h_out_bytes, [](const double* p) {
         cudaPointerAttributes at{};
-        if (cudaPointerGetAttributes(&at, out[0].dst) != cudaSuccess) (void)cudaGetLastError();
-        else stage = at.type == cudaMemoryTypeUnregistered;
-    }
-    char* h = ctx->h_out;
-    for (size_t i = 0, k; i < out.size(); i = k) {
-        /* staged results that lie side by side on the device: one copy */
-        size_t n = out[i].n;
-        for (k = i + 1; stage && k < out.size() && out[k].src == out[i].src + n; k++) n += out[k].n;
-        NSEM_CUDA(cudaMemcpyAsync(stage ? (void*)h : (void*)out[i].dst, out[i].src, n * sizeof(double),
-                                  cudaMemcpyDeviceToHost, ctx->stream));
-        h += n * sizeof(double);
-    }
+        if (cudaPointerGetAttributes(&at, p) == cudaSuccess) return at.type == cudaMemoryTypeUnregistered;
+        (void)cudaGetLastError();
+        return false;
+    });
+    double* h = stage ? (double*)ctx->h_out : nullptr;
+    const int e = nsem_copy_results(out.data(), n, h, [&](double* dst, const double* src, size_t m) {
+        return (int)cudaMemcpyAsync(dst, src, m * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
+    });
+    if (e) return cuda_fail(ctx, (cudaError_t)e, "copy of the results");
     const nsem_status s = check_status(ctx);
     if (!stage || (s != NSEM_OK && s != NSEM_NONFINITE)) return s;
-    h = ctx->h_out;
-    for (const HostCopy& c : out) {
+    for (const NsemHostCopy& c : out) {
         std::memcpy(c.dst, h, c.n * sizeof(double));
-        h += c.n * sizeof(double);
+        h += c.n;
     }
     return s;
 }
@@ -774,7 +767,7 @@ nsem_status nsem_tendency(nsem_ctx* ctx, nsem_precision prec, double* const L[5]
         return fail(ctx, NSEM_BAD_ARG, "unknown precision");
     }
     const size_t n = (size_t)D->n_int;
-    std::vector<HostCopy> out;
+    std::vector<NsemHostCopy> out;
     for (int c = 0; c < 5; c++) out.push_back({L[c], b->L[c], n});
     if (p_prime && prec == NSEM_FP64) out.push_back({p_prime, b->prim[4], n});
     return copy_out(ctx, out);
