@@ -421,10 +421,12 @@ nsem_status copy_out(nsem_ctx* ctx, const std::vector<NsemHostCopy>& out) {
     return s;
 }
 
-nsem_status copy_out(nsem_ctx* ctx, double* const dst[5], double* const src[5]) {
+/* five arrays; block: src is one allocation, as buf.L is */
+nsem_status copy_out(nsem_ctx* ctx, double* const dst[5], double* const src[5], bool block = false) {
     const size_t n = (size_t)ctx->dev.n_int;
-    return copy_out(ctx, {{dst[0], src[0], n}, {dst[1], src[1], n}, {dst[2], src[2], n},
-                          {dst[3], src[3], n}, {dst[4], src[4], n}});
+    return copy_out(ctx, {{dst[0], src[0], n, false}, {dst[1], src[1], n, block},
+                          {dst[2], src[2], n, block}, {dst[3], src[3], n, block},
+                          {dst[4], src[4], n, block}});
 }
 
 /* move the current state to the representation a form needs */
@@ -673,16 +675,16 @@ nsem_status nsem_get_state(nsem_ctx* ctx, double* rho, double* rhoU, double* rho
         int e = nsem_mixed_host_layout(&ctx->dev, &ctx->mbuf, 0, ctx->buf.u[0], ctx->scratch_aos,
                                        ctx->buf.u[4], ctx->stream);
         if (e) return cuda_fail(ctx, (cudaError_t)e, "state conversion");
-        return copy_out(ctx, {{rho, ctx->buf.u[0], n}, {rhoTheta, ctx->buf.u[4], n},
-                              {rhoU, ctx->scratch_aos, 3 * n}});
+        return copy_out(ctx, {{rho, ctx->buf.u[0], n, false}, {rhoTheta, ctx->buf.u[4], n, false},
+                              {rhoU, ctx->scratch_aos, 3 * n, false}});
     }
     nsem_status rs = materialise_conserved(ctx);
     if (rs != NSEM_OK) return rs;
     int e = nsem_soa_to_aos(ctx->buf.u[1], ctx->buf.u[2], ctx->buf.u[3], ctx->scratch_aos,
                             ctx->dev.n_int, ctx->stream);
     if (e) return cuda_fail(ctx, (cudaError_t)e, "soa_to_aos");
-    return copy_out(ctx, {{rho, ctx->buf.u[0], n}, {rhoTheta, ctx->buf.u[4], n},
-                          {rhoU, ctx->scratch_aos, 3 * n}});
+    return copy_out(ctx, {{rho, ctx->buf.u[0], n, false}, {rhoTheta, ctx->buf.u[4], n, false},
+                          {rhoU, ctx->scratch_aos, 3 * n, false}});
 }
 
 nsem_status nsem_set_fields(nsem_ctx* ctx, const double* rho, const double* U, const double* T) {
@@ -712,12 +714,12 @@ nsem_status nsem_get_pressure(nsem_ctx* ctx, double* p_prime) {
     NSEM_CUDA(cudaSetDevice(ctx->device));
     const size_t n = (size_t)ctx->dev.n_int;
     if (ctx->rep == 2 && ctx->seg_pp_valid) {
-        return copy_out(ctx, {{p_prime, ctx->sbuf.pp, n}});
+        return copy_out(ctx, {{p_prime, ctx->sbuf.pp, n, false}});
     }
     nsem_status rs = materialise_conserved(ctx);
     if (rs != NSEM_OK) return rs;
     if ((rs = fp64_prims(ctx, ctx->buf.u)) != NSEM_OK) return rs;
-    return copy_out(ctx, {{p_prime, ctx->buf.prim[4], n}});
+    return copy_out(ctx, {{p_prime, ctx->buf.prim[4], n, false}});
 }
 
 nsem_status nsem_get_fields(nsem_ctx* ctx, double* rho, double* U, double* T) {
@@ -730,7 +732,8 @@ nsem_status nsem_get_fields(nsem_ctx* ctx, double* rho, double* U, double* T) {
         int e = nsem_soa_to_aos(S.U[0], S.U[1], S.U[2], ctx->scratch_aos, n, ctx->stream);
         if (e) return cuda_fail(ctx, (cudaError_t)e, "soa_to_aos");
         const size_t nn = (size_t)n;
-        return copy_out(ctx, {{rho, S.rho[S.cur], nn}, {T, S.Tp, nn}, {U, ctx->scratch_aos, 3 * nn}});
+        return copy_out(ctx, {{rho, S.rho[S.cur], nn, false}, {T, S.Tp, nn, false},
+                              {U, ctx->scratch_aos, 3 * nn, false}});
     }
     std::vector<double> ru(3 * n), rt(n);
     nsem_status s = nsem_get_state(ctx, rho, ru.data(), rt.data());
@@ -768,8 +771,8 @@ nsem_status nsem_tendency(nsem_ctx* ctx, nsem_precision prec, double* const L[5]
     }
     const size_t n = (size_t)D->n_int;
     std::vector<NsemHostCopy> out;
-    for (int c = 0; c < 5; c++) out.push_back({L[c], b->L[c], n});
-    if (p_prime && prec == NSEM_FP64) out.push_back({p_prime, b->prim[4], n});
+    for (int c = 0; c < 5; c++) out.push_back({L[c], b->L[c], n, c > 0});
+    if (p_prime && prec == NSEM_FP64) out.push_back({p_prime, b->prim[4], n, false});
     return copy_out(ctx, out);
 }
 
@@ -1160,7 +1163,7 @@ extern "C" nsem_status nsem_vjp_prec(nsem_ctx* ctx, nsem_precision prec, const d
     e = nsem_mixed_vjp(&ctx->dev, &ctx->mbuf, b->L, b->L, ctx->mbuf.abar[0], ctx->mbuf.abar[1],
                        ctx->stream);
     if (e) return cuda_fail(ctx, (cudaError_t)e, "precision-form vjp");
-    return copy_out(ctx, g, b->L);
+    return copy_out(ctx, g, b->L, true);
 }
 
 /* the precision form's reverse sweep of the last checkpointed run */
@@ -1192,7 +1195,7 @@ static nsem_status mixed_adjoint(nsem_ctx* ctx, const double* const lam_final[5]
     NSEM_CUDA(cudaEventRecord(e1, ctx->stream));
     e = nsem_mixed_layout(&M, 1, nullptr, M.lam, b->L, ctx->stream);
     if (e) return cuda_fail(ctx, (cudaError_t)e, "adjoint layout");
-    s = copy_out(ctx, lam0, b->L);
+    s = copy_out(ctx, lam0, b->L, true);
     float ms = 0;
     cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
@@ -1416,7 +1419,7 @@ extern "C" nsem_status nsem_convection_get(nsem_ctx* ctx, double* T) {
     NsemConvBuf& C = ctx->cbuf;
     if (!C.ready) return fail(ctx, NSEM_BAD_ARG, "nsem_convection_set was not called");
     NSEM_CUDA(cudaSetDevice(ctx->device));
-    return copy_out(ctx, {{T, C.T[C.cur], (size_t)ctx->dev.n_int}});
+    return copy_out(ctx, {{T, C.T[C.cur], (size_t)ctx->dev.n_int, false}});
 }
 
 nsem_status nsem_profile(nsem_ctx* ctx, int nsteps, nsem_precision prec, double ms[8],

@@ -12,6 +12,7 @@ struct NsemHostCopy {
     double* dst;
     const double* src;
     size_t n;
+    bool joins;   /* src continues the result before it, within one allocation */
 };
 
 /* several results that fit the pinned buffer together are staged, when the host
@@ -33,9 +34,11 @@ bool nsem_stage_results(const NsemHostCopy* c, int n, size_t room, Pageable page
 template <typename Copy>
 int nsem_copy_results(const NsemHostCopy* c, int n, double* buffer, Copy copy) {
     for (int i = 0, k; i < n; i = k) {
-        /* staged results that lie side by side on the device: one copy */
+        /* staged results of one allocation side by side: one copy.  Equal
+         * addresses would not say so: allocations of their own can be neighbours,
+         * and a copy must not cross from one into the next */
         size_t m = c[i].n;
-        for (k = i + 1; buffer && k < n && c[k].src == c[i].src + m; k++) m += c[k].n;
+        for (k = i + 1; buffer && k < n && c[k].joins; k++) m += c[k].n;
         const int e = copy(buffer ? buffer : c[i].dst, c[i].src, m);
         if (e) return e;
         if (buffer) buffer += m;
