@@ -545,13 +545,7 @@ extern "C" int nsem_fp64_face(const NsemDev* m, NsemBuf* b, const double* rho, v
     for (int c = 0; c < 19; c++) a.mq[c] = b->mq[c];
     for (int c = 0; c < 15; c++) a.mf[c] = b->mf[c];
     for (int c = 0; c < 5; c++) a.dC[c] = b->dC[c];
-    /* a volume grid of less than a wave that fills the FP64 pipes (8 to 32 warps
-     * an SM) is started after this kernel: beside it, its CTAs gather on the
-     * SMs this grid leaves free (9 x 8 x 10 elements of order 4, forward and
-     * reverse: 9.2 against 7.8 ms); more waves even out (14 x 12 x 13: 6.14
-     * against 6.25 ms), fewer warps leave the pipes idle either way */
-    const int64_t warps = m->n_elem * ((m->np + 31) / 32) / 152;
-    a.early = warps < 8 || warps > 32;
+    a.early = m->early;
     const int64_t blocks = (m->n_slot + FACE - 1) / FACE;
     cudaStream_t st = (cudaStream_t)stream;
     const unsigned mb = (unsigned)((m->n_ms + 127) / 128);
@@ -574,6 +568,28 @@ extern "C" int nsem_fp64_prepare(NsemDev* m) {
                                              (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
+    /* Whether the volume kernel's CTAs may start beside the face kernel, where
+     * they gather on the SMs that its grid leaves free.  10 steps, after the face
+     * kernel and beside it:
+     *   - more than 32 warps an SM even out: 4 warps an element (order 4), 35 an
+     *     SM 2880 and 2838 us, 77 5215 and 5140;
+     *   - from 8 to 32, warps that share the pipes unevenly cost more: order 4,
+     *     10 an SM 1424 and 1548 us, 19 1859 and 2154; full metric 17 3037 and 3861
+     *     (above 26 the two are within 2 %, but one-warp elements of 2D lose up
+     *     to 13 % at 24);
+     *   - fewer leave the pipes idle either way, and starting early is worth 1 to
+     *     3 % (one-warp elements of order 1 5 to 14 %), where each SM has a few
+     *     CTAs to even out: order 2, 5.9 an SM 1181 and 1159 us; 2D, order 4, 8
+     *     1207 and 1169.  With up to two, one SM in many gets twice the others'
+     *     work: order 5, 0.4 elements an SM 1098 and 1327 us, 0.7 1216 and 1401;
+     *     order 4, 0.5 1044 and 1170; 2D, order 4, 2 984 and 1032.  (Order 7, half
+     *     an element, loses 1.5 % by this line.) */
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return (int)e;
+    const double elems = (double)m->n_elem / sms, warps = elems * ((m->np + 31) / 32);
+    m->early = warps > 32 || (warps < 8 && elems > 2.5);
     m->split = nsem_chain_split(NSEM_SPLIT, k_volume, (unsigned)m->n_elem, ((m->np + 31) / 32) * 32, smem);
     return 0;
 }

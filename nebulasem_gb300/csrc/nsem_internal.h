@@ -38,6 +38,7 @@ struct NsemDev {
     int64_t n_elem, n_int, n_slot;
     int32_t tame_tables; /* every dpsi entry zero or within 2^+-60 */
     int32_t split;       /* shared-memory split of the coupled form's launches */
+    int32_t early;       /* its volume kernel's CTAs may start beside the face kernel */
     int32_t tame_const;  /* P0, R, gamma R, nu, 1/Pr and T0 zero or within 2^+-60 */
     /* physical constants */
     double P0, R, gamma, gR, cv_heat, cp, T0;
