@@ -186,7 +186,10 @@ nsem_status nsem_diagnostics(nsem_ctx* ctx, double* mass, double* energy, double
  * nsem_adjoint: given lam_final = dJ/du at the final state of the last
  * nsem_forward_checkpointed call, return lam0 = dJ/du at its initial state
  * (reverse Shu-Osher sweep, each segment recomputed from its checkpoint with
- * its stage states kept; the last segment's are kept from the forward run).  The context's state is left at the final state.
+ * its stage states kept; the last segment's are kept from the forward run).
+ * The context's state is left at the final state.  A forward run that fails
+ * leaves nothing to differentiate; one that is refused before it begins (bad
+ * arguments, a form the mesh does not have) leaves the run before it.
  * ms_fwd / ms_adj (optional) receive the device time of the forward pass and
  * of the reverse sweep. */
 nsem_status nsem_vjp(nsem_ctx* ctx, const double* const w[5], double* const g[5]);

@@ -12,8 +12,7 @@
  *   Rusanov d = (cds F - n^ (x) lambda dq) . fN, lambda = (cds|U| + cds c) / 2
  *   ghosts  NEUMANN copies, SYMMETRY velocity (tangential projection
  *           rescaled to |U|, tensor.h:486-494), adjoint folded into the owner
- *   EOS     p = P0 (rho theta R / P0)^gamma -> dp/drho = gamma p / rho,
- *                                              dp/dtheta = gamma p / theta
+ *   EOS     p = P0 (E R / P0)^gamma, E = rho theta -> dp/dE = gamma p / E
  * Non-smooth points take the one-sided choice of the value's branch
  * (d|U| = U/|U|, 0 at U = 0; the SYMMETRY threshold |r| <= 1e-7 as forward).
  *
@@ -22,8 +21,8 @@
  * transposed volume gather, source, face contributions gathered through the
  * lift lists, primitive -> conserved chain rule).  The tangent-linear product
  * (k_tan_face, k_tan_volume) linearises the same chain in forward mode.
- * FP64 throughout; this file
- * may use FMA contraction (the adjoint is checked to 1e-6, not bitwise).
+ * FP64 throughout; this file may use FMA contraction (the adjoint is checked
+ * against the tangent-linear product, not bitwise).
  */
 #include <cuda_runtime.h>
 
@@ -364,7 +363,7 @@ struct VolAdjArgs {
 /* registers capped for the largest element: 736 threads (N+1 = 9) inviscid,
  * 512 (N+1 = 8) with the viscous terms */
 template <bool VISC>
-__global__ void __maxnreg__(VISC ? 128 : 88) k_adj_volume(const NsemDev m,                                                           VolAdjArgs a) {
+__global__ void __maxnreg__(VISC ? 128 : 88) k_adj_volume(const NsemDev m, VolAdjArgs a) {
     extern __shared__ double sm[];
     const int NPX = m.npx, NPY = m.npy, NPZ = m.npz, NP = m.np;
     double* rb = sm;                                 /* [5][NP] rbar of the element */

@@ -17,7 +17,8 @@ struct NsemAdjBuf {
     double* g[5] = {};      /* VJP output                                 */
     double* fin[5] = {};    /* final forward state (restored afterwards)  */
     double* ckpt = nullptr; /* [n_ckpt][5][n_int] states every k steps     */
-    double* seg = nullptr;  /* [k][3][5][n_int] u^n, u1, u2 of a segment   */
+    double* seg = nullptr;  /* [k][3][5][n_int] u^n, u1, u2 of a segment's steps (its first
+                               step's u^n is the checkpoint: that slot is free) */
     int64_t seg_slots = 0;  /* state slots allocated in seg                 */
     int64_t ckpt_slots = 0; /* states allocated in ckpt                     */
     int seg_of = -1;        /* the segment whose stage states seg holds (-1: none) */

@@ -22,7 +22,9 @@
  * FP64 operation count is the time:
  *   - products run on the integer pipes (nsem_mul_normal: the same correctly
  *     rounded product), beside the FP64 pipe's additions, on an element whose
- *     values are zero or of a size at which every product is normal (`tame`);
+ *     values are zero or of a size at which every product is normal (`tame`;
+ *     one value below 2^-400, as a wind far ahead of the sound front makes, sends
+ *     its element to the full products in FP64);
  *   - on an element whose metric is also diagonal (every off-diagonal component
  *     of every node is zero) a line source has dj = (0, .., J_cc D, .., 0), and
  *     the products with the zeros are zeros that change no sum: r starts at +0

@@ -1213,8 +1213,8 @@ int nsem_mixed_host_layout(const NsemDev* dev, NsemMixedBuf* mb, int to_pert, do
     return (int)cudaErrorNotSupported;
 }
 
-int nsem_mixed_steps(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf*, 
-                     int nsteps, double dt, void* stream) {
+int nsem_mixed_steps(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf*, int nsteps,
+                     double dt, void* stream) {
     int cur = mb->cur;
     for (int n = 0; n < nsteps; n++) {
         int e = nsem_mixed_step_bufs(dev, mb, mb->U[cur], mb->S[cur], mb->D[0], mb->D[1],
@@ -1225,8 +1225,7 @@ int nsem_mixed_steps(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf*,
     return 0;
 }
 
-int nsem_mixed_tendency(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf* b, 
-                        void* stream) {
+int nsem_mixed_tendency(const NsemDev* dev, NsemMixedBuf* mb, NsemBuf* b, void* stream) {
     StageArgs a = base_args(dev, mb, 0.0);
     a.U = mb->U[mb->cur];
     a.S = mb->S[mb->cur];

@@ -586,7 +586,6 @@ int launch_adj(const AdjArgs& a, int rs, cudaStream_t st, int passes) {
         case 2: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 2, false>, grid, G::block(), SMEM, st, a.split, a);
         default: return nsem_launch_chained(k_mixed_adj<NX, NY, NZ, 3, false>, grid, G::block(), SMEM, st, a.split, a);
     }
-    return (int)cudaGetLastError();
 }
 
 template <int NX, int NY, int NZ>

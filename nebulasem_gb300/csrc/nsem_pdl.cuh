@@ -44,7 +44,11 @@ constexpr int NSEM_SPLIT = 72;
 
 /* Grids of more than one wave keep the driver's choice: their own kernels
  * fill the SMs, and the best split of each counts for more (2184 elements of
- * order 3: 1323 us and 1358 with one split, of order 4 2151 and 2195). */
+ * order 3: 1323 us and 1358 with one split, of order 4 2151 and 2195).  The
+ * convection and the segregated scheme, whose kernels are shorter, name theirs
+ * at every size: convection, 20 steps, 343 elements of order 3 307 us with the
+ * driver's choices and 247, 1000 456 and 307, 4096 727 and 728, of order 4 1390
+ * and 1393; slower at 1728 of order 3, 491 and 541. */
 template <typename... P>
 inline int nsem_chain_split(int split, void (*kernel)(P...), unsigned grid, dim3 block, size_t smem) {
     int n = 0, dev = 0, sms = 0;
